@@ -447,3 +447,22 @@ def test_sampling_matches_oracle(bk):
     assert len(seen) > 3
     with pytest.raises(R.BunkerCudaError):
         ops.sample(dl.ptr, V, B, idx.ptr, top_k=65)
+
+
+@pytest.mark.parametrize("V", [1, 7, 63, 64, 8191, 8194, 40001])
+def test_sampling_row_lengths_and_clustered_logits(bk, V):
+    """The radix selection at rows shorter than top_k, not divisible into the cluster's slices or into vector loads, and at
+    logits that share their leading digits (several digits, then the index, decide)."""
+    B = 5
+    rng = np.random.default_rng(V)
+    logits = rng.normal(0, 2, (B, V)).astype(np.float32)
+    logits[1] = np.float32(1.0) + rng.integers(0, 4, V).astype(np.float32) * np.float32(2.0 ** -23)
+    logits[2] = np.where(rng.random(V) < 0.5, np.float32(0.0), np.float32(-0.0))
+    logits[3, rng.random(V) < 0.9] = np.nan
+    logits[4, :] = -np.inf
+    dl, idx, val = dev(logits), R.DeviceBuffer(B * 4), R.DeviceBuffer(B * 4)
+    for seed, (T, k, p) in enumerate(((1.0, 64, 1.0), (0.8, 40, 0.9), (0.0, 5, 1.0))):
+        ops.sample(dl.ptr, V, B, idx.ptr, val.ptr, temperature=T, top_k=k, top_p=p, seed=seed)
+        wi, wv = O.sample(logits, T, k, p, seed, np.zeros(B, np.int32), 0)
+        assert np.array_equal(idx.download(np.int32, (B,)), wi), (T, k, p)
+        assert_same_bits(val.download(np.float32, (B,)), wv, "sampled logit")
