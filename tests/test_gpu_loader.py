@@ -41,6 +41,22 @@ def test_quantize_q4k_matches_oracle(bk, bf16):
     dx.free(), out.free()
 
 
+@pytest.mark.parametrize("N,K", [(1, 256), (3, 256), (17, 256), (5, 768)])
+def test_quantize_q4k_odd_superblock_counts_and_ties(bk, N, K):
+    """Odd numbers of superblocks (two share a warp), and weights on rounding boundaries: multiples of half a step, where the
+    quotient must be the correctly rounded one."""
+    rng = np.random.default_rng(N * K)
+    x = rng.normal(0, 0.02, (N, K)).astype(np.float32)
+    x[0, :128] = (rng.integers(0, 31, 128) * 0.5).astype(np.float32)
+    x[0, 0], x[0, 1] = 15.0, 0.0
+    x[-1, 128:256] = (rng.integers(-15, 16, 128) * np.float32(0.125)).astype(np.float32)
+    dx, out = R.DeviceBuffer.from_numpy(x), R.DeviceBuffer(N * K // 256 * 144)
+    ops.quantize_q4k(dx.ptr, N, K, out.ptr)
+    assert R.cuSync() == 0
+    assert_same_bits(out.download(np.uint8, (N, K // 256 * 144)), O.q4k_quantize(x), "Q4_K superblocks")
+    dx.free(), out.free()
+
+
 def test_checkpoint_load_matches_host_quantised_model(bk, tmp_path):
     """A bf16 checkpoint with the reference's tensor names (model.language_model.layers.L...., tied embed_tokens) is
     loaded through the device quantiser; the model must decode exactly like one built from the same weights quantised
