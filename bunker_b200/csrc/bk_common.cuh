@@ -47,6 +47,18 @@ BK_DEVINL void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t 
                "l"(src), "r"(bytes), "r"(bar)
                : "memory");
 }
+// The same for weights: a step streams more of them than L2 holds, so their lines are the first to go and what is reused
+// every step (recurrent state, caches, activations, code) stays.
+BK_DEVINL uint64_t l2_evict_first() {
+  uint64_t p;
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+BK_DEVINL void bulk_g2s_stream(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar, uint64_t policy) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar), "l"(policy)
+               : "memory");
+}
 BK_DEVINL bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(

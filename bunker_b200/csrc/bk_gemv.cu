@@ -23,8 +23,8 @@
 // that lane 0 fills with one bulk async copy per contiguous run of rows (cp.async.bulk, completion on an
 // mbarrier).  The first copies are issued before the programmatic-dependency wait, so the weight stream of
 // this launch is in flight while the previous kernel drains and while the activation prologue runs; the
-// dot products then read weights from shared memory.  High nibbles stay in place (16*q as unsigned bytes);
-// the staged scale of odd blocks carries the 1/16.
+// dot products then read weights from shared memory.  High nibbles stay in place (16*q as unsigned bytes) and the
+// sum is shifted back.
 //
 // The activation lives in shared memory for the whole CTA: int8 quants padded to
 // 80 bytes per 64 (conflict-free 128-bit reads at lane stride), plus per-block

@@ -54,13 +54,14 @@ __device__ __forceinline__ WRegs decode_unit(const RowRegs& r, int p) {
   bk_q4k_scale_min_pair(r.hdr.y, r.hdr.z, r.hdr.w, p, sc2, mn2);
   w.sc0 = (int)(sc2 & 0xffu);
   w.sc1 = (int)(sc2 >> 8);
-  w.fm0 = (float)(int)(mn2 & 0xffu);
-  w.fm1 = (float)(int)(mn2 >> 8);
+  // the bytes as floats: placed in the mantissa of 2^23, which is then subtracted (exact)
+  w.fm0 = __fsub_rn(__uint_as_float(__byte_perm(mn2, 0x4B000000u, 0x7440)), 8388608.0f);
+  w.fm1 = __fsub_rn(__uint_as_float(__byte_perm(mn2, 0x4B000000u, 0x7441)), 8388608.0f);
   const uint32_t qw[8] = {r.qa.x, r.qa.y, r.qa.z, r.qa.w, r.qb.x, r.qb.y, r.qb.z, r.qb.w};
 #pragma unroll
   for (int k = 0; k < 8; k++) {
     w.lo[k] = qw[k] & 0x0f0f0f0fu;
-    w.hi[k] = qw[k] & 0xf0f0f0f0u;   // high nibbles stay in place: unsigned bytes 16*q, the staged d8 of odd blocks carries 1/16
+    w.hi[k] = qw[k] & 0xf0f0f0f0u;   // high nibbles stay in place: unsigned bytes 16*q
   }
   return w;
 }
@@ -83,10 +84,10 @@ __device__ __forceinline__ float unit_val(const WRegs& w, const XRegs& x) {
   i1 = bk_dp4a(w.hi[5], x.x3.y, i1);
   i1 = bk_dp4a(w.hi[6], x.x3.z, i1);
   i1 = bk_dp4a(w.hi[7], x.x3.w, i1);
-  // i1 = 16 * (sub-block sum): sc1*i1 < 2^26 is a multiple of 16, exact in f32, and x.d8.y = d8/16 (exact), so the
-  // fma rounds the same real number as fma(d8, f32(sc1*sum), accd)
-  float accd = __fmul_rn(x.d8.x, (float)(w.sc0 * i0));
-  accd = fmaf(x.d8.y, (float)(w.sc1 * i1), accd);
+  // i1 = 16 * (sub-block sum).  f32 of the integers sc*isum without conversion instructions (16 lanes per clock and SM):
+  // |sc*isum| < 2^22, so the sum with the bits of 1.5 * 2^23 is that float plus the integer, and both steps are exact.
+  float accd = __fmul_rn(x.d8.x, __fsub_rn(__int_as_float(w.sc0 * i0 + 0x4B400000), 12582912.0f));
+  accd = fmaf(x.d8.y, __fsub_rn(__int_as_float(w.sc1 * (i1 >> 4) + 0x4B400000), 12582912.0f), accd);
   float accm = __fmul_rn(x.s8.x, w.fm0);
   accm = fmaf(x.s8.y, w.fm1, accm);
   const float t = __fmul_rn(w.dmin, accm);

@@ -57,11 +57,11 @@ struct GemvParams {
 
 // ---- staged activation layouts ---------------------------------------------------
 // Plain (dp4a kernel): quants of block blk at xs[b*x_row_words + (blk>>1)*x_unit_words + (blk&1)*8 + w], w = 0..7;
-// scales d8s[b*x_scale_ld + blk] (odd blocks divided by 16, like the MMA layout), s8s likewise (undivided).
+// scales d8s[b*x_scale_ld + blk], s8s likewise.
 // MMA (TC = true): the eight words of a block are stored in the order 0,4,1,5,2,6,3,7 so that the two words a lane
 // feeds to one mma (w = j and j+4) are one 64-bit load; the scales of unit u = blk>>1 and column b form one float4
 // {d8 of block 2u, d8 of block 2u+1 divided by 16, s8 of 2u, s8 of 2u+1} at sc4[u*8 + b] (s8s is unused).
-// The division by 16 pairs with high nibbles left in place (16*q) in the integer dot: the product is unchanged.
+// The division by 16 pairs with high nibbles left in place (16*q) in the MMA's integer dot: the product is unchanged.
 template <bool TC>
 __device__ __forceinline__ uint32_t* x_block_ptr(const GemvParams& p, uint32_t* xs, int b, int blk) {
   return xs + (size_t)b * p.x_row_words + (blk >> 1) * p.x_unit_words + (blk & 1) * 8;
@@ -76,7 +76,7 @@ __device__ __forceinline__ void store_block_scales(const GemvParams& p, float* d
     e[0] = (blk & 1) ? __fmul_rn(d8, 0.0625f) : d8;
     e[2] = s8;
   } else {
-    d8s[b * p.x_scale_ld + blk] = (blk & 1) ? __fmul_rn(d8, 0.0625f) : d8;   // see unit_val() of the dp4a kernel
+    d8s[b * p.x_scale_ld + blk] = d8;
     s8s[b * p.x_scale_ld + blk] = s8;
   }
 }

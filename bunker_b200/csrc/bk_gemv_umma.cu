@@ -42,8 +42,6 @@
 //
 // No cluster, no multicast.  Every wait is bounded (and may sleep between polls); TMEM is released on every path out
 // of the kernel.
-#include <cuda.h>   // CUtensorMap and the types of its encoder; the encoder itself is looked up at run time
-
 #include "bk_gemv_shared.cuh"
 
 namespace {
@@ -553,33 +551,9 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
 
 size_t umma_smem_bytes() { return umma_smem_core_bytes() + 32 * 64 * sizeof(float); }
 
-// cuTensorMapEncodeTiled, looked up through the runtime so that the library needs no link against the driver
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_tiled_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static bool looked = false;
-  if (!looked) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qr;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qr) == cudaSuccess && qr == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(ptr);
-    looked = true;
-  }
-  return fn;
-}
-
 // uint8 matrix [n_rows][row_bytes], box = 32 rows x 144 bytes (one superblock column of 32 rows), no swizzle
 bool encode_weight_map(CUtensorMap* m, const uint8_t* W, int n_rows, size_t row_bytes) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn || (reinterpret_cast<uintptr_t>(W) & 15) || row_bytes % 16) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)n_rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
-  const cuuint32_t box[2] = {144, 32};
-  const cuuint32_t estr[2] = {1, 1};
-  return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(W), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return bk_encode_map_2d(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, (uint64_t)(uintptr_t)W, row_bytes, (uint64_t)n_rows, row_bytes, 144, 32);
 }
 
 }  // namespace

@@ -1,5 +1,6 @@
 // bk_internal.h -- host-side state shared by the translation units of libbunker_cuda.
 #pragma once
+#include <cuda.h>   // CUtensorMap and the types of its encoder; the encoder itself is looked up at run time
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -24,9 +25,8 @@ struct BkContext {
   int cta_trace_launch = -1;          // index (among GEMV launches since bkTraceCtas) of the launch to record
   int cta_trace_seen = 0;
   unsigned long long* step_trace = nullptr;  // per-phase timeline of the persistent step kernel (bkStepTraceEnable)
-  int step_trace_phases = 0;          // phases the buffer can hold (4 slots each)
+  int step_trace_phases = 0;          // phases the buffer can hold (8 slots each)
   int spin_limit = 0;                 // polls a bounded device-side wait may take (bkSetSpinLimit; 0 = built-in limits)
-  int step_barrier_mode = 1;          // grid barrier of the persistent step kernel: 0 one word per CTA, 1 one counter (faster, measured)
   int* d_status = nullptr;           // device word set by kernels whose bounded waits gave up
   float* tile_scratch = nullptr;     // dense tile GEMV cut along K: per-chunk partial sums [tile][chunk][32 columns][128 rows]
   int* tile_counters = nullptr;      // ... and one arrival counter per tile (self-resetting)
@@ -103,6 +103,11 @@ struct BkReduce {
   int spin_limit;              // polls before the bounded wait gives up (0 = default)
 };
 
+// tensor map of a matrix [n_rows][cols] with rows `stride` bytes apart, box box_rows x box_cols, no swizzle; false when the
+// encoder is missing or refuses
+bool bk_encode_map_2d(CUtensorMap* m, CUtensorMapDataType type, uint64_t base, uint64_t cols, uint64_t n_rows, uint64_t stride, uint32_t box_cols,
+                      uint32_t box_rows);
+
 // internal launchers shared between translation units
 bool bk_gemv_mma_fits(int K, int B);   // whether the batch-3..8 tensor-core GEMV can hold this K (else column pairs)
 bool bk_gemv_auto_tile(int rows, int K);   // whether BK_GEMV_ORDER_AUTO sends a launch of these shapes (>= 16 columns) to the dense tile path
@@ -153,22 +158,28 @@ int32_t bk_comm_argmax_merge(uint64_t comm, int slot, int B, uint64_t local_val,
 int32_t bk_comm_info(uint64_t comm, int* rank, int* nranks);
 
 // ---- persistent decode step (bk_persist.cu) ----------------------------------------------------------------
-// A plan is the list of phases of one batch-1 decode step on one GPU: GEMV phases (bkGemvArgs, prologues
-// BK_PRO_RMSNORM / BK_PRO_BF16) and conv1d + gated-DeltaNet phases (bkGdnArgs).  bk_plan_launch runs phases
-// [first, first+count) in ONE cooperative launch with device-side barriers between them.
-#define BK_PF_EMBED 1    /* GEMV phase: the activation is the embedded row of token ids_in[0] (also stored to x0) */
-#define BK_PF_ARGMAX 2   /* GEMV phase with one f32 segment: the launch ends with the argmax tail over its rows */
-struct BkStepIO {
-  uint64_t embed, ids_in, x0;                            // BK_PF_EMBED
-  uint64_t ids_out, val_out, pos, hist, host_out;        // BK_PF_ARGMAX tail (as bk_argmax_launch)
-  int32_t H, hist_ld, hist_rows, vocab_offset;
+// A plan is one batch-1 decode step on one GPU as the phases of a single cooperative launch.
+struct BkPlanDims {
+  int32_t H, Hk, Hv, Hq, Hkv, inter, max_len, split_len, rot_half;
+  float eps, scale;
+  uint64_t cos_t, sin_t;
 };
-int32_t bk_plan_create(uint64_t* out, int hidden);
-bool bk_plan_gemv_fits(uint64_t plan, int K);
-int32_t bk_plan_add_gemv(uint64_t plan, const bkGemvArgs& a, int flags);
-int32_t bk_plan_add_gdn(uint64_t plan, const bkGdnArgs& a);   // odd conv-state parity swaps conv_state_in / _new
-int32_t bk_plan_count(uint64_t plan);
-int32_t bk_plan_finish(uint64_t plan);
-int32_t bk_plan_launch(uint64_t plan, int first, int count, int parity, const BkStepIO& io);
+struct BkPlanLayer {   // device addresses of one layer's weights and state
+  bool full;
+  uint64_t in_ln, post_ln, gate, up, down, out_proj;   // out_proj: o_proj in an attention layer
+  uint64_t qkv, z, a, b, conv_w, A_log, dt_bias, gnorm, conv_state[2], S;
+  uint64_t q, k, v, q_norm, k_norm, kc, vc;
+  uint64_t x_out;      // untagged bf16 copy of the layer's output row
+};
+struct BkStepIO {
+  uint64_t embed, ids_in, x0;
+  uint64_t ids_out, val_out, pos, hist, host_out;        // as bk_argmax_launch
+  int32_t token;                                         // the input token, or -1: ids_in has it
+  int32_t hist_ld, hist_rows, vocab_offset;
+};
+int32_t bk_plan_create(uint64_t* out, const BkPlanDims& dims);   // *out = 0 when the shapes do not fit the kernel
+void bk_plan_add_layer(uint64_t plan, const BkPlanLayer& L);
+int32_t bk_plan_finish(uint64_t plan, uint64_t head, uint64_t final_norm, uint64_t logits, int vocab);
+int32_t bk_plan_launch(uint64_t plan, int parity, const BkStepIO& io);
 int32_t bk_plan_reset(uint64_t plan);
 void bk_plan_destroy(uint64_t plan);

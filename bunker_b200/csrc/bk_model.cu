@@ -67,12 +67,9 @@ struct Model {
   cudaGraphExec_t graph[2] = {nullptr, nullptr};       // token fed back on the device (embed reads m.ids)
   cudaGraphExec_t graph_host[2] = {nullptr, nullptr};  // token from the host (embed reads the mapped pinned ids)
   unsigned long long graph_kernels = 0;
-  // persistent step (batch 1, one GPU): the phases of the plan run as a few cooperative launches, with the attention
-  // kernel between them
+  // persistent step (batch 1, one GPU): the phases of the plan run as one cooperative launch
   int step_mode = 0;    // 0 = library's choice, 1 = one launch per op, 2 = persistent step kernel
   uint64_t plan = 0;
-  struct StepItem { int kind; int first, count; int layer; };   // kind 0: phases [first, first+count) of the plan; 1: attention of `layer`
-  std::vector<StepItem> items;
   long long steps = 0;  // steps taken since the last reset (host mirror of pos)
   int conv_cur = 0;     // which of the two conv-state buffers is current (flips with every decode step / prompt pass)
   // buffers of the multi-token prompt path (bkModelPrefill), sized for `cols` = tokens x sequences columns
@@ -164,113 +161,52 @@ bkAttnArgs step_attn_args(Model& m, LayerW& L, bool q8_handoff, bool o_staged) {
   return aa;
 }
 
-// The batch-1 single-GPU step as a plan for the persistent kernel (bk_persist.cu): the same ops in the same order as
-// enqueue_step, every GEMV and GDN launch becoming a phase; the attention kernel stays a launch of its own and cuts
-// the plan into segments.  Leaves m.plan = 0 when a shape does not fit the persistent kernel.
+// The batch-1 single-GPU step as a plan for the persistent kernel (bk_persist.cu): the ops of enqueue_step in the same
+// order.  Leaves m.plan = 0 when a shape does not fit the persistent kernel.
 int32_t build_plan(Model& m) {
   const bkModelConfig& c = m.cfg;
-  const int H = c.hidden, attn_w = m.Hq * c.head_dim;
-  if (H > 8192) return BK_OK;
-  TRY(bk_plan_create(&m.plan, H));
-  if (!bk_plan_gemv_fits(m.plan, H) || !bk_plan_gemv_fits(m.plan, m.ZD) || !bk_plan_gemv_fits(m.plan, attn_w) ||
-      !bk_plan_gemv_fits(m.plan, m.inter)) {
-    bk_plan_destroy(m.plan);
-    m.plan = 0;
-    return BK_OK;
-  }
-  int cur = 0, seg_first = 0;
-  auto close_segment = [&]() {
-    const int n = bk_plan_count(m.plan) - seg_first;
-    if (n > 0) m.items.push_back(Model::StepItem{0, seg_first, n, -1});
-    seg_first = bk_plan_count(m.plan);
-  };
-  auto gemv = [&](uint64_t x, int K, uint64_t norm_w) {
-    bkGemvArgs g;
-    memset(&g, 0, sizeof(g));
-    g.K = K; g.B = 1; g.eps = c.eps; g.x = x; g.norm_w = norm_w;
-    g.prologue = norm_w ? BK_PRO_RMSNORM : BK_PRO_BF16;
-    return g;
-  };
+  BkPlanDims D;
+  memset(&D, 0, sizeof(D));
+  D.H = c.hidden; D.Hk = m.Hk; D.Hv = m.Hv; D.Hq = m.Hq; D.Hkv = m.Hkv; D.inter = m.inter;
+  D.max_len = c.max_len; D.split_len = m.split_len; D.rot_half = c.rot_dim / 2;
+  D.eps = c.eps; D.scale = 1.0f / sqrtf((float)c.head_dim);
+  D.cos_t = m.cos_t; D.sin_t = m.sin_t;
+  TRY(bk_plan_create(&m.plan, D));
+  if (!m.plan) return BK_OK;
   for (int li = 0; li < c.n_layers; li++) {
-    LayerW& L = m.layers[li];
-    const int first_flags = li == 0 ? BK_PF_EMBED : 0;
-    bkGemvArgs g = gemv(m.x[cur], H, L.in_ln);
-    if (!L.full) {
-      g.n_segs = 4;
-      g.segs[0] = bkGemvSeg{L.qkv, 0, m.qkv, 0, m.Cw, BK_EPI_BF16, m.Cw, 0};
-      g.segs[1] = bkGemvSeg{L.z, 0, m.z, 0, m.ZD, BK_EPI_BF16, m.ZD, 0};
-      g.segs[2] = bkGemvSeg{L.a, 0, m.a, 0, m.Hv, BK_EPI_F32, m.Hv, 0};
-      g.segs[3] = bkGemvSeg{L.b, 0, m.b, 0, m.Hv, BK_EPI_F32, m.Hv, 0};
-      TRY(bk_plan_add_gemv(m.plan, g, first_flags));
-      bkGdnArgs ga;
-      memset(&ga, 0, sizeof(ga));
-      ga.qkv = m.qkv; ga.z = m.z; ga.a = m.a; ga.b = m.b;
-      ga.conv_w = L.conv_w; ga.conv_state_in = L.conv_state[0]; ga.conv_state_new = L.conv_state[1];
-      ga.A_log = L.A_log; ga.dt_bias = L.dt_bias; ga.norm_w = L.gnorm;
-      ga.S_in = L.S; ga.S_new = L.S;
-      ga.out = m.attn_out; ga.B = 1; ga.Hk = m.Hk; ga.Hv = m.Hv; ga.apply_conv = 1; ga.state_is_settled = 1;
-      TRY(bk_plan_add_gdn(m.plan, ga));
-      g = gemv(m.attn_out, m.ZD, 0);
-      g.n_segs = 1;
-      g.segs[0] = bkGemvSeg{L.out_proj, 0, m.h1, m.x[cur], H, BK_EPI_ADD_BF16, H, 0};
-      TRY(bk_plan_add_gemv(m.plan, g, 0));
-    } else {
-      g.n_segs = 3;
-      g.segs[0] = bkGemvSeg{L.q, 0, m.qg, 0, m.QG, BK_EPI_BF16, m.QG, 0};
-      g.segs[1] = bkGemvSeg{L.k, 0, m.kbuf, 0, m.KVD, BK_EPI_BF16, m.KVD, 0};
-      g.segs[2] = bkGemvSeg{L.v, 0, m.vbuf, 0, m.KVD, BK_EPI_BF16, m.KVD, 0};
-      TRY(bk_plan_add_gemv(m.plan, g, first_flags));
-      close_segment();
-      m.items.push_back(Model::StepItem{1, 0, 0, li});
-      g = gemv(m.attn_out, attn_w, 0);
-      g.n_segs = 1;
-      g.segs[0] = bkGemvSeg{L.o, 0, m.h1, m.x[cur], H, BK_EPI_ADD_BF16, H, 0};
-      TRY(bk_plan_add_gemv(m.plan, g, 0));
-    }
-    g = gemv(m.h1, H, L.post_ln);
-    g.n_segs = 1;
-    g.segs[0] = bkGemvSeg{L.gate, L.up, m.act, 0, m.inter, BK_EPI_SWIGLU, m.inter, 0};
-    TRY(bk_plan_add_gemv(m.plan, g, 0));
-    g = gemv(m.act, m.inter, 0);
-    g.n_segs = 1;
-    g.segs[0] = bkGemvSeg{L.down, 0, m.x[cur ^ 1], m.h1, H, BK_EPI_ADD_BF16, H, 0};
-    TRY(bk_plan_add_gemv(m.plan, g, 0));
-    cur ^= 1;
+    const LayerW& L = m.layers[li];
+    BkPlanLayer p;
+    memset(&p, 0, sizeof(p));
+    p.full = L.full;
+    p.in_ln = L.in_ln; p.post_ln = L.post_ln; p.gate = L.gate; p.up = L.up; p.down = L.down;
+    p.out_proj = L.full ? L.o : L.out_proj;
+    p.qkv = L.qkv; p.z = L.z; p.a = L.a; p.b = L.b; p.conv_w = L.conv_w; p.A_log = L.A_log; p.dt_bias = L.dt_bias; p.gnorm = L.gnorm;
+    p.conv_state[0] = L.conv_state[0]; p.conv_state[1] = L.conv_state[1]; p.S = L.S;
+    p.q = L.q; p.k = L.k; p.v = L.v; p.q_norm = L.q_norm; p.k_norm = L.k_norm; p.kc = L.kc; p.vc = L.vc;
+    p.x_out = m.x[(li & 1) ^ 1];
+    bk_plan_add_layer(m.plan, p);
   }
-  bkGemvArgs g = gemv(m.x[cur], H, m.final_norm);
-  g.n_segs = 1;
-  g.segs[0] = bkGemvSeg{m.embed, 0, m.logits, 0, m.vocab_local, BK_EPI_F32, m.vocab_local, 0};
-  TRY(bk_plan_add_gemv(m.plan, g, BK_PF_ARGMAX));
-  close_segment();
-  TRY(bk_plan_finish(m.plan));
-  return BK_OK;
+  return bk_plan_finish(m.plan, m.embed, m.final_norm, m.logits, m.vocab_local);
 }
 
-int32_t enqueue_step_persist(Model& m, int parity, bool host_tokens) {
+// token: the step's input, or -1 to take the device's own last one
+int32_t enqueue_step_persist(Model& m, int parity, int token = -1) {
   const bkModelConfig& c = m.cfg;
-  const bool mapped_io = m.pin_dev != 0;
   BkStepIO io;
   memset(&io, 0, sizeof(io));
   io.embed = m.embed;
-  io.ids_in = (host_tokens && mapped_io) ? m.pin_dev + (uint64_t)parity * 4 : m.ids;
+  io.ids_in = m.ids;
+  io.token = token;
   io.x0 = m.x[0];
   io.ids_out = m.ids; io.val_out = m.val; io.pos = m.pos; io.hist = m.hist;
-  io.host_out = mapped_io ? m.pin_dev + (uint64_t)2 * 4 : 0;
-  io.H = c.hidden; io.hist_ld = 1; io.hist_rows = c.max_len; io.vocab_offset = 0;
-  for (const Model::StepItem& it : m.items) {
-    if (it.kind == 0) {
-      TRY(bk_plan_launch(m.plan, it.first, it.count, parity, io));
-    } else {
-      bkAttnArgs aa = step_attn_args(m, m.layers[it.layer], false, false);
-      TRY(bkAttnDecode(&aa));
-    }
-  }
-  return BK_OK;
+  io.host_out = m.pin_dev ? m.pin_dev + (uint64_t)2 * 4 : 0;
+  io.hist_ld = 1; io.hist_rows = c.max_len; io.vocab_offset = 0;
+  return bk_plan_launch(m.plan, parity, io);
 }
 
 // enqueue one decode step on the library stream; parity selects the conv-state buffer pair
 int32_t enqueue_step(Model& m, int parity, bool host_tokens = false) {
-  if (m.plan && !g_prof.on) return enqueue_step_persist(m, parity, host_tokens);
+  if (m.plan && !g_prof.on) return enqueue_step_persist(m, parity);
   const bkModelConfig& c = m.cfg;
   const int B = m.B, H = c.hidden;
   int cur = 0;
@@ -795,9 +731,9 @@ int32_t bkModelFinalize(uint64_t model) {
     m.pin_dev = (uint64_t)(uintptr_t)dp;
   }
   BK_ARG(m.step_mode != 2 || (B == 1 && m.tp == 1), "bkModelFinalize: the persistent step needs batch 1 on one GPU");
-  // The library's own choice (mode 0) is one launch per op: on B200 the programmatic hand-off between dependent
-  // launches measures 0.7 us, a device-side barrier over 148 CTAs 1.8 us, and the step is a chain of ~120 of them.
-  if (m.step_mode == 2) TRY(build_plan(m));
+  // The library's own choice (mode 0) at batch 1 on one GPU is the persistent kernel wherever the shapes fit it: a
+  // hand-off inside it costs one L2 store and load, a dependent launch 2 us of completion, flush and wait.
+  if (m.step_mode == 2 || (m.step_mode == 0 && B == 1 && m.tp == 1)) TRY(build_plan(m));
   BK_ARG(m.step_mode != 2 || m.plan, "bkModelFinalize: this model's shapes do not fit the persistent step kernel");
   // one eager step sets the kernels' shared-memory attributes and validates every pointer, then the
   // state is cleared and the two parity graphs are captured
@@ -806,7 +742,7 @@ int32_t bkModelFinalize(uint64_t model) {
   TRY(reset_state(m));
   TRY(capture(m, 0));
   TRY(capture(m, 1));
-  if (m.tp == 1) {
+  if (m.tp == 1 && !m.plan) {
     TRY(capture(m, 0, true));
     TRY(capture(m, 1, true));
   }
@@ -851,9 +787,16 @@ int32_t bkDecodeStep(uint64_t model, const int32_t* tokens, int32_t* out_ids, fl
   BK_ARG(m.finalized, "bkDecodeStep: model is not finalized");
   cudaStream_t st = bk_ctx().stream;
   const int B = m.B;
-  const bool mapped_io = m.tp == 1 && m.graph_host[0] != nullptr;
+  const bool mapped_io = m.tp == 1;
   int32_t* const out_slot = m.pin_ids + 2 * B;   // ids out, then vals
-  if (tokens) {
+  if (tokens && m.plan) {
+    // The token travels in the launch's parameters: read from mapped host memory by all 148 CTAs it costs 18 us.
+    BK_ARG(tokens[0] >= 0 && tokens[0] < m.cfg.vocab, "bkDecodeStep: token %d outside the vocabulary", tokens[0]);
+    BK_ARG(m.steps < m.cfg.max_len, "bkDecodeStep: position %lld reached max_len=%d", m.steps, m.cfg.max_len);
+    TRY(enqueue_step_persist(m, m.conv_cur, tokens[0]));
+    m.steps++;
+    m.conv_cur ^= 1;
+  } else if (tokens) {
     const int p = m.conv_cur;                     // the graph about to run reads ids slot p
     int32_t* in_slot = m.pin_ids + (mapped_io ? p * B : 0);
     if (mapped_io && m.pin_busy[p]) {              // the step before last may still be reading this slot

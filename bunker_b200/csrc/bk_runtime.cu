@@ -16,6 +16,35 @@ int32_t bk_fail(int32_t code, const char* fmt, ...) {
   return code;
 }
 
+// cuTensorMapEncodeTiled, looked up through the runtime so that the library needs no link against the driver
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static EncodeTiledFn encode_tiled_fn() {
+  static EncodeTiledFn fn = nullptr;
+  static bool looked = false;
+  if (!looked) {
+    void* ptr = nullptr;
+    cudaDriverEntryPointQueryResult qr;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qr) == cudaSuccess && qr == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<EncodeTiledFn>(ptr);
+    looked = true;
+  }
+  return fn;
+}
+
+bool bk_encode_map_2d(CUtensorMap* m, CUtensorMapDataType type, uint64_t base, uint64_t cols, uint64_t n_rows, uint64_t stride, uint32_t box_cols,
+                      uint32_t box_rows) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn || (base & 15) || stride % 16) return false;
+  const cuuint64_t dims[2] = {cols, n_rows};
+  const cuuint64_t strides[1] = {stride};
+  const cuuint32_t box[2] = {box_cols, box_rows};
+  const cuuint32_t estr[2] = {1, 1};
+  return fn(m, type, 2, reinterpret_cast<void*>(static_cast<uintptr_t>(base)), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 extern "C" {
 
 int32_t bkInit(int32_t device) {
@@ -232,7 +261,6 @@ int32_t bkSetSpinLimit(int32_t polls) {
 int32_t bkStepBarrierMode(int32_t mode) {
   BK_REQUIRE_INIT();
   BK_ARG(mode == 0 || mode == 1, "bkStepBarrierMode: mode %d", mode);
-  g_ctx.step_barrier_mode = mode;
   return BK_OK;
 }
 

@@ -31,17 +31,17 @@ BK_API int32_t bkTuneGemvRing(int32_t warps, int32_t rows_per_group, int32_t max
 BK_API int32_t bkTuneTileMinRows(int32_t rows);
 /* Per-phase timeline of the persistent step kernel.  While enabled, every launch of that kernel stamps %globaltimer
  * (ns) into dev_buf[8*phase + k] for each phase it runs: 0 phase entered (CTA 0), 1 activation staged (CTA 0),
- * 2 CTA 0 finished its rows, 3 the latest CTA finished (atomic max; clear the buffer between steps), and for warp 0's
- * first row group of a GEMV phase 4 weights landed, 5 dot products done, 6 ring refilled, 7 epilogue stored.  Takes effect
- * for launches issued eagerly after the call (bkDecodeStepEager); captured graphs keep what they were captured with. */
+ * 2 CTA 0's warp 0 finished its part, 3 the latest warp of the grid finished (atomic max; clear the buffer between
+ * steps); slots 4 to 7 are not written.  Takes effect for launches issued eagerly after the call (bkDecodeStepEager);
+ * captured graphs keep what they were captured with. */
 BK_API int32_t bkStepTraceEnable(uint64_t dev_buf, int32_t max_phases);
 /* Polls a bounded device-side wait may take before it gives up and sets the status word that bkSync reports as
  * BK_ERR_TIMEOUT (0 restores the built-in limits).  Applies to the tensor-parallel exchange consumer
- * (bkReduceRmsNormQuantQ8_1 and the model's reducing launches) and the persistent step kernel's grid barrier, for
+ * (bkReduceRmsNormQuantQ8_1 and the model's reducing launches) and the persistent step kernel's waits for tagged words, for
  * launches issued after the call.  Lets a test make a wait run out in microseconds without hanging anything. */
 BK_API int32_t bkSetSpinLimit(int32_t polls);
-/* Grid barrier of the persistent step kernel, for models finalized after the call: 0 = one arrival word per CTA
- * , 1 = one atomic counter (the default: 1.8 us against 3-5 us per barrier on 148 CTAs). */
+/* Kept for hosts that bind it: the persistent step kernel has no grid barrier any more (its phases hand tagged words to
+ * one another), so the mode (0 or 1) is checked and has no effect. */
 BK_API int32_t bkStepBarrierMode(int32_t mode);
 /* One decode step enqueued without the CUDA graph (device-side token feedback), so that timelines enabled after
  * bkModelFinalize apply to it. */

@@ -356,6 +356,33 @@ def test_persistent_step_equals_per_op_step_and_oracle(bk, interval, n_layers):
     assert np.array_equal(outs[2][0], want)
 
 
+@pytest.mark.parametrize("hidden,inter,Hk,Hv,q_heads,kv_heads,vocab,T", [
+    (256, 256, 1, 2, 1, 1, 3, 3),              # fewer rows than SMs in every projection
+    (1280, 768, 20, 40, 3, 1, 997, 3),         # two recurrent items per SM, an odd number of query heads, ragged row splits
+    (512, 2816, 2, 6, 8, 1, 300, 600),         # several splits of the cache, eight query heads on one
+    (8192, 512, 2, 2, 2, 2, 64, 2),            # the widest normalised row
+    (8448, 512, 2, 2, 2, 2, 64, 2),            # past it: one launch per op
+])
+def test_persistent_step_shapes(bk, hidden, inter, Hk, Hv, q_heads, kv_heads, vocab, T):
+    """The one-launch step at the edges of what it takes, against the oracle: tokens and logits bit for bit."""
+    cfg = M.ModelConfig(hidden=hidden, n_layers=2, vocab=vocab, gdn_k_heads=Hk, gdn_v_heads=Hv, attn_q_heads=q_heads, attn_kv_heads=kv_heads,
+                        intermediate=inter, full_attn_interval=2, max_len=T + 16)
+    w = M.synth_weights(cfg, seed=hidden + T)
+    gm = M.DecodeModel(cfg, w, batch=1)
+    info = gm.info()
+    assert (info["kernels_per_step"] == 1) == (hidden <= 8192)
+    om = OracleModel(cfg, w, batch=1, split_len=info["split_len"], attn_warps=info["attn_warps"])
+    prompt = np.random.default_rng(T).integers(0, vocab, (T, 1)).astype(np.int32)
+    ids_g = ids_o = None
+    for t in range(T + 6):
+        ids_o, _ = om.step(prompt[t] if t < T else ids_o)
+        ids_g, _ = gm.step(prompt[t] if t < T else ids_g)
+        if t >= T - 1:
+            assert np.array_equal(ids_g, ids_o), f"step {t}"
+    assert_same_bits(gm.logits(), om.logits, "logits")
+    gm.destroy()
+
+
 def test_graph_front_end_decodes_like_the_step_graph(bk):
     """A runner.ts-style caller: build the declarative graph, take the static partition, resolve weights and
     double-buffered state through callbacks, rotate the state after every token.  Tokens must equal DecodeModel's and
