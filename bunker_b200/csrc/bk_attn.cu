@@ -36,7 +36,7 @@ struct AttnParams {
   const int32_t* pos;
   uint16_t* out;
   uint8_t* out_q8;
-  int out_q8_staged;
+  int out_q8_layout;
   float* scratch;
   const uint16_t* gate;
   int B, Hq, Hkv, rot_half, max_len, split_len, max_splits, fused;
@@ -161,7 +161,8 @@ __device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, flo
       y[2 * e] = __uint_as_float(o[e] << 16);
       y[2 * e + 1] = __uint_as_float(o[e] & 0xffff0000u);
     }
-    if (p.out_q8_staged) bk_staged_store<8>(p.out_q8, p.Hq * kHD, p.B, b, (h * kHD + lane * 8) >> 5, y, (lane & 3) * 8);
+    if (p.out_q8_layout == BK_Q8_TILE) bk_tile_store<8>(p.out_q8, p.Hq * kHD, p.B, b, (h * kHD + lane * 8) >> 5, y, (lane & 3) * 8);
+    else if (p.out_q8_layout == BK_Q8_STAGED) bk_staged_store<8>(p.out_q8, p.Hq * kHD, p.B, b, (h * kHD + lane * 8) >> 5, y, (lane & 3) * 8);
     else bk_q8_1_store<8>(p.out_q8 + ((((size_t)b * p.Hq + h) * kHD + lane * 8) >> 5) * 36, y, (lane & 3) * 8);
   }
 }
@@ -489,6 +490,7 @@ uint64_t bkAttnScratchBytes(int32_t B, int32_t Hq, int32_t HD, int32_t max_len, 
 int32_t bkAttnDecode(const bkAttnArgs* args) {
   BK_REQUIRE_INIT();
   BK_ARG(args != nullptr, "bkAttnDecode: args is null");
+  BK_ARG(args->out_q8_layout == BK_Q8_BLOCKS || args->out_q8_layout == BK_Q8_STAGED, "bkAttnDecode: out_q8_layout %d", args->out_q8_layout);
   return bk_attn_launch(*args, 0, 0);
 }
 
@@ -538,8 +540,7 @@ int32_t bk_attn_launch(const bkAttnArgs& args, int n_seq, int layout_B) {
   p.pos = bk_ptr<int32_t>(a.pos);
   p.out = bk_ptr<uint16_t>(a.out);
   p.out_q8 = bk_ptr<uint8_t>(a.out_q8);
-  p.out_q8_staged = a.out_q8_layout == BK_Q8_STAGED;
-  BK_ARG(a.out_q8_layout == BK_Q8_BLOCKS || a.out_q8_layout == BK_Q8_STAGED, "bkAttnDecode: out_q8_layout %d", a.out_q8_layout);
+  p.out_q8_layout = a.out_q8_layout;
   p.scratch = bk_ptr<float>(a.scratch);
   p.gate = bk_ptr<uint16_t>(a.gate);
   p.B = a.B;

@@ -370,6 +370,80 @@ BK_DEVINL void bk_staged_store(uint8_t* img, int K, int B, int b, int blk, const
   }
 }
 
+// ---- activation image of the dense tile GEMV (9 to 64 columns) ---------------------------
+// For np = 16, 32 or 64 columns (unused ones are never read into a result).  First, per 64-value unit, operand B of its MMAs: f16
+// [2 blocks][4 chunks of 8 values][np][8], the values of four in the order 0, 2, 1, 3; then per unit the column factors
+// [2 blocks][np / 2] {d8 of columns 2i, 2i+1, s8 of columns 2i, 2i+1}.
+__host__ __device__ __forceinline__ int bk_tile_columns(int B) { return B <= 16 ? 16 : B <= 32 ? 32 : 64; }
+__host__ __device__ __forceinline__ size_t bk_tile_image_bytes(int K, int B) { return (size_t)(K / 64) * bk_tile_columns(B) * 144; }
+// words w0, w1 (eight quants) of chunk c of block blk
+BK_DEVINL void bk_tile_store_quants(uint8_t* img, int B, int b, int blk, int c, uint32_t w0, uint32_t w1) {
+  const int np = bk_tile_columns(B);
+  uint32_t o[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {   // 1024 + (q + 128) in f16, minus 1152
+    const uint32_t v = __byte_perm((i < 2 ? w0 : w1) ^ 0x80808080u, 0x64646464u, (i & 1) ? 0x4341 : 0x4240);
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(o[i]) : "r"(v), "r"(0xE480E480u));
+  }
+  *reinterpret_cast<uint4*>(img + (size_t)(blk >> 1) * np * 128 + ((size_t)((blk & 1) * 4 + c) * np + b) * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+BK_DEVINL void bk_tile_store_factors(uint8_t* img, int K, int B, int b, int blk, float d8, float s8) {
+  const int np = bk_tile_columns(B);
+  float* f = reinterpret_cast<float*>(img + (size_t)(K / 64) * np * 128 + ((size_t)blk * (np / 2) + (b >> 1)) * 16) + (b & 1);
+  f[0] = d8;
+  f[2] = s8;
+}
+
+// Same contract as bk_q8_1_store, writing block blk of column b into an image.
+template <int PER>
+BK_DEVINL void bk_tile_store(uint8_t* img, int K, int B, int b, int blk, const float (&y)[PER], int idx_in_block) {
+  static_assert(PER == 1 || PER == 4 || PER == 8, "values per lane");
+  constexpr int GROUP = 32 / PER;
+  float amax = 0.0f;
+#pragma unroll
+  for (int e = 0; e < PER; e++) amax = fmaxf(amax, fabsf(y[e]));
+#pragma unroll
+  for (int off = GROUP / 2; off >= 1; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+  const float d = __fdiv_rn(amax, 127.0f);
+  const float id = (d == 0.0f) ? 1.0f : __fdiv_rn(1.0f, d);
+  int sum = 0;
+  int qs[PER];
+#pragma unroll
+  for (int e = 0; e < PER; e++) {
+    const int v = __float2int_rd(fmaf(y[e], id, 0.5f));
+    qs[e] = max(-128, min(127, v));
+    sum += qs[e];
+  }
+#pragma unroll
+  for (int off = GROUP / 2; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+  if (PER == 1) {
+    const int np = bk_tile_columns(B), e = idx_in_block & 7;
+    const int pos = (e & 4) | ((e & 1) << 1) | ((e >> 1) & 1);   // the order 0, 2, 1, 3
+    const int biased = qs[0] + 128;
+    uint32_t h;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(h) : "r"(0x6400u | (uint32_t)biased), "r"(0xE480u));
+    *reinterpret_cast<uint16_t*>(img + (size_t)(blk >> 1) * np * 128 + ((size_t)((blk & 1) * 4 + (idx_in_block >> 3)) * np + b) * 16 + pos * 2) = (uint16_t)h;
+  } else if (PER == 4) {
+    const int np = bk_tile_columns(B);
+    const uint32_t w = ((uint32_t)(qs[0] & 0xff) | ((uint32_t)(qs[1 % PER] & 0xff) << 8) | ((uint32_t)(qs[2 % PER] & 0xff) << 16) | ((uint32_t)(qs[3 % PER] & 0xff) << 24)) ^ 0x80808080u;
+    uint32_t o0, o1;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(o0) : "r"(__byte_perm(w, 0x64646464u, 0x4240)), "r"(0xE480E480u));
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(o1) : "r"(__byte_perm(w, 0x64646464u, 0x4341)), "r"(0xE480E480u));
+    *reinterpret_cast<uint2*>(img + (size_t)(blk >> 1) * np * 128 + ((size_t)((blk & 1) * 4 + (idx_in_block >> 3)) * np + b) * 16 + (idx_in_block & 4) * 2) = make_uint2(o0, o1);
+  } else {
+    uint32_t w[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+      w[i] = (uint32_t)(qs[4 * i % PER] & 0xff) | ((uint32_t)(qs[(4 * i + 1) % PER] & 0xff) << 8) | ((uint32_t)(qs[(4 * i + 2) % PER] & 0xff) << 16) |
+             ((uint32_t)(qs[(4 * i + 3) % PER] & 0xff) << 24);
+    bk_tile_store_quants(img, B, b, blk, idx_in_block >> 3, w[0], w[1]);
+  }
+  if (idx_in_block == 0) {
+    const float d8 = bk_q8half_to_f32(bk_f32_to_f16_trunc(d));
+    bk_tile_store_factors(img, K, B, b, blk, d8, __fmul_rn(d8, (float)sum));
+  }
+}
+
 // ---- Q4_K superblock header -------------------------------------------------
 // bytes [4,16) of a superblock as three words w0,w1,w2; sub-block j in 0..7
 BK_DEVINL void bk_q4k_scale_min(uint32_t w0, uint32_t w1, uint32_t w2, int j, int& sc, int& mn) {

@@ -29,7 +29,7 @@ struct GdnParams {
   float* o_raw;
   uint16_t* conv_out;
   uint8_t* out_q8;
-  int out_q8_staged;
+  int out_q8_layout;
   int B, Hk, Hv, apply_conv;
   int T;      // tokens per sequence handled by this launch, in order (1 in the decode step)
   int early;  // state / conv state / weights are not outputs of the immediately preceding launch
@@ -219,7 +219,8 @@ __device__ __forceinline__ void gdn_step_body(const GdnParams& p, GdnSmem& sm, c
       p.out[(row * p.Hv + hv) * D + t] = ob;
       if (p.out_q8) {  // warp w of the first four holds block w of this head
         const float y[1] = {bk_bf16_to_f32(ob)};
-        if (p.out_q8_staged) bk_staged_store<1>(p.out_q8, p.Hv * D, p.B * T, (int)row, hv * 4 + warp, y, lane);
+        if (p.out_q8_layout == BK_Q8_TILE) bk_tile_store<1>(p.out_q8, p.Hv * D, p.B * T, (int)row, hv * 4 + warp, y, lane);
+        else if (p.out_q8_layout == BK_Q8_STAGED) bk_staged_store<1>(p.out_q8, p.Hv * D, p.B * T, (int)row, hv * 4 + warp, y, lane);
         else bk_q8_1_store<1>(p.out_q8 + ((row * p.Hv + hv) * 4 + warp) * 36, y, lane);
       }
     }

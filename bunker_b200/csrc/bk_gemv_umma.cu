@@ -1,86 +1,89 @@
-// bk_gemv_umma.cu -- Q4_K x Q8_1 GEMM for 16 or more activation columns on the 5th-generation tensor cores:
-// tcgen05.mma kind::i8 with the accumulators in tensor memory (TMEM).
+// bk_gemv_umma.cu -- Q4_K x Q8_1 GEMM for 16 to 64 activation columns on the 5th-generation tensor cores (tcgen05.mma kind::f16,
+// operand A and the accumulators in tensor memory).
 //
-// From 16 columns on the product is a dense contraction: the weights are streamed ONCE for all columns (the batch 2..8
-// kernel would stream them once per group of 8).  The reference's nearest thing is its int8 tensor-core GEMM experiment
+// From 16 columns on the product is a dense contraction: the weights are streamed ONCE for all columns (the batch 2..8 kernel
+// streams them once per group of 8).  The reference's nearest thing is its int8 tensor-core GEMM experiment
 // (src/kernel.ts:396-456: 4-bit blocks expanded to int8 tiles, int32 accumulators, scales applied afterwards,
-// experiments/q4k_q81_final.ts:217); this is that scheme on the 144-byte Q4_K layout.
+// experiments/q4k_q81_final.ts:217); this is that idea on the 144-byte Q4_K layout.
 //
-// One CTA of 768 threads per SM walks over its 128-row tiles, as five groups of warps that meet only at mbarriers:
-//   * one PRODUCER warp keeps a ring of two stages filled: a stage holds two superblock columns (288 bytes) of each of
-//     the 128 rows; the ring runs ahead across tile boundaries and starts before the dependency wait (see "Weight
-//     feed" below for the two ways a stage is filled);
-//   * four EXPANDER warps (thread <-> tile row).  Per 256-weight superblock column every expander thread
-//     unpacks its row's 128 quant bytes into eight 32-byte rows of unsigned int8 (one per sub-block), stored in the
-//     K-major "core matrix" layout the MMA reads (8 rows x 16 bytes contiguous, no swizzle), and decodes the eight
-//     6-bit scales and mins into a table;
-//   * two STAGER warps put the superblock's Q8_1 activation blocks into the same layout (signed int8, N = columns)
-//     with their d8 and s8 scales, reading one superblock ahead;
-//   * one MMA warp: when all 128 expander threads have arrived, one thread issues eight MMAs (M = 128, N = 16 or 32,
-//     K = 32: exactly one sub-block each) into eight separate TMEM accumulators -- the integer dot of every (row,
-//     column, sub-block), exact -- and commits to an mbarrier (issue and commit keep that thread busy for about a
-//     thousand cycles per superblock, which is why it is not an expander);
-//   * sixteen SCALER warps (four per TMEM lane quarter, each a quarter of the columns) run the f32 part of a
-//     superblock as soon as its MMAs have completed: tcgen05.ld brings a thread its row's int32 sums, and
-//     accd = fma(d8, f32(sc*isum), accd), accm = fma(s8, f32(m), accm)  over the sub-blocks in ascending order, then
-//     yc += fma(d, accd, -(dmin*accm));  every four superblocks  y += yc.  They hand the buffers back through two more
-//     mbarriers: the shared-memory side (tiles and tables, three buffers, so that the unpacking runs up to two steps
-//     ahead) to the expanders and stagers, the accumulators (two buffers of 256 TMEM columns) to the MMA warp.
-// That f32 order ("tile order": per (row, column) one chain per chunk of four superblocks, chunks added in order) is
-// fixed and mirrored by the CPU checker; it differs from the batch <= 8 kernels' lane / butterfly order by a few ulp.
+// The integer dots are exact in f16 operands and f32 accumulators: A holds sc*q (a 6-bit scale times a nibble, <= 945, an
+// integer below 2^11), B the signed 8-bit quants, and every partial sum of a 32-value sub-block is an integer below 2^22.  So
+// an accumulator IS f32(sc*isum), and what is left per (row, column, sub-block) are two fused multiply-adds: d8 * it and
+// s8 * m.  (With int8 operands the product sc*isum and its conversion cost an integer multiply, at half rate, and an
+// addition per element more, and were what bounded this kernel: 2.2 us per 128 x 256 weights and 32 columns.)
 //
-// A launch of few tiles (fewer than half the SMs) is cut along K: thread block (tile, part) runs a contiguous range of
-// whole chunks and leaves each chunk's partial sums in a scratch buffer; the block that arrives last at the tile's
-// counter adds the chunks in ascending order -- the same chain as an uncut launch -- and runs the epilogue.
+// A step is (superblock, sub-block pair p): 128 rows x 64 weights.  A CTA of 640 threads runs as groups of warps that meet only at
+// mbarriers:
+//   * one PRODUCER warp keeps a ring of stages filled: a stage holds one superblock (or the pairs of it that this CTA handles)
+//     of the 128 rows and the activations of that superblock, which are ready-made operand B tiles (see the image below);
+//   * eight EXPANDER warps (two per 32 rows, taking turns; thread <-> row) turn a row's 32 bytes into 64 f16 in tensor memory
+//     (operand A; the shared-memory bandwidth that it would cost is needed by the scalers) and its header into {d, -dmin, m0, m1};
+//   * one MMA warp issues four MMAs (M = 128, N = columns, K = 16) per step into two accumulators of N tensor-memory columns
+//     (measured: 47 cycles each whatever N, 43 for a commit, both of them the issuing thread's);
+//   * eight SCALER warps (two per TMEM lane quarter, half of the columns each) read the accumulators as 16x256b fragments (a thread
+//     holds 4 rows x 2 columns of every 8 columns, so that a column's d8 and s8 are loaded once for 4 rows and a row's minima
+//     once for all columns) and run the f32 part, two columns per instruction; four such blocks (one step at N = 64, four at
+//     N = 16) per wait;
+//   * two EPILOGUE warps add up what the scalers hand over and write the outputs while the scalers are at the next tile.
 //
-// Weight feed: when every segment's row count is a multiple of 32 (all shapes of the model) a stage is filled with one
-// tiled TMA load per 32-row box and superblock column (cp.async.bulk.tensor.2d through a tensor map of the weight
-// matrix; 8 instructions per stage instead of 128 row copies -- the row copies cap the feed at about 7 GB/s per SM
-// and cost 5 us before the first stage has landed).  A SwiGLU launch then keeps its 64 gate rows in tile rows 0..63
-// and the 64 up rows in 64..127 (boxes are contiguous rows of one matrix), and the epilogue passes the up values to
-// the gate rows' threads through shared memory.  Other shapes keep the per-row copies.
+// Two orders of the f32 part, both fixed and mirrored by the CPU checker:
+//   LANES (the order of the batch <= 8 kernels, for prompts of 17 columns and more): per unit u = (s, p)
+//     val = fma(d, fma(d8_1, x1, d8_0*x0), -(dmin * fma(s8_1, m1, s8_0*m0))); class c = s mod 8 of pair p adds its units in
+//     ascending s; T_p = ((P0+P4)+(P2+P6)) + ((P1+P5)+(P3+P7)); y = (T0+T2) + (T1+T3).  The classes are walked in the order
+//     0,4,2,6,1,5,3,7, so that a stack of three values per (row, column, pair) holds what is still to be added: one in
+//     registers, two in shared memory, 64 KB, which is why a CTA takes 2 pairs at N = 32 and one at N = 64.
+//   TILE (16 and more sequences): accd = fma(d8, x, accd), accm = fma(s8, m, accm) over the eight sub-blocks; yc += fma(d, accd,
+//     -(dmin*accm)); every four superblocks y += yc.
 //
-// No cluster, no multicast.  Every wait is bounded (and may sleep between polls); TMEM is released on every path out
-// of the kernel.
+// A cluster of CTAs shares a tile: the four pairs (LANES), and where there are few tiles also the classes (LANES) or the
+// four-superblock chunks (TILE).  Every CTA sends each value it ends up with to the CTA of the cluster that owns the column
+// (one bulk copy through distributed shared memory per owner); the owner adds them in the fixed order and runs the epilogue.
+//
+// Weight feed: tiled TMA loads of 32-row boxes (cp.async.bulk.tensor.2d) where every segment's row count is a multiple of 32; a
+// SwiGLU launch then keeps its 64 gate rows in tile rows 0..63 and their up rows in 64..127.  Other shapes (TILE only)
+// copy row by row.  No multicast.  Every wait is bounded; TMEM is released on every path out of the kernel.
+#include <cuda_fp16.h>
+
 #include "bk_gemv_shared.cuh"
 
 namespace {
 
 constexpr int kTileM = 128;
-// The supporting roles come first: their work per step is short but the scalers wait for it
-constexpr int kExpanderWarps = 4;   // warps 0..3: thread <-> tile row
-constexpr int kStagerWarp0 = 4;     // warps 4, 5 stage the activation blocks
-constexpr int kStagerWarps = 2;
-constexpr int kProducerWarp = 6;    // keeps the weight ring filled
-constexpr int kMmaWarp = 7;         // issues the MMAs
-constexpr int kScalerWarp0 = 8;     // warps 8..23: warp w reads TMEM lanes 32*(w mod 4)..+31, columns of quarter (w - 8) / 4
-constexpr int kScalerWarps = 16;
-constexpr int kUT = (kScalerWarp0 + kScalerWarps) * 32;
-constexpr int kStages = 2;          // ring stages, two superblock columns each
-constexpr int kSB = 3;              // shared-memory buffers (A / B tiles, scale tables): the unpacking runs up to two steps
-                                    // ahead of the two TMEM accumulator buffers
-constexpr int kRowPitch = 2 * 144 + 16;   // bytes between rows of a stage: 76 words, so 16-byte reads of 8 rows hit 8 bank groups
-constexpr int kStageBytes = kTileM * kRowPitch;
-constexpr int kPlaneBytes = kTileM * 144;   // tensor-map feed: a stage is two planes [128 rows][144 bytes], one per superblock column
+constexpr int kProducerWarp = 8, kMmaWarp = 9, kEpilogueWarp0 = 10, kScalerWarp0 = 12;
+constexpr int kUT = 640;
+constexpr int kScalers = 256;
 constexpr int kTmemCols = 512;
-constexpr int kScsLd = 72;          // floats per sub-block of the column scales: 32 d8, 32 s8, 8 of padding (bank spread)
+constexpr int kXPitch = 132;       // floats between columns of the exchange buffers: fragments hit 32 banks
+constexpr int kMaxStages = 8;
 
-// dynamic shared memory without the SwiGLU exchange buffer, which follows it: ring, A tiles (3 x 8 x 4 KB), B tiles,
-// column scales, row scale table, row {d, dmin}, barriers and flags
-__host__ __device__ constexpr size_t umma_smem_core_bytes() {
-  return (size_t)kStages * kStageBytes + kSB * 8 * 4096 + kSB * 8 * 32 * 32 + kSB * 8 * kScsLd * 4 + kSB * 8 * kTileM * 2 +
-         kSB * kTileM * 8 + 160;
-}
+// per-instance constants: NB = columns / 16
+template <int NB, bool LANES>
+struct Cfg {
+  static constexpr int N = 16 * NB;
+  static constexpr int PS = LANES ? 4 / NB : 4;                       // sub-block pairs of a superblock that a CTA handles
+  // TMEM: kBatches batches of accumulators (128 columns each) and kA steps of operand A (32 each), handed over kHalf at a time.
+  // What a step costs the MMA thread beside its MMAs is mostly waits, so few columns take larger halves and fewer batches -- but in the
+  // lane order, whose scalers pause at the end of a class, three batches are better (32 columns, 152k rows: 176 us, with two 199).
+  static constexpr int kBatches = LANES || NB == 4 ? 3 : 2, kA = LANES || NB == 4 ? 4 : 8, kHalf = kA / 2;
+  static constexpr int BT = 4 / NB;                                   // steps per batch of the scalers: 128 TMEM columns
+  static constexpr int kTabs = kA + kBatches * BT;               // row tables: a step's is read before its successor's is written (see there)
+  static constexpr int kWBytes = kTileM * (PS == 4 ? 144 : 16 + 32 * PS);
+  static constexpr int kBBytes = N * 128;                             // operand B of a step
+  static constexpr int kStage = (kWBytes + PS * kBBytes + 1023) & ~1023;
+  // registers of expanders, the single warps, scalers: 640 x 96 at launch = 256 E + 128 M + 256 S at most
+  static constexpr int kRegE = 64, kRegM = 64, kRegS = 144;
+  static constexpr int kColBytes = PS * N * 16;                       // column factors of a superblock
+};
 
 struct UmmaParams {
-  GemvParams g;   // K, segments, total_vrows, x = Q8_1 blocks [B][K/32][36], status
-  int B;          // activation columns of this launch, 1..32
-  int Npad;       // MMA N: 16 or 32
-  int use_maps;   // weights are fed by tiled TMA loads through maps[] (segment i -> maps[i]; the up matrix of a SwiGLU launch -> maps[4])
-  int ksplit;     // > 1: every tile is cut along K over ksplit thread blocks (launches of few tiles)
-  float* scratch; // ksplit > 1: per-chunk partial sums [tile][chunk][32 columns][128 rows]
-  int* counters;  // ksplit > 1: arrivals per tile; the last block to arrive adds the chunks in order and resets the count
-  CUtensorMap maps[5];   // use_maps: uint8 [n_rows][row bytes], box 32 rows x 144 bytes
+  GemvParams g;       // K, segments, total_vrows, x = image (see bk_tile_image_bytes), status
+  int B;              // activation columns, 1..64
+  int use_maps;       // weights come by tiled TMA loads through maps[]
+  int stages;         // ring stages
+  int csplit;         // LANES: CTAs that share the classes of a pair; TILE: CTAs that share the chunks (= cluster size)
+  int levels;         // LANES: stack levels in shared memory
+  uint32_t xbuf_bytes, stg_bytes;   // received values; values to send (clusters of more than one)
+  CUtensorMap maps[10];   // [2i], [2i+1]: headers and quants of segment i (whole superblocks: only [2i]); i = 4: the up matrix
 };
 
 BK_DEVINL uint64_t umma_desc(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
@@ -90,101 +93,189 @@ BK_DEVINL uint64_t umma_desc(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sb
          ((uint64_t)((sbo_bytes >> 4) & 0x3fffu) << 32) | (1ull << 46);
 }
 
-// f32 of the integer sc*isum, |sc*isum| < 2^22: the product lands in the mantissa of 1.5 * 2^23, which is then
-// subtracted -- both steps exact, so the value equals the integer-to-float conversion
-BK_DEVINL float scaled_sum_f32(int sc, int isum) { return __fsub_rn(__int_as_float(sc * isum + 0x4B400000), 12582912.0f); }
-
-// NC accumulator columns of this thread's TMEM lane, starting at column taddr; the load is complete after tmem_wait.
-// No memory clobber on either: they touch tensor memory only, their order among themselves is kept by `volatile`, and
-// without the clobber the compiler may move shared-memory loads of later sub-blocks across them (their latency was
-// the largest stall of the scaler warps).
-template <int NC>
-BK_DEVINL void tmem_ld(uint32_t taddr, uint32_t (&r)[NC]) {
-  if constexpr (NC == 8) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-  } else {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(taddr));
-  }
+// Four registers of a 16x256b fragment (16 lanes x 8 columns): rows lane/4 and lane/4 + 8, columns 2(lane mod 4) and the next;
+// complete after tmem_wait.  No memory clobber: they touch tensor memory only and `volatile` keeps their order.
+BK_DEVINL void tmem_ld_frag(uint32_t taddr, float (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];" : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]) : "r"(taddr));
 }
 // the registers are operands so that no use of them can be scheduled before the wait
-template <int NC>
-BK_DEVINL void tmem_wait(uint32_t (&r)[NC]) {
-  if constexpr (NC == 8) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]));
-  } else {
-    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]));
-  }
+BK_DEVINL void tmem_wait16(float (&a)[4], float (&b)[4], float (&c)[4], float (&d)[4]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+f"(a[0]), "+f"(a[1]), "+f"(a[2]), "+f"(a[3]), "+f"(b[0]), "+f"(b[1]), "+f"(b[2]), "+f"(b[3]), "+f"(c[0]), "+f"(c[1]), "+f"(c[2]),
+                 "+f"(c[3]), "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]));
 }
 
-// Bounded wait whose polls may sleep: the hint lets the hardware keep the warp suspended for up to a millisecond per
-// try (it wakes as soon as the phase completes), so that waiting roles do not spend issue slots on polling.  2048 tries
-// bound a wait to about two seconds; the first wait of a CTA that gives up sets the status word and a flag in shared
-// memory, after which every other wait of that CTA returns at once -- the kernel then runs to its end (results
-// undefined, status BK_ERR_TIMEOUT) instead of timing out step after step.
+// Bounded wait whose polls may sleep (a waiting role should not spend issue slots on polling).  The first wait of a CTA that gives
+// up sets the status word and a flag in shared memory, after which every other wait of that CTA returns at once -- the kernel
+// then runs to its end (results undefined, status BK_ERR_TIMEOUT) instead of timing out step after step.
+template <bool CLUSTER = false>
+BK_DEVINL bool mbar_poll(uint32_t bar, uint32_t parity, bool may_sleep) {
+  uint32_t ok;
+  if (CLUSTER)
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(ok)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+  else if (may_sleep)
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  else
+    asm volatile("{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+template <bool CLUSTER = false>
 BK_DEVINL void mbar_wait_idle(uint32_t bar, uint32_t parity, int* status, volatile int* dead) {
-  for (int it = 0; it < 2048; it++) {
-    uint32_t ok;
-    asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(1000000u)
-        : "memory");
-    if (ok || *dead) return;
-  }
+  if (!CLUSTER && mbar_poll(bar, parity, false)) return;
+#pragma unroll 1
+  for (int it = 0; it < (1 << 22); it++)
+    if (mbar_poll<CLUSTER>(bar, parity, true) || *dead) return;
   *dead = 1;
   if (status) atomicExch(status, 10003 /* BK_ERR_TIMEOUT */);
 }
 
 BK_DEVINL void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+BK_DEVINL void mbar_arrive_remote(uint32_t bar, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(bar), "r"(rank));
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(r) : "memory");
+}
+// bytes at src (this CTA) to the same kind of address in another CTA of the cluster, whose barrier counts them
+BK_DEVINL void bulk_s2cluster(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar, uint32_t rank) {
+  uint32_t d, b;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(dst), "r"(rank));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(bar), "r"(rank));
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(d), "r"(src), "r"(bytes), "r"(b) : "memory");
+}
+BK_DEVINL void umma_commit(uint32_t bar) {   // arrives when every MMA issued so far has completed
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+template <bool ACC>   // D (+)= A * B, K = 16
+BK_DEVINL void umma_f16(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc) {
+  asm volatile("{\n\t.reg .pred pz;\n\tsetp.ne.b32 pz, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, pz;\n\t}" ::"r"(d), "r"(a), "l"(bdesc),
+               "r"(idesc), "n"(ACC ? 1 : 0)
+               : "memory");
+}
+BK_DEVINL void scalers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kScalers) : "memory"); }
+BK_DEVINL void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
-// NC: accumulator columns per scaler thread (MMA N / 4): 4 or 8
-template <int NC>
+// The superblocks of a tile that a CTA handles, in order.
+// LANES: class positions [pos0, pos1) of the order 0,4,2,6,1,5,3,7, within a class ascending.  TILE: [pos0, pos1) themselves.
+template <bool LANES>
+struct Walk {
+  int pos, pos1, s, nsb;
+  BK_DEVINL static int cls(int pos) { return (int)((0x73516240u >> (4 * pos)) & 7u); }
+  BK_DEVINL void start(int pos0, int end, int n) {
+    nsb = n;
+    pos1 = end;
+    pos = pos0;
+    if (LANES) {
+      s = cls(pos);
+      settle();
+    } else s = pos;
+  }
+  BK_DEVINL bool done() const { return LANES ? pos >= pos1 : s >= pos1; }
+  BK_DEVINL void settle() {   // to the next class that has a superblock
+    while (pos < pos1 && s >= nsb) {
+      pos++;
+      s = cls(pos & 7);
+    }
+  }
+  BK_DEVINL void next() {
+    if (LANES) {
+      s += 8;
+      settle();
+    } else s++;
+  }
+};
+
+BK_DEVINL float2 mul2(float2 a, float2 b) {
+  unsigned long long ra, rb, rd;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
+  return d;
+}
+BK_DEVINL float2 add2(float2 a, float2 b) {
+  unsigned long long ra, rb, rd;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
+  return d;
+}
+BK_DEVINL float2 dup2(float a) { return make_float2(a, a); }
+BK_DEVINL uint32_t hfma2(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t d;
+  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+BK_DEVINL uint32_t hadd2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+BK_DEVINL uint32_t hmul2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+
+template <int NB, bool LANES>
 __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_constant__ UmmaParams P) {
+  using C = Cfg<NB, LANES>;
+  constexpr int N = C::N, PS = C::PS, BT = C::BT;
   bk_pdl_trigger();
   const GemvParams& p = P.g;
   extern __shared__ __align__(1024) uint8_t smem[];
-  constexpr int Npad = 4 * NC;
-  uint8_t* raw = smem;                                             // [kStages][128 rows][kRowPitch]
-  uint8_t* As = raw + (size_t)kStages * kStageBytes;               // [kSB][8][4096]
-  uint8_t* Bs = As + kSB * 8 * 4096;                               // [kSB][8][Npad*32]
-  float* scs = reinterpret_cast<float*>(Bs + kSB * 8 * 32 * 32);   // [kSB][8][d8 of 32 columns | s8 of 32 columns | pad]
-  uint16_t* scm = reinterpret_cast<uint16_t*>(scs + kSB * 8 * kScsLd);   // [kSB][8][128] sc | m << 8 of (sub-block, row)
-  float2* dd = reinterpret_cast<float2*>(scm + kSB * 8 * kTileM);  // [kSB][128] {d, dmin} of a row's superblock
-  uint64_t* full = reinterpret_cast<uint64_t*>(dd + kSB * kTileM); // [kStages] weights of a stage have landed
-  uint64_t* empty = full + kStages;                                // [kStages] every row of a stage has been unpacked (4 arrivals)
-  uint64_t* ab_full = empty + kStages;                             // [kSB] tiles and tables of a step written (192 arrivals)
-  uint64_t* smem_free = ab_full + kSB;                             // [kSB] the scalers are done with a shared-memory buffer (16 arrivals)
-  uint64_t* mma_done = smem_free + kSB;                            // [2] the step's MMAs have completed
-  uint64_t* tmem_free = mma_done + 2;                              // [2] the scalers have read an accumulator buffer (16 arrivals)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_free + 2);
-  int* last_flag = reinterpret_cast<int*>(tmem_slot + 1);   // K cut: this block arrived last at its tile's counter
-  volatile int* dead = last_flag + 1;                        // a bounded wait of this CTA has given up
-  float* xchg = reinterpret_cast<float*>(smem + umma_smem_core_bytes());   // [32 columns][64]: up values of a SwiGLU tile (tensor-map feed)
-  const bool swiglu_halves = P.use_maps && p.segs[0].epi == BK_EPI_SWIGLU;   // tile rows 0..63 gate, 64..127 up
+  const int nst = P.stages;
+  uint8_t* raw = smem;                                              // [nst] weights | operand B
+  uint8_t* rows = raw + (size_t)nst * C::kStage;                    // [kTabs] float4 {d, -dmin, m0, m1} [128] of a step
+  uint8_t* cols = rows + C::kTabs * kTileM * 16;                    // [nst + 3] column factors of a superblock: [pair] float4 {d8, d8', s8, s8'} [2][N/2]
+  const int ncols = nst + 3;
+  float* xbuf = reinterpret_cast<float*>(cols + ncols * C::kColBytes);   // values received: [value][own column][kXPitch rows]
+  uint8_t* stg = reinterpret_cast<uint8_t*>(xbuf) + P.xbuf_bytes;   // values to send: [owner][value][column of the owner][kXPitch rows]
+  float2* stack = reinterpret_cast<float2*>(stg + P.stg_bytes);     // [levels][16][256]
+  uint64_t* wfull = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(stack) + (size_t)P.levels * 32768);   // [kMaxStages] a stage has landed
+  uint64_t* wempty = wfull + kMaxStages;                            // [kMaxStages] its readers are done
+  uint64_t* a_full = wempty + kMaxStages;                           // [2] operand A and row tables of half a ring are written
+  uint64_t* a_free = a_full + 2;                           // [2] its MMAs have completed
+  uint64_t* d_full = a_free + 2;                          // [kBatches] accumulators of a batch complete, tables visible
+  uint64_t* d_free = d_full + C::kBatches;                             // [kBatches] the scalers are done with it
+  uint64_t* xfull = d_free + C::kBatches;                              // the cluster's values of a tile have arrived
+  uint64_t* xempty = xfull + 1;                                     // every owner has read this CTA's values
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xempty + 1);
+  volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);   // a bounded wait of this CTA has given up
 
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const int K = p.K, nsb = K / 256, nblk = K / 32;
+  const int nsb = p.K / 256;
+  constexpr int PSPLIT = 4 / PS;
+  const int CS = P.csplit * PSPLIT;
+  uint32_t rank;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
 
   if (t == 0) {
     *dead = 0;
-    for (int i = 0; i < kStages; i++) {
-      mbar_init(smem_u32(full + i), 1);
-      mbar_init(smem_u32(empty + i), kExpanderWarps);
-    }
-    for (int i = 0; i < kSB; i++) {
-      mbar_init(smem_u32(ab_full + i), (kExpanderWarps + kStagerWarps) * 32);
-      mbar_init(smem_u32(smem_free + i), kScalerWarps);
+    for (int i = 0; i < nst; i++) {
+      mbar_init(smem_u32(wfull + i), 1);
+      mbar_init(smem_u32(wempty + i), (PS == 1 ? 4 : 8) + 1);   // expander warps, and a scaler for the MMAs
     }
     for (int i = 0; i < 2; i++) {
-      mbar_init(smem_u32(mma_done + i), 1);
-      mbar_init(smem_u32(tmem_free + i), kScalerWarps);
+      mbar_init(smem_u32(a_full + i), C::kHalf * kTileM);
+      mbar_init(smem_u32(a_free + i), 1);
     }
+    for (int i = 0; i < C::kBatches; i++) {
+      mbar_init(smem_u32(d_full + i), 2);
+      mbar_init(smem_u32(d_free + i), kScalers / 32);
+    }
+    mbar_init(smem_u32(xfull), 1);
+    mbar_init(smem_u32(xempty), CS);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols)
@@ -193,350 +284,459 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  cluster_sync();   // every CTA's barriers exist
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+  const uint32_t tmem_a = tmem + C::kBatches * 128;
 
   const int n_tiles = (p.total_vrows + kTileM - 1) / kTileM;
   const int n_chunks = (nsb + 3) / 4;
-  // this CTA's tiles tile0, tile0 + tile_step, ... (n_my of them) and, of each, superblocks [s_begin, s_begin + n_s)
-  int tile0 = (int)blockIdx.x, tile_step = (int)gridDim.x, s_begin = 0, n_s = nsb;
-  int n_my = (n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-  if (P.ksplit > 1) {
-    const int part = (int)blockIdx.x % P.ksplit;
-    const int c0 = part * n_chunks / P.ksplit, c1 = (part + 1) * n_chunks / P.ksplit;   // whole chunks, at least one
-    tile0 = (int)blockIdx.x / P.ksplit;
-    tile_step = 0;
-    n_my = 1;
-    s_begin = 4 * c0;
-    n_s = min(nsb, 4 * c1) - s_begin;
-  }
-  const int npairs = (n_s + 1) / 2;
-  const int G = n_my * n_s;       // superblock steps of this CTA, tile after tile
-  const int Q = n_my * npairs;    // ring fills: pairs of superblock columns, never across a tile boundary
+  const int tile0 = (int)blockIdx.x / CS, tile_step = (int)gridDim.x / CS;   // the cluster's tiles
+  const int n_my = (n_tiles - tile0 + tile_step - 1) / tile_step;
+  const int p0 = LANES ? ((int)rank % PSPLIT) * PS : 0, part = LANES ? (int)rank / PSPLIT : (int)rank;
+  const int pos0 = LANES ? part * 8 / P.csplit : 4 * (part * n_chunks / P.csplit);
+  const int pos1 = LANES ? (part + 1) * 8 / P.csplit : min(nsb, 4 * ((part + 1) * n_chunks / P.csplit));
+  int n_sb = 0;   // superblocks of a tile that this CTA handles, and of all its tiles
+  for (int pos = pos0; pos < pos1; pos++) n_sb += LANES ? max(0, (nsb - Walk<LANES>::cls(pos) + 7) / 8) : 1;
+  const int total = n_my * n_sb;
+  const int own = N / CS;   // columns of a tile that a CTA of the cluster owns
+  const bool swiglu_halves = P.use_maps && p.segs[0].epi == BK_EPI_SWIGLU;   // tile rows 0..63 gate, 64..127 up
 
-  if (warp >= kStagerWarp0 && warp < kStagerWarp0 + kStagerWarps) {
-    // ================= stagers: Q8_1 activation blocks of step g -> B tiles and scales of buffer g&1 =================
-    const int te = t - kStagerWarp0 * 32;
-    const uint32_t* xq = reinterpret_cast<const uint32_t*>(p.x);
-    // activation blocks of a superblock: Npad*8 items (column b, sub-block j); eight neighbouring threads take eight
-    // neighbouring columns of one sub-block, whose 16-byte rows are contiguous in the B tile (no bank conflicts);
-    // stager thread te takes items te, te + 64, ...
-    constexpr int kXI = Npad * 8 / 64;   // 2 or 4
-    uint32_t xw[kXI][9];
-    auto load_x = [&](int s) {
+  if (warp < kProducerWarp) {
+    // ================= expanders: row te of every second step =================
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegE));
+    const int grp = warp >> 2, te = t & (kTileM - 1);
+    int stage = 0, g = grp, tab = grp, sbc = 0;   // g: step
+    uint32_t spar = 0;
+    const uint32_t ta = tmem_a + ((uint32_t)((warp & 3) * 32) << 16);
+    {
+      for (; sbc < total; sbc++) {
+        if (PS > 1 || (sbc & 1) == grp) {
+          mbar_wait_idle(smem_u32(wfull + stage), spar, p.status, dead);
+          const uint8_t* base = raw + (size_t)stage * C::kStage;
+          uint4 hdr, qv[PS > 1 ? PS : 2];
+          if (PS == 4) {
+            hdr = *reinterpret_cast<const uint4*>(base + te * 144);
 #pragma unroll
-      for (int i = 0; i < kXI; i++) {
-        const int it = te + 64 * i, j = (it >> 3) & 7, b = (it & 7) + 8 * (it >> 6);
+            for (int i = 0; i < PS; i++) qv[i] = *reinterpret_cast<const uint4*>(base + te * 144 + 16 + (2 * (i >> 1) + grp) * 32 + (i & 1) * 16);
+          } else {
+            hdr = *reinterpret_cast<const uint4*>(base + te * 16);
+            const uint8_t* qr = base + kTileM * 16 + te * 32 * PS;   // boxes are swizzled: 16-byte chunk c of a row lies at c ^ f(row)
+            const int sw = PS == 1 ? (te >> 2) & 1 : (te >> 1) & 3, c0 = PS == 1 ? 0 : 2 * grp;
+            qv[0] = *reinterpret_cast<const uint4*>(qr + ((c0 ^ sw) * 16));
+            qv[1] = *reinterpret_cast<const uint4*>(qr + (((c0 + 1) ^ sw) * 16));
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(wempty + stage));   // this warp's rows are in registers
+          const float d = bk_f16_to_f32((uint16_t)(hdr.x & 0xffffu)), nmin = -bk_f16_to_f32((uint16_t)(hdr.x >> 16));
 #pragma unroll
-        for (int k = 0; k < 9; k++) xw[i][k] = b < P.B ? __ldcg(xq + ((size_t)b * nblk + (size_t)s * 8 + j) * 9 + k) : 0u;
-      }
-    };
-    auto store_x = [&](int buf) {
+          for (int i = 0; i < (PS > 1 ? PS / 2 : 1); i++) {
+            const int pi = PS > 1 ? 2 * i + grp : 0;
+            uint32_t sc2, mn2;
+            bk_q4k_scale_min_pair(hdr.y, hdr.z, hdr.w, p0 + pi, sc2, mn2);
+            // half2 of the scales: (1024 + sc) - 1024; the nibble in the mantissa of 1024: (1024 + q) * sc - 1024 * sc, exact
+            const uint32_t s0 = hadd2(__byte_perm(sc2, 0x64u, 0x4040), 0xE400E400u), s1 = hadd2(__byte_perm(sc2, 0x64u, 0x4141), 0xE400E400u);
+            const uint32_t n0 = hmul2(s0, 0xE400E400u), s1s = hmul2(s1, 0x2C002C00u), n1 = hmul2(s1, 0xD400D400u);   // -1024 sc0, sc1 / 16, -64 sc1
+            uint32_t a[32];
 #pragma unroll
-      for (int i = 0; i < kXI; i++) {
-        const int it = te + 64 * i, j = (it >> 3) & 7, b = (it & 7) + 8 * (it >> 6);
-        uint8_t* tile_j = Bs + (size_t)buf * 8 * (Npad * 32) + (size_t)j * (Npad * 32) + (b >> 3) * 128 + (b & 7) * 16;
-        *reinterpret_cast<uint4*>(tile_j) = make_uint4(xw[i][0], xw[i][1], xw[i][2], xw[i][3]);
-        *reinterpret_cast<uint4*>(tile_j + Npad * 16) = make_uint4(xw[i][4], xw[i][5], xw[i][6], xw[i][7]);
-        int qsum = 0;
-#pragma unroll
-        for (int k = 0; k < 8; k++) qsum = bk_dp4a_ss(xw[i][k], 0x01010101u, qsum);
-        const float d8 = bk_q8half_to_f32((uint16_t)(xw[i][8] & 0xffffu));
-        scs[(size_t)buf * 8 * kScsLd + j * kScsLd + b] = d8;
-        scs[(size_t)buf * 8 * kScsLd + j * kScsLd + 32 + b] = __fmul_rn(d8, (float)qsum);
-      }
-    };
-
-    bk_pdl_wait();
-    load_x(s_begin);
-    int s = 0;
-    int buf = 0;          // shared-memory buffer g mod kSB, and the parity of its use number g / kSB
-    uint32_t upar = 0;
-    for (int g = 0; g < G; g++) {
-      if (g >= kSB) mbar_wait_idle(smem_u32(smem_free + buf), upar ^ 1u, p.status, dead);   // the scalers have finished step g - kSB
-      store_x(buf);
-      s = s + 1 == n_s ? 0 : s + 1;
-      if (g + 1 < G) load_x(s_begin + s);   // in flight until the next step
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      mbar_arrive(smem_u32(ab_full + buf));
-      if (++buf == kSB) {
-        buf = 0;
-        upar ^= 1u;
+            for (int j = 0; j < 8; j++) {
+              const uint4 qq = qv[2 * i + (j >> 2)];
+              const uint32_t wv = (j & 3) == 0 ? qq.x : (j & 3) == 1 ? qq.y : (j & 3) == 2 ? qq.z : qq.w, w8 = wv >> 8;
+              a[2 * j] = hfma2((wv & 0x000f000fu) | 0x64006400u, s0, n0);            // bytes 0, 2
+              a[2 * j + 1] = hfma2((w8 & 0x000f000fu) | 0x64006400u, s0, n0);        // bytes 1, 3
+              a[16 + 2 * j] = hfma2((wv & 0x00f000f0u) | 0x64006400u, s1s, n1);
+              a[17 + 2 * j] = hfma2((w8 & 0x00f000f0u) | 0x64006400u, s1s, n1);
+            }
+            if (g >= C::kA) mbar_wait_idle(smem_u32(a_free + ((g / C::kHalf) & 1)), (uint32_t)(g / C::kA - 1) & 1u, p.status, dead);   // step g - kA has been multiplied
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            asm volatile(
+                "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
+                "%20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(ta + (g % C::kA) * 32),
+                "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(a[8]), "r"(a[9]), "r"(a[10]), "r"(a[11]),
+                "r"(a[12]), "r"(a[13]), "r"(a[14]), "r"(a[15]), "r"(a[16]), "r"(a[17]), "r"(a[18]), "r"(a[19]), "r"(a[20]), "r"(a[21]), "r"(a[22]),
+                "r"(a[23]), "r"(a[24]), "r"(a[25]), "r"(a[26]), "r"(a[27]), "r"(a[28]), "r"(a[29]), "r"(a[30]), "r"(a[31])
+                : "memory");
+            // (step g - kTabs, whose table this was, has been scaled: the MMAs of step g - kA waited for that)
+            reinterpret_cast<float4*>(rows + tab * (kTileM * 16))[te] =
+                make_float4(d, nmin, __fsub_rn(__uint_as_float(__byte_perm(mn2, 0x4B000000u, 0x7440)), 8388608.0f),
+                            __fsub_rn(__uint_as_float(__byte_perm(mn2, 0x4B000000u, 0x7441)), 8388608.0f));
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            mbar_arrive(smem_u32(a_full + ((g / C::kHalf) & 1)));
+            g += 2;
+            tab += 2;
+            if (tab >= C::kTabs) tab -= C::kTabs;
+          }
+        }
+        if (++stage == nst) {
+          stage = 0;
+          spar ^= 1u;
+        }
       }
     }
-  } else if (warp == kMmaWarp) {
-    // ================= MMA issue: eight MMAs, one per sub-block, into accumulator buffer g&1 =================
-    // M = 128, N = Npad, int32 accumulators, A unsigned 8-bit, B signed 8-bit, both K-major
-    const uint32_t idesc = (2u << 4) | (0u << 7) | (1u << 10) | ((uint32_t)(Npad >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
-    int buf = 0;
-    uint32_t upar = 0;
-    for (int g = 0; g < G; g++) {
-      const int tb = g & 1;   // accumulator buffer
-      mbar_wait_idle(smem_u32(ab_full + buf), upar, p.status, dead);   // all 128 rows and the activations are in place
-      if (g >= 2) mbar_wait_idle(smem_u32(tmem_free + tb), (uint32_t)(((g >> 1) & 1) ^ 1), p.status, dead);   // step g-2 has been read out
+    for (const int end = (total * PS + C::kHalf - 1) / C::kHalf * C::kHalf; g < end; g += 2) mbar_arrive(smem_u32(a_full + ((g / C::kHalf) & 1)));   // steps that the last half lacks
+  } else if (warp < kScalerWarp0) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegM));
+    if (warp >= kEpilogueWarp0) {
+      // ================= epilogue: the columns this CTA owns, in the fixed order of addition =================
+      const int et = t - kEpilogueWarp0 * 32;
+      bk_pdl_wait();
+      const int vs = own * kXPitch;   // floats between values
+      auto value = [&](int c, int r) {
+        const float* v = xbuf + c * kXPitch + r;
+        if constexpr (!LANES) {
+          if (CS == 1) return v[0];
+          float y = 0.0f;
+          for (int ch = 0; ch < n_chunks; ch++) y = __fadd_rn(y, v[ch * vs]);
+          return y;
+        } else {
+          float T[4];
+#pragma unroll
+          for (int pp = 0; pp < 4; pp++) {   // value of (part, pair): sent by CTA part * PSPLIT + pair / PS
+            const float* vp = v + pp * vs;
+            if (P.csplit == 1) T[pp] = vp[0];
+            else if (P.csplit == 2) T[pp] = __fadd_rn(vp[0], vp[4 * vs]);
+            else if (P.csplit == 4) T[pp] = __fadd_rn(__fadd_rn(vp[0], vp[4 * vs]), __fadd_rn(vp[8 * vs], vp[12 * vs]));
+            else
+              T[pp] = __fadd_rn(__fadd_rn(__fadd_rn(vp[0], vp[4 * vs]), __fadd_rn(vp[8 * vs], vp[12 * vs])),
+                                __fadd_rn(__fadd_rn(vp[16 * vs], vp[20 * vs]), __fadd_rn(vp[24 * vs], vp[28 * vs])));
+          }
+          return __fadd_rn(__fadd_rn(T[0], T[2]), __fadd_rn(T[1], T[3]));
+        }
+      };
+      const uint32_t xbytes = (uint32_t)((LANES ? 4 * P.csplit : n_chunks) * vs * 4);
+      const int b0 = (int)rank * own;
+      for (int k = 0; k < n_my; k++) {
+        const int tile = tile0 + k * tile_step;
+        if (CS > 1 && et == 0) mbar_expect_tx(smem_u32(xfull), xbytes);
+        mbar_wait_idle(smem_u32(xfull), (uint32_t)k & 1u, p.status, dead);
+        for (int h = 0; h < (swiglu_halves ? 1 : 2); h++) {
+          const int r = et + 64 * h;
+          VRow vr = {nullptr, 0, 0};
+          bool have;
+          int up = 0;   // distance to the up row of a SwiGLU pair
+          if (swiglu_halves) {
+            vr.n = tile * 64 + r;
+            have = vr.n < p.segs[0].n_rows;
+            up = 64;
+          } else {
+            have = tile * kTileM + r < p.total_vrows;
+            if (have) vr = decode_vrow(p, tile * kTileM + r);
+            if (p.segs[vr.si].epi == BK_EPI_SWIGLU) {
+              up = 1;
+              have = have && !(r & 1);
+            }
+          }
+          const SegDev& sg = p.segs[vr.si];
+          if (!have) continue;
+          const size_t o0 = (size_t)b0 * sg.ld_out + sg.col_off + vr.n, ld = sg.ld_out;
+          const int nc = min(own, P.B - b0), epi = sg.epi;
+          if (epi == BK_EPI_F32) {
+            float* o = static_cast<float*>(sg.out) + o0;
+#pragma unroll 4
+            for (int c = 0; c < nc; c++) o[c * ld] = value(c, r);
+          } else if (epi == BK_EPI_BF16) {
+            uint16_t* o = static_cast<uint16_t*>(sg.out) + o0;
+#pragma unroll 4
+            for (int c = 0; c < nc; c++) o[c * ld] = bk_f32_to_bf16(value(c, r));
+          } else if (epi == BK_EPI_SWIGLU) {
+            uint16_t* o = static_cast<uint16_t*>(sg.out) + o0;
+#pragma unroll 4
+            for (int c = 0; c < nc; c++) {
+              const float y = value(c, r);
+              o[c * ld] = bk_f32_to_bf16(__fmul_rn(__fmul_rn(y, bk_sigmoidf(y)), value(c, r + up)));
+            }
+          } else {   // BK_EPI_ADD_BF16
+            uint16_t* o = static_cast<uint16_t*>(sg.out) + o0;
+            const uint16_t* res = sg.res + o0;
+#pragma unroll 1
+            for (int c0 = 0; c0 < nc; c0 += 8) {   // eight residuals in flight (the outputs may alias them)
+              uint16_t rs[8];
+#pragma unroll
+              for (int j = 0; j < 8; j++) rs[j] = c0 + j < nc ? res[(c0 + j) * ld] : (uint16_t)0;
+#pragma unroll
+              for (int j = 0; j < 8; j++)
+                if (c0 + j < nc) o[(c0 + j) * ld] = bk_f32_to_bf16(__fadd_rn(value(c0 + j, r), bk_bf16_to_f32(rs[j])));
+            }
+          }
+        }
+        asm volatile("bar.sync 2, 64;" ::: "memory");
+        if (et < CS) mbar_arrive_remote(smem_u32(xempty), et);
+      }
+    } else if (warp == kMmaWarp) {
+      // ================= MMA issue: per step two sub-blocks of K = 32 =================
+      // One lane only, and few instructions: this thread has to keep up with four warps per scheduler.
+      // f32 accumulators, f16 operands, both K-major
+      constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
       if (lane == 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a0 = smem_u32(As + (size_t)buf * 8 * 4096);
-        const uint32_t b0 = smem_u32(Bs + (size_t)buf * 8 * (Npad * 32));
+        int stage = 0, batch = 0, g = 0;
+        uint32_t spar = 0, bpar = 1;   // a fresh barrier counts as freed
+        {
+          for (int i = 0; i < total; i++) {
+            mbar_wait_idle(smem_u32(wfull + stage), spar, p.status, dead);   // operand B and the column factors
+            uint64_t bd = umma_desc(smem_u32(raw + (size_t)stage * C::kStage + C::kWBytes), N * 16, 128);
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-          const uint64_t ad = umma_desc(a0 + j * 4096, 2048, 128);
-          const uint64_t bd = umma_desc(b0 + j * (Npad * 32), (uint32_t)Npad * 16, 128);
-          const uint32_t dcol = tmem + (uint32_t)(tb * 256 + j * Npad);
-          asm volatile(
-              "{\n\t.reg .pred pz;\n\tsetp.ne.b32 pz, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, pz;\n\t}"
-              ::"r"(dcol), "l"(ad), "l"(bd), "r"(idesc), "r"(0u), "r"(0u)
-              : "memory");
-        }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(mma_done + tb))
-                     : "memory");
-      }
-      __syncwarp();
-      if (++buf == kSB) {
-        buf = 0;
-        upar ^= 1u;
-      }
-    }
-  } else if (warp == kProducerWarp) {
-    // ================= producer: fill ring stage q mod kStages with pair q (weights depend on no earlier kernel) ==========
-    for (int q = 0; q < Q; q++) {
-      if (q >= kStages) mbar_wait_idle(smem_u32(empty + q % kStages), (uint32_t)((q / kStages - 1) & 1), p.status, dead);
-      const int tl = q / npairs, pp = q - tl * npairs;
-      const int tile = tile0 + tl * tile_step;
-      const uint32_t bytes = (uint32_t)((n_s - 2 * pp) >= 2 ? 288 : 144);
-      const int rows_here = min(kTileM, p.total_vrows - tile * kTileM);
-      const uint32_t bar = smem_u32(full + q % kStages);
-      const uint32_t dst0 = smem_u32(raw + (size_t)(q % kStages) * kStageBytes);
-      if (P.use_maps) {
-        // lane l < 8: 32-row box l & 3 of the tile, superblock column l >> 2 of the pair
-        const int k = lane & 3, sbi = lane >> 2;
-        bool valid = lane < 8 && (uint32_t)sbi * 144 < bytes;
-        int mi = 0, row0 = 0;
-        if (swiglu_halves) {   // boxes 0, 1: gate rows tile*64 + 32k; boxes 2, 3: the same rows of the up matrix
-          row0 = tile * 64 + 32 * (k & 1);
-          mi = k < 2 ? 0 : 4;
-          valid = valid && row0 < p.segs[0].n_rows;
-        } else {
-          const int v0 = tile * kTileM + 32 * k;
-          valid = valid && v0 < p.total_vrows;
-#pragma unroll
-          for (int i = 1; i < 4; i++)
-            if (i < p.n_segs && v0 >= p.segs[i].vrow_begin) mi = i;
-          row0 = v0 - p.segs[mi].vrow_begin;
-        }
-        const unsigned n_valid = __popc(__ballot_sync(0xffffffffu, valid));
-        if (lane == 0) mbar_expect_tx(bar, n_valid * 32u * 144u);
-        __syncwarp();
-        if (valid) {
-          const int x = (s_begin + 2 * pp + sbi) * 144;
-          asm volatile(
-              "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-              ::"r"(dst0 + (uint32_t)(sbi * kPlaneBytes + 32 * k * 144)), "l"(reinterpret_cast<uint64_t>(&P.maps[mi])), "r"(x), "r"(row0),
-              "r"(bar)
-              : "memory");
-        }
-        continue;
-      }
-      if (lane == 0) mbar_expect_tx(bar, (uint32_t)rows_here * bytes);
-      __syncwarp();
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        const int r = lane + 32 * k;
-        if (r < rows_here) bulk_g2s(dst0 + r * kRowPitch, decode_vrow(p, tile * kTileM + r).row + (size_t)s_begin * 144 + (size_t)pp * 288, bytes, bar);
-      }
-    }
-  } else if (warp >= kScalerWarp0) {
-    // ================= scalers: f32 part of step g from accumulator buffer g&1 =================
-    const int row_t = t & (kTileM - 1);   // tile row (= TMEM lane) of this thread
-    const int qd = (t >> 7) - kScalerWarp0 / 4;   // which quarter of the columns
-    bk_pdl_wait();
-    float y[NC], yc[NC];
-#pragma unroll
-    for (int c = 0; c < NC; c++) y[c] = yc[c] = 0.0f;
-    int s = 0, tl = 0;
-    int buf = 0;
-    uint32_t upar = 0;
-    for (int g = 0; g < G; g++) {
-      const int tb = g & 1;   // accumulator buffer
-      mbar_wait_idle(smem_u32(ab_full + buf), upar, p.status, dead);    // the tables of this step are visible
-      mbar_wait_idle(smem_u32(mma_done + tb), (uint32_t)((g >> 1) & 1), p.status, dead);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const float2 dm = dd[buf * kTileM + row_t];
-      const float4* sb4 = reinterpret_cast<const float4*>(scs + (size_t)buf * 8 * kScsLd + qd * NC);   // d8 of this thread's columns; s8 8 float4 further
-      const uint16_t* sm_ = scm + (size_t)buf * 8 * kTileM + row_t;
-      const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(tb * 256 + qd * NC);
-      float2 accd[NC / 2], accm[NC / 2];   // columns (2i, 2i+1) side by side: one packed FMA serves both
-#pragma unroll
-      for (int c = 0; c < NC / 2; c++) accd[c] = accm[c] = make_float2(0.0f, 0.0f);
-      uint32_t r[NC], rn[NC];
-      tmem_ld<NC>(taddr, r);
-      tmem_wait<NC>(r);
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        if (j < 7) tmem_ld<NC>(taddr + (uint32_t)((j + 1) * Npad), rn);   // in flight during this sub-block's arithmetic
-        const uint32_t scmv = sm_[j * kTileM];
-        const int2 s2 = make_int2((int)(scmv & 0xffu), 0);
-        const float fm = __fsub_rn(__int_as_float((int)(scmv >> 8) + 0x4B400000), 12582912.0f);   // f32(m), exact
-        const float2 fm2 = make_float2(fm, fm);
-#pragma unroll
-        for (int c = 0; c < NC; c += 4) {
-          const float4 d4 = sb4[j * (kScsLd / 4) + (c >> 2)], s4 = sb4[j * (kScsLd / 4) + 8 + (c >> 2)];   // d8, s8 of columns c..c+3
-          accd[c / 2] = bk_fma2(make_float2(d4.x, d4.y),
-                             make_float2(scaled_sum_f32(s2.x, (int)r[c]), scaled_sum_f32(s2.x, (int)r[c + 1])), accd[c / 2]);
-          accd[c / 2 + 1] = bk_fma2(make_float2(d4.z, d4.w),
-                                 make_float2(scaled_sum_f32(s2.x, (int)r[c + 2]), scaled_sum_f32(s2.x, (int)r[c + 3])), accd[c / 2 + 1]);
-          accm[c / 2] = bk_fma2(make_float2(s4.x, s4.y), fm2, accm[c / 2]);
-          accm[c / 2 + 1] = bk_fma2(make_float2(s4.z, s4.w), fm2, accm[c / 2 + 1]);
-        }
-        if (j < 7) {
-          tmem_wait<NC>(rn);
-#pragma unroll
-          for (int c = 0; c < NC; c++) r[c] = rn[c];
-        }
-      }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) {   // tables and accumulators of this step may be overwritten
-        mbar_arrive(smem_u32(smem_free + buf));
-        mbar_arrive(smem_u32(tmem_free + tb));
-      }
-      if (++buf == kSB) {
-        buf = 0;
-        upar ^= 1u;
-      }
-#pragma unroll
-      for (int c = 0; c < NC; c += 2) {
-        yc[c] = __fadd_rn(yc[c], fmaf(dm.x, accd[c / 2].x, -__fmul_rn(dm.y, accm[c / 2].x)));
-        yc[c + 1] = __fadd_rn(yc[c + 1], fmaf(dm.x, accd[c / 2].y, -__fmul_rn(dm.y, accm[c / 2].y)));
-      }
-      const bool last = s == n_s - 1;
-      const int tile = tile0 + tl * tile_step;
-      if ((s & 3) == 3 || last) {   // a chunk of four superblocks ends
-        if (P.ksplit > 1) {         // its partial sums go to the scratch buffer; the last block of the tile adds them up
-          float* dst = P.scratch + (((size_t)tile * n_chunks + ((s_begin + s) >> 2)) * 32 + qd * NC) * kTileM + row_t;
-#pragma unroll
-          for (int c = 0; c < NC; c++) {
-            __stcg(dst + c * kTileM, yc[c]);
-            yc[c] = 0.0f;
-          }
-        } else {
-#pragma unroll
-          for (int c = 0; c < NC; c++) {
-            y[c] = __fadd_rn(y[c], yc[c]);
-            yc[c] = 0.0f;
+            for (int pi = 0; pi < PS; pi++, g++) {
+              const int bi = pi % BT;
+              if (bi == 0) mbar_wait_idle(smem_u32(d_free + batch), bpar, p.status, dead);
+              if (g % C::kHalf == 0) mbar_wait_idle(smem_u32(a_full + ((g / C::kHalf) & 1)), (uint32_t)(g / C::kA) & 1u, p.status, dead);
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              const uint32_t a0 = tmem_a + (g % C::kA) * 32, d0 = tmem + batch * 128 + bi * 2 * N;
+              umma_f16<false>(d0, a0, bd, idesc);
+              umma_f16<true>(d0, a0 + 8, bd + N * 2, idesc);
+              umma_f16<false>(d0 + N, a0 + 16, bd + N * 4, idesc);
+              umma_f16<true>(d0 + N, a0 + 24, bd + N * 6, idesc);
+              bd += N * 8;
+              if (bi == BT - 1) {
+                umma_commit(smem_u32(d_full + batch));
+                mbar_arrive(smem_u32(d_full + batch));   // passes on what the expanders and the copies have written
+                if (++batch == C::kBatches) {
+                  batch = 0;
+                  bpar ^= 1u;
+                }
+              }
+              if (g % C::kHalf == C::kHalf - 1) umma_commit(smem_u32(a_free + ((g / C::kHalf) & 1)));
+            }
+            if (++stage == nst) {
+              stage = 0;
+              spar ^= 1u;
+            }
           }
         }
       }
-      bool merge = true;
-      if (last && P.ksplit > 1) {
-        __threadfence();                                   // this thread's partial sums before the arrival
-        asm volatile("bar.sync 1, %0;" ::"n"(kScalerWarps * 32) : "memory");
-        if (t == kScalerWarp0 * 32) {
-          const int old = atomicAdd(P.counters + tile, 1);
-          if (old == P.ksplit - 1) P.counters[tile] = 0;   // everyone has arrived: ready for the next launch
-          *last_flag = old == P.ksplit - 1;
+      __syncwarp();
+    } else {
+      // ================= producer: superblock after superblock, tile after tile =================
+      int cslot = 0;
+      Walk<LANES> w, wx;
+      const int first = min(total, nst);
+      const uint64_t policy = l2_evict_first();
+      const uint8_t* img_b = static_cast<const uint8_t*>(p.x) + (size_t)p0 * C::kBBytes;   // image: operand B of all units, then their factors
+      const uint8_t* img_c = static_cast<const uint8_t*>(p.x) + (size_t)(p.K / 64) * C::kBBytes + (size_t)p0 * (N * 16);
+      auto fill_x = [&](int s, int stage) {
+        if (lane == 0) {
+          const uint32_t bar = smem_u32(wfull + stage);
+          bulk_g2s(smem_u32(raw + (size_t)stage * C::kStage + C::kWBytes), img_b + (size_t)s * 4 * C::kBBytes, PS * C::kBBytes, bar);
+          bulk_g2s(smem_u32(cols + cslot * C::kColBytes), img_c + (size_t)s * (4 * N * 16), C::kColBytes, bar);
         }
-        asm volatile("bar.sync 1, %0;" ::"n"(kScalerWarps * 32) : "memory");
-        merge = *last_flag != 0;
-        if (merge) {
-          __threadfence();
-          const float* src = P.scratch + (((size_t)tile * n_chunks) * 32 + qd * NC) * kTileM + row_t;
-          for (int ch = 0; ch < n_chunks; ch++)
+        if (++cslot == ncols) cslot = 0;   // (three superblocks more than stages: the scalers are at most that far behind the MMAs)
+      };
+      constexpr uint32_t kXBytes = PS * C::kBBytes + C::kColBytes;
+      int tile = tile0, stage = 0;
+      uint32_t spar = 1;   // parity of the readers' arrivals on the previous use
+      w.start(pos0, pos1, nsb);
+      for (int i = 0; i < total; i++) {
+        if (i >= nst) mbar_wait_idle(smem_u32(wempty + stage), spar, p.status, dead);
+        const uint32_t bar = smem_u32(wfull + stage), dst0 = smem_u32(raw + (size_t)stage * C::kStage);
+        if (P.use_maps) {
+          // lanes 0..3: the 32-row boxes of the tile (whole superblocks, or headers); lanes 4..7: their quants
+          const int bx = lane & 3;
+          bool valid = lane < (PS == 4 ? 4 : 8);
+          int mi = 0, row0 = 0;
+          if (swiglu_halves) {   // boxes 0, 1: gate rows tile*64 + 32k; boxes 2, 3: the same rows of the up matrix
+            row0 = tile * 64 + 32 * (bx & 1);
+            mi = bx < 2 ? 0 : 4;
+            valid = valid && row0 < p.segs[0].n_rows;
+          } else {
+            const int v0 = tile * kTileM + 32 * bx;
+            valid = valid && v0 < p.total_vrows;
 #pragma unroll
-            for (int c = 0; c < NC; c++) y[c] = __fadd_rn(y[c], __ldcg(src + ((size_t)ch * 32 + c) * kTileM));
+            for (int si = 1; si < 4; si++)
+              if (si < p.n_segs && v0 >= p.segs[si].vrow_begin) mi = si;
+            row0 = v0 - p.segs[mi].vrow_begin;
+          }
+          const unsigned boxes = __popc(__ballot_sync(0xffffffffu, valid && lane < 4));
+          if (lane == 0) mbar_expect_tx(bar, boxes * (uint32_t)(C::kWBytes / 4) + kXBytes);
+          __syncwarp();
+          if (valid) {
+            const bool quants = lane >= 4;
+            const int x = w.s * 144 + (quants ? 16 + 32 * p0 : 0);
+            const uint32_t dst = dst0 + (PS == 4 ? bx * 32 * 144 : quants ? kTileM * 16 + bx * 32 * 32 * PS : bx * 32 * 16);
+            asm volatile(
+                "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;" ::"r"(dst),
+                "l"(reinterpret_cast<uint64_t>(&P.maps[2 * mi + (quants ? 1 : 0)])), "r"(x), "r"(row0), "r"(bar), "l"(policy)
+                : "memory");
+          }
+        } else {
+          const int rows_here = min(kTileM, p.total_vrows - tile * kTileM);
+          if (lane == 0) mbar_expect_tx(bar, (uint32_t)rows_here * 144 + kXBytes);
+          __syncwarp();
+#pragma unroll 1
+          for (int r = lane; r < rows_here; r += 32) bulk_g2s(dst0 + r * 144, decode_vrow(p, tile * kTileM + r).row + (size_t)w.s * 144, 144, bar);
         }
-      }
-      if (last && merge && swiglu_halves) {   // gate rows in tile rows 0..63, their up rows 64 further on (other warps)
-        if (row_t >= 64) {
-#pragma unroll
-          for (int c = 0; c < NC; c++) xchg[(qd * NC + c) * 64 + row_t - 64] = y[c];
+        if (i == first - 1) {   // the ring is full of weights, which depend on nothing: now the activations of these stages
+          bk_pdl_wait();
+          int f = 0;
+          while (f < first) {
+            for (wx.start(pos0, pos1, nsb); !wx.done() && f < first; wx.next(), f++) fill_x(wx.s, f);
+          }
+        } else if (i >= first) {
+          fill_x(w.s, stage);
         }
-        asm volatile("bar.sync 1, %0;" ::"n"(kScalerWarps * 32) : "memory");
-        const SegDev& sg = p.segs[0];
-        const int n = tile * 64 + row_t;
-#pragma unroll
-        for (int c = 0; c < NC; c++) {
-          const int b = qd * NC + c;
-          if (row_t < 64 && b < P.B && n < sg.n_rows)
-            store_epilogue<false>(p, sg, (size_t)b * sg.ld_out + sg.col_off + n, y[c], xchg[b * 64 + row_t]);
-          y[c] = 0.0f;
+        w.next();
+        if (w.done()) {
+          tile += tile_step;
+          w.start(pos0, pos1, nsb);
         }
-        asm volatile("bar.sync 1, %0;" ::"n"(kScalerWarps * 32) : "memory");   // the values have been read: the next tile may overwrite them
-        s = 0;
-        tl++;
-      } else if (last && merge) {   // fused epilogue of the tile; uniform over the CTA
-        const int vrow = tile * kTileM + row_t;
-        const bool have_row = vrow < p.total_vrows;
-        VRow vr = {nullptr, 0, 0};
-        if (have_row) vr = decode_vrow(p, vrow);
-        const SegDev& sg = p.segs[vr.si];
-        const bool swiglu = have_row && sg.epi == BK_EPI_SWIGLU;
-#pragma unroll
-        for (int c = 0; c < NC; c++) {
-          const int b = qd * NC + c;
-          const float yup = __shfl_xor_sync(0xffffffffu, y[c], 1);   // the odd neighbour row: the "up" row of a SwiGLU pair
-          if (b < P.B && have_row && !(swiglu && (row_t & 1)))
-            store_epilogue<false>(p, sg, (size_t)b * sg.ld_out + sg.col_off + vr.n, y[c], yup);
-          y[c] = 0.0f;
+        if (++stage == nst) {
+          stage = 0;
+          spar ^= 1u;
         }
-        s = 0;
-        tl++;
-      } else {
-        s++;
       }
     }
   } else {
-    // ================= expanders: unpacking, scale tables =================
-    const int te = t;                 // tile row of this thread
-    bk_pdl_wait();
-    int s = 0, tl = 0;
-    int buf = 0;
-    uint32_t upar = 0;
-    for (int g = 0; g < G; g++) {
-      const int q = tl * npairs + (s >> 1);
-      const int stage = q % kStages;
-      if ((s & 1) == 0) mbar_wait_idle(smem_u32(full + stage), (uint32_t)((q / kStages) & 1), p.status, dead);
-      if (g >= kSB) mbar_wait_idle(smem_u32(smem_free + buf), upar ^ 1u, p.status, dead);   // the scalers have finished step g - kSB
-      const int s_next = s + 1 == n_s ? 0 : s + 1;
-      // header -> scale table; 4-bit quants -> unsigned int8 rows, sub-block 2p from the low nibbles of group p,
-      //     2p+1 from the high nibbles
-      const uint8_t* rw = raw + (size_t)stage * kStageBytes +
-                          (P.use_maps ? (size_t)(s & 1) * kPlaneBytes + (size_t)te * 144 : (size_t)te * kRowPitch + (s & 1) * 144);
-      const uint4 hdr = *reinterpret_cast<const uint4*>(rw);
-      dd[buf * kTileM + te] = make_float2(bk_f16_to_f32((uint16_t)(hdr.x & 0xffffu)), bk_f16_to_f32((uint16_t)(hdr.x >> 16)));
-      uint16_t* sm_w = scm + (size_t)buf * 8 * kTileM + te;
-      uint8_t* Ab = As + (size_t)buf * 8 * 4096 + (te >> 3) * 128 + (te & 7) * 16;
-      uint4 qv[8];
+    // ================= scalers: f32 part =================
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kRegS));
+    const int st = t - kScalerWarp0 * 32, q = warp & 3, half = st >> 7;
+    const int row0 = 32 * q + (lane >> 2);              // this thread's rows: row0 + 8i
+    const int col0 = half * (N / 2) + 2 * (lane & 3);   // and columns: col0 + 8cb and the next
+    const int own_shift = __ffs(own) - 1;
+    const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + half * (N / 2);
+    int batch = 0, tab = 0, col = 0, stage = 0;
+    uint32_t bpar = 0;
+    // One batch: BT steps from the current row table and pair pi0 of the current column factors on, as four blocks of 8 columns;
+    // f(m, i, x0, x1, c0, c1, r): the two columns of block m = step * NB + column block, row i, accumulators of both sub-blocks,
+    // column factors {d8, d8', s8, s8'} of both, row factors
+    auto run_batch = [&](int pi0, auto&& f) {
+      mbar_wait_idle(smem_u32(d_full + batch), bpar, p.status, dead);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const float4* ct = reinterpret_cast<const float4*>(cols + col * C::kColBytes) + pi0 * N + (col0 >> 1);
+      const uint32_t td = ta + batch * 128;
+      float x[2][2][2][4];   // [buffer][sub-block][lanes 0..15 / 16..31][fragment]
+      auto request = [&](int m) {
 #pragma unroll
-      for (int k = 0; k < 8; k++) qv[k] = *reinterpret_cast<const uint4*>(rw + 16 + 16 * k);
-      if ((s & 1) || s == n_s - 1) {   // this warp's rows of the stage are in registers: hand the stage back
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(empty + stage));
-      }
+        for (int j = 0; j < 4; j++)
+          tmem_ld_frag(td + (m / NB) * 2 * N + (m % NB) * 8 + (j >> 1) * N + ((uint32_t)(16 * (j & 1)) << 16), x[m & 1][j >> 1][j & 1]);
+      };
+      request(0);
+      float4 r4[4];
 #pragma unroll
-      for (int pq = 0; pq < 4; pq++) {
-        uint32_t sc2, mn2;
-        bk_q4k_scale_min_pair(hdr.y, hdr.z, hdr.w, pq, sc2, mn2);
-        sm_w[(2 * pq) * kTileM] = (uint16_t)((sc2 & 0xffu) | ((mn2 & 0xffu) << 8));
-        sm_w[(2 * pq + 1) * kTileM] = (uint16_t)((sc2 >> 8) | (mn2 & 0xff00u));
-        const uint4 qa = qv[2 * pq], qb = qv[2 * pq + 1];
-        uint8_t* A0 = Ab + (size_t)(2 * pq) * 4096;
-        *reinterpret_cast<uint4*>(A0) = make_uint4(qa.x & 0x0f0f0f0fu, qa.y & 0x0f0f0f0fu, qa.z & 0x0f0f0f0fu, qa.w & 0x0f0f0f0fu);
-        *reinterpret_cast<uint4*>(A0 + 2048) = make_uint4(qb.x & 0x0f0f0f0fu, qb.y & 0x0f0f0f0fu, qb.z & 0x0f0f0f0fu, qb.w & 0x0f0f0f0fu);
-        *reinterpret_cast<uint4*>(A0 + 4096) =
-            make_uint4((qa.x >> 4) & 0x0f0f0f0fu, (qa.y >> 4) & 0x0f0f0f0fu, (qa.z >> 4) & 0x0f0f0f0fu, (qa.w >> 4) & 0x0f0f0f0fu);
-        *reinterpret_cast<uint4*>(A0 + 4096 + 2048) =
-            make_uint4((qb.x >> 4) & 0x0f0f0f0fu, (qb.y >> 4) & 0x0f0f0f0fu, (qb.z >> 4) & 0x0f0f0f0fu, (qb.w >> 4) & 0x0f0f0f0fu);
+      for (int m = 0; m < 4; m++) {
+        const int u = m & 1, cb = m % NB, bi = m / NB;
+        if (cb == 0) {
+          const float4* rt = reinterpret_cast<const float4*>(rows + tab * (kTileM * 16)) + row0;
+#pragma unroll
+          for (int i = 0; i < 4; i++) r4[i] = rt[8 * i];
+          if (++tab == C::kTabs) tab = 0;
+        }
+        tmem_wait16(x[u][0][0], x[u][0][1], x[u][1][0], x[u][1][1]);
+        if (m < 3) request(m + 1);   // in flight during this block's arithmetic
+        const float4 c0 = ct[bi * N + cb * 4], c1 = ct[bi * N + N / 2 + cb * 4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          f(m, i, make_float2(x[u][0][i >> 1][2 * (i & 1)], x[u][0][i >> 1][2 * (i & 1) + 1]),
+            make_float2(x[u][1][i >> 1][2 * (i & 1)], x[u][1][i >> 1][2 * (i & 1) + 1]), c0, c1, r4[i]);
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMA reads shared memory through the async proxy
-      mbar_arrive(smem_u32(ab_full + buf));
-      if (++buf == kSB) {
-        buf = 0;
-        upar ^= 1u;
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(d_free + batch));
+      if (++batch == C::kBatches) {
+        batch = 0;
+        bpar ^= 1u;
       }
-      s = s_next;
-      if (s == 0) tl++;
+    };
+    auto next_superblock = [&]() {
+      if (st == 0) mbar_arrive(smem_u32(wempty + stage));   // its MMAs are through with operand B
+      if (++stage == nst) stage = 0;
+      if (++col == ncols) col = 0;
+    };
+    // value v (of nv that this CTA sends) of column block cb and row i into the buffer the owners read or are sent
+    float* const out = CS > 1 ? reinterpret_cast<float*>(stg) : xbuf;
+    auto place = [&](int v, int nv, int cb, int i) {
+      const int c = col0 + 8 * cb;
+      return out + ((((c >> own_shift) * nv + v) << own_shift) + (c & (own - 1))) * kXPitch + row0 + 8 * i;
+    };
+    auto send = [&](int first, int nv) {   // nv values, the owner's buffer index of the first
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      scalers_sync();
+      if (CS == 1) {
+        if (st == 0) mbar_arrive(smem_u32(xfull));
+      } else if (st < CS && nv > 0) {
+        const uint32_t bytes = (uint32_t)(nv * own * kXPitch * 4), dst = (uint32_t)(first * own * kXPitch * 4);
+        bulk_s2cluster(smem_u32(xbuf) + dst, smem_u32(stg) + st * bytes, bytes, smem_u32(xfull), st);
+      }
+    };
+
+    for (int k = 0; k < n_my; k++) {
+      if constexpr (LANES) {
+        float2 S[16], L0[16];
+        int sp = 0;
+        for (int lp = 0; lp < pos1 - pos0; lp++) {
+#pragma unroll
+          for (int e = 0; e < 16; e++) S[e] = make_float2(0.0f, 0.0f);
+          for (int s = Walk<LANES>::cls(pos0 + lp); s < nsb; s += 8) {
+            run_batch(0, [&](int m, int i, float2 x0, float2 x1, const float4& c0, const float4& c1, const float4& r) {
+              float2 a = mul2(make_float2(c0.x, c0.y), x0);
+              a = bk_fma2(make_float2(c1.x, c1.y), x1, a);
+              float2 mm = mul2(make_float2(c0.z, c0.w), dup2(r.z));
+              mm = bk_fma2(make_float2(c1.z, c1.w), dup2(r.w), mm);
+              S[m * 4 + i] = add2(S[m * 4 + i], bk_fma2(dup2(r.x), a, mul2(dup2(r.y), mm)));
+            });
+            next_superblock();
+          }
+          if (lp & 1) {
+#pragma unroll
+            for (int e = 0; e < 16; e++) S[e] = add2(L0[e], S[e]);
+            for (int m = lp >> 1; m & 1; m >>= 1) {
+              sp--;
+#pragma unroll
+              for (int e = 0; e < 16; e++) S[e] = add2(stack[(sp * 16 + e) * kScalers + st], S[e]);
+            }
+            if (lp + 1 < pos1 - pos0) {
+#pragma unroll
+              for (int e = 0; e < 16; e++) stack[(sp * 16 + e) * kScalers + st] = S[e];
+              sp++;
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 16; e++) L0[e] = S[e];
+          }
+        }
+        if (k > 0) mbar_wait_idle<true>(smem_u32(xempty), (uint32_t)(k - 1) & 1u, p.status, dead);   // what was sent before has been read
+#pragma unroll
+        for (int e = 0; e < 16; e++) {
+          float* o = place(e / (4 * NB), PS, (e / 4) % NB, e & 3);
+          o[0] = pos1 - pos0 == 1 ? L0[e].x : S[e].x;
+          o[kXPitch] = pos1 - pos0 == 1 ? L0[e].y : S[e].y;
+        }
+        send((int)rank * PS, PS);
+      } else {
+        float2 yc[NB * 4];
+        const int ch0 = pos0 >> 2, nv = CS > 1 ? (pos1 + 3) / 4 - ch0 : 1;
+        if (k > 0 && pos0 >= pos1) mbar_wait_idle<true>(smem_u32(xempty), (uint32_t)(k - 1) & 1u, p.status, dead);
+        for (int s = pos0; s < pos1; s++) {
+          float2 A[NB * 4], M[NB * 4];
+#pragma unroll
+          for (int e = 0; e < NB * 4; e++) A[e] = M[e] = make_float2(0.0f, 0.0f);
+          float rd[4], rm[4];
+#pragma unroll 1
+          for (int pi = 0; pi < 4; pi += BT)
+            run_batch(pi, [&](int m, int i, float2 x0, float2 x1, const float4& c0, const float4& c1, const float4& r) {
+              const int e = (m % NB) * 4 + i;
+              A[e] = bk_fma2(make_float2(c0.x, c0.y), x0, A[e]);
+              M[e] = bk_fma2(make_float2(c0.z, c0.w), dup2(r.z), M[e]);
+              A[e] = bk_fma2(make_float2(c1.x, c1.y), x1, A[e]);
+              M[e] = bk_fma2(make_float2(c1.z, c1.w), dup2(r.w), M[e]);
+              rd[i] = r.x;
+              rm[i] = r.y;
+            });
+          next_superblock();
+#pragma unroll
+          for (int e = 0; e < NB * 4; e++)
+            yc[e] = add2((s & 3) == 0 ? make_float2(0.0f, 0.0f) : yc[e], bk_fma2(dup2(rd[e & 3]), A[e], mul2(dup2(rm[e & 3]), M[e])));
+          if ((s & 3) == 3 || s == nsb - 1) {   // a chunk ends: its own value, or y += yc in place
+            if (k > 0 && s - pos0 < 4) mbar_wait_idle<true>(smem_u32(xempty), (uint32_t)(k - 1) & 1u, p.status, dead);
+            const bool first = CS > 1 || s < 4;
+#pragma unroll
+            for (int e = 0; e < NB * 4; e++) {
+              float* o = place(CS > 1 ? (s >> 2) - ch0 : 0, nv, e / 4, e & 3);
+              o[0] = __fadd_rn(first ? 0.0f : o[0], yc[e].x);
+              o[kXPitch] = __fadd_rn(first ? 0.0f : o[kXPitch], yc[e].y);
+            }
+          }
+        }
+        send(ch0, nv);
+      }
     }
   }
 
@@ -547,63 +747,139 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
   }
+  cluster_sync();   // nobody leaves while another CTA may still reach its shared memory
 }
 
-size_t umma_smem_bytes() { return umma_smem_core_bytes() + 32 * 64 * sizeof(float); }
+// Q8_1 blocks [B][K/32][36] -> image
+__global__ void __launch_bounds__(256) tile_image_kernel(const uint32_t* x, int nblk, int B, uint8_t* img) {
+  bk_pdl_trigger();
+  bk_pdl_wait();
+  const int i = blockIdx.x * 256 + threadIdx.x, b = i % B, blk = i / B;
+  if (blk >= nblk) return;
+  const uint32_t* src = x + ((size_t)b * nblk + blk) * 9;
+  uint32_t w[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) w[k] = __ldg(src + k);
+  int qsum = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) qsum = bk_dp4a_ss(w[k], 0x01010101u, qsum);
+#pragma unroll
+  for (int c = 0; c < 4; c++) bk_tile_store_quants(img, B, b, blk, c, w[2 * c], w[2 * c + 1]);
+  const float d8 = bk_q8half_to_f32((uint16_t)(w[8] & 0xffffu));
+  bk_tile_store_factors(img, nblk * 32, B, b, blk, d8, __fmul_rn(d8, (float)qsum));
+}
 
-// uint8 matrix [n_rows][row_bytes], box = 32 rows x 144 bytes (one superblock column of 32 rows), no swizzle
-bool encode_weight_map(CUtensorMap* m, const uint8_t* W, int n_rows, size_t row_bytes) {
-  return bk_encode_map_2d(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, (uint64_t)(uintptr_t)W, row_bytes, (uint64_t)n_rows, row_bytes, 144, 32);
+// Matrix of Q4_K rows; header < 0: whole superblock columns (box 32 rows x 144 bytes), 1: their headers (x 16 bytes), 0: the quants
+// of `pairs` sub-block pairs (x 32 * pairs bytes, swizzled so that the expanders' 16-byte reads hit all banks).
+bool encode_weight_map(CUtensorMap* m, const uint8_t* W, int n_rows, size_t row_bytes, int header, int pairs) {
+  const uint32_t box = header < 0 ? 144 : header ? 16 : 32 * pairs;
+  const CUtensorMapSwizzle sw = header == 0 ? (pairs == 1 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B) : CU_TENSOR_MAP_SWIZZLE_NONE;
+  return bk_encode_map_2d(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, (uint64_t)(uintptr_t)W, row_bytes, (uint64_t)n_rows, row_bytes, box, 32, sw);
+}
+
+template <int NB, bool LANES>
+int32_t launch_tile(UmmaParams& P) {
+  using C = Cfg<NB, LANES>;
+  BkContext& c = bk_ctx();
+  GemvParams& g = P.g;
+  // tensor-map feed: 32-row boxes that never straddle two segments
+  bool ok = true;
+  for (int i = 0; i < g.n_segs; i++) ok = ok && g.segs[i].n_rows % 32 == 0;
+  const size_t row_bytes = (size_t)(g.K / 256) * 144;
+  for (int i = 0; ok && i < g.n_segs; i++) {
+    for (int up = 0; ok && up < (g.segs[i].epi == BK_EPI_SWIGLU ? 2 : 1); up++) {
+      const uint8_t* W = up ? g.segs[i].W2 : g.segs[i].W;
+      CUtensorMap* m = P.maps + (up ? 8 : 2 * i);
+      ok = C::PS == 4 ? encode_weight_map(m, W, g.segs[i].n_rows, row_bytes, -1, 4)
+                      : encode_weight_map(m, W, g.segs[i].n_rows, row_bytes, 1, 0) && encode_weight_map(m + 1, W, g.segs[i].n_rows, row_bytes, 0, C::PS);
+    }
+  }
+  BK_ARG(ok || !LANES, "tile GEMV: the lane order needs segments of whole 32-row boxes");
+  P.use_maps = ok ? 1 : 0;
+
+  auto kernel = gemv_q4k_umma_kernel<NB, LANES>;
+  static int clusters[4] = {0, 0, 0, 0};   // resident clusters of 1, 2, 4, 8 CTAs
+  const size_t limit = c.smem_optin - 1024;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kUT);
+  cfg.dynamicSmemBytes = limit;
+  cfg.stream = c.stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  if (!clusters[0]) {
+    BK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+    for (int i = 3; i >= 0; i--) {
+      attr[0].val.clusterDim.x = 1 << i;
+      cfg.gridDim = dim3((c.sm_count >> i) << i);
+      cfg.numAttrs = 1;
+      BK_CUDA(cudaOccupancyMaxActiveClusters(&clusters[i], kernel, &cfg));
+      if (clusters[i] < 1) return bk_fail(BK_ERR_UNSUPPORTED, "tile GEMV: a cluster of %d does not fit the device", 1 << i);
+    }
+  }
+  // How many CTAs share the classes (or chunks) of a tile: the fewest steps of the longest CTA, a tile's exchange and pipeline
+  // fill counted as one superblock.
+  const int tiles = (g.total_vrows + kTileM - 1) / kTileM, nsb = g.K / 256, n_chunks = (nsb + 3) / 4;
+  int best = 1, best_cost = 0x7fffffff;
+  for (int s = 1; s * (4 / C::PS) <= 8; s *= 2) {
+    const int cs = s * (4 / C::PS), n = clusters[__builtin_ctz(cs)];
+    const int rounds = (tiles + n - 1) / n, len = LANES ? (nsb + 7) / 8 * (8 / s) : 4 * ((n_chunks + s - 1) / s);
+    const size_t buf = LANES ? 0 : (size_t)((s > 1 ? n_chunks * (C::N / cs) : C::N) + (s > 1 ? (n_chunks + s - 1) / s * C::N : 0)) * kXPitch * 4;
+    if (buf + (size_t)C::kTabs * kTileM * 16 + 2 * C::kStage + 5 * C::kColBytes + 512 > limit) continue;   // (one CTA a tile always fits)
+    const int cost = rounds * (len + 1);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = s;
+    }
+  }
+  P.csplit = best;
+  const int cs = best * (4 / C::PS), n = clusters[__builtin_ctz(cs)];
+  P.levels = LANES && best <= 2 ? 2 - __builtin_ctz(best) : 0;
+  P.xbuf_bytes = (uint32_t)((LANES ? 64 : cs > 1 ? n_chunks * (C::N / cs) : C::N) * kXPitch * 4);
+  P.stg_bytes = cs == 1 ? 0 : (uint32_t)((LANES ? 64 : (n_chunks + best - 1) / best * C::N) * kXPitch * 4);
+  const size_t fixed = (size_t)C::kTabs * kTileM * 16 + 3 * C::kColBytes + P.xbuf_bytes + P.stg_bytes + (size_t)P.levels * 32768 + 512;
+  constexpr size_t per_stage = C::kStage + C::kColBytes;
+  BK_ARG(fixed + 2 * per_stage <= limit, "tile GEMV: K=%d does not fit in shared memory", g.K);
+  P.stages = (int)((limit - fixed) / per_stage);
+  if (P.stages > kMaxStages) P.stages = kMaxStages;
+  attr[0].val.clusterDim.x = cs;
+  cfg.gridDim = dim3((tiles < n ? tiles : n) * cs);
+  cfg.dynamicSmemBytes = fixed + (size_t)P.stages * per_stage;
+  cfg.numAttrs = 2;
+  BK_CUDA(cudaLaunchKernelEx(&cfg, kernel, P));
+  BK_CHECK_LAUNCH();
+  return BK_OK;
 }
 
 }  // namespace
 
-// Launch for at most 32 columns (the caller cuts wider batches into groups of 32).  p: a filled GemvParams.
-int32_t bk_gemv_umma_launch(void* params, int B) {
+// 16 to 64 columns (17 in the lane order); p: a filled GemvParams whose x is an image, or Q8_1 blocks (prologue BK_PRO_Q8).
+int32_t bk_gemv_umma_launch(void* params, int B, bool lanes) {
   BkContext& c = bk_ctx();
   UmmaParams P;
   P.g = *static_cast<GemvParams*>(params);
-  BK_ARG(B >= 1 && B <= 32, "tile GEMV: %d columns per launch (1..32)", B);
   P.B = B;
-  P.Npad = B <= 16 ? 16 : 32;
-  // tensor-map feed: whole rows in memory, 32-row boxes that never straddle two segments, and a SwiGLU segment alone
-  {
-    const GemvParams& g = P.g;
-    bool ok = g.row_stride == 0 && g.row_off == 0;
-    bool any_swiglu = false;
-    for (int i = 0; i < g.n_segs; i++) {
-      ok = ok && g.segs[i].n_rows % 32 == 0;
-      any_swiglu = any_swiglu || g.segs[i].epi == BK_EPI_SWIGLU;
+  if (P.g.prologue == BK_PRO_Q8) {
+    const size_t need = bk_tile_image_bytes(P.g.K, B);
+    if (c.tile_image_bytes < need) {
+      if (c.capturing) return bk_fail(BK_ERR_STATE, "bkGemvQ4K: the tile path's image buffer must be sized by an eager launch before a capture");
+      BK_CUDA(cudaStreamSynchronize(c.stream));
+      cudaFree(c.tile_image);
+      c.tile_image = nullptr;
+      c.tile_image_bytes = 0;
+      void* q = nullptr;
+      BK_CUDA(cudaMalloc(&q, need));
+      c.tile_image = static_cast<uint8_t*>(q);
+      c.tile_image_bytes = need;
     }
-    ok = ok && (!any_swiglu || g.n_segs == 1);
-    const size_t row_bytes = (size_t)(g.K / 256) * 144;
-    for (int i = 0; ok && i < g.n_segs; i++) {
-      ok = encode_weight_map(&P.maps[i], g.segs[i].W, g.segs[i].n_rows, row_bytes);
-      if (ok && g.segs[i].epi == BK_EPI_SWIGLU) ok = encode_weight_map(&P.maps[4], g.segs[i].W2, g.segs[i].n_rows, row_bytes);
-    }
-    P.use_maps = ok ? 1 : 0;
+    const int nblk = P.g.K / 32;
+    BK_CUDA(bk_launch_pdl(tile_image_kernel, dim3((nblk * B + 255) / 256), dim3(256), 0, static_cast<const uint32_t*>(P.g.x), nblk, B, c.tile_image));
+    BK_CHECK_LAUNCH();
+    P.g.x = c.tile_image;
   }
-  static bool configured = false;
-  const size_t smem = umma_smem_bytes();
-  if (!configured) {
-    BK_CUDA(cudaFuncSetAttribute(gemv_q4k_umma_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    BK_CUDA(cudaFuncSetAttribute(gemv_q4k_umma_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
-  }
-  const int tiles = (P.g.total_vrows + kTileM - 1) / kTileM;
-  int grid = tiles < c.sm_count ? tiles : c.sm_count;
-  // few tiles: cut each along K into parts of whole chunks (four superblocks), as many as there are SMs for
-  const int n_chunks = (P.g.K / 256 + 3) / 4;
-  P.ksplit = 1;
-  P.scratch = c.tile_scratch;
-  P.counters = c.tile_counters;
-  if (tiles * 2 <= c.sm_count && n_chunks >= 2 && tiles <= 256 &&
-      (size_t)tiles * n_chunks * 32 * kTileM * sizeof(float) <= c.tile_scratch_bytes) {
-    P.ksplit = c.sm_count / tiles < n_chunks ? c.sm_count / tiles : n_chunks;
-    if (P.ksplit > 1) grid = tiles * P.ksplit;
-  }
-  if (P.Npad == 16) BK_CUDA(bk_launch_pdl(gemv_q4k_umma_kernel<4>, dim3(grid), dim3(kUT), smem, P));
-  else BK_CUDA(bk_launch_pdl(gemv_q4k_umma_kernel<8>, dim3(grid), dim3(kUT), smem, P));
-  BK_CHECK_LAUNCH();
-  return BK_OK;
+  if (lanes) return B <= 32 ? launch_tile<2, true>(P) : launch_tile<4, true>(P);   // (17 columns and more)
+  return B <= 16 ? launch_tile<1, false>(P) : B <= 32 ? launch_tile<2, false>(P) : launch_tile<4, false>(P);
 }

@@ -28,9 +28,8 @@ struct BkContext {
   int step_trace_phases = 0;          // phases the buffer can hold (8 slots each)
   int spin_limit = 0;                 // polls a bounded device-side wait may take (bkSetSpinLimit; 0 = built-in limits)
   int* d_status = nullptr;           // device word set by kernels whose bounded waits gave up
-  float* tile_scratch = nullptr;     // dense tile GEMV cut along K: per-chunk partial sums [tile][chunk][32 columns][128 rows]
-  int* tile_counters = nullptr;      // ... and one arrival counter per tile (self-resetting)
-  size_t tile_scratch_bytes = 0;
+  uint8_t* tile_image = nullptr;     // activation image of the dense tile GEMV when its caller has Q8_1 blocks
+  size_t tile_image_bytes = 0;
   float* gemv_carry = nullptr;       // class accumulators handed from one K part of a split GEMV to the next
   size_t gemv_carry_bytes = 0;
   char err[512] = {0};
@@ -103,16 +102,22 @@ struct BkReduce {
   int spin_limit;              // polls before the bounded wait gives up (0 = default)
 };
 
-// tensor map of a matrix [n_rows][cols] with rows `stride` bytes apart, box box_rows x box_cols, no swizzle; false when the
+// tensor map of a matrix [n_rows][cols] with rows `stride` bytes apart, box box_rows x box_cols; false when the
 // encoder is missing or refuses
 bool bk_encode_map_2d(CUtensorMap* m, CUtensorMapDataType type, uint64_t base, uint64_t cols, uint64_t n_rows, uint64_t stride, uint32_t box_cols,
-                      uint32_t box_rows);
+                      uint32_t box_rows, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_NONE);
+
+// internal: the activation image of the dense tile GEMV (bk_common.cuh) as an output layout and as a GEMV input
+#define BK_Q8_TILE 2
+#define BK_PRO_TILE 5
 
 // internal launchers shared between translation units
 bool bk_gemv_mma_fits(int K, int B);   // whether the batch-3..8 tensor-core GEMV can hold this K (else column pairs)
+bool bk_gemv_dense_lanes(int B);           // whether B columns are enough for the dense tile kernel in the lane order
 bool bk_gemv_auto_tile(int rows, int K);   // whether BK_GEMV_ORDER_AUTO sends a launch of these shapes (>= 16 columns) to the dense tile path
 int32_t bk_gemv_launch(const bkGemvArgs& a);
-// decode attention; n_seq > 0: the B entries are prompt columns of n_seq sequences (append launch + attention launch)
+int32_t bk_gdn_launch(const bkGdnArgs& a);   // bkGdnStep, also with out_q8_layout BK_Q8_TILE
+// decode attention (out_q8_layout BK_Q8_TILE too); n_seq > 0: the B entries are prompt columns of n_seq sequences (append launch + attention launch)
 int32_t bk_attn_launch(const bkAttnArgs& a, int n_seq, int layout_B);
 // same with the fused exchange: push (may be null) for BK_EPI_PUSH_F32 segments, reduce (may be null) for
 // BK_PRO_REDUCE_RMSNORM; ctas_out (may be null) receives the number of CTAs that will signal arrival

@@ -16,6 +16,7 @@
 
 #include <string>
 #include <unordered_map>
+#include <algorithm>
 #include <vector>
 
 #include "bk_common.cuh"
@@ -146,13 +147,13 @@ struct ProfScope {
 
 
 // arguments of the attention launch of layer L for the decode step (one token per sequence)
-bkAttnArgs step_attn_args(Model& m, LayerW& L, bool q8_handoff, bool o_staged) {
+bkAttnArgs step_attn_args(Model& m, LayerW& L, bool q8_handoff, int o_layout) {
   const bkModelConfig& c = m.cfg;
   bkAttnArgs aa;
   memset(&aa, 0, sizeof(aa));
   aa.qg = m.qg; aa.k = m.kbuf; aa.v = m.vbuf; aa.q_norm_w = L.q_norm; aa.k_norm_w = L.k_norm;
   aa.cos_t = m.cos_t; aa.sin_t = m.sin_t; aa.k_cache = L.kc; aa.v_cache = L.vc; aa.pos = m.pos;
-  aa.out = m.attn_out; aa.out_q8 = q8_handoff ? m.attn_q8 : 0; aa.out_q8_layout = o_staged ? BK_Q8_STAGED : BK_Q8_BLOCKS;
+  aa.out = m.attn_out; aa.out_q8 = q8_handoff ? m.attn_q8 : 0; aa.out_q8_layout = o_layout;
   aa.scratch = m.attn_scratch;
   aa.B = m.B; aa.Hq = m.Hq; aa.Hkv = m.Hkv; aa.HD = c.head_dim; aa.rot_half = c.rot_dim / 2; aa.max_len = c.max_len;
   aa.split_len = m.split_len; aa.max_pos = c.max_len - 1; aa.scale = 1.0f / sqrtf((float)c.head_dim);
@@ -222,6 +223,12 @@ int32_t enqueue_step(Model& m, int parity, bool host_tokens = false) {
   auto staged_ok = [&](int K, int rows) {
     return !(tile_path && bk_gemv_auto_tile(rows, K)) && bk_gemv_mma_fits(K, B < 8 ? B : 8) && !(B > 8 && B % 8 == 1);
   };
+  // A projection that goes to the dense tile kernel (bk_gemv_launch_tp has the rule) reads that kernel's image.
+  auto layout_for = [&](int K, int rows, int row_gcd) {
+    if (tile_path && (bk_gemv_auto_tile(rows, K) || (row_gcd % 32 == 0 && bk_gemv_dense_lanes(B)))) return BK_Q8_TILE;
+    return staged_ok(K, rows) ? BK_Q8_STAGED : BK_Q8_BLOCKS;
+  };
+  auto prologue_of = [](int layout) { return layout == BK_Q8_TILE ? BK_PRO_TILE : layout == BK_Q8_STAGED ? BK_PRO_STAGED : BK_PRO_Q8; };
   // Input of a projection: fused RMSNorm/quantise prologue at batch 1; at batch >= 2 one small launch
   // normalises and quantises the rows once and every CTA of the projection just copies the blocks.
   // Tensor parallel: a row-parallel GEMV pushes its partial sums to every rank (BK_EPI_PUSH_F32); the sum over ranks,
@@ -230,7 +237,8 @@ int32_t enqueue_step(Model& m, int parity, bool host_tokens = false) {
   unsigned int n_exchanges = 0;   // fused exchanges enqueued so far in this step
   BkReduce red_desc;
   bool use_red = false;   // the GEMV being set up carries the reduce prologue (batch 1)
-  auto set_input = [&](bkGemvArgs& g, uint64_t x, int K, uint64_t norm_w, int rows) -> int32_t {
+  // row_gcd: a number that divides every segment's row count
+  auto set_input = [&](bkGemvArgs& g, uint64_t x, int K, uint64_t norm_w, int rows, int row_gcd) -> int32_t {
     g.K = K; g.B = B; g.eps = c.eps; g.order = gemv_order;
     use_red = false;
     const bool reduce = pending.on && norm_w && x == pending.out;
@@ -242,10 +250,9 @@ int32_t enqueue_step(Model& m, int parity, bool host_tokens = false) {
       pending.on = false;
     }
     if (q8_handoff) {
-      const bool staged = staged_ok(K, rows);   // else the GEMV is cut along K (or runs as column pairs) reading plain blocks
-      PROF(PC_QUANT, bk_quant_rows_launch(x, norm_w, K, B, c.eps, m.xq, staged ? BK_Q8_STAGED : BK_Q8_BLOCKS,
-                                          reduce ? &red_desc : nullptr));
-      g.prologue = staged ? BK_PRO_STAGED : BK_PRO_Q8; g.x = m.xq;
+      const int layout = layout_for(K, rows, row_gcd);   // (plain blocks: the GEMV is cut along K or runs as column pairs)
+      PROF(PC_QUANT, bk_quant_rows_launch(x, norm_w, K, B, c.eps, m.xq, layout, reduce ? &red_desc : nullptr));
+      g.prologue = prologue_of(layout); g.x = m.xq;
     } else {
       g.prologue = reduce ? BK_PRO_REDUCE_RMSNORM : norm_w ? BK_PRO_RMSNORM : BK_PRO_BF16; g.x = x; g.norm_w = norm_w;
       use_red = reduce;
@@ -274,7 +281,7 @@ int32_t enqueue_step(Model& m, int parity, bool host_tokens = false) {
     bkGemvArgs g;
     if (!L.full) {
       memset(&g, 0, sizeof(g));
-      TRY(set_input(g, m.x[cur], H, L.in_ln, m.Cw + m.ZD + 2 * m.Hv));
+      TRY(set_input(g, m.x[cur], H, L.in_ln, m.Cw + m.ZD + 2 * m.Hv, m.Hv));   // Cw and ZD are multiples of 128
       g.n_segs = 4;
       g.segs[0] = bkGemvSeg{L.qkv, 0, m.qkv, 0, m.Cw, BK_EPI_BF16, m.Cw, 0};
       g.segs[1] = bkGemvSeg{L.z, 0, m.z, 0, m.ZD, BK_EPI_BF16, m.ZD, 0};
@@ -287,14 +294,14 @@ int32_t enqueue_step(Model& m, int parity, bool host_tokens = false) {
       ga.conv_w = L.conv_w; ga.conv_state_in = L.conv_state[parity]; ga.conv_state_new = L.conv_state[parity ^ 1];
       ga.A_log = L.A_log; ga.dt_bias = L.dt_bias; ga.norm_w = L.gnorm;
       ga.S_in = L.S; ga.S_new = L.S;  // in place: each thread rewrites exactly the rows it read
-      const bool zd_staged = q8_handoff && staged_ok(m.ZD, H);
-      ga.out = m.attn_out; ga.out_q8 = q8_handoff ? m.attn_q8 : 0; ga.out_q8_layout = zd_staged ? BK_Q8_STAGED : BK_Q8_BLOCKS;
+      const int zd_layout = q8_handoff ? layout_for(m.ZD, H, H) : BK_Q8_BLOCKS;
+      ga.out = m.attn_out; ga.out_q8 = q8_handoff ? m.attn_q8 : 0; ga.out_q8_layout = zd_layout;
       ga.B = B; ga.Hk = m.Hk; ga.Hv = m.Hv; ga.apply_conv = 1;
       ga.state_is_settled = 1;  // this layer's state was last written one whole step ago
-      PROF(PC_GDN, bkGdnStep(&ga));
+      PROF(PC_GDN, bk_gdn_launch(ga));
       memset(&g, 0, sizeof(g));
       g.K = m.ZD; g.B = B; g.n_segs = 1; g.order = gemv_order;
-      g.prologue = zd_staged ? BK_PRO_STAGED : q8_handoff ? BK_PRO_Q8 : BK_PRO_BF16; g.x = q8_handoff ? m.attn_q8 : m.attn_out;
+      g.prologue = q8_handoff ? prologue_of(zd_layout) : BK_PRO_BF16; g.x = q8_handoff ? m.attn_q8 : m.attn_out;
       if (m.tp == 1) {
         g.segs[0] = bkGemvSeg{L.out_proj, 0, m.h1, m.x[cur], H, BK_EPI_ADD_BF16, H, 0};
         PROF(PC_GEMV_OUT, launch(g));
@@ -303,18 +310,18 @@ int32_t enqueue_step(Model& m, int parity, bool host_tokens = false) {
       }
     } else {
       memset(&g, 0, sizeof(g));
-      TRY(set_input(g, m.x[cur], H, L.in_ln, m.QG + 2 * m.KVD));
+      TRY(set_input(g, m.x[cur], H, L.in_ln, m.QG + 2 * m.KVD, 32));
       g.n_segs = 3;
       g.segs[0] = bkGemvSeg{L.q, 0, m.qg, 0, m.QG, BK_EPI_BF16, m.QG, 0};
       g.segs[1] = bkGemvSeg{L.k, 0, m.kbuf, 0, m.KVD, BK_EPI_BF16, m.KVD, 0};
       g.segs[2] = bkGemvSeg{L.v, 0, m.vbuf, 0, m.KVD, BK_EPI_BF16, m.KVD, 0};
       PROF(PC_GEMV_PROJ, launch(g));
-      const bool o_staged = q8_handoff && staged_ok(m.Hq * c.head_dim, H);
-      bkAttnArgs aa = step_attn_args(m, L, q8_handoff, o_staged);
-      PROF(PC_ATTN, bkAttnDecode(&aa));
+      const int o_layout = q8_handoff ? layout_for(m.Hq * c.head_dim, H, H) : BK_Q8_BLOCKS;
+      bkAttnArgs aa = step_attn_args(m, L, q8_handoff, o_layout);
+      PROF(PC_ATTN, bk_attn_launch(aa, 0, 0));
       memset(&g, 0, sizeof(g));
       g.K = m.Hq * c.head_dim; g.B = B; g.n_segs = 1; g.order = gemv_order;
-      g.prologue = o_staged ? BK_PRO_STAGED : q8_handoff ? BK_PRO_Q8 : BK_PRO_BF16; g.x = q8_handoff ? m.attn_q8 : m.attn_out;
+      g.prologue = q8_handoff ? prologue_of(o_layout) : BK_PRO_BF16; g.x = q8_handoff ? m.attn_q8 : m.attn_out;
       if (m.tp == 1) {
         g.segs[0] = bkGemvSeg{L.o, 0, m.h1, m.x[cur], H, BK_EPI_ADD_BF16, H, 0};
         PROF(PC_GEMV_OUT, launch(g));
@@ -323,12 +330,12 @@ int32_t enqueue_step(Model& m, int parity, bool host_tokens = false) {
       }
     }
     memset(&g, 0, sizeof(g));
-    TRY(set_input(g, m.h1, H, L.post_ln, 2 * m.inter));
+    TRY(set_input(g, m.h1, H, L.post_ln, 2 * m.inter, m.inter));
     g.n_segs = 1;
     g.segs[0] = bkGemvSeg{L.gate, L.up, m.act, 0, m.inter, BK_EPI_SWIGLU, m.inter, 0};
     PROF(PC_GEMV_GATEUP, launch(g));
     memset(&g, 0, sizeof(g));
-    TRY(set_input(g, m.act, m.inter, 0, H));
+    TRY(set_input(g, m.act, m.inter, 0, H, H));
     g.n_segs = 1;
     if (m.tp == 1) {
       g.segs[0] = bkGemvSeg{L.down, 0, m.x[cur ^ 1], m.h1, H, BK_EPI_ADD_BF16, H, 0};
@@ -340,7 +347,7 @@ int32_t enqueue_step(Model& m, int parity, bool host_tokens = false) {
   }
   bkGemvArgs g;
   memset(&g, 0, sizeof(g));
-  TRY(set_input(g, m.x[cur], H, m.final_norm, m.vocab_local));
+  TRY(set_input(g, m.x[cur], H, m.final_norm, m.vocab_local, m.vocab_local));
   g.n_segs = 1;
   g.segs[0] = bkGemvSeg{m.embed + (uint64_t)m.vocab_offset * (H / 256) * 144, 0, m.logits, 0, m.vocab_local, BK_EPI_F32,
                         m.vocab_local, 0};
@@ -387,7 +394,7 @@ int32_t alloc_prefill(Model& m, int cols) {
   if (m.ZD > kmax) kmax = m.ZD;
   if (attn_w > kmax) kmax = attn_w;
   const size_t blocks = C * kmax / 32 * 36, staged = bk_staged_total_bytes(kmax, cols);
-  TRY(dev_alloc(m, blocks > staged ? blocks : staged, &f.xq));
+  TRY(dev_alloc(m, std::max(std::max(blocks, staged), bk_tile_image_bytes(kmax, cols)), &f.xq));
   TRY(dev_alloc(m, C * 4, &f.ids));
   TRY(dev_alloc(m, C * 4, &f.pos));
   TRY(dev_alloc(m, bkAttnScratchBytes(cols, m.Hq, c.head_dim, c.max_len, m.split_len), &f.attn_scratch));
@@ -404,17 +411,28 @@ int32_t enqueue_prefill(Model& m, int T) {
   const int B = m.B, H = c.hidden, C = T * B;
   Model::Prefill& f = m.pf;
   auto staged_ok = [&](int K, int cols) { return cols >= 2 && bk_gemv_mma_fits(K, cols < 8 ? cols : 8) && !(cols > 8 && cols % 8 == 1); };
+  // many columns: the dense tile kernel, in the lane order, where the row counts are whole boxes of 32
+  auto layout_for = [&](int K, int cols, int row_gcd) {
+    if (bk_gemv_dense_lanes(cols) && row_gcd % 32 == 0) return BK_Q8_TILE;
+    return staged_ok(K, cols) ? BK_Q8_STAGED : BK_Q8_BLOCKS;
+  };
+  auto point_at = [&](bkGemvArgs& g, int K, int cols, int layout) {
+    g.K = K; g.B = cols; g.eps = c.eps;
+    g.order = BK_GEMV_ORDER_LANES;   // every column must get the bits of a single decode step
+    g.prologue = layout == BK_Q8_TILE ? BK_PRO_TILE : layout == BK_Q8_STAGED ? BK_PRO_STAGED : BK_PRO_Q8; g.x = f.xq;
+  };
   // quantise `cols` rows once (optionally RMSNorm first) and point the GEMV at the result
-  auto set_input = [&](bkGemvArgs& g, uint64_t x, int K, uint64_t norm_w, int cols) -> int32_t {
+  // row_gcd: a number that divides every segment's row count
+  auto set_input = [&](bkGemvArgs& g, uint64_t x, int K, uint64_t norm_w, int cols, int row_gcd) -> int32_t {
     g.K = K; g.B = cols; g.eps = c.eps;
     g.order = BK_GEMV_ORDER_LANES;   // every column must get the bits of a single decode step
     if (cols == 1) {
       g.prologue = norm_w ? BK_PRO_RMSNORM : BK_PRO_BF16; g.x = x; g.norm_w = norm_w;
       return BK_OK;
     }
-    const bool staged = staged_ok(K, cols);
-    TRY(bk_quant_rows_launch(x, norm_w, K, cols, c.eps, f.xq, staged ? BK_Q8_STAGED : BK_Q8_BLOCKS, nullptr));
-    g.prologue = staged ? BK_PRO_STAGED : BK_PRO_Q8; g.x = f.xq;
+    const int layout = layout_for(K, cols, row_gcd);
+    TRY(bk_quant_rows_launch(x, norm_w, K, cols, c.eps, f.xq, layout, nullptr));
+    point_at(g, K, cols, layout);
     return BK_OK;
   };
   prefill_positions_kernel<<<(C + 127) / 128, 128, 0, bk_ctx().stream>>>(bk_ptr<int32_t>(m.pos), bk_ptr<int32_t>(f.pos), T, B);
@@ -425,7 +443,7 @@ int32_t enqueue_prefill(Model& m, int T) {
     LayerW& L = m.layers[li];
     bkGemvArgs g;
     memset(&g, 0, sizeof(g));
-    TRY(set_input(g, f.x[cur], H, L.in_ln, C));
+    TRY(set_input(g, f.x[cur], H, L.in_ln, C, L.full ? 32 : m.Hv));   // (the other row counts are multiples of 128)
     if (!L.full) {
       g.n_segs = 4;
       g.segs[0] = bkGemvSeg{L.qkv, 0, f.qkv, 0, m.Cw, BK_EPI_BF16, m.Cw, 0};
@@ -441,12 +459,15 @@ int32_t enqueue_prefill(Model& m, int T) {
         ga.conv_w = L.conv_w; ga.conv_state_in = L.conv_state[parity]; ga.conv_state_new = L.conv_state[parity ^ 1];
         ga.A_log = L.A_log; ga.dt_bias = L.dt_bias; ga.norm_w = L.gnorm;
         ga.S_in = L.S; ga.S_new = L.S;
-        ga.out = f.attn_out; ga.B = B; ga.Hk = m.Hk; ga.Hv = m.Hv; ga.apply_conv = 1; ga.n_tokens = T;
+        const int layout = layout_for(m.ZD, C, H);
+        ga.out = f.attn_out; ga.out_q8 = C > 1 ? f.xq : 0; ga.out_q8_layout = C > 1 ? layout : BK_Q8_BLOCKS;
+        ga.B = B; ga.Hk = m.Hk; ga.Hv = m.Hv; ga.apply_conv = 1; ga.n_tokens = T;
         ga.state_is_settled = 1;   // written by the previous pass, many launches ago
-        TRY(bkGdnStep(&ga));
+        TRY(bk_gdn_launch(ga));
       }
       memset(&g, 0, sizeof(g));
-      TRY(set_input(g, f.attn_out, m.ZD, 0, C));
+      if (C > 1) point_at(g, m.ZD, C, layout_for(m.ZD, C, H));   // quantised by the launch before
+      else TRY(set_input(g, f.attn_out, m.ZD, 0, C, H));
       g.n_segs = 1;
       g.segs[0] = bkGemvSeg{L.out_proj, 0, f.h1, f.x[cur], H, BK_EPI_ADD_BF16, H, 0};
       TRY(bk_gemv_launch(g));
@@ -466,24 +487,29 @@ int32_t enqueue_prefill(Model& m, int T) {
         aa.q_norm_w = L.q_norm; aa.k_norm_w = L.k_norm;
         aa.cos_t = m.cos_t; aa.sin_t = m.sin_t; aa.k_cache = L.kc; aa.v_cache = L.vc; aa.pos = f.pos;
         aa.out = f.attn_out; aa.scratch = f.attn_scratch;
+        if (C > 1) {
+          aa.out_q8 = f.xq;
+          aa.out_q8_layout = layout_for(attn_w, C, H);
+        }
         aa.B = C; aa.Hq = m.Hq; aa.Hkv = m.Hkv; aa.HD = c.head_dim; aa.rot_half = c.rot_dim / 2; aa.max_len = c.max_len;
         aa.split_len = m.split_len; aa.max_pos = c.max_len - 1; aa.scale = 1.0f / sqrtf((float)c.head_dim);
         aa.fused_norm_rope = 1;
         TRY(bk_attn_launch(aa, B, m.pf.cols));
       }
       memset(&g, 0, sizeof(g));
-      TRY(set_input(g, f.attn_out, attn_w, 0, C));
+      if (C > 1) point_at(g, attn_w, C, layout_for(attn_w, C, H));
+      else TRY(set_input(g, f.attn_out, attn_w, 0, C, H));
       g.n_segs = 1;
       g.segs[0] = bkGemvSeg{L.o, 0, f.h1, f.x[cur], H, BK_EPI_ADD_BF16, H, 0};
       TRY(bk_gemv_launch(g));
     }
     memset(&g, 0, sizeof(g));
-    TRY(set_input(g, f.h1, H, L.post_ln, C));
+    TRY(set_input(g, f.h1, H, L.post_ln, C, m.inter));
     g.n_segs = 1;
     g.segs[0] = bkGemvSeg{L.gate, L.up, f.act, 0, m.inter, BK_EPI_SWIGLU, m.inter, 0};
     TRY(bk_gemv_launch(g));
     memset(&g, 0, sizeof(g));
-    TRY(set_input(g, f.act, m.inter, 0, C));
+    TRY(set_input(g, f.act, m.inter, 0, C, H));
     g.n_segs = 1;
     g.segs[0] = bkGemvSeg{L.down, 0, f.x[cur ^ 1], f.h1, H, BK_EPI_ADD_BF16, H, 0};
     TRY(bk_gemv_launch(g));
@@ -492,7 +518,7 @@ int32_t enqueue_prefill(Model& m, int T) {
   // logits and argmax of the last token only
   bkGemvArgs g;
   memset(&g, 0, sizeof(g));
-  TRY(set_input(g, f.x[cur] + (uint64_t)(C - B) * H * 2, H, m.final_norm, B));
+  TRY(set_input(g, f.x[cur] + (uint64_t)(C - B) * H * 2, H, m.final_norm, B, m.vocab_local));
   g.n_segs = 1;
   g.segs[0] = bkGemvSeg{m.embed, 0, m.logits, 0, m.vocab_local, BK_EPI_F32, m.vocab_local, 0};
   TRY(bk_gemv_launch(g));
@@ -693,8 +719,9 @@ int32_t bkModelFinalize(uint64_t model) {
     const int ka = m.ZD > attn_w ? m.ZD : attn_w, kx = m.inter > H ? m.inter : H;
     const size_t ba = (size_t)B * ka / 32 * 36, bx = (size_t)B * kx / 32 * 36;
     const size_t sa = bk_staged_total_bytes(ka, B), sx = bk_staged_total_bytes(kx, B);
-    TRY(dev_alloc(m, ba > sa ? ba : sa, &m.attn_q8));
-    TRY(dev_alloc(m, bx > sx ? bx : sx, &m.xq));
+    const size_t ta = bk_tile_image_bytes(ka, B), tx = bk_tile_image_bytes(kx, B);
+    TRY(dev_alloc(m, std::max(std::max(ba, sa), ta), &m.attn_q8));
+    TRY(dev_alloc(m, std::max(std::max(bx, sx), tx), &m.xq));
   }
   TRY(dev_alloc(m, (size_t)B * m.QG * 2, &m.qg));
   TRY(dev_alloc(m, (size_t)B * m.KVD * 2, &m.kbuf));

@@ -72,9 +72,9 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const uint16_t* x, const u
 // At batch >= 2 the projection kernels read their activation as ready Q8_1 blocks instead of each of the
 // 148 CTAs normalising and quantising all batch rows again.  NORM: one CTA per batch row (the canonical
 // 256-thread sum of squares).  Plain: 256 chunks of 8 values per CTA.  Output blocks [B][K/32][36].
-// STAGED: the output is the staged image of the tensor-core GEMV instead of 36-byte blocks.
+// LAYOUT: 36-byte blocks, the staged image of the batch 2..8 GEMV or the image of the dense tile GEMV.
 // rd.n > 0 (NORM only): row b is not read from x but formed from the tensor-parallel partial sums + residual.
-template <bool NORM, bool STAGED>
+template <bool NORM, int LAYOUT>
 __global__ void __launch_bounds__(256) quant_rows_kernel(const uint16_t* x, const uint16_t* w, int K, float eps,
                                                          uint8_t* out, const BkReduce rd, int* status) {
   bk_pdl_trigger();
@@ -125,7 +125,8 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const uint16_t* x, cons
 #pragma unroll
       for (int e = 0; e < 8; e++)
         y[e] = bk_bf16_to_f32(bk_f32_to_bf16(__fmul_rn(__fmul_rn(v[e], rstd), __fadd_rn(1.0f, wv[e]))));
-      if (STAGED) bk_staged_store<8>(out, K, gridDim.y, b, q >> 2, y, (q & 3) * 8);
+      if (LAYOUT == BK_Q8_STAGED) bk_staged_store<8>(out, K, gridDim.y, b, q >> 2, y, (q & 3) * 8);
+      else if (LAYOUT == BK_Q8_TILE) bk_tile_store<8>(out, K, gridDim.y, b, q >> 2, y, (q & 3) * 8);
       else bk_q8_1_store<8>(orow + (size_t)(q >> 2) * 36, y, (q & 3) * 8);
     }
   } else {
@@ -134,7 +135,8 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const uint16_t* x, cons
     if (q < nchunk) {
       float y[8];
       load8_bf16(row + (size_t)q * 8, y);
-      if (STAGED) bk_staged_store<8>(out, K, gridDim.y, b, q >> 2, y, (q & 3) * 8);
+      if (LAYOUT == BK_Q8_STAGED) bk_staged_store<8>(out, K, gridDim.y, b, q >> 2, y, (q & 3) * 8);
+      else if (LAYOUT == BK_Q8_TILE) bk_tile_store<8>(out, K, gridDim.y, b, q >> 2, y, (q & 3) * 8);
       else bk_q8_1_store<8>(orow + (size_t)(q >> 2) * 36, y, (q & 3) * 8);
     }
   }
@@ -343,9 +345,8 @@ int32_t bk_quant_rows_launch(uint64_t x, uint64_t w, int32_t K, int32_t B, float
                              const BkReduce* reduce) {
   BK_ARG(K > 0 && K % 256 == 0 && B > 0, "bkRmsNormQuantQ8_1: bad shape K=%d B=%d (K a multiple of 256)", K, B);
   BK_ARG((x || reduce) && out && ((x | w) & 15) == 0 && (out & 3) == 0, "bkRmsNormQuantQ8_1: null or misaligned pointer");
-  BK_ARG(layout == BK_Q8_BLOCKS || layout == BK_Q8_STAGED, "bkRmsNormQuantQ8_1: unknown layout %d", layout);
   BK_ARG(!reduce || w, "bkRmsNormQuantQ8_1: the reduce input exists with the norm only");
-  if (layout == BK_Q8_STAGED) BK_ARG((out & 15) == 0, "bkRmsNormQuantQ8_1: a staged image is 16-byte aligned");
+  if (layout != BK_Q8_BLOCKS) BK_ARG((out & 15) == 0, "bkRmsNormQuantQ8_1: a staged image is 16-byte aligned");
   const dim3 grid = w ? dim3(1, B) : dim3((K / 8 + 255) / 256, B);
   auto* px = bk_ptr<uint16_t>(x);
   auto* pw = bk_ptr<uint16_t>(w);
@@ -355,13 +356,9 @@ int32_t bk_quant_rows_launch(uint64_t x, uint64_t w, int32_t K, int32_t B, float
   if (reduce) red = *reduce;
   red.spin_limit = bk_ctx().spin_limit;
   int* st = bk_ctx().d_status;
-  if (w) {
-    if (layout == BK_Q8_STAGED) BK_CUDA(bk_launch_pdl(quant_rows_kernel<true, true>, grid, dim3(256), 0, px, pw, K, eps, po, red, st));
-    else BK_CUDA(bk_launch_pdl(quant_rows_kernel<true, false>, grid, dim3(256), 0, px, pw, K, eps, po, red, st));
-  } else {
-    if (layout == BK_Q8_STAGED) BK_CUDA(bk_launch_pdl(quant_rows_kernel<false, true>, grid, dim3(256), 0, px, pw, K, eps, po, red, st));
-    else BK_CUDA(bk_launch_pdl(quant_rows_kernel<false, false>, grid, dim3(256), 0, px, pw, K, eps, po, red, st));
-  }
+  auto kernel = w ? (layout == BK_Q8_TILE ? quant_rows_kernel<true, BK_Q8_TILE> : layout == BK_Q8_STAGED ? quant_rows_kernel<true, BK_Q8_STAGED> : quant_rows_kernel<true, BK_Q8_BLOCKS>)
+                  : (layout == BK_Q8_TILE ? quant_rows_kernel<false, BK_Q8_TILE> : layout == BK_Q8_STAGED ? quant_rows_kernel<false, BK_Q8_STAGED> : quant_rows_kernel<false, BK_Q8_BLOCKS>);
+  BK_CUDA(bk_launch_pdl(kernel, grid, dim3(256), 0, px, pw, K, eps, po, red, st));
   BK_CHECK_LAUNCH();
   return BK_OK;
 }
@@ -370,6 +367,7 @@ extern "C" {
 int32_t bkRmsNormQuantQ8_1(uint64_t x, uint64_t w, int32_t K, int32_t B, float eps, uint64_t out, int32_t layout) {
   BK_REQUIRE_INIT();
   BK_ARG(x != 0, "bkRmsNormQuantQ8_1: x is null");
+  BK_ARG(layout == BK_Q8_BLOCKS || layout == BK_Q8_STAGED, "bkRmsNormQuantQ8_1: unknown layout %d", layout);
   return bk_quant_rows_launch(x, w, K, B, eps, out, layout, nullptr);
 }
 
@@ -379,6 +377,7 @@ int32_t bkReduceRmsNormQuantQ8_1(uint64_t words, int32_t n_ranks, uint64_t strid
   BK_REQUIRE_INIT();
   BK_ARG(words && epoch && residual && sum_out && w && n_ranks >= 1 && n_ranks <= 8 && (words & 15) == 0 && stride_words % 2 == 0,
          "bkReduceRmsNormQuantQ8_1: bad arguments");
+  BK_ARG(layout == BK_Q8_BLOCKS || layout == BK_Q8_STAGED, "bkRmsNormQuantQ8_1: unknown layout %d", layout);
   BkReduce rd;
   memset(&rd, 0, sizeof(rd));
   rd.src = bk_ptr<uint2>(words);
@@ -419,49 +418,8 @@ int32_t bkConv1dStep(uint64_t x, uint64_t state_in, uint64_t w, int32_t C, int32
 int32_t bkGdnStep(const bkGdnArgs* args) {
   BK_REQUIRE_INIT();
   BK_ARG(args != nullptr, "bkGdnStep: args is null");
-  bkGdnArgs a = *args;
-  BK_ARG(a.B > 0 && a.Hk > 0 && a.Hv > 0 && a.Hv % a.Hk == 0, "bkGdnStep: bad head counts B=%d Hk=%d Hv=%d", a.B, a.Hk,
-         a.Hv);
-  BK_ARG(a.qkv && a.z && a.a && a.b && a.A_log && a.dt_bias && a.norm_w && a.S_in && a.S_new && a.out,
-         "bkGdnStep: null pointer among required arguments");
-  if (a.apply_conv) {
-    BK_ARG(a.conv_w && a.conv_state_in && a.conv_state_new && (a.conv_w & 7) == 0,
-           "bkGdnStep: conv weights/state missing or misaligned");
-    BK_ARG(a.conv_state_in != a.conv_state_new, "bkGdnStep: conv state buffers must be distinct");
-  }
-  GdnParams p;
-  p.qkv = bk_ptr<uint16_t>(a.qkv);
-  p.z = bk_ptr<uint16_t>(a.z);
-  p.a = bk_ptr<float>(a.a);
-  p.b = bk_ptr<float>(a.b);
-  p.conv_w = bk_ptr<uint16_t>(a.conv_w);
-  p.cs_in = bk_ptr<uint16_t>(a.conv_state_in);
-  p.cs_new = bk_ptr<uint16_t>(a.conv_state_new);
-  p.A_log = bk_ptr<float>(a.A_log);
-  p.dt_bias = bk_ptr<uint16_t>(a.dt_bias);
-  p.norm_w = bk_ptr<float>(a.norm_w);
-  p.S_in = bk_ptr<float>(a.S_in);
-  p.S_new = bk_ptr<float>(a.S_new);
-  p.out = bk_ptr<uint16_t>(a.out);
-  p.o_raw = bk_ptr<float>(a.o_raw);
-  p.conv_out = bk_ptr<uint16_t>(a.conv_out);
-  p.out_q8 = bk_ptr<uint8_t>(a.out_q8);
-  p.out_q8_staged = a.out_q8_layout == BK_Q8_STAGED;
-  BK_ARG(a.out_q8_layout == BK_Q8_BLOCKS || (a.out_q8_layout == BK_Q8_STAGED && (a.Hv * 128) % 256 == 0),
-         "bkGdnStep: out_q8_layout %d (a staged image needs Hv*128 a multiple of 256)", a.out_q8_layout);
-  p.B = a.B;
-  p.Hk = a.Hk;
-  p.Hv = a.Hv;
-  p.apply_conv = a.apply_conv;
-  p.early = a.state_is_settled;
-  p.T = a.n_tokens > 1 ? a.n_tokens : 1;
-  BK_ARG(a.n_tokens >= 0 && (p.out_q8_staged == 0 || (size_t)a.B * p.T <= 64), "bkGdnStep: n_tokens=%d", a.n_tokens);
-  p.trace = bk_trace_slot();
-  if (p.T > 1) BK_CUDA(bk_launch_pdl(gdn_step_kernel_multi, dim3(a.Hv, a.B), dim3(576), 0, p));
-  else if (a.Hv * a.B > bk_ctx().sm_count) BK_CUDA(bk_launch_pdl(gdn_step_kernel_x2, dim3(a.Hv, a.B), dim3(512), 0, p));
-  else BK_CUDA(bk_launch_pdl(gdn_step_kernel, dim3(a.Hv, a.B), dim3(576), 0, p));
-  BK_CHECK_LAUNCH();
-  return BK_OK;
+  BK_ARG(args->out_q8_layout == BK_Q8_BLOCKS || args->out_q8_layout == BK_Q8_STAGED, "bkGdnStep: out_q8_layout %d", args->out_q8_layout);
+  return bk_gdn_launch(*args);
 }
 
 int32_t bkRopeTables(int32_t max_len, int32_t rot_dim, double theta, float* cos_out, float* sin_out) {
@@ -499,6 +457,52 @@ int32_t bkArgmax(uint64_t logits, int32_t V, int32_t B, uint64_t idx, uint64_t v
 }
 
 }  // extern "C"
+
+int32_t bk_gdn_launch(const bkGdnArgs& a) {
+  BK_ARG(a.B > 0 && a.Hk > 0 && a.Hv > 0 && a.Hv % a.Hk == 0, "bkGdnStep: bad head counts B=%d Hk=%d Hv=%d", a.B, a.Hk,
+         a.Hv);
+  BK_ARG(a.qkv && a.z && a.a && a.b && a.A_log && a.dt_bias && a.norm_w && a.S_in && a.S_new && a.out,
+         "bkGdnStep: null pointer among required arguments");
+  if (a.apply_conv) {
+    BK_ARG(a.conv_w && a.conv_state_in && a.conv_state_new && (a.conv_w & 7) == 0,
+           "bkGdnStep: conv weights/state missing or misaligned");
+    BK_ARG(a.conv_state_in != a.conv_state_new, "bkGdnStep: conv state buffers must be distinct");
+  }
+  GdnParams p;
+  p.qkv = bk_ptr<uint16_t>(a.qkv);
+  p.z = bk_ptr<uint16_t>(a.z);
+  p.a = bk_ptr<float>(a.a);
+  p.b = bk_ptr<float>(a.b);
+  p.conv_w = bk_ptr<uint16_t>(a.conv_w);
+  p.cs_in = bk_ptr<uint16_t>(a.conv_state_in);
+  p.cs_new = bk_ptr<uint16_t>(a.conv_state_new);
+  p.A_log = bk_ptr<float>(a.A_log);
+  p.dt_bias = bk_ptr<uint16_t>(a.dt_bias);
+  p.norm_w = bk_ptr<float>(a.norm_w);
+  p.S_in = bk_ptr<float>(a.S_in);
+  p.S_new = bk_ptr<float>(a.S_new);
+  p.out = bk_ptr<uint16_t>(a.out);
+  p.o_raw = bk_ptr<float>(a.o_raw);
+  p.conv_out = bk_ptr<uint16_t>(a.conv_out);
+  p.out_q8 = bk_ptr<uint8_t>(a.out_q8);
+  p.out_q8_layout = a.out_q8_layout;
+  BK_ARG(a.out_q8_layout == BK_Q8_BLOCKS || (a.Hv * 128) % 256 == 0,
+         "bkGdnStep: out_q8_layout %d (a staged image needs Hv*128 a multiple of 256)", a.out_q8_layout);
+  p.B = a.B;
+  p.Hk = a.Hk;
+  p.Hv = a.Hv;
+  p.apply_conv = a.apply_conv;
+  p.early = a.state_is_settled;
+  p.T = a.n_tokens > 1 ? a.n_tokens : 1;
+  BK_ARG(a.n_tokens >= 0 && (p.out_q8_layout == BK_Q8_BLOCKS || (size_t)a.B * p.T <= 64), "bkGdnStep: n_tokens=%d", a.n_tokens);
+  p.trace = bk_trace_slot();
+  if (p.T > 1) BK_CUDA(bk_launch_pdl(gdn_step_kernel_multi, dim3(a.Hv, a.B), dim3(576), 0, p));
+  else if (a.Hv * a.B > bk_ctx().sm_count) BK_CUDA(bk_launch_pdl(gdn_step_kernel_x2, dim3(a.Hv, a.B), dim3(512), 0, p));
+  else BK_CUDA(bk_launch_pdl(gdn_step_kernel, dim3(a.Hv, a.B), dim3(576), 0, p));
+  BK_CHECK_LAUNCH();
+  return BK_OK;
+}
+
 
 int32_t bk_argmax_launch(uint64_t logits, int32_t V, int32_t B, uint64_t idx, uint64_t val, uint64_t scratch,
                          uint64_t pos, uint64_t hist, int32_t hist_ld, int32_t hist_rows, uint64_t host_out) {

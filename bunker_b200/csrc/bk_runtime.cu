@@ -34,7 +34,7 @@ static EncodeTiledFn encode_tiled_fn() {
 }
 
 bool bk_encode_map_2d(CUtensorMap* m, CUtensorMapDataType type, uint64_t base, uint64_t cols, uint64_t n_rows, uint64_t stride, uint32_t box_cols,
-                      uint32_t box_rows) {
+                      uint32_t box_rows, CUtensorMapSwizzle swizzle) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn || (base & 15) || stride % 16) return false;
   const cuuint64_t dims[2] = {cols, n_rows};
@@ -42,7 +42,7 @@ bool bk_encode_map_2d(CUtensorMap* m, CUtensorMapDataType type, uint64_t base, u
   const cuuint32_t box[2] = {box_cols, box_rows};
   const cuuint32_t estr[2] = {1, 1};
   return fn(m, type, 2, reinterpret_cast<void*>(static_cast<uintptr_t>(base)), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+            swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 extern "C" {
@@ -70,10 +70,8 @@ int32_t bkInit(int32_t device) {
   BK_CUDA(cudaStreamCreateWithFlags(&g_ctx.stream, cudaStreamNonBlocking));
   BK_CUDA(cudaMalloc((void**)&g_ctx.d_status, sizeof(int)));
   BK_CUDA(cudaMemsetAsync(g_ctx.d_status, 0, sizeof(int), g_ctx.stream));   // ordered on the library stream, then awaited
-  g_ctx.tile_scratch_bytes = (size_t)24 << 20;
-  BK_CUDA(cudaMalloc((void**)&g_ctx.tile_scratch, g_ctx.tile_scratch_bytes));
-  BK_CUDA(cudaMalloc((void**)&g_ctx.tile_counters, 256 * sizeof(int)));
-  BK_CUDA(cudaMemsetAsync(g_ctx.tile_counters, 0, 256 * sizeof(int), g_ctx.stream));
+  g_ctx.tile_image_bytes = (size_t)4 << 20;   // K up to 52,428 at 64 columns; more by the first launch that needs it
+  BK_CUDA(cudaMalloc((void**)&g_ctx.tile_image, g_ctx.tile_image_bytes));
   BK_CUDA(cudaStreamSynchronize(g_ctx.stream));
   g_ctx.launches = 0;
   g_ctx.ready = true;
@@ -85,11 +83,10 @@ int32_t bkShutdown(void) {
   cudaStreamSynchronize(g_ctx.stream);
   cudaStreamDestroy(g_ctx.stream);
   cudaFree(g_ctx.d_status);
-  cudaFree(g_ctx.tile_scratch);
-  cudaFree(g_ctx.tile_counters);
+  cudaFree(g_ctx.tile_image);
   g_ctx.d_status = nullptr;
-  g_ctx.tile_scratch = nullptr;
-  g_ctx.tile_counters = nullptr;
+  g_ctx.tile_image = nullptr;
+  g_ctx.tile_image_bytes = 0;
   g_ctx.stream = nullptr;
   g_ctx.ready = false;
   return BK_OK;

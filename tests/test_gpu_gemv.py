@@ -306,3 +306,27 @@ def test_gemv_automatic_order_follows_the_row_count(bk):
     ops.gemv(dxq.ptr, K, B, [ops.gemv_seg(dWg.ptr, N, act.ptr, R.BK_EPI_SWIGLU, W2=dWu.ptr)])
     assert_same_bits(act.download(np.uint16, (B, N)),
                      O.swiglu(O.gemv_q4k_q8_tile(Wg, N, K, xq), O.gemv_q4k_q8_tile(Wu, N, K, xq)), "SwiGLU pair of 2 x 2048 rows")
+
+
+@pytest.mark.parametrize("B,K,N", [(9, 256, 32), (16, 768, 2080), (17, 2304, 96), (20, 256, 32), (32, 4096, 2048), (31, 6144, 4128), (33, 256, 160),
+                                   (64, 2048, 9216), (48, 6144, 2048), (64, 17408, 64), (24, 17408, 5120)])
+def test_gemv_dense_tiles_in_lane_order(bk, B, K, N):
+    """17 and more columns of Q8_1 blocks with rows in whole boxes of 32: the dense tile kernel in the batch <= 8 order (fewer
+    columns: the batch <= 8 kernels), for the
+    largest integer dots (all nibbles 15, scales 63, quants at their limits) as well as random ones, two segments and a pair."""
+    rng = np.random.default_rng(900 + B + K)
+    W, W2 = synth.q4k_weights(rng, N, K), synth.q4k_weights(rng, 32, K)
+    W.reshape(N, -1, 144)[::7, :, 4:] = 0xFF
+    x = rng.normal(0, 1, (B, K)).astype(np.float32)
+    x[0] = 1.0
+    x[B - 1] = -1.0
+    xq = O.q8_1_quantize(x)
+    want, want2 = O.gemv_q4k_q8(W, N, K, xq), O.gemv_q4k_q8(W2, 32, K, xq)
+    dW, dW2, dxq = dev(W), dev(W2), dev(xq)
+    y, y2 = R.DeviceBuffer(B * N * 2), R.DeviceBuffer(B * 32 * 4)
+    for _ in range(2):
+        ops.gemv(dxq.ptr, K, B, [ops.gemv_seg(dW.ptr, N, y.ptr, R.BK_EPI_BF16), ops.gemv_seg(dW2.ptr, 32, y2.ptr, R.BK_EPI_F32)], order=R.BK_GEMV_ORDER_LANES)
+    assert_same_bits(y.download(np.uint16, (B, N)), O.epilogue_cast(want), "bf16 segment")
+    assert_same_bits(y2.download(np.float32, (B, 32)), want2, "f32 segment")
+    ops.gemv(dxq.ptr, K, B, [ops.gemv_seg(dW2.ptr, 32, y2.ptr, R.BK_EPI_SWIGLU, W2=dW2.ptr)], order=R.BK_GEMV_ORDER_LANES)
+    assert_same_bits(y2.download(np.uint16, (B, 32)), O.swiglu(want2, want2), "SwiGLU pair")
