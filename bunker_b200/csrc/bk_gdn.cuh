@@ -1,6 +1,5 @@
 // bk_gdn.cuh -- the fused conv1d + gated-DeltaNet step body (emitConv1d + emitGDN, src/emitters.ts:48-120;
-// buildGDNDecode, prototypes/decode.ts:314-388), shared by the per-op kernels (bk_ops.cu) and the persistent
-// decode-step kernel (bk_persist.cu).
+// buildGDNDecode, prototypes/decode.ts:314-388), the per-op kernels of one token (bk_ops.cu).
 #pragma once
 #include "bk_common.cuh"
 #include "bk_internal.h"
@@ -31,7 +30,7 @@ struct GdnParams {
   uint8_t* out_q8;
   int out_q8_layout;
   int B, Hk, Hv, apply_conv;
-  int T;      // tokens per sequence handled by this launch, in order (1 in the decode step)
+  int T;      // tokens per sequence (gdn_step_body<true>)
   int early;  // state / conv state / weights are not outputs of the immediately preceding launch
   unsigned long long* trace;
 };
@@ -39,20 +38,14 @@ struct GdnParams {
 // Two builds of this body.  gdn_step_kernel: launched with 576 threads when the grid has at most one CTA per SM; the
 // two extra warps only keep a second CTA of this grid off the SM (register file), so no SM finishes last with two.
 // gdn_step_kernel_x2: 64 registers, two CTAs per SM, for grids larger than the SM count (batch 8: 256 CTAs, one wave).
-// MULTI = false compiles the single-token body of the decode step (no loop, no carried taps).
-// PERSIST: the body runs as one phase of the persistent decode-step kernel (bk_persist.cu): head and sequence come
-// from the caller, no programmatic-launch calls, and the activations another CTA of the same launch produced
-// (qkv, z, a, b) are read past this SM's L1.
 struct GdnSmem {
   float s_q[128], s_k[128], s_v[128], s_o[128];
   float s_part[4][128];
   float s_scal[4];  // q scale, k rstd, decay, beta
 };
 
-template <bool PERSIST, typename T>
-__device__ __forceinline__ T gdn_ld_act(const T* p) { return PERSIST ? __ldcg(p) : *p; }
-
-template <bool MULTI, bool PERSIST = false>
+// MULTI: a few tokens one after the other (T of them), the state and the three conv taps in registers between them.
+template <bool MULTI>
 __device__ __forceinline__ void gdn_step_body(const GdnParams& p, GdnSmem& sm, const int hv, const int b) {
   constexpr int D = 128;
   float (&s_q)[D] = sm.s_q;
@@ -61,10 +54,8 @@ __device__ __forceinline__ void gdn_step_body(const GdnParams& p, GdnSmem& sm, c
   float (&s_o)[D] = sm.s_o;
   float (&s_part)[4][D] = sm.s_part;
   float (&s_scal)[4] = sm.s_scal;
-  if (!PERSIST) {
-    bk_pdl_trigger();
-    bk_stamp(p.trace, 0);
-  }
+  bk_pdl_trigger();
+  bk_stamp(p.trace, 0);
   const int t = threadIdx.x;
   const int ratio = p.Hv / p.Hk, hk = hv / ratio;
   const int keydim = p.Hk * D, C = 2 * keydim + p.Hv * D;
@@ -104,25 +95,19 @@ __device__ __forceinline__ void gdn_step_body(const GdnParams& p, GdnSmem& sm, c
     }
     if (t < D) nw = p.norm_w[t];
   };
-  if (PERSIST) {
-    load_static();
-  } else {
-    if (p.early) load_static();
-    bk_pdl_wait();
-    bk_stamp(p.trace, 2);
-    if (!p.early) load_static();
-  }
+  if (p.early) load_static();
+  bk_pdl_wait();
+  bk_stamp(p.trace, 2);
+  if (!p.early) load_static();
 
-  // Tokens tk = 0..T-1 of this sequence in order (T = 1 in the decode step): rows tk*B + b of the per-token inputs and
-  // outputs.  The state and the three conv taps stay in registers between tokens; both are written back after the last.
-  const int T = MULTI ? p.T : 1;
+  const int T = MULTI ? p.T : 1;   // rows tk*B + b of the per-token inputs and outputs
   for (int tk = 0; tk < T; tk++) {
     const size_t row = (size_t)tk * p.B + b;
     const bool last = !MULTI || tk == T - 1;
     float zv = 0.0f;
-    if (t < D) zv = bk_bf16_to_f32(gdn_ld_act<PERSIST>(p.z + (row * p.Hv + hv) * D + t));
+    if (t < D) zv = bk_bf16_to_f32(p.z[(row * p.Hv + hv) * D + t]);
     if (t < 3 * D) {
-      uint16_t hx = gdn_ld_act<PERSIST>(p.qkv + row * C + ch);
+      uint16_t hx = p.qkv[row * C + ch];
       float val;
       if (p.apply_conv) {
         float w0 = __uint_as_float(cw.x << 16), w1 = __uint_as_float(cw.x & 0xffff0000u);
@@ -154,9 +139,9 @@ __device__ __forceinline__ void gdn_step_body(const GdnParams& p, GdnSmem& sm, c
       else s_v[ci] = val;
     } else if (t == 3 * D) {
       // gates on an otherwise idle warp, overlapping the conv above
-      float sp = bk_softplusf(__fadd_rn(gdn_ld_act<PERSIST>(p.a + row * p.Hv + hv), dtb));
+      float sp = bk_softplusf(__fadd_rn(p.a[row * p.Hv + hv], dtb));
       s_scal[2] = bk_expf(-__fmul_rn(bk_expf(alog), sp));
-      s_scal[3] = bk_sigmoidf(gdn_ld_act<PERSIST>(p.b + row * p.Hv + hv));
+      s_scal[3] = bk_sigmoidf(p.b[row * p.Hv + hv]);
     }
     __syncthreads();
     if (warp < 2) {
@@ -226,7 +211,224 @@ __device__ __forceinline__ void gdn_step_body(const GdnParams& p, GdnSmem& sm, c
     }
     if (!last) __syncthreads();   // s_scal[0] and s_o are rewritten by the next token
   }
-  if (!PERSIST) bk_stamp(p.trace, 5);
+  bk_stamp(p.trace, 5);
+}
+
+// ---- several tokens per sequence -----------------------------------------------------------
+// Only the recurrence itself is serial.  Convolution, norms and gates of all tokens come first (gdn_prepare_kernel, one warp per
+// token and head), then the recurrence, four CTAs per value head (32 columns of the state each, in registers for all tokens),
+// then the gated norm (gdn_finish_kernel).  Per token the recurrence is two chains of 32 dependent FMAs and two barriers of
+// four warps, 0.3 us; as one CTA per head that did everything token after token it took 2.7 us.  (64 tokens, 32 value heads:
+// 176 us before, see below for now.)  The operations and their order are those of gdn_step_body.
+struct GdnTokens {
+  GdnParams g;
+  int T;            // tokens per sequence of this launch
+  int t0, t_all;    // its first token, and the tokens of all launches
+  float *qn, *kn;   // [T*B][Hk][128] normalised
+  float* v;         // [T*B][Hv][128]
+  float2* gates;    // [T*B][Hv] decay, beta
+  float* o;         // [T*B][Hv][128]
+};
+__host__ __device__ inline size_t gdn_row_floats(int Hk, int Hv) { return (size_t)Hk * 256 + (size_t)Hv * 258; }
+
+// four values of a caller's buffer, which need not be aligned to them
+__device__ __forceinline__ uint2 gdn_ld4(const uint16_t* p) {
+  if ((reinterpret_cast<uintptr_t>(p) & 7) == 0) return *reinterpret_cast<const uint2*>(p);
+  return make_uint2((uint32_t)p[0] | (uint32_t)p[1] << 16, (uint32_t)p[2] | (uint32_t)p[3] << 16);
+}
+__device__ __forceinline__ void gdn_st4(uint16_t* p, uint2 v) {
+  if ((reinterpret_cast<uintptr_t>(p) & 7) == 0) {
+    *reinterpret_cast<uint2*>(p) = v;
+    return;
+  }
+  p[0] = (uint16_t)v.x;
+  p[1] = (uint16_t)(v.x >> 16);
+  p[2] = (uint16_t)v.y;
+  p[3] = (uint16_t)(v.y >> 16);
+}
+
+// one warp per (row, head): heads 0..Hk-1 of q, of k, then the value heads; lane: channels 4 lane .. 4 lane + 3
+__global__ void __launch_bounds__(128) gdn_prepare_kernel(const GdnTokens w) {
+  bk_pdl_trigger();
+  bk_pdl_wait();
+  const GdnParams& p = w.g;
+  const int lane = threadIdx.x & 31, heads = 2 * p.Hk + p.Hv, C = heads * 128;
+  const int item = blockIdx.x * 4 + (threadIdx.x >> 5), row = item / heads, head = item - row * heads;
+  if (row >= w.T * p.B) return;
+  const int tk = w.t0 + row / p.B, b = row - row / p.B * p.B;
+  const int ch = head * 128 + 4 * lane;
+  auto taps = [&](int t) {   // the channels' raw values at token t; before token 0 the conv state
+    const uint16_t* src = t >= 0 ? p.qkv + ((size_t)t * p.B + b) * C + ch : p.cs_in + ((size_t)b * 3 + t + 3) * C + ch;
+    return gdn_ld4(src);
+  };
+  float x[4];
+  const uint2 hx = taps(tk);
+  if (p.apply_conv) {
+    const uint2 h[3] = {taps(tk - 3), taps(tk - 2), taps(tk - 1)};
+    auto at = [](const uint2& v, int e) { return e & 1 ? __uint_as_float((e < 2 ? v.x : v.y) & 0xffff0000u) : __uint_as_float((e < 2 ? v.x : v.y) << 16); };
+    uint32_t ob[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const uint2 cw = *reinterpret_cast<const uint2*>(p.conv_w + 4 * (size_t)(ch + e));
+      const float w0 = __uint_as_float(cw.x << 16), w1 = __uint_as_float(cw.x & 0xffff0000u);
+      const float w2 = __uint_as_float(cw.y << 16), w3 = __uint_as_float(cw.y & 0xffff0000u);
+      const float raw = __fadd_rn(__fadd_rn(__fmul_rn(w0, at(h[0], e)), __fmul_rn(w1, at(h[1], e))),
+                                  __fadd_rn(__fmul_rn(w2, at(h[2], e)), __fmul_rn(w3, at(hx, e))));
+      ob[e] = bk_f32_to_bf16(__fmul_rn(raw, bk_sigmoidf(raw)));
+      x[e] = bk_bf16_to_f32((uint16_t)ob[e]);
+    }
+    if (p.conv_out) gdn_st4(p.conv_out + ((size_t)tk * p.B + b) * C + ch, make_uint2(ob[0] | ob[1] << 16, ob[2] | ob[3] << 16));
+    if (tk == w.t_all - 1) {
+      uint16_t* d = p.cs_new + (size_t)b * 3 * C + ch;
+      gdn_st4(d, h[1]);
+      gdn_st4(d + C, h[2]);
+      gdn_st4(d + 2 * C, hx);
+    }
+  } else {
+    x[0] = __uint_as_float(hx.x << 16);
+    x[1] = __uint_as_float(hx.x & 0xffff0000u);
+    x[2] = __uint_as_float(hx.y << 16);
+    x[3] = __uint_as_float(hx.y & 0xffff0000u);
+  }
+  if (head >= 2 * p.Hk) {
+    const int hv = head - 2 * p.Hk;
+    const size_t o = (size_t)row * p.Hv + hv, in = ((size_t)tk * p.B + b) * p.Hv + hv;
+    reinterpret_cast<float4*>(w.v + o * 128)[lane] = make_float4(x[0], x[1], x[2], x[3]);
+    if (lane == 0) {
+      const float sp = bk_softplusf(__fadd_rn(p.a[in], bk_bf16_to_f32(p.dt_bias[hv])));
+      w.gates[o] = make_float2(bk_expf(-__fmul_rn(bk_expf(p.A_log[hv]), sp)), bk_sigmoidf(p.b[in]));
+    }
+    return;
+  }
+  float acc = 0.0f;
+#pragma unroll
+  for (int e = 0; e < 4; e++) acc = fmaf(x[e], x[e], acc);
+  float f = bk_rcp_sqrt(__fadd_rn(bk_warp_sum(acc), 1e-6f));
+  if (head < p.Hk) f = __fmul_rn(f, 0.088388347648318441f);
+  float* dst = head < p.Hk ? w.qn + ((size_t)row * p.Hk + head) * 128 : w.kn + ((size_t)row * p.Hk + head - p.Hk) * 128;
+  reinterpret_cast<float4*>(dst)[lane] = make_float4(__fmul_rn(x[0], f), __fmul_rn(x[1], f), __fmul_rn(x[2], f), __fmul_rn(x[3], f));
+}
+
+// CTA (4 hv + quarter, b): warp r has rows 32r..32r+31 of column 32 quarter + lane.  Dynamic shared memory: per token kn and qn
+// [256], v of the quarter [32]; then the gates.  The loop has no global load and one barrier a token: the sums over the warps
+// of token t's outputs are formed after token t+1's barrier.
+__host__ __device__ inline size_t gdn_recur_smem(int T) { return (size_t)T * (256 + 32 + 2) * 4; }
+__global__ void __launch_bounds__(128) gdn_recur_kernel(const GdnTokens w) {
+  extern __shared__ __align__(16) float gdn_tok[];
+  __shared__ float part[2][2][4][32];   // [parity of the token][sum][warp][column]
+  bk_pdl_trigger();
+  const GdnParams& p = w.g;
+  const int t = threadIdx.x, lane = t & 31, r = t >> 5, hv = blockIdx.x >> 2, b = blockIdx.y, hk = hv / (p.Hv / p.Hk), T = w.T;
+  const int col = (blockIdx.x & 3) * 32 + lane;
+  const size_t so = (((size_t)b * p.Hv + hv) * 128 + 32 * r) * 128 + col;
+  float s[32];
+  auto load_state = [&]() {
+#pragma unroll
+    for (int i = 0; i < 32; i++) s[i] = p.S_in[so + (size_t)i * 128];
+  };
+  if (p.early) load_state();
+  bk_pdl_wait();
+  if (!p.early) load_state();
+  float* kq = gdn_tok;
+  float* vs = gdn_tok + T * 256;
+  float2* gs = reinterpret_cast<float2*>(vs + T * 32);
+  auto copy16 = [](float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+  };
+  for (int i = t; i < T * 64; i += 128) {
+    const int tk = i >> 6, q = i & 63;
+    copy16(kq + i * 4, (q < 32 ? w.kn : w.qn) + (((size_t)tk * p.B + b) * p.Hk + hk) * 128 + (q & 31) * 4);
+  }
+  for (int i = t; i < T * 8; i += 128) copy16(vs + i * 4, w.v + (((size_t)(i >> 3) * p.B + b) * p.Hv + hv) * 128 + (blockIdx.x & 3) * 32 + (i & 7) * 4);
+  for (int i = t; i < T; i += 128) gs[i] = __ldcg(w.gates + ((size_t)i * p.B + b) * p.Hv + hv);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  float* out = w.o + ((size_t)b * p.Hv + hv) * 128 + col;
+  const size_t out_step = (size_t)p.B * p.Hv * 128;
+  auto finish = [&](int tk) {   // output of token tk
+    if (r == 0) {
+      const float(*q)[32] = part[tk & 1][1];
+      out[tk * out_step] = __fadd_rn(__fadd_rn(__fadd_rn(q[0][lane], q[1][lane]), q[2][lane]), q[3][lane]);
+    }
+  };
+#pragma unroll 1
+  for (int tk = 0; tk < T; tk++) {
+    const float4* k4 = reinterpret_cast<const float4*>(kq + tk * 256) + 8 * r;
+    const float2 gate = gs[tk];
+    const float v = vs[tk * 32 + lane];
+    float4 k[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) k[i] = k4[i];
+    float acc = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 32; i++) s[i] = __fmul_rn(s[i], gate.x);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      acc = fmaf(k[i].x, s[4 * i], acc);
+      acc = fmaf(k[i].y, s[4 * i + 1], acc);
+      acc = fmaf(k[i].z, s[4 * i + 2], acc);
+      acc = fmaf(k[i].w, s[4 * i + 3], acc);
+    }
+    float(*pp)[4][32] = part[tk & 1];
+    pp[0][r][lane] = acc;
+    __syncthreads();
+    const float kS = __fadd_rn(__fadd_rn(__fadd_rn(pp[0][0][lane], pp[0][1][lane]), pp[0][2][lane]), pp[0][3][lane]);
+    const float delta = __fmul_rn(__fsub_rn(v, kS), gate.y);
+    if (tk > 0) finish(tk - 1);
+    acc = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const float4 q = k4[32 + i];
+      s[4 * i] = fmaf(k[i].x, delta, s[4 * i]);
+      s[4 * i + 1] = fmaf(k[i].y, delta, s[4 * i + 1]);
+      s[4 * i + 2] = fmaf(k[i].z, delta, s[4 * i + 2]);
+      s[4 * i + 3] = fmaf(k[i].w, delta, s[4 * i + 3]);
+      acc = fmaf(q.x, s[4 * i], acc);
+      acc = fmaf(q.y, s[4 * i + 1], acc);
+      acc = fmaf(q.z, s[4 * i + 2], acc);
+      acc = fmaf(q.w, s[4 * i + 3], acc);
+    }
+    pp[1][r][lane] = acc;
+  }
+  __syncthreads();
+  finish(T - 1);
+#pragma unroll
+  for (int i = 0; i < 32; i++) p.S_new[so + (size_t)i * 128] = s[i];
+}
+
+// one warp per (row, value head)
+__global__ void __launch_bounds__(128) gdn_finish_kernel(const GdnTokens w) {
+  bk_pdl_trigger();
+  const GdnParams& p = w.g;
+  const int lane = threadIdx.x & 31, item = blockIdx.x * 4 + (threadIdx.x >> 5), row = item / p.Hv, hv = item - row * p.Hv;
+  bk_pdl_wait();
+  if (row >= w.T * p.B) return;
+  const size_t orow = (size_t)w.t0 * p.B + row;   // row of the outputs
+  const uint2 zz = gdn_ld4(p.z + (orow * p.Hv + hv) * 128 + 4 * lane);
+  const float4 o4 = __ldcg(reinterpret_cast<const float4*>(w.o + (size_t)item * 128) + lane);
+  const float o[4] = {o4.x, o4.y, o4.z, o4.w}, n[4] = {p.norm_w[4 * lane], p.norm_w[4 * lane + 1], p.norm_w[4 * lane + 2], p.norm_w[4 * lane + 3]};
+  const float z[4] = {__uint_as_float(zz.x << 16), __uint_as_float(zz.x & 0xffff0000u), __uint_as_float(zz.y << 16), __uint_as_float(zz.y & 0xffff0000u)};
+  if (p.o_raw)
+    for (int e = 0; e < 4; e++) p.o_raw[(orow * p.Hv + hv) * 128 + 4 * lane + e] = o[e];
+  float a2 = 0.0f;
+#pragma unroll
+  for (int e = 0; e < 4; e++) a2 = fmaf(o[e], o[e], a2);
+  const float rstd = bk_rcp_sqrt(__fadd_rn(__fdiv_rn(bk_warp_sum(a2), 128.0f), 1e-6f));
+  uint32_t ob[4];
+  float y[4];
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    ob[e] = bk_f32_to_bf16(__fmul_rn(__fmul_rn(__fmul_rn(o[e], rstd), n[e]), __fmul_rn(z[e], bk_sigmoidf(z[e]))));
+    y[e] = bk_bf16_to_f32((uint16_t)ob[e]);
+  }
+  gdn_st4(p.out + (orow * p.Hv + hv) * 128 + 4 * lane, make_uint2(ob[0] | ob[1] << 16, ob[2] | ob[3] << 16));
+  if (p.out_q8) {   // eight lanes hold one 32-value block
+    const int blk = hv * 4 + (lane >> 3), cols = p.B * w.t_all;
+    if (p.out_q8_layout == BK_Q8_TILE) bk_tile_store<4>(p.out_q8, p.Hv * 128, cols, (int)orow, blk, y, (lane & 7) * 4);
+    else if (p.out_q8_layout == BK_Q8_STAGED) bk_staged_store<4>(p.out_q8, p.Hv * 128, cols, (int)orow, blk, y, (lane & 7) * 4);
+    else bk_q8_1_store<4>(p.out_q8 + (orow * p.Hv * 4 + blk) * 36, y, (lane & 7) * 4);
+  }
 }
 
 }  // namespace

@@ -30,6 +30,8 @@ struct BkContext {
   int* d_status = nullptr;           // device word set by kernels whose bounded waits gave up
   uint8_t* tile_image = nullptr;     // activation image of the dense tile GEMV when its caller has Q8_1 blocks
   size_t tile_image_bytes = 0;
+  float* gdn_ws = nullptr;           // intermediate rows of a gated-DeltaNet launch of several tokens
+  size_t gdn_ws_bytes = 0;
   float* gemv_carry = nullptr;       // class accumulators handed from one K part of a split GEMV to the next
   size_t gemv_carry_bytes = 0;
   char err[512] = {0};

@@ -72,6 +72,8 @@ int32_t bkInit(int32_t device) {
   BK_CUDA(cudaMemsetAsync(g_ctx.d_status, 0, sizeof(int), g_ctx.stream));   // ordered on the library stream, then awaited
   g_ctx.tile_image_bytes = (size_t)4 << 20;   // K up to 52,428 at 64 columns; more by the first launch that needs it
   BK_CUDA(cudaMalloc((void**)&g_ctx.tile_image, g_ctx.tile_image_bytes));
+  g_ctx.gdn_ws_bytes = (size_t)8 << 20;       // 127 rows of 16 key and 48 value heads
+  BK_CUDA(cudaMalloc((void**)&g_ctx.gdn_ws, g_ctx.gdn_ws_bytes));
   BK_CUDA(cudaStreamSynchronize(g_ctx.stream));
   g_ctx.launches = 0;
   g_ctx.ready = true;
@@ -84,9 +86,12 @@ int32_t bkShutdown(void) {
   cudaStreamDestroy(g_ctx.stream);
   cudaFree(g_ctx.d_status);
   cudaFree(g_ctx.tile_image);
+  cudaFree(g_ctx.gdn_ws);
   g_ctx.d_status = nullptr;
   g_ctx.tile_image = nullptr;
   g_ctx.tile_image_bytes = 0;
+  g_ctx.gdn_ws = nullptr;
+  g_ctx.gdn_ws_bytes = 0;
   g_ctx.stream = nullptr;
   g_ctx.ready = false;
   return BK_OK;

@@ -164,6 +164,33 @@ def test_gdn_step_several_tokens_in_one_launch(bk):
                   O.q8_1_quantize_bf16(np.concatenate(want_out, axis=0)), Hv * 128, T * B)
 
 
+@pytest.mark.parametrize("B,T,Hk,Hv", [(1, 2, 1, 1), (1, 64, 2, 4), (3, 5, 8, 8), (1, 300, 16, 32), (7, 9, 2, 6)])
+def test_gdn_step_many_tokens(bk, B, T, Hk, Hv):
+    """T tokens in one call (prepared, recurred and finished for as many at a time as the workspace holds) equal T single calls."""
+    c = synth.gdn_case(B, Hk=Hk, Hv=Hv, config_id=30 + T)
+    C = (2 * Hk + Hv) * 128
+    rng = np.random.default_rng(T)
+    x = {"qkv": synth.normal_bf16(rng, (T, B, C)), "z": synth.normal_bf16(rng, (T, B, Hv * 128)),
+         "a": rng.normal(0, 1, (T, B, Hv)).astype(np.float32), "b": rng.normal(0, 1, (T, B, Hv)).astype(np.float32)}
+    w = {k: dev(c[k]) for k in ("conv_w", "A_log", "dt_bias", "norm_w")}
+    kw = dict(conv_w=w["conv_w"].ptr, A_log=w["A_log"].ptr, dt_bias=w["dt_bias"].ptr, norm_w=w["norm_w"].ptr, B=B, Hk=Hk, Hv=Hv, apply_conv=1)
+    d = {k: dev(v) for k, v in x.items()}
+    S1, S2, cs = dev(c["S"]), dev(c["S"]), [dev(c["conv_state"]), R.DeviceBuffer(B * 3 * C * 2)]
+    cs2, out1, out2 = R.DeviceBuffer(B * 3 * C * 2), R.DeviceBuffer(T * B * Hv * 256), R.DeviceBuffer(T * B * Hv * 256)
+    conv1, conv2 = R.DeviceBuffer(T * B * C * 2), R.DeviceBuffer(T * B * C * 2)
+    raw1, raw2 = R.DeviceBuffer(T * B * Hv * 512), R.DeviceBuffer(T * B * Hv * 512)
+    ops.gdn_step(qkv=d["qkv"].ptr, z=d["z"].ptr, a=d["a"].ptr, b=d["b"].ptr, conv_state_in=cs[0].ptr, conv_state_new=cs2.ptr, S_in=S1.ptr, S_new=S1.ptr,
+                 out=out1.ptr, o_raw=raw1.ptr, conv_out=conv1.ptr, n_tokens=T, **kw)
+    for t in range(T):
+        ops.gdn_step(qkv=d["qkv"].ptr + t * B * C * 2, z=d["z"].ptr + t * B * Hv * 256, a=d["a"].ptr + t * B * Hv * 4, b=d["b"].ptr + t * B * Hv * 4,
+                     conv_state_in=cs[t & 1].ptr, conv_state_new=cs[(t & 1) ^ 1].ptr, S_in=S2.ptr, S_new=S2.ptr, out=out2.ptr + t * B * Hv * 256,
+                     o_raw=raw2.ptr + t * B * Hv * 512, conv_out=conv2.ptr + t * B * C * 2, **kw)
+    for a, b, n, what in ((out1, out2, T * B * Hv * 128, "out"), (conv1, conv2, T * B * C, "conv"), (cs2, cs[T & 1], B * 3 * C, "conv state")):
+        assert_same_bits(a.download(np.uint16, (n,)), b.download(np.uint16, (n,)), what)
+    for a, b, n, what in ((raw1, raw2, T * B * Hv * 128, "raw"), (S1, S2, B * Hv * 128 * 128, "state")):
+        assert_same_bits(a.download(np.float32, (n,)), b.download(np.float32, (n,)), what)
+
+
 def test_gdn_step_without_conv(bk):
     c = synth.gdn_case(2, Hk=2, Hv=4, config_id=21)
     Hk, Hv, B = 2, 4, 2
