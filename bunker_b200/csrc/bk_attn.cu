@@ -21,7 +21,6 @@ namespace {
 constexpr int kW = 8;        // warps per split CTA
 constexpr int kHD = 256;     // head dim (8 per lane)
 constexpr int kMaxSplits = 1024;
-constexpr int kCh = 4;       // rows of one warp per register chunk (two chunks are live: the one in use and the next)
 
 struct AttnParams {
   const uint16_t* qg;
@@ -175,8 +174,8 @@ __device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, flo
 //   s_s   : split_len*8 f32
 //   o_s   : kW*8*256 f32              65536   (reused by the split merge)
 // One CTA per (split, KV head, batch).  Rows of the cache that were written in earlier steps do not depend on
-// the kernel running just before this one, so (p.settled) the first 8 K rows and 8 V rows of every warp are
-// requested before the dependency wait; longer splits stream further chunks of 8 rows per warp with the next
+// the kernel running just before this one, so (p.settled) the first chunk of K rows and of V rows of every warp is
+// requested before the dependency wait; longer splits stream further chunks with the next
 // chunk in flight while the current one is reduced.  The CTA that finishes a (batch, KV head) last merges the splits.
 // Two CTAs per SM (at most 128 registers): with one CTA of 8 warps an SM cannot hide the latency of the per-row
 // shuffle reductions and the stream stalls.
@@ -200,8 +199,24 @@ __global__ void __launch_bounds__(32) attn_append_kernel(const AttnParams p) {
       *reinterpret_cast<const uint4*>(p.v + ((size_t)b * p.Hkv + kvh) * kHD + lane * 8);
 }
 
+// warp_sum8 of values in the order g ^ (4 bit4 + 2 bit3 + bit2 of the lane): the same sums, addition for addition
+__device__ __forceinline__ float warp_sum8_swapped(const float (&v)[8]) {
+  float w[4], x[2];
+#pragma unroll
+  for (int i = 0; i < 4; i++) w[i] = __fadd_rn(v[i], __shfl_xor_sync(0xffffffffu, v[i + 4], 16));
+#pragma unroll
+  for (int i = 0; i < 2; i++) x[i] = __fadd_rn(w[i], __shfl_xor_sync(0xffffffffu, w[i + 2], 8));
+  float y = __fadd_rn(x[0], __shfl_xor_sync(0xffffffffu, x[1], 4));
+  y = __fadd_rn(y, __shfl_xor_sync(0xffffffffu, y, 2));
+  return __fadd_rn(y, __shfl_xor_sync(0xffffffffu, y, 1));
+}
+
 template <int G>
 __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams p) {
+  // Rows of one warp per register chunk (two chunks are live, the one in use and the next): as many as 128 registers hold
+  // without spilling, since the bytes in flight bound the few-head case (8 sequences, 20,000 rows, 4 heads: 4 rows 84 us, 6 rows 78) and
+  // the FMAs the many-head one (32,768 rows, 8 heads: 4 rows with 24 bytes spilled 218 us, 3 rows and the head order below 208).
+  constexpr int kCh = G <= 4 ? 6 : G >= 7 ? 3 : 4;
   bk_pdl_trigger();
   bk_stamp(p.trace, 0);
   extern __shared__ __align__(16) uint8_t smem[];
@@ -300,15 +315,18 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
     // query heads in pairs {q_g[d], q_g+1[d]}: one packed FMA advances the dot products of two heads (each its own
     // chain over d, as before)
     float2 qp[(G + 1) / 2][8];
+    const int hsel = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);   // the head whose score this lane ends up with
+    // Eight heads: a lane takes them in the order g ^ hsel, so that in each of the first three levels of the reduction it keeps the
+    // first half of its values and sends the second -- nothing to select.
+    const int swap = G == 8 ? hsel : 0;
 #pragma unroll
     for (int g = 0; g < G; g += 2) {
       float q0[8], q1[8];
-      bf16x8_to_f32(*reinterpret_cast<const uint4*>(q_st + g * kHD + lane * 8), q0);
-      if (g + 1 < G) bf16x8_to_f32(*reinterpret_cast<const uint4*>(q_st + (g + 1) * kHD + lane * 8), q1);
+      bf16x8_to_f32(*reinterpret_cast<const uint4*>(q_st + (g ^ swap) * kHD + lane * 8), q0);
+      if (g + 1 < G) bf16x8_to_f32(*reinterpret_cast<const uint4*>(q_st + ((g + 1) ^ swap) * kHD + lane * 8), q1);
 #pragma unroll
       for (int d = 0; d < 8; d++) qp[g >> 1][d] = make_float2(q0[d], g + 1 < G ? q1[d] : 0.0f);
     }
-    const int hsel = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
     for (int c = 0; c < nchunks; c++) {
       uint4 kn[kCh];
       if (c + 1 < nchunks) load_chunk(Kb, c + 1, kn, false);
@@ -328,7 +346,7 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
             pa[g] = a2.x;
             pa[g + 1] = a2.y;
           }
-          const float s1 = warp_sum8(pa);
+          const float s1 = G == 8 ? warp_sum8_swapped(pa) : warp_sum8(pa);
           if ((lane & 3) == 0) s_s[(size_t)jj * 8 + hsel] = __fmul_rn(s1, p.scale);
         }
       }
@@ -368,10 +386,11 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   // ---- phase 3: o = sum p * V ----
   {
     float2 acc[G][4];   // dims (2i, 2i+1) side by side: one packed FMA per pair
-    float lw[G];
+    float2 lw[(G + 1) / 2];   // heads 2i, 2i+1
+#pragma unroll
+    for (int g = 0; g < (G + 1) / 2; g++) lw[g] = make_float2(0.0f, 0.0f);
 #pragma unroll
     for (int g = 0; g < G; g++) {
-      lw[g] = 0.0f;
 #pragma unroll
       for (int e = 0; e < 4; e++) acc[g][e] = make_float2(0.0f, 0.0f);
     }
@@ -388,8 +407,9 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
           const float4 p1 = *reinterpret_cast<const float4*>(s_s + (size_t)jj * 8 + 4);
           const float pp[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
 #pragma unroll
+          for (int g = 0; g < G; g += 2) lw[g >> 1] = bk_add2(lw[g >> 1], make_float2(pp[g], pp[g + 1]));
+#pragma unroll
           for (int g = 0; g < G; g++) {
-            lw[g] = __fadd_rn(lw[g], pp[g]);
             const float2 p2 = make_float2(pp[g], pp[g]);
 #pragma unroll
             for (int d = 0; d < 4; d++) acc[g][d] = bk_fma2(p2, make_float2(vf[2 * d], vf[2 * d + 1]), acc[g][d]);
@@ -406,7 +426,7 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
       float4* d = reinterpret_cast<float4*>(o_s + ((size_t)(warp * 8 + g)) * kHD + lane * 8);
       d[0] = make_float4(acc[g][0].x, acc[g][0].y, acc[g][1].x, acc[g][1].y);
       d[1] = make_float4(acc[g][2].x, acc[g][2].y, acc[g][3].x, acc[g][3].y);
-      if (lane == 0) l_s[warp * 8 + g] = lw[g];
+      if (lane == 0) l_s[warp * 8 + g] = g & 1 ? lw[g >> 1].y : lw[g >> 1].x;
     }
   }
   __syncthreads();

@@ -199,22 +199,13 @@ BK_DEVINL float2 mul2(float2 a, float2 b) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
   return d;
 }
-BK_DEVINL float2 add2(float2 a, float2 b) {
-  unsigned long long ra, rb, rd;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
-  float2 d;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
-  return d;
-}
 BK_DEVINL float2 dup2(float a) { return make_float2(a, a); }
 BK_DEVINL uint32_t hfma2(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t d;
   asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
   return d;
 }
-BK_DEVINL uint32_t hadd2(uint32_t a, uint32_t b) {
+BK_DEVINL uint32_t hbk_add2(uint32_t a, uint32_t b) {
   uint32_t d;
   asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
@@ -335,7 +326,7 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
             uint32_t sc2, mn2;
             bk_q4k_scale_min_pair(hdr.y, hdr.z, hdr.w, p0 + pi, sc2, mn2);
             // half2 of the scales: (1024 + sc) - 1024; the nibble in the mantissa of 1024: (1024 + q) * sc - 1024 * sc, exact
-            const uint32_t s0 = hadd2(__byte_perm(sc2, 0x64u, 0x4040), 0xE400E400u), s1 = hadd2(__byte_perm(sc2, 0x64u, 0x4141), 0xE400E400u);
+            const uint32_t s0 = hbk_add2(__byte_perm(sc2, 0x64u, 0x4040), 0xE400E400u), s1 = hbk_add2(__byte_perm(sc2, 0x64u, 0x4141), 0xE400E400u);
             const uint32_t n0 = hmul2(s0, 0xE400E400u), s1s = hmul2(s1, 0x2C002C00u), n1 = hmul2(s1, 0xD400D400u);   // -1024 sc0, sc1 / 16, -64 sc1
             uint32_t a[32];
 #pragma unroll
@@ -670,17 +661,17 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
               a = bk_fma2(make_float2(c1.x, c1.y), x1, a);
               float2 mm = mul2(make_float2(c0.z, c0.w), dup2(r.z));
               mm = bk_fma2(make_float2(c1.z, c1.w), dup2(r.w), mm);
-              S[m * 4 + i] = add2(S[m * 4 + i], bk_fma2(dup2(r.x), a, mul2(dup2(r.y), mm)));
+              S[m * 4 + i] = bk_add2(S[m * 4 + i], bk_fma2(dup2(r.x), a, mul2(dup2(r.y), mm)));
             });
             next_superblock();
           }
           if (lp & 1) {
 #pragma unroll
-            for (int e = 0; e < 16; e++) S[e] = add2(L0[e], S[e]);
+            for (int e = 0; e < 16; e++) S[e] = bk_add2(L0[e], S[e]);
             for (int m = lp >> 1; m & 1; m >>= 1) {
               sp--;
 #pragma unroll
-              for (int e = 0; e < 16; e++) S[e] = add2(stack[(sp * 16 + e) * kScalers + st], S[e]);
+              for (int e = 0; e < 16; e++) S[e] = bk_add2(stack[(sp * 16 + e) * kScalers + st], S[e]);
             }
             if (lp + 1 < pos1 - pos0) {
 #pragma unroll
@@ -723,7 +714,7 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
           next_superblock();
 #pragma unroll
           for (int e = 0; e < NB * 4; e++)
-            yc[e] = add2((s & 3) == 0 ? make_float2(0.0f, 0.0f) : yc[e], bk_fma2(dup2(rd[e & 3]), A[e], mul2(dup2(rm[e & 3]), M[e])));
+            yc[e] = bk_add2((s & 3) == 0 ? make_float2(0.0f, 0.0f) : yc[e], bk_fma2(dup2(rd[e & 3]), A[e], mul2(dup2(rm[e & 3]), M[e])));
           if ((s & 3) == 3 || s == nsb - 1) {   // a chunk ends: its own value, or y += yc in place
             if (k > 0 && s - pos0 < 4) mbar_wait_idle<true>(smem_u32(xempty), (uint32_t)(k - 1) & 1u, p.status, dead);
             const bool first = CS > 1 || s < 4;
