@@ -22,9 +22,20 @@ constexpr int kQWarps = 8;   // warps of a CTA, two superblocks each
 constexpr float kTieBand = 2e-5f;
 BK_DEVINL int quant4_exact(float t, float dl) { return max(0, min(15, (int)floorf(__fadd_rn(__fdiv_rn(t, dl), 0.5f)))); }
 
+BK_DEVINL float2 add2_rd(float2 a, float2 b) {   // rounding down
+  unsigned long long ra, rb, rd;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
+  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
+  return d;
+}
+
 // 16 lanes per superblock, 16 weights each (half a sub-block): two superblocks per warp share the scalar work, and a
-// superblock leaves through shared memory as 16-byte stores.  Issue-bound: 17408 x 5120 bf16 took 123 us with eight
-// IEEE divisions per thread and byte stores (1.86 TB/s), 78 us like this (2.9 TB/s).
+// superblock leaves through shared memory as 16-byte stores.  Issue-bound, the half-rate minima and maxima above all: 17408 x
+// 5120 bf16 took 123 us with eight IEEE divisions per thread and byte stores (1.86 TB/s), 78 us with one weight at a time, 73 us with
+// two (3.1 TB/s).
 template <bool BF16>
 __global__ void __launch_bounds__(kQWarps * 32) quantize_q4k_kernel(const void* x, size_t n_superblocks, uint8_t* out) {
   __shared__ __align__(16) uint8_t stage[kQWarps][2 * 144];
@@ -81,14 +92,24 @@ __global__ void __launch_bounds__(kQWarps * 32) quantize_q4k_kernel(const void* 
   if (dl > 0.0f) {
     float r;
     asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(dl));
-    bool near_tie = false;
+    // floor without conversions: y + 1.5 * 2^23 rounded down has floor(y) in its low bits, and the clamp to 0..15 is one of floats
+    float off_tie = 0.0f;   // largest distance of a fraction from 1/2
+    uint32_t t[16];
+    const float2 ml2 = make_float2(ml, ml), r2 = make_float2(r, r), half2 = make_float2(0.5f, 0.5f);
 #pragma unroll
-    for (int e = 0; e < 16; e++) {
-      const float y = fmaf(__fadd_rn(v[e], ml), r, 0.5f);
-      const float fl = floorf(y);
-      near_tie = near_tie || fabsf(__fsub_rn(__fsub_rn(y, fl), 0.5f)) > 0.5f - kTieBand;
-      q[e >> 2] |= (uint32_t)max(0, min(15, (int)fl)) << (8 * (e & 3));
+    for (int e = 0; e < 16; e += 2) {   // two weights per instruction
+      const float2 y = bk_fma2(bk_add2(make_float2(v[e], v[e + 1]), ml2), r2, half2);
+      const float2 f = add2_rd(y, make_float2(12582912.0f, 12582912.0f));
+      const float2 fl = bk_add2(f, make_float2(-12582912.0f, -12582912.0f));
+      const float2 o = bk_add2(bk_fma2(fl, make_float2(-1.0f, -1.0f), y), make_float2(-0.5f, -0.5f));
+      off_tie = fmaxf(off_tie, fmaxf(fabsf(o.x), fabsf(o.y)));
+      t[e] = __float_as_uint(fminf(fmaxf(f.x, 12582912.0f), 12582927.0f));
+      t[e + 1] = __float_as_uint(fminf(fmaxf(f.y, 12582912.0f), 12582927.0f));
     }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      q[k] = __byte_perm(__byte_perm(t[4 * k], t[4 * k + 1], 0x0040), __byte_perm(t[4 * k + 2], t[4 * k + 3], 0x0040), 0x5410);
+    const bool near_tie = off_tie > 0.5f - kTieBand;
     if (near_tie) {
       q[0] = q[1] = q[2] = q[3] = 0u;
 #pragma unroll
