@@ -160,7 +160,7 @@ __device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, flo
       y[2 * e] = __uint_as_float(o[e] << 16);
       y[2 * e + 1] = __uint_as_float(o[e] & 0xffff0000u);
     }
-    if (p.out_q8_layout == BK_Q8_TILE) bk_tile_store<8>(p.out_q8, p.Hq * kHD, p.B, b, (h * kHD + lane * 8) >> 5, y, (lane & 3) * 8);
+    if (p.out_q8_layout >= BK_Q8_TILE) bk_tile_store<8>(p.out_q8, p.Hq * kHD, p.B, b, (h * kHD + lane * 8) >> 5, y, (lane & 3) * 8, p.out_q8_layout == BK_Q8_TILE32);
     else if (p.out_q8_layout == BK_Q8_STAGED) bk_staged_store<8>(p.out_q8, p.Hq * kHD, p.B, b, (h * kHD + lane * 8) >> 5, y, (lane & 3) * 8);
     else bk_q8_1_store<8>(p.out_q8 + ((((size_t)b * p.Hq + h) * kHD + lane * 8) >> 5) * 36, y, (lane & 3) * 8);
   }

@@ -405,7 +405,12 @@ BK_DEVINL void bk_tile_store_factors(uint8_t* img, int K, int B, int b, int blk,
 
 // Same contract as bk_q8_1_store, writing block blk of column b into an image.
 template <int PER>
-BK_DEVINL void bk_tile_store(uint8_t* img, int K, int B, int b, int blk, const float (&y)[PER], int idx_in_block) {
+BK_DEVINL void bk_tile_store(uint8_t* img, int K, int B, int b, int blk, const float (&y)[PER], int idx_in_block, bool split = false) {
+  if (split) {   // an image per 32 columns
+    img += (size_t)(b >> 5) * bk_tile_image_bytes(K, 32);
+    b &= 31;
+    B = 32;
+  }
   static_assert(PER == 1 || PER == 4 || PER == 8, "values per lane");
   constexpr int GROUP = 32 / PER;
   float amax = 0.0f;

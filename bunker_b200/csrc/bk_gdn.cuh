@@ -204,7 +204,7 @@ __device__ __forceinline__ void gdn_step_body(const GdnParams& p, GdnSmem& sm, c
       p.out[(row * p.Hv + hv) * D + t] = ob;
       if (p.out_q8) {  // warp w of the first four holds block w of this head
         const float y[1] = {bk_bf16_to_f32(ob)};
-        if (p.out_q8_layout == BK_Q8_TILE) bk_tile_store<1>(p.out_q8, p.Hv * D, p.B * T, (int)row, hv * 4 + warp, y, lane);
+        if (p.out_q8_layout >= BK_Q8_TILE) bk_tile_store<1>(p.out_q8, p.Hv * D, p.B * T, (int)row, hv * 4 + warp, y, lane, p.out_q8_layout == BK_Q8_TILE32);
         else if (p.out_q8_layout == BK_Q8_STAGED) bk_staged_store<1>(p.out_q8, p.Hv * D, p.B * T, (int)row, hv * 4 + warp, y, lane);
         else bk_q8_1_store<1>(p.out_q8 + ((row * p.Hv + hv) * 4 + warp) * 36, y, lane);
       }
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(128) gdn_finish_kernel(const GdnTokens w) {
   gdn_st4(p.out + (orow * p.Hv + hv) * 128 + 4 * lane, make_uint2(ob[0] | ob[1] << 16, ob[2] | ob[3] << 16));
   if (p.out_q8) {   // eight lanes hold one 32-value block
     const int blk = hv * 4 + (lane >> 3), cols = p.B * w.t_all;
-    if (p.out_q8_layout == BK_Q8_TILE) bk_tile_store<4>(p.out_q8, p.Hv * 128, cols, (int)orow, blk, y, (lane & 7) * 4);
+    if (p.out_q8_layout >= BK_Q8_TILE) bk_tile_store<4>(p.out_q8, p.Hv * 128, cols, (int)orow, blk, y, (lane & 7) * 4, p.out_q8_layout == BK_Q8_TILE32);
     else if (p.out_q8_layout == BK_Q8_STAGED) bk_staged_store<4>(p.out_q8, p.Hv * 128, cols, (int)orow, blk, y, (lane & 7) * 4);
     else bk_q8_1_store<4>(p.out_q8 + (orow * p.Hv * 4 + blk) * 36, y, (lane & 7) * 4);
   }

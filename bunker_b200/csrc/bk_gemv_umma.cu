@@ -78,6 +78,7 @@ struct Cfg {
 struct UmmaParams {
   GemvParams g;       // K, segments, total_vrows, x = image (see bk_tile_image_bytes), status
   int B;              // activation columns, 1..64
+  int groups;         // column groups (N > 32 columns of few rows: two groups of 32, each with its own image and its own tiles)
   int use_maps;       // weights come by tiled TMA loads through maps[]
   int stages;         // ring stages
   int csplit;         // LANES: CTAs that share the classes of a pair; TILE: CTAs that share the chunks (= cluster size)
@@ -280,7 +281,8 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
   const uint32_t tmem_a = tmem + C::kBatches * 128;
 
-  const int n_tiles = (p.total_vrows + kTileM - 1) / kTileM;
+  const bool two = LANES && NB == 2 && P.groups == 2;   // tile index: row tile * 2 + column group
+  const int n_tiles = (p.total_vrows + kTileM - 1) / kTileM * (two ? 2 : 1);
   const int n_chunks = (nsb + 3) / 4;
   const int tile0 = (int)blockIdx.x / CS, tile_step = (int)gridDim.x / CS;   // the cluster's tiles
   const int n_my = (n_tiles - tile0 + tile_step - 1) / tile_step;
@@ -396,9 +398,9 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
         }
       };
       const uint32_t xbytes = (uint32_t)((LANES ? 4 * P.csplit : n_chunks) * vs * 4);
-      const int b0 = (int)rank * own;
+      const int b00 = (int)rank * own;
       for (int k = 0; k < n_my; k++) {
-        const int tile = tile0 + k * tile_step;
+        const int vt = tile0 + k * tile_step, tile = two ? vt >> 1 : vt, b0 = b00 + (two ? (vt & 1) * N : 0);
         if (CS > 1 && et == 0) mbar_expect_tx(smem_u32(xfull), xbytes);
         mbar_wait_idle(smem_u32(xfull), (uint32_t)k & 1u, p.status, dead);
         for (int h = 0; h < (swiglu_halves ? 1 : 2); h++) {
@@ -504,21 +506,24 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
       const uint64_t policy = l2_evict_first();
       const uint8_t* img_b = static_cast<const uint8_t*>(p.x) + (size_t)p0 * C::kBBytes;   // image: operand B of all units, then their factors
       const uint8_t* img_c = static_cast<const uint8_t*>(p.x) + (size_t)(p.K / 64) * C::kBBytes + (size_t)p0 * (N * 16);
-      auto fill_x = [&](int s, int stage) {
+      const size_t img_bytes = (size_t)(p.K / 64) * (C::kBBytes + N * 16);
+      auto fill_x = [&](int s, int stage, int vt) {
+        const size_t go = two ? (size_t)(vt & 1) * img_bytes : 0;
         if (lane == 0) {
           const uint32_t bar = smem_u32(wfull + stage);
-          bulk_g2s(smem_u32(raw + (size_t)stage * C::kStage + C::kWBytes), img_b + (size_t)s * 4 * C::kBBytes, PS * C::kBBytes, bar);
-          bulk_g2s(smem_u32(cols + cslot * C::kColBytes), img_c + (size_t)s * (4 * N * 16), C::kColBytes, bar);
+          bulk_g2s(smem_u32(raw + (size_t)stage * C::kStage + C::kWBytes), img_b + go + (size_t)s * 4 * C::kBBytes, PS * C::kBBytes, bar);
+          bulk_g2s(smem_u32(cols + cslot * C::kColBytes), img_c + go + (size_t)s * (4 * N * 16), C::kColBytes, bar);
         }
         if (++cslot == ncols) cslot = 0;   // (three superblocks more than stages: the scalers are at most that far behind the MMAs)
       };
       constexpr uint32_t kXBytes = PS * C::kBBytes + C::kColBytes;
-      int tile = tile0, stage = 0;
+      int vt = tile0, stage = 0;
       uint32_t spar = 1;   // parity of the readers' arrivals on the previous use
       w.start(pos0, pos1, nsb);
       for (int i = 0; i < total; i++) {
         if (i >= nst) mbar_wait_idle(smem_u32(wempty + stage), spar, p.status, dead);
         const uint32_t bar = smem_u32(wfull + stage), dst0 = smem_u32(raw + (size_t)stage * C::kStage);
+        const int tile = two ? vt >> 1 : vt;
         if (P.use_maps) {
           // lanes 0..3: the 32-row boxes of the tile (whole superblocks, or headers); lanes 4..7: their quants
           const int bx = lane & 3;
@@ -557,16 +562,14 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
         }
         if (i == first - 1) {   // the ring is full of weights, which depend on nothing: now the activations of these stages
           bk_pdl_wait();
-          int f = 0;
-          while (f < first) {
-            for (wx.start(pos0, pos1, nsb); !wx.done() && f < first; wx.next(), f++) fill_x(wx.s, f);
-          }
+          for (int f = 0, vx = tile0; f < first; vx += tile_step)
+            for (wx.start(pos0, pos1, nsb); !wx.done() && f < first; wx.next(), f++) fill_x(wx.s, f, vx);
         } else if (i >= first) {
-          fill_x(w.s, stage);
+          fill_x(w.s, stage, vt);
         }
         w.next();
         if (w.done()) {
-          tile += tile_step;
+          vt += tile_step;
           w.start(pos0, pos1, nsb);
         }
         if (++stage == nst) {
@@ -742,10 +745,11 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
 }
 
 // Q8_1 blocks [B][K/32][36] -> image
-__global__ void __launch_bounds__(256) tile_image_kernel(const uint32_t* x, int nblk, int B, uint8_t* img) {
+__global__ void __launch_bounds__(256) tile_image_kernel(const uint32_t* x, int nblk, const int B_all, uint8_t* img, const bool split) {
   bk_pdl_trigger();
   bk_pdl_wait();
-  const int i = blockIdx.x * 256 + threadIdx.x, b = i % B, blk = i / B;
+  const int i = blockIdx.x * 256 + threadIdx.x, blk = i / B_all;
+  int b = i % B_all, B = B_all;
   if (blk >= nblk) return;
   const uint32_t* src = x + ((size_t)b * nblk + blk) * 9;
   uint32_t w[9];
@@ -754,6 +758,11 @@ __global__ void __launch_bounds__(256) tile_image_kernel(const uint32_t* x, int 
   int qsum = 0;
 #pragma unroll
   for (int k = 0; k < 8; k++) qsum = bk_dp4a_ss(w[k], 0x01010101u, qsum);
+  if (split) {   // an image per 32 columns
+    img += (size_t)(b >> 5) * bk_tile_image_bytes(nblk * 32, 32);
+    b &= 31;
+    B = 32;
+  }
 #pragma unroll
   for (int c = 0; c < 4; c++) bk_tile_store_quants(img, B, b, blk, c, w[2 * c], w[2 * c + 1]);
   const float d8 = bk_q8half_to_f32((uint16_t)(w[8] & 0xffffu));
@@ -813,7 +822,7 @@ int32_t launch_tile(UmmaParams& P) {
   }
   // How many CTAs share the classes (or chunks) of a tile: the fewest steps of the longest CTA, a tile's exchange and pipeline
   // fill counted as one superblock.
-  const int tiles = (g.total_vrows + kTileM - 1) / kTileM, nsb = g.K / 256, n_chunks = (nsb + 3) / 4;
+  const int tiles = (g.total_vrows + kTileM - 1) / kTileM * P.groups, nsb = g.K / 256, n_chunks = (nsb + 3) / 4;
   int best = 1, best_cost = 0x7fffffff;
   for (int s = 1; s * (4 / C::PS) <= 8; s *= 2) {
     const int cs = s * (4 / C::PS), n = clusters[__builtin_ctz(cs)];
@@ -853,6 +862,8 @@ int32_t bk_gemv_umma_launch(void* params, int B, bool lanes) {
   UmmaParams P;
   P.g = *static_cast<GemvParams*>(params);
   P.B = B;
+  const bool split = lanes && bk_tile_split(P.g.total_vrows, B);
+  P.groups = split ? 2 : 1;
   if (P.g.prologue == BK_PRO_Q8) {
     const size_t need = bk_tile_image_bytes(P.g.K, B);
     if (c.tile_image_bytes < need) {
@@ -867,10 +878,10 @@ int32_t bk_gemv_umma_launch(void* params, int B, bool lanes) {
       c.tile_image_bytes = need;
     }
     const int nblk = P.g.K / 32;
-    BK_CUDA(bk_launch_pdl(tile_image_kernel, dim3((nblk * B + 255) / 256), dim3(256), 0, static_cast<const uint32_t*>(P.g.x), nblk, B, c.tile_image));
+    BK_CUDA(bk_launch_pdl(tile_image_kernel, dim3((nblk * B + 255) / 256), dim3(256), 0, static_cast<const uint32_t*>(P.g.x), nblk, B, c.tile_image, split));
     BK_CHECK_LAUNCH();
     P.g.x = c.tile_image;
   }
-  if (lanes) return B <= 32 ? launch_tile<2, true>(P) : launch_tile<4, true>(P);   // (17 columns and more)
+  if (lanes) return B <= 32 || split ? launch_tile<2, true>(P) : launch_tile<4, true>(P);   // (17 columns and more)
   return B <= 16 ? launch_tile<1, false>(P) : B <= 32 ? launch_tile<2, false>(P) : launch_tile<4, false>(P);
 }

@@ -225,10 +225,11 @@ int32_t enqueue_step(Model& m, int parity, bool host_tokens = false) {
   };
   // A projection that goes to the dense tile kernel (bk_gemv_launch_tp has the rule) reads that kernel's image.
   auto layout_for = [&](int K, int rows, int row_gcd) {
-    if (tile_path && (bk_gemv_auto_tile(rows, K) || (row_gcd % 32 == 0 && bk_gemv_dense_lanes(B)))) return BK_Q8_TILE;
+    if (tile_path && bk_gemv_auto_tile(rows, K)) return BK_Q8_TILE;
+    if (tile_path && row_gcd % 32 == 0 && bk_gemv_dense_lanes(B)) return bk_tile_split(rows, B) ? BK_Q8_TILE32 : BK_Q8_TILE;
     return staged_ok(K, rows) ? BK_Q8_STAGED : BK_Q8_BLOCKS;
   };
-  auto prologue_of = [](int layout) { return layout == BK_Q8_TILE ? BK_PRO_TILE : layout == BK_Q8_STAGED ? BK_PRO_STAGED : BK_PRO_Q8; };
+  auto prologue_of = [](int layout) { return layout >= BK_Q8_TILE ? BK_PRO_TILE : layout == BK_Q8_STAGED ? BK_PRO_STAGED : BK_PRO_Q8; };
   // Input of a projection: fused RMSNorm/quantise prologue at batch 1; at batch >= 2 one small launch
   // normalises and quantises the rows once and every CTA of the projection just copies the blocks.
   // Tensor parallel: a row-parallel GEMV pushes its partial sums to every rank (BK_EPI_PUSH_F32); the sum over ranks,
@@ -412,25 +413,25 @@ int32_t enqueue_prefill(Model& m, int T) {
   Model::Prefill& f = m.pf;
   auto staged_ok = [&](int K, int cols) { return cols >= 2 && bk_gemv_mma_fits(K, cols < 8 ? cols : 8) && !(cols > 8 && cols % 8 == 1); };
   // many columns: the dense tile kernel, in the lane order, where the row counts are whole boxes of 32
-  auto layout_for = [&](int K, int cols, int row_gcd) {
-    if (bk_gemv_dense_lanes(cols) && row_gcd % 32 == 0) return BK_Q8_TILE;
+  auto layout_for = [&](int K, int cols, int rows, int row_gcd) {
+    if (bk_gemv_dense_lanes(cols) && row_gcd % 32 == 0) return bk_tile_split(rows, cols) ? BK_Q8_TILE32 : BK_Q8_TILE;
     return staged_ok(K, cols) ? BK_Q8_STAGED : BK_Q8_BLOCKS;
   };
   auto point_at = [&](bkGemvArgs& g, int K, int cols, int layout) {
     g.K = K; g.B = cols; g.eps = c.eps;
     g.order = BK_GEMV_ORDER_LANES;   // every column must get the bits of a single decode step
-    g.prologue = layout == BK_Q8_TILE ? BK_PRO_TILE : layout == BK_Q8_STAGED ? BK_PRO_STAGED : BK_PRO_Q8; g.x = f.xq;
+    g.prologue = layout >= BK_Q8_TILE ? BK_PRO_TILE : layout == BK_Q8_STAGED ? BK_PRO_STAGED : BK_PRO_Q8; g.x = f.xq;
   };
   // quantise `cols` rows once (optionally RMSNorm first) and point the GEMV at the result
   // row_gcd: a number that divides every segment's row count
-  auto set_input = [&](bkGemvArgs& g, uint64_t x, int K, uint64_t norm_w, int cols, int row_gcd) -> int32_t {
+  auto set_input = [&](bkGemvArgs& g, uint64_t x, int K, uint64_t norm_w, int cols, int rows, int row_gcd) -> int32_t {
     g.K = K; g.B = cols; g.eps = c.eps;
     g.order = BK_GEMV_ORDER_LANES;   // every column must get the bits of a single decode step
     if (cols == 1) {
       g.prologue = norm_w ? BK_PRO_RMSNORM : BK_PRO_BF16; g.x = x; g.norm_w = norm_w;
       return BK_OK;
     }
-    const int layout = layout_for(K, cols, row_gcd);
+    const int layout = layout_for(K, cols, rows, row_gcd);
     TRY(bk_quant_rows_launch(x, norm_w, K, cols, c.eps, f.xq, layout, nullptr));
     point_at(g, K, cols, layout);
     return BK_OK;
@@ -443,7 +444,7 @@ int32_t enqueue_prefill(Model& m, int T) {
     LayerW& L = m.layers[li];
     bkGemvArgs g;
     memset(&g, 0, sizeof(g));
-    TRY(set_input(g, f.x[cur], H, L.in_ln, C, L.full ? 32 : m.Hv));   // (the other row counts are multiples of 128)
+    TRY(set_input(g, f.x[cur], H, L.in_ln, C, L.full ? m.QG + 2 * m.KVD : m.Cw + m.ZD + 2 * m.Hv, L.full ? 32 : m.Hv));   // (the other row counts are multiples of 128)
     if (!L.full) {
       g.n_segs = 4;
       g.segs[0] = bkGemvSeg{L.qkv, 0, f.qkv, 0, m.Cw, BK_EPI_BF16, m.Cw, 0};
@@ -459,15 +460,15 @@ int32_t enqueue_prefill(Model& m, int T) {
         ga.conv_w = L.conv_w; ga.conv_state_in = L.conv_state[parity]; ga.conv_state_new = L.conv_state[parity ^ 1];
         ga.A_log = L.A_log; ga.dt_bias = L.dt_bias; ga.norm_w = L.gnorm;
         ga.S_in = L.S; ga.S_new = L.S;
-        const int layout = layout_for(m.ZD, C, H);
+        const int layout = layout_for(m.ZD, C, H, H);
         ga.out = f.attn_out; ga.out_q8 = C > 1 ? f.xq : 0; ga.out_q8_layout = C > 1 ? layout : BK_Q8_BLOCKS;
         ga.B = B; ga.Hk = m.Hk; ga.Hv = m.Hv; ga.apply_conv = 1; ga.n_tokens = T;
         ga.state_is_settled = 1;   // written by the previous pass, many launches ago
         TRY(bk_gdn_launch(ga));
       }
       memset(&g, 0, sizeof(g));
-      if (C > 1) point_at(g, m.ZD, C, layout_for(m.ZD, C, H));   // quantised by the launch before
-      else TRY(set_input(g, f.attn_out, m.ZD, 0, C, H));
+      if (C > 1) point_at(g, m.ZD, C, layout_for(m.ZD, C, H, H));   // quantised by the launch before
+      else TRY(set_input(g, f.attn_out, m.ZD, 0, C, H, H));
       g.n_segs = 1;
       g.segs[0] = bkGemvSeg{L.out_proj, 0, f.h1, f.x[cur], H, BK_EPI_ADD_BF16, H, 0};
       TRY(bk_gemv_launch(g));
@@ -489,7 +490,7 @@ int32_t enqueue_prefill(Model& m, int T) {
         aa.out = f.attn_out; aa.scratch = f.attn_scratch;
         if (C > 1) {
           aa.out_q8 = f.xq;
-          aa.out_q8_layout = layout_for(attn_w, C, H);
+          aa.out_q8_layout = layout_for(attn_w, C, H, H);
         }
         aa.B = C; aa.Hq = m.Hq; aa.Hkv = m.Hkv; aa.HD = c.head_dim; aa.rot_half = c.rot_dim / 2; aa.max_len = c.max_len;
         aa.split_len = m.split_len; aa.max_pos = c.max_len - 1; aa.scale = 1.0f / sqrtf((float)c.head_dim);
@@ -497,19 +498,19 @@ int32_t enqueue_prefill(Model& m, int T) {
         TRY(bk_attn_launch(aa, B, m.pf.cols));
       }
       memset(&g, 0, sizeof(g));
-      if (C > 1) point_at(g, attn_w, C, layout_for(attn_w, C, H));
-      else TRY(set_input(g, f.attn_out, attn_w, 0, C, H));
+      if (C > 1) point_at(g, attn_w, C, layout_for(attn_w, C, H, H));
+      else TRY(set_input(g, f.attn_out, attn_w, 0, C, H, H));
       g.n_segs = 1;
       g.segs[0] = bkGemvSeg{L.o, 0, f.h1, f.x[cur], H, BK_EPI_ADD_BF16, H, 0};
       TRY(bk_gemv_launch(g));
     }
     memset(&g, 0, sizeof(g));
-    TRY(set_input(g, f.h1, H, L.post_ln, C, m.inter));
+    TRY(set_input(g, f.h1, H, L.post_ln, C, 2 * m.inter, m.inter));
     g.n_segs = 1;
     g.segs[0] = bkGemvSeg{L.gate, L.up, f.act, 0, m.inter, BK_EPI_SWIGLU, m.inter, 0};
     TRY(bk_gemv_launch(g));
     memset(&g, 0, sizeof(g));
-    TRY(set_input(g, f.act, m.inter, 0, C, H));
+    TRY(set_input(g, f.act, m.inter, 0, C, H, H));
     g.n_segs = 1;
     g.segs[0] = bkGemvSeg{L.down, 0, f.x[cur ^ 1], f.h1, H, BK_EPI_ADD_BF16, H, 0};
     TRY(bk_gemv_launch(g));
@@ -518,7 +519,7 @@ int32_t enqueue_prefill(Model& m, int T) {
   // logits and argmax of the last token only
   bkGemvArgs g;
   memset(&g, 0, sizeof(g));
-  TRY(set_input(g, f.x[cur] + (uint64_t)(C - B) * H * 2, H, m.final_norm, B, m.vocab_local));
+  TRY(set_input(g, f.x[cur] + (uint64_t)(C - B) * H * 2, H, m.final_norm, B, m.vocab_local, m.vocab_local));
   g.n_segs = 1;
   g.segs[0] = bkGemvSeg{m.embed, 0, m.logits, 0, m.vocab_local, BK_EPI_F32, m.vocab_local, 0};
   TRY(bk_gemv_launch(g));

@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const uint16_t* x, const u
 // rd.n > 0 (NORM only): row b is not read from x but formed from the tensor-parallel partial sums + residual.
 template <bool NORM, int LAYOUT>
 __global__ void __launch_bounds__(256) quant_rows_kernel(const uint16_t* x, const uint16_t* w, int K, float eps,
-                                                         uint8_t* out, const BkReduce rd, int* status) {
+                                                         uint8_t* out, const BkReduce rd, int* status, const bool split) {
   bk_pdl_trigger();
   __shared__ float red[8];
   const int b = blockIdx.y, nchunk = K / 8, tid = threadIdx.x;
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const uint16_t* x, cons
       for (int e = 0; e < 8; e++)
         y[e] = bk_bf16_to_f32(bk_f32_to_bf16(__fmul_rn(__fmul_rn(v[e], rstd), __fadd_rn(1.0f, wv[e]))));
       if (LAYOUT == BK_Q8_STAGED) bk_staged_store<8>(out, K, gridDim.y, b, q >> 2, y, (q & 3) * 8);
-      else if (LAYOUT == BK_Q8_TILE) bk_tile_store<8>(out, K, gridDim.y, b, q >> 2, y, (q & 3) * 8);
+      else if (LAYOUT == BK_Q8_TILE) bk_tile_store<8>(out, K, gridDim.y, b, q >> 2, y, (q & 3) * 8, split);
       else bk_q8_1_store<8>(orow + (size_t)(q >> 2) * 36, y, (q & 3) * 8);
     }
   } else {
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const uint16_t* x, cons
       float y[8];
       load8_bf16(row + (size_t)q * 8, y);
       if (LAYOUT == BK_Q8_STAGED) bk_staged_store<8>(out, K, gridDim.y, b, q >> 2, y, (q & 3) * 8);
-      else if (LAYOUT == BK_Q8_TILE) bk_tile_store<8>(out, K, gridDim.y, b, q >> 2, y, (q & 3) * 8);
+      else if (LAYOUT == BK_Q8_TILE) bk_tile_store<8>(out, K, gridDim.y, b, q >> 2, y, (q & 3) * 8, split);
       else bk_q8_1_store<8>(orow + (size_t)(q >> 2) * 36, y, (q & 3) * 8);
     }
   }
@@ -358,9 +358,11 @@ int32_t bk_quant_rows_launch(uint64_t x, uint64_t w, int32_t K, int32_t B, float
   if (reduce) red = *reduce;
   red.spin_limit = bk_ctx().spin_limit;
   int* st = bk_ctx().d_status;
+  const bool split = layout == BK_Q8_TILE32;
+  if (split) layout = BK_Q8_TILE;
   auto kernel = w ? (layout == BK_Q8_TILE ? quant_rows_kernel<true, BK_Q8_TILE> : layout == BK_Q8_STAGED ? quant_rows_kernel<true, BK_Q8_STAGED> : quant_rows_kernel<true, BK_Q8_BLOCKS>)
                   : (layout == BK_Q8_TILE ? quant_rows_kernel<false, BK_Q8_TILE> : layout == BK_Q8_STAGED ? quant_rows_kernel<false, BK_Q8_STAGED> : quant_rows_kernel<false, BK_Q8_BLOCKS>);
-  BK_CUDA(bk_launch_pdl(kernel, grid, dim3(256), 0, px, pw, K, eps, po, red, st));
+  BK_CUDA(bk_launch_pdl(kernel, grid, dim3(256), 0, px, pw, K, eps, po, red, st, split));
   BK_CHECK_LAUNCH();
   return BK_OK;
 }
