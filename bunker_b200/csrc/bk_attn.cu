@@ -36,12 +36,11 @@ struct AttnParams {
   uint16_t* out;
   uint8_t* out_q8;
   int out_q8_layout;
-  float* scratch;
+  float *part_ml, *part_o;   // partials of all entries: (m, l) pairs, and 256 sums 16-byte aligned
+  unsigned int* counters;    // splits done per (entry, KV head); they reset themselves
   const uint16_t* gate;
   int B, Hq, Hkv, rot_half, max_len, split_len, max_splits, fused;
   int settled;  // cache rows of earlier steps and pos[] are not outputs of the immediately preceding launch
-  int layout_B; // entries the scratch buffer is laid out for (>= B): partials of all entries, then the completion counters,
-                // which must stay where they are from launch to launch (they reset themselves)
   int n_seq;    // > 0: prompt columns.  Entry b of the launch is token b / n_seq of sequence b mod n_seq: it reads that
                 // sequence's cache, and its own K/V row has already been appended (attn_append_kernel)
   float scale;
@@ -119,8 +118,8 @@ __device__ __forceinline__ float warp_sum8(const float (&v)[8]) {
 // L = fma(w_s, l_s, L) and O = fma(w_s, o_s, O) in ascending s; out = (O/L) * sigmoid(gate).
 __device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, float* w_s) {
   const int lane = threadIdx.x & 31;
-  const float* sc_ml = p.scratch + ((size_t)b * p.Hq + h) * p.max_splits * 2;
-  const float* sc_o = p.scratch + (size_t)p.layout_B * p.Hq * p.max_splits * 2 + ((size_t)b * p.Hq + h) * p.max_splits * kHD;
+  const float* sc_ml = p.part_ml + ((size_t)b * p.Hq + h) * p.max_splits * 2;
+  const float* sc_o = p.part_o + ((size_t)b * p.Hq + h) * p.max_splits * kHD;
   float m = -INFINITY;
   for (int s = lane; s < ns; s += 32) {
     float ms = __ldcg(sc_ml + 2 * s);
@@ -433,8 +432,7 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   bk_stamp(p.trace, 6);
 
   // ---- cross-warp sums in warp order, partial out ----
-  float* sc_ml = p.scratch;
-  float* sc_o = p.scratch + (size_t)p.layout_B * p.Hq * p.max_splits * 2;
+  float *sc_ml = p.part_ml, *sc_o = p.part_o;
   for (int idx = tid; idx < G * kHD; idx += kW * 32) {
     const int g = idx >> 8, d = idx & 255;
     float o = o_s[(size_t)g * kHD + d];
@@ -455,7 +453,7 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   __threadfence();
   __syncthreads();
   bk_stamp(p.trace, 7);
-  unsigned int* cnt = reinterpret_cast<unsigned int*>(p.scratch + (size_t)p.layout_B * p.Hq * p.max_splits * (kHD + 2)) + b * p.Hkv + kvh;
+  unsigned int* cnt = p.counters + b * p.Hkv + kvh;
   if (tid == 0) {
     const unsigned int done = atomicAdd(cnt, 1u);
     s_last = (done == (unsigned int)(nsplits - 1));
@@ -561,7 +559,6 @@ int32_t bk_attn_launch(const bkAttnArgs& args, int n_seq, int layout_B) {
   p.out = bk_ptr<uint16_t>(a.out);
   p.out_q8 = bk_ptr<uint8_t>(a.out_q8);
   p.out_q8_layout = a.out_q8_layout;
-  p.scratch = bk_ptr<float>(a.scratch);
   p.gate = bk_ptr<uint16_t>(a.gate);
   p.B = a.B;
   p.Hq = a.Hq;
@@ -575,7 +572,18 @@ int32_t bk_attn_launch(const bkAttnArgs& args, int n_seq, int layout_B) {
   p.trace = bk_trace_slot();
   p.settled = n_seq ? 0 : a.cache_is_settled;
   p.n_seq = n_seq;
-  p.layout_B = layout_B ? layout_B : a.B;
+  {
+    // The scratch buffer: the partials of layout_B entries, then the completion counters, which must stay where they are from launch to
+    // launch.  The sums are read 16 bytes at a time: they lie behind the pairs (8 bytes each) or, where an odd number of
+    // pairs would leave them off the boundary, in front of them.
+    const size_t n = (size_t)(layout_B ? layout_B : a.B) * a.Hq * max_splits;
+    const bool pairs_first = ((a.scratch + n * 8) & 15) == 0;
+    BK_ARG(pairs_first || (a.scratch & 15) == 0, "bkAttnDecode: scratch must be 16-byte aligned");
+    float* base = bk_ptr<float>(a.scratch);
+    p.part_ml = pairs_first ? base : base + n * kHD;
+    p.part_o = pairs_first ? base + n * 2 : base;
+    p.counters = reinterpret_cast<unsigned int*>(base + n * (kHD + 2));
+  }
   if (n_seq) {
     BK_CUDA(bk_launch_pdl(attn_append_kernel, dim3(a.Hkv, a.B), dim3(32), 0, p));
     BK_CHECK_LAUNCH();

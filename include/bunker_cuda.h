@@ -215,8 +215,8 @@ BK_API int32_t bkHeadNormRope(uint64_t in, int32_t in_stride, uint64_t w, uint64
  * qg: bf16 [B][Hq][2*HD] = per head q | gate (q_proj output); k, v: bf16 [B][Hkv*HD] projections.
  * The kernel norms+rotates q and k, appends k,v at row pos[b], attends over rows 0..pos[b],
  * and writes out bf16 [B][Hq*HD] = attention * sigmoid(gate).
- * caches: bf16 [B][Hkv][max_len][HD].  scratch: bkAttnScratchBytes() bytes, zeroed once before its first use
- * (it ends with completion counters that the kernel re-arms itself). */
+ * caches: bf16 [B][Hkv][max_len][HD].  scratch: bkAttnScratchBytes() bytes, 16-byte aligned, zeroed once before its
+ * first use (it ends with completion counters that the kernel re-arms itself). */
 typedef struct bkAttnArgs {
   uint64_t qg, k, v;
   uint64_t q_norm_w, k_norm_w, cos_t, sin_t;

@@ -280,6 +280,38 @@ def test_attn_decode(bk, B, L):
     assert_same_bits(got, want, f"attention B={B} L={L} split_len={split_len}")
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,L,split_len", [(1, 1, 1, 1, 64), (1, 5, 1, 60, 64), (1, 3, 1, 150, 64), (3, 7, 1, 9, 64), (1, 9, 3, 200, 40)])
+def test_attn_decode_odd_number_of_partials(bk, B, Hq, Hkv, L, split_len):
+    """Heads, sequences and splits all odd: the splits' sums start 8 bytes off a 16-byte boundary when they follow the (m, l) pairs."""
+    assert B * Hq * ((L + split_len - 1) // split_len) % 2 == 1
+    cos_t, sin_t = ops.rope_tables(max(L, 64))
+    c = synth.attn_case(B, L, Hq=Hq, Hkv=Hkv)
+    got, Kg, Vg, split_len, W = _run_attn(c, cos_t, sin_t, split_len=split_len)
+    q, Kc, Vc, want = _attn_oracle(c, cos_t, sin_t, split_len, W)
+    assert_same_bits(Kg, Kc, "k cache after append")
+    assert_same_bits(got, want, "attention")
+
+
+@pytest.mark.parametrize("Hq,taken", [(5, True), (4, False)])
+def test_attn_decode_scratch_off_the_boundary(bk, Hq, taken):
+    """A scratch buffer at 8 modulo 16: an odd number of pairs puts the sums on a boundary, an even one is refused."""
+    L, HD = 30, 256
+    cos_t, sin_t = ops.rope_tables(64)
+    c = synth.attn_case(1, L, Hq=Hq, Hkv=1)
+    d = {k: dev(v) for k, v in c.items() if isinstance(v, np.ndarray)}
+    dc, ds, out = dev(cos_t), dev(sin_t), R.DeviceBuffer(Hq * HD * 2)
+    scratch = R.DeviceBuffer.zeros(ops.attn_scratch_bytes(1, Hq, HD, c["max_len"], 64) + 16)
+    run = lambda: ops.attn_decode(qg=d["qg"].ptr, k=d["k"].ptr, v=d["v"].ptr, q_norm_w=d["q_norm_w"].ptr, k_norm_w=d["k_norm_w"].ptr, cos_t=dc.ptr,
+                                  sin_t=ds.ptr, k_cache=d["k_cache"].ptr, v_cache=d["v_cache"].ptr, pos=d["pos"].ptr, out=out.ptr, scratch=scratch.ptr + 8,
+                                  B=1, Hq=Hq, Hkv=1, HD=HD, rot_half=32, max_len=c["max_len"], split_len=64, max_pos=L - 1, scale=1.0 / 16.0, fused_norm_rope=1)
+    if not taken:
+        with pytest.raises(R.BunkerCudaError):
+            run()
+        return
+    run()
+    assert_same_bits(out.download(np.uint16, (1, Hq * HD)), _attn_oracle(c, cos_t, sin_t, 64, ops.attn_plan(L, 1, 1)[1])[3], "attention")
+
+
 def test_attn_decode_ragged_positions_and_plain(bk):
     """Sequences of different lengths in one batch; one head also checked against the plain softmax."""
     B, L = 4, 700
