@@ -664,6 +664,8 @@ int32_t bkGemvQ4K(const bkGemvArgs* args) {
   BK_REQUIRE_INIT();
   BK_ARG(args != nullptr, "bkGemvQ4K: args is null");
   bkGemvArgs a = *args;  // copied before any asynchronous use
+  // the activation image of the dense tile kernel is the library's own hand-off: a caller's buffer read as one would be read past its end
+  BK_ARG(a.prologue != BK_PRO_TILE, "bkGemvQ4K: unknown prologue %d", a.prologue);
   return bk_gemv_launch(a);
 }
 

@@ -331,3 +331,16 @@ def test_gemv_dense_tiles_in_lane_order(bk, B, K, N):
     assert_same_bits(y2.download(np.float32, (B, 32)), want2, "f32 segment")
     ops.gemv(dxq.ptr, K, B, [ops.gemv_seg(dW2.ptr, 32, y2.ptr, R.BK_EPI_SWIGLU, W2=dW2.ptr)], order=R.BK_GEMV_ORDER_LANES)
     assert_same_bits(y2.download(np.uint16, (B, 32)), O.swiglu(want2, want2), "SwiGLU pair")
+
+
+@pytest.mark.parametrize("B", [1, 8, 17, 64])
+@pytest.mark.parametrize("prologue", [4, 5, 6, -1])
+def test_gemv_refuses_internal_prologues(bk, B, prologue):
+    """The prologues that only the library's own launches use are unknown to a caller at every column count (x is as large as the
+    largest of their inputs)."""
+    K, N = 512, 64
+    dW, y, x = dev(synth.q4k_weights(np.random.default_rng(B), N, K)), R.DeviceBuffer.zeros(B * N * 4), R.DeviceBuffer.zeros(K // 64 * 64 * 144)
+    with pytest.raises(R.BunkerCudaError) as e:
+        ops.gemv(x.ptr, K, B, [ops.gemv_seg(dW.ptr, N, y.ptr)], prologue=prologue, norm_w=x.ptr)
+    assert e.value.code == R.BK_ERR_ARG
+    assert R.cuSync() == 0
