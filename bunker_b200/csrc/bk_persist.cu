@@ -16,7 +16,8 @@
 // Hand-off.  There is no grid barrier.  Every activation word carries the generation it belongs to: bf16 values as 32-bit
 // words {value, 16-bit tag}, f32 values as 64-bit words {value, 32-bit tag}.  A producer stores the word; a consumer loads
 // the words it needs (past L1) until their tags match -- one L2 store and one L2 load on the critical path, no fence, no
-// flag.  A buffer is rewritten once per layer; a writer of generation g+1 has, through the chain of phases in between,
+// flag.  A value and its tag are one element of the access on both sides (the elements of a vector access are not ordered among
+// themselves, so a 64-bit word is never read as two of 32 bits).  A buffer is rewritten once per layer; a writer of generation g+1 has, through the chain of phases in between,
 // waited for every reader of generation g (each full-vector input is complete only when all its writers have finished
 // reading the vector before it), so one buffer per activation is enough and a tag can never be skipped or reused early.
 //
@@ -217,7 +218,6 @@ BK_DEVINL bool keep_polling(const Ctl& c, int it) {
 }
 // bits of the upper halves that differ from the tag
 BK_DEVINL uint32_t stale16(const uint4& v, uint32_t th) { return ((v.x ^ th) | (v.y ^ th) | (v.z ^ th) | (v.w ^ th)) & 0xffff0000u; }
-BK_DEVINL uint32_t stale32(const uint4& v, uint32_t tag) { return (v.y ^ tag) | (v.w ^ tag); }
 BK_DEVINL uint32_t wait_word(const uint32_t* p, uint32_t first, uint32_t tag, const Ctl& c) {
   uint32_t w = first;
   for (int it = 0; ((w ^ (tag << 16)) & 0xffff0000u) != 0; it++) {
@@ -1054,13 +1054,15 @@ BK_DEVINL void phase_merge(const StepParams& P, const Phase& ph, uint8_t* scratc
   for (int h = (int)gridDim.x - 1 - (int)blockIdx.x; h < P.Hq; h += gridDim.x) {
 #pragma unroll 1
     for (int s = tid; s < ns; s += kCT) {
-      uint4 v;
+      const unsigned long long* ml = P.pml + ((size_t)h * P.max_splits + s) * 2;
+      uint2 m, l;
       for (int it = 0;; it++) {
-        v = ld_vec(P.pml + ((size_t)h * P.max_splits + s) * 2);
-        if (!stale32(v, tag) || !keep_polling(ctl, it)) break;
+        m = ld_pair(ml);
+        l = ld_pair(ml + 1);
+        if (!((m.y ^ tag) | (l.y ^ tag)) || !keep_polling(ctl, it)) break;
       }
-      m_s[s] = __uint_as_float(v.x);
-      l_s[s] = __uint_as_float(v.z);
+      m_s[s] = __uint_as_float(m.x);
+      l_s[s] = __uint_as_float(l.x);
     }
     consumers_sync();
     float m = -INFINITY;

@@ -383,6 +383,26 @@ def test_persistent_step_shapes(bk, hidden, inter, Hk, Hv, q_heads, kv_heads, vo
     gm.destroy()
 
 
+@pytest.mark.parametrize("q_heads,kv_heads,T,max_len", [(8, 1, 2950, 3008), (6, 2, 2950, 3008), (3, 1, 1500, 20000)])
+def test_persistent_step_long_context(bk, q_heads, kv_heads, T, max_len):
+    """Thousands of cached rows: several attention items per CTA and tens of splits to merge.  The one-launch step gives the bits of
+    the launch chain."""
+    cfg = M.ModelConfig(hidden=256, n_layers=2, vocab=300, gdn_k_heads=1, gdn_v_heads=2, attn_q_heads=q_heads, attn_kv_heads=kv_heads, intermediate=512,
+                        full_attn_interval=2, max_len=max_len)
+    w = M.synth_weights(cfg, seed=T + q_heads)
+    prompt = np.random.default_rng(T).integers(0, cfg.vocab, (T, 1)).astype(np.int32)
+    outs = []
+    for mode in (1, 2):
+        gm = M.DecodeModel(cfg, w, batch=1, step_mode=mode)
+        gm.prefill(prompt)
+        gm.run(12)
+        assert R.cuSync() == 0
+        outs.append((gm.tokens(T - 1, 13), gm.logits()))
+        gm.destroy()
+    assert np.array_equal(outs[0][0], outs[1][0])
+    assert_same_bits(outs[1][1], outs[0][1], "logits")
+
+
 def test_graph_front_end_decodes_like_the_step_graph(bk):
     """A runner.ts-style caller: build the declarative graph, take the static partition, resolve weights and
     double-buffered state through callbacks, rotate the state after every token.  Tokens must equal DecodeModel's and
