@@ -26,8 +26,10 @@
 // weights depend on nothing, so the next phases' rows arrive while the activations of this one are waited for.  It also
 // prefetches the small per-layer data (norm weights, recurrent state, conv taps, cached keys and values) into L2.
 //
-// Every wait is bounded: one that gives up sets the status word and a flag in shared memory, after which no wait of that
-// CTA waits again; the CTA runs through its remaining phases (its words keep their tags, so nobody waits for it) and ends.
+// Every wait -- for words, weights, state slices and free buffers -- is bounded by the same number of polls: one that gives up sets the
+// status word and a flag in shared memory, after which no wait of that CTA waits again.  Its consumers run through the remaining
+// phases on whatever lies in shared memory (its words keep their tags, so nobody waits for it); its producer requests no more,
+// waits until what it has requested has landed, and ends.
 #include <string.h>
 
 #include <vector>
@@ -216,6 +218,12 @@ BK_DEVINL bool keep_polling(const Ctl& c, int it) {
   atomicExch(c.status, BK_ERR_TIMEOUT);
   return false;
 }
+// whether the phase of an mbarrier completed before the wait gave up
+BK_DEVINL bool wait_bar(uint32_t bar, uint32_t parity, const Ctl& c) {
+  for (int it = 0; !mbar_try_wait(bar, parity); it++)
+    if (!keep_polling(c, it)) return false;
+  return true;
+}
 // bits of the upper halves that differ from the tag
 BK_DEVINL uint32_t stale16(const uint4& v, uint32_t th) { return ((v.x ^ th) | (v.y ^ th) | (v.z ^ th) | (v.w ^ th)) & 0xffff0000u; }
 BK_DEVINL uint32_t wait_word(const uint32_t* p, uint32_t first, uint32_t tag, const Ctl& c) {
@@ -281,6 +289,11 @@ BK_DEVINL void group_range(const Share& s, int round, int w, int& g0, int& g1) {
 }
 
 // ---- producer warp --------------------------------------------------------------------
+// copies that have been requested land by themselves; the limit is a last resort
+__device__ __noinline__ void wait_landed(uint32_t bar, uint32_t parity) {
+  for (int it = 0; it < (1 << 22) && !mbar_try_wait(bar, parity); it++) {
+  }
+}
 BK_DEVINL void l2_prefetch(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 BK_DEVINL bool mbar_test(uint32_t bar, uint32_t parity) {
@@ -294,7 +307,11 @@ BK_DEVINL bool mbar_test(uint32_t bar, uint32_t parity) {
 
 // Lane w < kCW serves consumer warp w: it places the group in the FIFO (a prefix sum over the round), waits until the space
 // is free and issues the copies.  Entries are freed in order; the lanes look at 32 entries' barriers at a time.
-__device__ __forceinline__ void producer_warp(const StepParams& P, uint8_t* smem, const SmemLayout& L, const Ctl& ctl, int pos) {
+struct Requested {
+  uint32_t entries, partial;   // entries of whole rounds; bit i: entry `entries` + i of a round that was given up
+  uint32_t slices[2];          // state slices, by slot
+};
+__device__ __forceinline__ void producer_warp(const StepParams& P, uint8_t* smem, const SmemLayout& L, const Ctl& ctl, int pos, Requested& rq) {
   const int lane = threadIdx.x & 31;
   const uint32_t full0 = smem_u32(smem + L.full), empty0 = smem_u32(smem + L.empty), ring0 = smem_u32(smem + L.ring);
   volatile uint32_t* ent = reinterpret_cast<volatile uint32_t*>(smem + L.ent);
@@ -302,11 +319,10 @@ __device__ __forceinline__ void producer_warp(const StepParams& P, uint8_t* smem
   constexpr int kDescVec = (int)(sizeof(Phase) / 16);
   const uint32_t size = P.ring_bytes;
   uint32_t h = 0, A = 0, tail_abs = 0;   // ring position of the head; absolute positions of head and tail
-  uint32_t seq = 0, tail = 0;            // entries issued and freed
+  uint32_t &seq = rq.entries, tail = 0;  // entries issued and freed
   uint32_t end0 = 0, end1 = 0;           // absolute end of the entries e = lane and e = lane + 32 (mod 64)
   const int c = blockIdx.x;
   const uint64_t policy = l2_evict_first();
-  uint32_t n_gdn = 0;   // GDN phases so far
   uint4 next = make_uint4(0, 0, 0, 0);
   if (lane < kDescVec) next = __ldg(reinterpret_cast<const uint4*>(P.phases) + lane);
   for (int k = 0; k < P.n_phases; k++) {
@@ -379,13 +395,12 @@ __device__ __forceinline__ void producer_warp(const StepParams& P, uint8_t* smem
             const uint32_t a0 = __shfl_sync(0xffffffffu, end0, last & 31), a1 = __shfl_sync(0xffffffffu, end1, last & 31);
             tail_abs = last & 32u ? a1 : a0;
             tail += n;
-          } else if (it < (1 << 16)) {
-            mbar_try_wait(empty0 + 8 * (tail % kEnt), (tail / kEnt) & 1u);   // suspends the warp until the oldest entry is free, or a while
           } else {
-            *ctl.dead = 1;
-            if (lane == 0) atomicExch(ctl.status, BK_ERR_TIMEOUT);
-            tail_abs = A;   // go on without waiting: the results are lost anyway
-            tail = seq;
+            mbar_try_wait(empty0 + 8 * (tail % kEnt), (tail / kEnt) & 1u);   // suspends the warp until the oldest entry is free, or a while
+            if (!__all_sync(0xffffffffu, keep_polling(ctl, it))) {
+              rq.partial = __ballot_sync(0xffffffffu, lane < kCW && !todo);
+              return;
+            }
           }
         }
         A += total + pad;
@@ -400,7 +415,10 @@ __device__ __forceinline__ void producer_warp(const StepParams& P, uint8_t* smem
         if (item >= P.Hv * 4) break;
         const int hv = item >> 2, hk = hv / (P.Hv / P.Hk), Cw = (2 * P.Hk + P.Hv) * 128;
         const uint32_t bar = smem_u32(smem + L.gfull) + 8 * i;
-        if (n_gdn > 0) mbar_wait_bounded(smem_u32(smem + L.gfree) + 8 * i, (n_gdn - 1) & 1u, P.status);   // the previous layer's slice has left
+        // the previous layer's slice has left
+        const uint32_t n = i ? rq.slices[1] : rq.slices[0];
+        if (n > 0 && !__all_sync(0xffffffffu, wait_bar(smem_u32(smem + L.gfree) + 8 * i, (n - 1) & 1u, ctl))) return;
+        (i ? rq.slices[1] : rq.slices[0]) = n + 1;
         if (lane == 0) {
           mbar_expect_tx(bar, kGdnBytes);
           asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
@@ -416,7 +434,6 @@ __device__ __forceinline__ void producer_warp(const StepParams& P, uint8_t* smem
           else l2_prefetch(ph.d.conv_w + (size_t)4 * ch + (k3 - 6) * 64);
         }
       }
-      n_gdn++;
     } else if (ph.type == PH_ATTN) {
       const int nsplits = pos / P.split_len + 1;
       if (c < nsplits * P.Hkv) {   // a row block that some CTA will read
@@ -430,7 +447,20 @@ __device__ __forceinline__ void producer_warp(const StepParams& P, uint8_t* smem
       }
     }
     __syncwarp();   // the descriptor has been read by every lane
+    if (__any_sync(0xffffffffu, *ctl.dead)) return;
   }
+}
+// After a wait of this CTA has given up: the copies of the last entries and slices, before the CTA may end.
+__device__ __noinline__ void producer_drain(uint32_t full0, uint32_t gfull0, Requested rq) {
+  const int lane = threadIdx.x & 31;
+  for (uint32_t slot = lane; slot < (uint32_t)kEnt; slot += 32) {
+    const uint32_t i = (slot - rq.entries) % kEnt;   // (kEnt is a power of two)
+    uint32_t n = rq.entries + i + 1;                 // the last entry in this slot, counted from one
+    if (i >= 32 || !((rq.partial >> i) & 1u)) n = n > (uint32_t)kEnt ? n - kEnt : 0;
+    if (n > 0) wait_landed(full0 + 8 * slot, ((n - 1) / kEnt) & 1u);
+  }
+  const uint32_t s = lane == 0 ? rq.slices[0] : lane == 1 ? rq.slices[1] : 0;
+  if (s > 0) wait_landed(gfull0 + 8 * lane, (s - 1) & 1u);
 }
 
 // ---- consumer side ------------------------------------------------------------------------
@@ -790,7 +820,7 @@ BK_DEVINL void phase_gdn(const StepParams& P, const Phase& ph, uint8_t* smem, co
     sm.kn[t] = __fmul_rn(sm.k[t], bk_rcp_sqrt(__fadd_rn(ak, 1e-6f)));
     __syncwarp();
   }
-  mbar_wait_bounded(smem_u32(smem + L.gfull) + 8 * quad, n_gdn & 1u, P.status);
+  wait_bar(smem_u32(smem + L.gfull) + 8 * quad, n_gdn & 1u, ctl);
   float* S = reinterpret_cast<float*>(smem + L.gdn + (size_t)quad * kGdnBytes) + 32 * r * kGdnCols + lane;
   float sd[32];
 #pragma unroll
@@ -1132,7 +1162,9 @@ __global__ void __launch_bounds__(kPT, 1) decode_step_kernel(const __grid_consta
   const uint32_t base = (ep + 1u) * (uint32_t)P.tags;
   __syncthreads();
   if (warp == kCW) {
-    producer_warp(P, smem, L, ctl, pos);
+    Requested rq = {0, 0, {0, 0}};
+    producer_warp(P, smem, L, ctl, pos, rq);
+    if (__any_sync(0xffffffffu, *ctl.dead)) producer_drain(smem_u32(smem + L.full), smem_u32(smem + L.gfull), rq);
     return;
   }
 
@@ -1160,9 +1192,10 @@ __global__ void __launch_bounds__(kPT, 1) decode_step_kernel(const __grid_consta
         const uint32_t e = (entry + r * kCW) % kEnt, parity = ((entry + r * kCW) / kEnt) & 1u;
         int g0, g1;
         group_range(s, r, warp, g0, g1);
-        if (!landed) mbar_wait_bounded(smem_u32(smem + L.full) + 8 * e, parity, P.status);
+        if (!landed) landed = wait_bar(smem_u32(smem + L.full) + 8 * e, parity, ctl);
+        // (a CTA that has given up multiplies whatever lies at the ring's start: its entries may be anybody's)
+        const uint32_t off = landed && !*ctl.dead ? reinterpret_cast<const volatile uint32_t*>(smem + L.ent)[e] : 0u;
         landed = false;
-        const uint32_t off = reinterpret_cast<const volatile uint32_t*>(smem + L.ent)[e];
         group_rows(P, ph, st, smem + L.ring + off, smem_u32(smem + L.empty) + 8 * e, reinterpret_cast<float*>(smem + L.accs) + warp * kGroupMax * kAccPitch,
                                      (s.u0 + g0) * s.upr, (g1 - g0) * s.upr, base, ctl, best_s + warp * kGroupMax);
       }

@@ -126,10 +126,10 @@ def test_full_size_model_256_greedy_steps_match_oracle(bk):
 
 
 def test_persistent_step_barrier_gives_up_cleanly(bk):
-    """The grid barrier of the persistent step kernel with a poll limit of 1: some CTA's first look at the arrival
-    counter comes too early, its barrier gives up, sets the status word and the launch winds down by itself (every
-    other wait ends as soon as it sees the status).  bkSync must report BK_ERR_TIMEOUT and clear it; afterwards, with
-    the limit restored and the state reset, the same model must decode exactly like a fresh one."""
+    """The waits of the persistent step kernel -- for tagged words, weights, state slices and ring space -- with a poll limit of 1: some
+    CTA's look comes too early, the wait gives up, sets the status word, and the launch winds down by itself (no wait of that CTA
+    waits again, its copies land before it ends).  bkSync must report BK_ERR_TIMEOUT and clear it; afterwards, with the limit
+    restored and the state reset, the same model must decode exactly like a fresh one."""
     cfg = M.CONFIG_TINY.with_(max_len=64)
     w = M.synth_weights(cfg, seed=9)
     prompt = np.random.default_rng(2).integers(0, cfg.vocab, (4, 1)).astype(np.int32)
@@ -146,7 +146,7 @@ def test_persistent_step_barrier_gives_up_cleanly(bk):
             rc = R.cuSync()
             assert rc in (0, R.BK_ERR_TIMEOUT)
             seen += rc == R.BK_ERR_TIMEOUT
-        assert seen > 0, "no barrier ran out with a poll limit of 1"
+        assert seen > 0, "no wait ran out with a poll limit of 1"
     finally:
         R._check(lib.bkSetSpinLimit(0))
     assert R.cuSync() == 0
