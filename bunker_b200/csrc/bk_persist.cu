@@ -28,10 +28,11 @@
 //
 // Every wait -- for words, weights, state slices and free buffers -- is bounded by the same number of polls: one that gives up sets the
 // status word and a flag in shared memory, after which no wait of that CTA waits again.  Its consumers run through the remaining
-// phases on whatever lies in shared memory (its words keep their tags, so nobody waits for it); its producer requests no more,
+// phases on whatever lies in shared memory (their words keep their tags, so nobody waits for them); its producer requests no more,
 // waits until what it has requested has landed, and ends.
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 
 #include <cuda.h>   // CUtensorMap
@@ -163,13 +164,12 @@ __host__ __device__ inline SmemLayout smem_layout(uint32_t xs_bytes, uint32_t sc
   L.misc = o; o += 256;                // [0] dead flag, [1] last flag, [8..24) argmax values, [24..40) indices
   L.best = o; o += (size_t)kCW * kGroupMax * 8;   // running argmax of the lm_head rows
   o = (o + 127) & ~(size_t)127;
+  L.ring = o; o += ring_bytes;         // in front of the rest: a CTA that has given up reads up to a group past any offset in it
   L.accs = o; o += (size_t)kCW * kGroupMax * kAccPitch * 4;   // lane sums of a row group, per warp
   L.xs = o; o += xs_bytes;             // both staged activations
   L.scratch = o; o += scratch_bytes;
   o = (o + 127) & ~(size_t)127;
   L.gdn = o; o += gdn_bytes;           // state slices of the CTA's GDN items
-  o = (o + 127) & ~(size_t)127;
-  L.ring = o; o += ring_bytes;
   L.total = o;
   return L;
 }
@@ -1155,6 +1155,7 @@ __global__ void __launch_bounds__(kPT, 1) decode_step_kernel(const __grid_consta
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  if (tid < kEnt) reinterpret_cast<uint32_t*>(smem + L.ent)[tid] = 0u;
   for (int i = tid; i < 2 * kDescVec && i < P.n_phases * kDescVec; i += kPT)
     reinterpret_cast<uint4*>(smem + L.desc)[i] = __ldg(reinterpret_cast<const uint4*>(P.phases) + i);
   const unsigned int ep = *reinterpret_cast<const volatile unsigned int*>(P.epoch);
@@ -1192,10 +1193,9 @@ __global__ void __launch_bounds__(kPT, 1) decode_step_kernel(const __grid_consta
         const uint32_t e = (entry + r * kCW) % kEnt, parity = ((entry + r * kCW) / kEnt) & 1u;
         int g0, g1;
         group_range(s, r, warp, g0, g1);
-        if (!landed) landed = wait_bar(smem_u32(smem + L.full) + 8 * e, parity, ctl);
-        // (a CTA that has given up multiplies whatever lies at the ring's start: its entries may be anybody's)
-        const uint32_t off = landed && !*ctl.dead ? reinterpret_cast<const volatile uint32_t*>(smem + L.ent)[e] : 0u;
+        if (!landed) wait_bar(smem_u32(smem + L.full) + 8 * e, parity, ctl);
         landed = false;
+        const uint32_t off = reinterpret_cast<const volatile uint32_t*>(smem + L.ent)[e];   // (after giving up: of any group, or 0)
         group_rows(P, ph, st, smem + L.ring + off, smem_u32(smem + L.empty) + 8 * e, reinterpret_cast<float*>(smem + L.accs) + warp * kGroupMax * kAccPitch,
                                      (s.u0 + g0) * s.upr, (g1 - g0) * s.upr, base, ctl, best_s + warp * kGroupMax);
       }
@@ -1379,7 +1379,12 @@ int32_t bk_plan_create(uint64_t* out, const BkPlanDims& dims) {
     return BK_OK;   // the caller keeps one launch per op
   }
   pl->ring_bytes = (uint32_t)((limit - fixed) & ~(size_t)127);
-  pl->smem = smem_layout(pl->xs_bytes, pl->scratch_bytes, pl->gdn_bytes, pl->ring_bytes).total;
+  const SmemLayout lay = smem_layout(pl->xs_bytes, pl->scratch_bytes, pl->gdn_bytes, pl->ring_bytes);
+  pl->smem = lay.total;
+  if (lay.total - lay.accs < std::max((size_t)pl->ring_bytes * 3 / 4 / kCW, 2 * widest)) {   // a group (group_max) must fit behind the ring
+    delete pl;
+    return BK_OK;
+  }
   // tagged buffers
   size_t o = 0;
   auto take = [&](size_t bytes) {
