@@ -480,21 +480,48 @@ BK_DEVINL Stage stage_of(uint8_t* base, int K) {
   s.s8s = s.d8s + K / 32;
   return s;
 }
+BK_DEVINL float max_nan(float a, float b) {   // a NaN wins
+  float m;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+  return m;
+}
+// A block with a NaN or an infinity, or of values too small for a finite factor, as bk_q8_1_store has it: a NaN does not count for the
+// maximum and becomes 0.  Out of line: it is hardly ever fetched.
+__device__ __noinline__ uint4 stage8_general(float4 a, float4 c) {
+  const float y[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
+  const unsigned block = 0xfu << (threadIdx.x & 28u);
+  float amax = 0.0f;
+#pragma unroll
+  for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(y[e]));
+  amax = fmaxf(amax, __shfl_xor_sync(block, amax, 1));
+  amax = fmaxf(amax, __shfl_xor_sync(block, amax, 2));
+  const float d = __fdiv_rn(amax, 127.0f), id = (d == 0.0f) ? 1.0f : __fdiv_rn(1.0f, d);
+  uint32_t o[2] = {0u, 0u};
+#pragma unroll
+  for (int e = 0; e < 8; e++) o[e >> 2] |= ((uint32_t)max(-128, min(127, __float2int_rd(fmaf(y[e], id, 0.5f)))) & 0xffu) << (8 * (e & 3));
+  return make_uint4(o[0], o[1], __float_as_uint(d), 0u);
+}
 // Chunk q of eight values -> Q8_1; four neighbouring lanes hold a block.
 BK_DEVINL void stage8(const Stage& st, const float (&y)[8], int q) {
   float amax = 0.0f;
 #pragma unroll
-  for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(y[e]));
-  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-  const float d = __fdiv_rn(amax, 127.0f);
+  for (int e = 0; e < 8; e++) amax = max_nan(amax, fabsf(y[e]));
+  amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+  amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+  float d = __fdiv_rn(amax, 127.0f);
   const float id = (d == 0.0f) ? 1.0f : __fdiv_rn(1.0f, d);
   // floor(y * id + 0.5), |.| <= 127: rounding down to the unit of 1.5 * 2^23 leaves it in the low byte
   uint32_t b[8];
 #pragma unroll
   for (int e = 0; e < 8; e++) b[e] = __float_as_uint(__fadd_rd(fmaf(y[e], id, 0.5f), 12582912.0f));
-  const uint32_t w0 = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
-  const uint32_t w1 = __byte_perm(__byte_perm(b[4], b[5], 0x0040), __byte_perm(b[6], b[7], 0x0040), 0x5410);
+  uint32_t w0 = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+  uint32_t w1 = __byte_perm(__byte_perm(b[4], b[5], 0x0040), __byte_perm(b[6], b[7], 0x0040), 0x5410);
+  if (!(amax < INFINITY && id < INFINITY)) {
+    const uint4 g = stage8_general(make_float4(y[0], y[1], y[2], y[3]), make_float4(y[4], y[5], y[6], y[7]));
+    w0 = g.x;
+    w1 = g.y;
+    d = __uint_as_float(g.z);
+  }
   int qsum = bk_dp4a_ss(w1, 0x01010101u, bk_dp4a_ss(w0, 0x01010101u, 0));
   qsum += __shfl_xor_sync(0xffffffffu, qsum, 1);
   qsum += __shfl_xor_sync(0xffffffffu, qsum, 2);
@@ -1253,7 +1280,7 @@ __global__ void __launch_bounds__(kPT, 1) decode_step_kernel(const __grid_consta
     best_merge(best, ov, oi);
   }
   if (lane == 0) {
-    const int id = best.i == 0x7fffffff ? 0 : best.i;
+    const int id = best.v == -INFINITY ? 0 : best.i;   // nothing above it: token 0, as argmax_kernel has it
     P.io.ids_out[0] = id;
     P.io.val_out[0] = best.v;
     if (P.io.host_out) {   // pinned host memory mapped into the device

@@ -403,6 +403,29 @@ def test_persistent_step_long_context(bk, q_heads, kv_heads, T, max_len):
     assert_same_bits(outs[1][1], outs[0][1], "logits")
 
 
+@pytest.mark.parametrize("name,value", [("model.layers.0.post_attention_layernorm.weight", 0x7fc0), ("model.layers.1.input_layernorm.weight", 0xffc0),
+                                        ("model.layers.0.input_layernorm.weight", 0x7f80), ("final.norm.weight", 0x7fc0), ("final.norm.weight", 0xff80),
+                                        ("final.norm.weight", 0x0001)])
+def test_persistent_step_of_values_that_are_not_finite(bk, name, value):
+    """NaN and infinite activations (from a norm weight) and a weight of the smallest magnitude: the one-launch step quantises them as
+    the launch chain does -- the same tokens and the same logits, NaN where it has NaN."""
+    cfg = M.CONFIG_TINY.with_(max_len=32)
+    w = M.synth_weights(cfg, seed=4)
+    w[name] = w[name].copy()
+    w[name].reshape(-1)[[3, 70, 71]] = value
+    prompt = np.random.default_rng(1).integers(0, cfg.vocab, (5, 1)).astype(np.int32)
+    outs = []
+    for mode in (1, 2):
+        gm = M.DecodeModel(cfg, w, batch=1, step_mode=mode)
+        toks = M.runGraphDecode(gm, prompt, 6)
+        outs.append((toks, gm.logits()))
+        gm.destroy()
+    assert np.array_equal(outs[0][0], outs[1][0])
+    nan = np.isnan(outs[0][1])
+    assert np.array_equal(nan, np.isnan(outs[1][1]))
+    assert_same_bits(np.where(nan, np.float32(0), outs[1][1]), np.where(nan, np.float32(0), outs[0][1]), "logits")
+
+
 def test_graph_front_end_decodes_like_the_step_graph(bk):
     """A runner.ts-style caller: build the declarative graph, take the static partition, resolve weights and
     double-buffered state through callbacks, rotate the state after every token.  Tokens must equal DecodeModel's and
