@@ -188,6 +188,9 @@ struct BkStepIO {
   int32_t hist_ld, hist_rows, vocab_offset;
 };
 int32_t bk_plan_create(uint64_t* out, const BkPlanDims& dims);   // *out = 0 when the shapes do not fit the kernel
+// whether a model goes on with one launch per op after its plan failed with rc: what this device cannot do is an error only to a
+// caller who asked for the persistent step (step mode 2)
+static inline bool bk_plan_optional(int step_mode, int32_t rc) { return step_mode == 0 && rc == BK_ERR_UNSUPPORTED; }
 void bk_plan_add_layer(uint64_t plan, const BkPlanLayer& L);
 int32_t bk_plan_finish(uint64_t plan, uint64_t head, uint64_t final_norm, uint64_t logits, int vocab);
 int32_t bk_plan_launch(uint64_t plan, int parity, const BkStepIO& io);

@@ -163,8 +163,8 @@ bkAttnArgs step_attn_args(Model& m, LayerW& L, bool q8_handoff, int o_layout) {
 }
 
 // The batch-1 single-GPU step as a plan for the persistent kernel (bk_persist.cu): the ops of enqueue_step in the same
-// order.  Leaves m.plan = 0 when a shape does not fit the persistent kernel.
-int32_t build_plan(Model& m) {
+// order.  Leaves m.plan = 0 when a shape does not fit the persistent kernel, and on an error.
+int32_t fill_plan(Model& m) {
   const bkModelConfig& c = m.cfg;
   BkPlanDims D;
   memset(&D, 0, sizeof(D));
@@ -188,6 +188,13 @@ int32_t build_plan(Model& m) {
     bk_plan_add_layer(m.plan, p);
   }
   return bk_plan_finish(m.plan, m.embed, m.final_norm, m.logits, m.vocab_local);
+}
+int32_t build_plan(Model& m) {
+  const int32_t rc = fill_plan(m);
+  if (rc == BK_OK) return BK_OK;
+  if (m.plan) bk_plan_destroy(m.plan);
+  m.plan = 0;
+  return bk_plan_optional(m.step_mode, rc) ? BK_OK : rc;
 }
 
 // token: the step's input, or -1 to take the device's own last one
