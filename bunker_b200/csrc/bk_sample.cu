@@ -9,13 +9,14 @@
 //      total is the token.
 //
 // Selection.  Every candidate is a 64-bit key, unique and totally ordered: the logit's bits made monotonic above the
-// complement of its index.  A cluster of eight CTAs per sequence runs a radix selection over 11-bit digits from the top:
+// complement of its index.  A cluster of one to eight CTAs per sequence runs a radix selection over 11-bit digits from the top:
 // histogram of the digit among the keys that share the prefix chosen so far (shared memory per CTA, added up over
 // distributed shared memory), then the digit in which the top_k-th key lies.  As soon as the keys at or above that
 // prefix fit the candidate list, they are collected, and each finds its rank by counting the larger ones.  Ordinary logits
 // need one digit (two reads of the row, the second from L2); equal or clustered logits take further digits, at most six.
-// What bounds it: two passes over V floats by eight SMs plus four cluster barriers.  Measured at V = 151936,
-// top_k = 40, one sequence: 772 us with top_k rounds of a full scan by one CTA, about 14 us like this.
+// What bounds it: two passes over V floats by the cluster's SMs plus four cluster barriers.  Measured at V = 151936,
+// top_k = 40, one sequence: 774 us with top_k rounds of a full scan by one CTA, 15.6 us like this.  One pick or two are rounds of a
+// full scan all the same (sample_rounds_kernel; bkSample has the rule).
 #include <math.h>
 
 #include "bk_common.cuh"
@@ -32,7 +33,6 @@ BK_DEVINL unsigned long long splitmix64(unsigned long long x) {
   return x ^ (x >> 31);
 }
 
-constexpr int kSampleCtas = 8;       // CTAs of a sequence's cluster (the portable maximum)
 constexpr int kSampleThreads = 1024;
 constexpr int kDigitBits = 11, kBins = 1 << kDigitBits;
 constexpr int kListMax = 2048;       // candidates collected before the ranking
@@ -44,7 +44,12 @@ BK_DEVINL unsigned long long cand_key(float v, int i) {
   u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
   return ((unsigned long long)u << 32) | (uint32_t)~i;
 }
+template <int CTAS>
 BK_DEVINL void cluster_sync() {
+  if (CTAS == 1) {
+    __syncthreads();
+    return;
+  }
   asm volatile("barrier.cluster.arrive;" ::: "memory");
   asm volatile("barrier.cluster.wait;" ::: "memory");
 }
@@ -66,9 +71,124 @@ BK_DEVINL unsigned long long ld_cluster_u64(uint32_t a) {
   return v;
 }
 
-__global__ void __cluster_dims__(kSampleCtas, 1, 1) __launch_bounds__(kSampleThreads)
-    sample_kernel(const float* logits, int V, float temperature, int top_k, float top_p, unsigned long long seed, const int32_t* step_dev,
-                  unsigned int step_add, int32_t* idx_out, float* val_out) {
+struct SampleParams {
+  const float* logits;
+  int V;
+  float temperature;
+  int top_k;
+  float top_p;
+  unsigned long long seed;
+  const int32_t* step_dev;
+  unsigned int step_add;
+  int32_t* idx_out;
+  float* val_out;
+};
+
+// The top_k largest logits of sequence b lie in cv / ci; pr: room for their weights.  By all threads of a CTA.
+BK_DEVINL void pick_token(const SampleParams& p, int b, int top_k, const float* cv, const int* ci, float* pr) {
+  const int tid = threadIdx.x;
+  __syncthreads();
+  if (p.temperature > 0.0f && tid < top_k) pr[tid] = bk_expf(__fmul_rn(__fsub_rn(cv[tid], cv[0]), __fdiv_rn(1.0f, p.temperature)));
+  __syncthreads();
+  if (tid == 0) {
+    int pick = 0;
+    if (top_k <= 0) {
+      p.idx_out[b] = 0;
+      if (p.val_out) p.val_out[b] = -INFINITY;
+      return;
+    }
+    if (p.temperature > 0.0f && top_k > 1) {
+      float total = 0.0f;
+      for (int i = 0; i < top_k; i++) total = __fadd_rn(total, pr[i]);
+      const float need = __fmul_rn(p.top_p, total);
+      int m = top_k;
+      float run = 0.0f;
+      for (int i = 0; i < top_k; i++) {
+        run = __fadd_rn(run, pr[i]);
+        if (run >= need) {
+          m = i + 1;
+          break;
+        }
+      }
+      float prefix_sum = 0.0f;
+      for (int i = 0; i < m; i++) prefix_sum = __fadd_rn(prefix_sum, pr[i]);
+      const unsigned int step = (p.step_dev ? (unsigned int)p.step_dev[b] : 0u) + p.step_add;
+      const unsigned long long h = splitmix64(splitmix64(p.seed ^ ((unsigned long long)step << 20)) + (unsigned long long)b);
+      const float u = __fmul_rn((float)(unsigned int)(h >> 40), 5.9604644775390625e-8f);   // 24 bits -> [0,1)
+      const float target = __fmul_rn(u, prefix_sum);
+      pick = m - 1;
+      run = 0.0f;
+      for (int i = 0; i < m; i++) {
+        run = __fadd_rn(run, pr[i]);
+        if (run > target) {
+          pick = i;
+          break;
+        }
+      }
+    }
+    p.idx_out[b] = ci[pick];
+    if (p.val_out) p.val_out[b] = cv[pick];
+  }
+}
+
+// One pick or two: one CTA per sequence, round r finds the candidate that follows round r-1's (larger logit first, then lower index).
+// A round is one pass over the row in two comparisons a logit.
+BK_DEVINL bool before(float v, int i, float w, int j) { return v > w || (v == w && i < j); }
+BK_DEVINL void warp_first(float& v, int& i) {
+  for (int off = 16; off >= 1; off >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, v, off);
+    const int oi = __shfl_xor_sync(0xffffffffu, i, off);
+    if (before(ov, oi, v, i)) {
+      v = ov;
+      i = oi;
+    }
+  }
+}
+__global__ void __launch_bounds__(kSampleThreads) sample_rounds_kernel(const __grid_constant__ SampleParams p) {
+  __shared__ float sv[32], cv[kSampleMaxK], pr[kSampleMaxK];
+  __shared__ int si[32], ci[kSampleMaxK];
+  bk_pdl_trigger();
+  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, V = p.V;
+  const float* l = p.logits + (size_t)b * V;
+  bk_pdl_wait();
+  float last_v = INFINITY;
+  int last_i = -1, top_k = p.top_k;
+  for (int r = 0; r < top_k; r++) {
+    float v = -INFINITY;
+    int at = 0x7fffffff;
+    for (int i = tid; i < V; i += kSampleThreads) {
+      const float x = __ldcg(l + i);   // (a NaN is before nothing)
+      if (before(x, i, v, at) && before(last_v, last_i, x, i)) {
+        v = x;
+        at = i;
+      }
+    }
+    warp_first(v, at);
+    if (lane == 0) {
+      sv[warp] = v;
+      si[warp] = at;
+    }
+    __syncthreads();
+    v = sv[lane];
+    at = si[lane];
+    warp_first(v, at);
+    __syncthreads();
+    if (at == 0x7fffffff) {   // fewer than top_k logits that are not NaN
+      top_k = r;
+      break;
+    }
+    if (tid == 0) {
+      cv[r] = v;
+      ci[r] = at;
+    }
+    last_v = v;
+    last_i = at;
+  }
+  pick_token(p, b, top_k, cv, ci, pr);
+}
+
+template <int CTAS>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kSampleThreads) sample_kernel(const __grid_constant__ SampleParams p) {
   __shared__ unsigned int hist[kBins];
   __shared__ unsigned long long list[kListMax];
   __shared__ unsigned int n_list;
@@ -78,9 +198,10 @@ __global__ void __cluster_dims__(kSampleCtas, 1, 1) __launch_bounds__(kSampleThr
   __shared__ float cv[kSampleMaxK], pr[kSampleMaxK];
   __shared__ int ci[kSampleMaxK];
   bk_pdl_trigger();
-  const int rank = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const float* l = logits + (size_t)b * V;
-  const int per = ((V + kSampleCtas - 1) / kSampleCtas + 3) & ~3;
+  const int rank = blockIdx.x % CTAS, b = blockIdx.x / CTAS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, V = p.V;
+  int top_k = p.top_k;
+  const float* l = p.logits + (size_t)b * V;
+  const int per = ((V + CTAS - 1) / CTAS + 3) & ~3;
   const int lo = min(V, rank * per), hi = min(V, lo + per);
   if (tid == 0) {
     n_list = 0;
@@ -113,12 +234,12 @@ __global__ void __cluster_dims__(kSampleCtas, 1, 1) __launch_bounds__(kSampleThr
     for_each([&](unsigned long long key) {
       if (key != 0 && (shift == 64 || (key >> shift) == prefix)) atomicAdd(&hist[(unsigned int)(key >> next) & ((1u << bits) - 1u)], 1u);
     });
-    cluster_sync();
+    cluster_sync<CTAS>();
     if (rank == 0) {
       // thread t owns bins kBins-1-2t and kBins-2-2t (largest first); running count from the top
       unsigned int c0 = 0, c1 = 0;
       const int b0 = kBins - 1 - 2 * tid, b1 = b0 - 1;
-      for (int r = 0; r < kSampleCtas; r++) {
+      for (int r = 0; r < CTAS; r++) {
         c0 += ld_cluster_u32(cluster_addr(&hist[b0], r));
         c1 += ld_cluster_u32(cluster_addr(&hist[b1], r));
       }
@@ -144,7 +265,7 @@ __global__ void __cluster_dims__(kSampleCtas, 1, 1) __launch_bounds__(kSampleThr
         s_need = short_ ? need : need - (first ? before : before + c0);
       }
     }
-    cluster_sync();
+    cluster_sync<CTAS>();
     const int decided = 0;
     prefix = ld_cluster_u64(cluster_addr(&s_prefix, decided));
     // keys above this prefix are fewer than top_k, so the list holds what it says if the chosen digit's bin is small
@@ -165,7 +286,7 @@ __global__ void __cluster_dims__(kSampleCtas, 1, 1) __launch_bounds__(kSampleThr
       if (at < (unsigned int)kListMax) asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(list_addr + 8 * at), "l"(key) : "memory");
     }
   });
-  cluster_sync();
+  cluster_sync<CTAS>();
   if (rank != 0) return;
   const int n = min((int)n_list, kListMax);
   for (int i = tid; i < n; i += kSampleThreads) {
@@ -178,48 +299,7 @@ __global__ void __cluster_dims__(kSampleCtas, 1, 1) __launch_bounds__(kSampleThr
     }
   }
   if (n < top_k) top_k = n;   // fewer than top_k logits that are not NaN
-  __syncthreads();
-  if (temperature > 0.0f && tid < top_k) pr[tid] = bk_expf(__fmul_rn(__fsub_rn(cv[tid], cv[0]), __fdiv_rn(1.0f, temperature)));
-  __syncthreads();
-  if (tid == 0) {
-    int pick = 0;
-    if (top_k <= 0) {
-      idx_out[b] = 0;
-      if (val_out) val_out[b] = -INFINITY;
-      return;
-    }
-    if (temperature > 0.0f && top_k > 1) {
-      float total = 0.0f;
-      for (int i = 0; i < top_k; i++) total = __fadd_rn(total, pr[i]);
-      const float need = __fmul_rn(top_p, total);
-      int m = top_k;
-      float run = 0.0f;
-      for (int i = 0; i < top_k; i++) {
-        run = __fadd_rn(run, pr[i]);
-        if (run >= need) {
-          m = i + 1;
-          break;
-        }
-      }
-      float prefix_sum = 0.0f;
-      for (int i = 0; i < m; i++) prefix_sum = __fadd_rn(prefix_sum, pr[i]);
-      const unsigned int step = (step_dev ? (unsigned int)step_dev[b] : 0u) + step_add;
-      const unsigned long long h = splitmix64(splitmix64(seed ^ ((unsigned long long)step << 20)) + (unsigned long long)b);
-      const float u = __fmul_rn((float)(unsigned int)(h >> 40), 5.9604644775390625e-8f);   // 24 bits -> [0,1)
-      const float target = __fmul_rn(u, prefix_sum);
-      pick = m - 1;
-      run = 0.0f;
-      for (int i = 0; i < m; i++) {
-        run = __fadd_rn(run, pr[i]);
-        if (run > target) {
-          pick = i;
-          break;
-        }
-      }
-    }
-    idx_out[b] = ci[pick];
-    if (val_out) val_out[b] = cv[pick];
-  }
+  pick_token(p, b, top_k, cv, ci, pr);
 }
 
 }  // namespace
@@ -230,8 +310,21 @@ extern "C" int32_t bkSample(uint64_t logits, int32_t V, int32_t B, float tempera
   BK_ARG(logits && idx && V > 0 && B > 0, "bkSample: bad arguments");
   BK_ARG(top_k >= 1 && top_k <= kSampleMaxK, "bkSample: top_k=%d outside 1..%d", top_k, kSampleMaxK);
   BK_ARG(temperature >= 0.0f && top_p > 0.0f && top_p <= 1.0f, "bkSample: temperature=%g top_p=%g", (double)temperature, (double)top_p);
-  BK_CUDA(bk_launch_pdl(sample_kernel, dim3(kSampleCtas, B), dim3(kSampleThreads), 0, bk_ptr<float>(logits), V, temperature, top_k, top_p,
-                        (unsigned long long)seed, bk_ptr<int32_t>(step_dev), step_add, bk_ptr<int32_t>(idx), bk_ptr<float>(val)));
+  SampleParams p = {bk_ptr<float>(logits), V, temperature, top_k, top_p, (unsigned long long)seed, bk_ptr<int32_t>(step_dev), step_add, bk_ptr<int32_t>(idx), bk_ptr<float>(val)};
+  // CTAs per sequence: a short row is one CTA's (V 4,096, one sequence: 5 us with one, 7 with eight); a longer one takes as many as still
+  // leave each CTA an SM of its own -- beyond that the clusters wait for one another (V 32,000, top_k 40, 64 sequences: 22 us with one, 15
+  // with two, 23 with four, 39 with eight) -- and eight only where rows are long and sequences few (64,000, one sequence: 12.5 us, with four
+  // 13.6; 151,936: 15.6 and 20.4).
+  const int sms = bk_ctx().sm_count;
+  const int ctas = V <= 8192 ? 1 : V > 40000 && B <= 8 ? 8 : B <= sms / 4 ? 4 : B <= sms / 2 ? 2 : 1;
+  // Rounds of a full pass where the two passes of the selection, or its barriers, cost more: top_k 1 of 64 sequences, V 151,936: 23 us against
+  // 29; of one, V 16,000: 5 against 7 (V 64,000: 11 against 9); top_k 2 of 200, V 151,936: 86 against 90 (top_k 3: 124 against 90).
+  const bool rounds = top_k * ctas <= 2 || (top_k == 1 && V <= 32768);
+  if (rounds) BK_CUDA(bk_launch_pdl(sample_rounds_kernel, dim3(B), dim3(kSampleThreads), 0, p));
+  else if (ctas == 1) BK_CUDA(bk_launch_pdl(sample_kernel<1>, dim3(B), dim3(kSampleThreads), 0, p));
+  else if (ctas == 2) BK_CUDA(bk_launch_pdl(sample_kernel<2>, dim3(2u * B), dim3(kSampleThreads), 0, p));
+  else if (ctas == 4) BK_CUDA(bk_launch_pdl(sample_kernel<4>, dim3(4u * B), dim3(kSampleThreads), 0, p));
+  else BK_CUDA(bk_launch_pdl(sample_kernel<8>, dim3(8u * B), dim3(kSampleThreads), 0, p));
   BK_CHECK_LAUNCH();
   return BK_OK;
 }

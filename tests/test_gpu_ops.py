@@ -525,3 +525,22 @@ def test_sampling_row_lengths_and_clustered_logits(bk, V):
         wi, wv = O.sample(logits, T, k, p, seed, np.zeros(B, np.int32), 0)
         assert np.array_equal(idx.download(np.int32, (B,)), wi), (T, k, p)
         assert_same_bits(val.download(np.float32, (B,)), wv, "sampled logit")
+
+
+@pytest.mark.parametrize("V,B", [(8192, 3), (8193, 3), (40000, 8), (40001, 8), (40001, 9), (33000, 37), (33000, 38), (33000, 75), (32768, 75), (5, 65600)])
+def test_sampling_at_the_edges_of_its_rule(bk, V, B):
+    """Row lengths and sequence counts on both sides of the lines between one, two, four and eight CTAs a sequence and between rounds of
+    a full scan and the radix selection; more sequences than a grid's second dimension holds."""
+    rng = np.random.default_rng(V + B)
+    logits = rng.normal(0, 2, (min(B, 80), V)).astype(np.float32)
+    logits[0, :] = np.where(rng.random(V) < 0.9, np.float32(1.5), logits[0])   # ties decided by the index
+    logits[1, ::2] = np.nan
+    logits[2, 1:] = np.nan
+    n = logits.shape[0]
+    full = np.tile(logits, ((B + n - 1) // n, 1))[:B]
+    dl, idx, val = dev(full), R.DeviceBuffer(B * 4), R.DeviceBuffer(B * 4)
+    for seed, (T, k, p) in enumerate(((1.0, 1, 1.0), (0.8, 2, 1.0), (1.0, 3, 0.9), (0.8, 40, 0.9))):
+        ops.sample(dl.ptr, V, B, idx.ptr, val.ptr, temperature=T, top_k=k, top_p=p, seed=seed)
+        wi, wv = O.sample(full, T, k, p, seed, np.zeros(B, np.int32), 0)
+        assert np.array_equal(idx.download(np.int32, (B,)), wi), (T, k, p)
+        assert_same_bits(val.download(np.float32, (B,)), wv, "sampled logit")
