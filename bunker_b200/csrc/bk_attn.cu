@@ -210,12 +210,14 @@ __device__ __forceinline__ float warp_sum8_swapped(const float (&v)[8]) {
   return __fadd_rn(y, __shfl_xor_sync(0xffffffffu, y, 1));
 }
 
-template <int G>
+template <int G, bool LONG>
 __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams p) {
   // Rows of one warp per register chunk (two chunks are live, the one in use and the next): as many as 128 registers hold
   // without spilling, since the bytes in flight bound the few-head case (8 sequences, 20,000 rows, 4 heads: 4 rows 84 us, 6 rows 78) and
   // the FMAs the many-head one (32,768 rows, 8 heads: 4 rows with 24 bytes spilled 218 us, 3 rows and the head order below 208).
-  constexpr int kCh = G <= 4 ? 6 : G >= 7 ? 3 : 4;
+  // A short split of few heads takes 4 rows all the same: it has 8 to 32 rows a warp, and what a chunk of six holds beyond them is
+  // cleared and tested for nothing (launch_split).
+  constexpr int kCh = G <= 4 ? (LONG ? 6 : 4) : G >= 7 ? 3 : 4;
   bk_pdl_trigger();
   bk_stamp(p.trace, 0);
   extern __shared__ __align__(16) uint8_t smem[];
@@ -469,16 +471,24 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
 
 size_t attn_smem_bytes(int split_len) { return 4096 + 512 + 64 + 256 + (size_t)split_len * 32 + (size_t)kW * 8 * kHD * 4; }
 
-template <int G>
-int32_t launch_split(const AttnParams& p, dim3 grid, size_t smem) {
+template <int G, bool LONG>
+int32_t launch_split_rows(const AttnParams& p, dim3 grid, size_t smem) {
   static size_t configured = 0;
   if (smem > configured) {
-    BK_CUDA(cudaFuncSetAttribute(attn_split_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BK_CUDA(cudaFuncSetAttribute(attn_split_kernel<G, LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = smem;
   }
-  BK_CUDA(bk_launch_pdl(attn_split_kernel<G>, grid, dim3(kW * 32), smem, p));
+  BK_CUDA(bk_launch_pdl(attn_split_kernel<G, LONG>, grid, dim3(kW * 32), smem, p));
   BK_CHECK_LAUNCH();
   return BK_OK;
+}
+// Chunks of six rows from splits of more than 256 rows on.  Two heads per KV head, 2 KV heads, chunks of 4 / 6 rows: splits of 64 rows (1
+// sequence, 1,000 rows) 10.5 / 11.1 us, of 256 (8 sequences, 4,096 rows) 23.2 / 22.8, of 512 (8 sequences, 32,768 rows) 163 / 149.
+template <int G>
+int32_t launch_split(const AttnParams& p, dim3 grid, size_t smem) {
+  if constexpr (G <= 4)
+    if (p.split_len > 256) return launch_split_rows<G, true>(p, grid, smem);
+  return launch_split_rows<G, false>(p, grid, smem);
 }
 
 }  // namespace
