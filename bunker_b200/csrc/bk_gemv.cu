@@ -350,6 +350,21 @@ static const KView* g_view = nullptr;
 
 int32_t bk_gemv_launch(const bkGemvArgs& a) { return bk_gemv_launch_tp(a, nullptr, nullptr, nullptr); }
 
+// Whether the lane-order dense kernel, with the launch that makes its image (2 us), is faster than one launch per 8 columns.  A short K is
+// few steps per tile and row round, so the kernel's fixed part weighs more the more rounds there are.  Measured (groups of 8 / dense, us):
+// 24 columns, K 2048: 4,096 rows 16.0 / 15.4, 9,472 20.2 / 24.9; K 2560: 12,352 rows 34.0 / 28.7; K 256: 1,024 rows 11.1 / 9.3, 12,352 14.5 / 20.8.
+// 32 columns, K 256: 8,192 rows 14.3 / 12.9, 20,480 23.6 / 31.3; K 1024: 12,352 rows 24.4 / 24.7.  40 columns, K 1024: 4,096 rows 19.7 / 16.4, 49,152
+// 76.8 / 84.1; K 2048: 49,152 rows 118.7 / 110.4.  48 columns, K 256: 12,352 rows 28.5 / 24.9, 49,152 62.4 / 74.2.
+static bool dense_blocks_pay(int rows, int K, int B) {
+  switch ((B + 7) / 8) {
+    case 3: return K >= 2560 || rows <= 1024 || (K >= 2048 && rows <= 4096);
+    case 4: return K > 512 || rows <= 8192;
+    case 5: return K > 1024 || rows <= 8192;
+    case 6: return K > 512 || rows <= 16384;
+    default: return true;
+  }
+}
+
 int32_t bk_gemv_launch_tp(const bkGemvArgs& a, const BkPush* push, const BkReduce* reduce, int* ctas_out) {
   BkContext& c = bk_ctx();
   BK_ARG(a.K > 0 && a.K % 256 == 0, "bkGemvQ4K: K=%d is not a positive multiple of 256", a.K);
@@ -358,7 +373,8 @@ int32_t bk_gemv_launch_tp(const bkGemvArgs& a, const BkPush* push, const BkReduc
   // once for all columns.  From 16 columns on it has an f32 order of its own (see there), which order = BK_GEMV_ORDER_LANES
   // declines and AUTO takes for launches of many rows; the rule depends on the shapes only.  In the lane order it takes
   // 17 columns and more of rows in whole boxes of 32: two launches of 8 columns on the mma.sync kernel are as fast at 16 (K 2048,
-  // 12,352 rows: 18 us, here 20), three or four are not (32 columns: 37 us, here 27; 64: 74 us, here 36).
+  // 12,352 rows: 18 us, here 20), three or four are not (32 columns: 37 us, here 27; 64: 74 us, here 36).  A caller's Q8_1 blocks have to be
+  // made into its image first, which few columns of a short K do not pay back (dense_blocks_pay).
   int launch_rows = 0;
   bool whole_boxes = true;
   for (int i = 0; i < a.n_segs && i < 4; i++) {
@@ -367,7 +383,8 @@ int32_t bk_gemv_launch_tp(const bkGemvArgs& a, const BkPush* push, const BkReduc
   }
   const bool dense = a.B > 8 && (a.prologue == BK_PRO_Q8 || a.prologue == BK_PRO_TILE) && !push && !reduce && !g_view;
   const bool tile_order = dense && a.B >= 16 && (a.order == BK_GEMV_ORDER_TILE || (a.order == BK_GEMV_ORDER_AUTO && bk_gemv_auto_tile(launch_rows, a.K)));
-  const bool tile_path = tile_order || (dense && whole_boxes && bk_gemv_dense_lanes(a.B));
+  const bool tile_path = tile_order || (dense && whole_boxes && bk_gemv_dense_lanes(a.B) &&
+                                        (a.prologue == BK_PRO_TILE || dense_blocks_pay(launch_rows, a.K, a.B)));
   BK_ARG(a.prologue != BK_PRO_TILE || tile_path, "bkGemvQ4K: unknown prologue %d", a.prologue);
   if (a.B > 8 && !tile_path) {
     // Everything else of more than 8 columns: groups of 8 on the mma.sync kernel, one launch per group (the weights

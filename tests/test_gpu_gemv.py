@@ -310,7 +310,10 @@ def test_gemv_automatic_order_follows_the_row_count(bk):
 
 @pytest.mark.parametrize("B,K,N", [(9, 256, 32), (16, 768, 2080), (17, 2304, 96), (20, 256, 32), (32, 4096, 2048), (31, 6144, 4128), (33, 256, 160),
                                    (64, 2048, 9216), (48, 6144, 2048), (64, 17408, 64), (24, 17408, 5120),
-                                   (33, 2048, 2272), (64, 768, 2272), (64, 768, 2304)])   # 18 row tiles of more than 32 columns are two column groups, 19 one
+                                   (33, 2048, 2272), (64, 768, 2272), (64, 768, 2304),   # 18 row tiles of more than 32 columns are two column groups, 19 one
+                                   # both sides of the lines between this kernel and one launch per 8 columns (the second segment has 32 rows)
+                                   (24, 2304, 992), (24, 2304, 1024), (24, 2048, 4064), (24, 2048, 4096), (24, 2560, 4096), (25, 512, 8160), (32, 512, 8192),
+                                   (33, 1024, 8160), (40, 1024, 8192), (41, 512, 16352), (48, 512, 16384), (49, 512, 16384)])
 def test_gemv_dense_tiles_in_lane_order(bk, B, K, N):
     """17 and more columns of Q8_1 blocks with rows in whole boxes of 32: the dense tile kernel in the batch <= 8 order (fewer
     columns: the batch <= 8 kernels), for the
