@@ -655,9 +655,6 @@ int32_t bk_gemv_launch_tp(const bkGemvArgs& a, const BkPush* push, const BkReduc
 }
 
 bool bk_gemv_dense_lanes(int B) { return B > 16; }
-// At 64 columns a 128-row tile takes a cluster of four CTAs, so up to 18 tiles leave half of the SMs idle (clusters of eight, which
-// would share the classes too, do not fit sixteen times).  As two groups of 32 columns they take twice as many clusters.
-bool bk_tile_split(int rows, int B) { return B > 32 && (rows + 127) / 128 * 8 <= bk_ctx().sm_count; }
 bool bk_gemv_auto_tile(int rows, int K) { return rows >= g_tile_min_rows || (rows >= g_tile_min_rows_cut && K >= 2048); }
 
 extern "C" {

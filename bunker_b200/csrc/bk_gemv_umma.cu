@@ -36,13 +36,16 @@
 //     -(dmin*accm)); every four superblocks y += yc.
 //
 // A cluster of CTAs shares a tile: the four pairs (LANES), and where there are few tiles also the classes (LANES) or the
-// four-superblock chunks (TILE).  Every CTA sends each value it ends up with to the CTA of the cluster that owns the column
-// (one bulk copy through distributed shared memory per owner); the owner adds them in the fixed order and runs the epilogue.
+// four-superblock chunks (TILE, by any number of CTAs up to eight).  Every CTA sends each value it ends up with to the CTA of the cluster
+// that owns the column (one bulk copy through distributed shared memory per owner; the first 1, 2, 4 or 8 CTAs own columns); the owner adds
+// them in the fixed order and runs the epilogue.
 //
 // Weight feed: tiled TMA loads of 32-row boxes (cp.async.bulk.tensor.2d) where every segment's row count is a multiple of 32; a
 // SwiGLU launch then keeps its 64 gate rows in tile rows 0..63 and their up rows in 64..127.  Other shapes (TILE only)
 // copy row by row.  No multicast.  Every wait is bounded; TMEM is released on every path out of the kernel.
 #include <cuda_fp16.h>
+
+#include <algorithm>
 
 #include "bk_gemv_shared.cuh"
 
@@ -81,7 +84,7 @@ struct UmmaParams {
   int groups;         // column groups (N > 32 columns of few rows: two groups of 32, each with its own image and its own tiles)
   int use_maps;       // weights come by tiled TMA loads through maps[]
   int stages;         // ring stages
-  int csplit;         // LANES: CTAs that share the classes of a pair; TILE: CTAs that share the chunks (= cluster size)
+  int csplit;         // LANES: CTAs that share the classes of a pair; TILE: CTAs that share the chunks (= cluster size, 1 to 8)
   int levels;         // LANES: stack levels in shared memory
   uint32_t xbuf_bytes, stg_bytes;   // received values; values to send (clusters of more than one)
   CUtensorMap maps[10];   // [2i], [2i+1]: headers and quants of segment i (whole superblocks: only [2i]); i = 4: the up matrix
@@ -247,6 +250,7 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
   const int nsb = p.K / 256;
   constexpr int PSPLIT = 4 / PS;
   const int CS = P.csplit * PSPLIT;
+  const int owners = CS >= 8 ? 8 : CS >= 4 ? 4 : CS >= 2 ? 2 : 1;   // CTAs of a cluster that own columns: its size, or the power of two below it
   uint32_t rank;
   asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
 
@@ -265,7 +269,7 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
       mbar_init(smem_u32(d_free + i), kScalers / 32);
     }
     mbar_init(smem_u32(xfull), 1);
-    mbar_init(smem_u32(xempty), CS);
+    mbar_init(smem_u32(xempty), owners);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -281,7 +285,7 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
   const uint32_t tmem_a = tmem + C::kBatches * 128;
 
-  const bool two = LANES && NB == 2 && P.groups == 2;   // tile index: row tile * 2 + column group
+  const bool two = NB == 2 && P.groups == 2;   // tile index: row tile * 2 + column group
   const int n_tiles = (p.total_vrows + kTileM - 1) / kTileM * (two ? 2 : 1);
   const int n_chunks = (nsb + 3) / 4;
   const int tile0 = (int)blockIdx.x / CS, tile_step = (int)gridDim.x / CS;   // the cluster's tiles
@@ -292,7 +296,7 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
   int n_sb = 0;   // superblocks of a tile that this CTA handles, and of all its tiles
   for (int pos = pos0; pos < pos1; pos++) n_sb += LANES ? max(0, (nsb - Walk<LANES>::cls(pos) + 7) / 8) : 1;
   const int total = n_my * n_sb;
-  const int own = N / CS;   // columns of a tile that a CTA of the cluster owns
+  const int own = N / owners;   // columns of a tile that each of the cluster's first CTAs owns
   const bool swiglu_halves = P.use_maps && p.segs[0].epi == BK_EPI_SWIGLU;   // tile rows 0..63 gate, 64..127 up
 
   if (warp < kProducerWarp) {
@@ -399,7 +403,7 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
       };
       const uint32_t xbytes = (uint32_t)((LANES ? 4 * P.csplit : n_chunks) * vs * 4);
       const int b00 = (int)rank * own;
-      for (int k = 0; k < n_my; k++) {
+      for (int k = 0; k < ((int)rank < owners ? n_my : 0); k++) {
         const int vt = tile0 + k * tile_step, tile = two ? vt >> 1 : vt, b0 = b00 + (two ? (vt & 1) * N : 0);
         if (CS > 1 && et == 0) mbar_expect_tx(smem_u32(xfull), xbytes);
         mbar_wait_idle(smem_u32(xfull), (uint32_t)k & 1u, p.status, dead);
@@ -645,7 +649,7 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
       scalers_sync();
       if (CS == 1) {
         if (st == 0) mbar_arrive(smem_u32(xfull));
-      } else if (st < CS && nv > 0) {
+      } else if (st < owners && nv > 0) {
         const uint32_t bytes = (uint32_t)(nv * own * kXPitch * 4), dst = (uint32_t)(first * own * kXPitch * 4);
         bulk_s2cluster(smem_u32(xbuf) + dst, smem_u32(stg) + st * bytes, bytes, smem_u32(xfull), st);
       }
@@ -777,6 +781,91 @@ bool encode_weight_map(CUtensorMap* m, const uint8_t* W, int n_rows, size_t row_
   return bk_encode_map_2d(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, (uint64_t)(uintptr_t)W, row_bytes, (uint64_t)n_rows, row_bytes, box, 32, sw);
 }
 
+// How a launch of `tiles` tiles is cut: CTAs of a cluster that share the classes (or chunks) of a tile.
+struct TilePlan {
+  int csplit, clusters, rounds, len;   // len: superblocks of the longest CTA
+  float cost;                          // superblocks, see plan_tiles
+  uint32_t xbuf_bytes, stg_bytes;
+  int levels, stages;
+  size_t smem;
+};
+constexpr int kMaxCluster = 8;
+int owners_of(int cs) { return cs >= 8 ? 8 : cs >= 4 ? 4 : cs >= 2 ? 2 : 1; }
+
+// clusters of each size that are resident at once (0: that size does not fit)
+template <int NB, bool LANES>
+int32_t resident_clusters(const int** out) {
+  static int clusters[kMaxCluster + 1] = {};
+  BkContext& c = bk_ctx();
+  if (!clusters[1]) {
+    auto kernel = gemv_q4k_umma_kernel<NB, LANES>;
+    const size_t limit = c.smem_optin - 1024;
+    BK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(kUT);
+    cfg.dynamicSmemBytes = limit;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    for (int cs = kMaxCluster; cs >= 1; cs--) {
+      attr[0].val.clusterDim.x = cs;
+      cfg.gridDim = dim3(c.sm_count / cs * cs);
+      if (cudaOccupancyMaxActiveClusters(&clusters[cs], kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        clusters[cs] = 0;
+      }
+    }
+    if (clusters[1] < 1) return bk_fail(BK_ERR_UNSUPPORTED, "tile GEMV: the kernel does not fit the device");
+  }
+  *out = clusters;
+  return BK_OK;
+}
+
+template <int NB, bool LANES>
+int32_t plan_tiles(int tiles, int K, TilePlan* best) {
+  // The cheapest of 1, 2, 4 and 8 parts: the steps of the longest CTA, a tile's exchange and pipeline fill counted as one superblock; with
+  // two stages only, superblocks of one tile after another come half as fast (17 chunks, 48 tiles of 32 columns: 1.8 times, rounds of
+  // one tile hardly at all).  The lane order shares its classes by powers of two; other numbers of parts are taken in the tile order
+  // where they save 30 % (K 5120, 2,048 rows, 32 columns: five parts of one chunk 15.4 us, four of one or two 20.2): by less they are
+  // slower, since fewer CTAs own columns.
+  using C = Cfg<NB, LANES>;
+  constexpr int PSPLIT = 4 / C::PS;
+  constexpr size_t per_stage = C::kStage + C::kColBytes;
+  const size_t limit = bk_ctx().smem_optin - 1024;
+  const int* clusters = nullptr;
+  const int32_t rc = resident_clusters<NB, LANES>(&clusters);
+  if (rc != BK_OK) return rc;
+  const int nsb = K / 256, n_chunks = (nsb + 3) / 4;
+  auto candidate = [&](int s, TilePlan& p) {
+    const int cs = s * PSPLIT, n = clusters[cs], own = C::N / owners_of(cs);
+    p.csplit = s;
+    p.clusters = n;
+    p.levels = LANES && s <= 2 ? 2 - __builtin_ctz(s) : 0;
+    p.xbuf_bytes = (uint32_t)((LANES ? 64 : cs > 1 ? n_chunks * own : C::N) * kXPitch * 4);
+    p.stg_bytes = cs == 1 ? 0 : (uint32_t)((LANES ? 64 : (n_chunks + s - 1) / s * C::N) * kXPitch * 4);
+    const size_t fixed = (size_t)C::kTabs * kTileM * 16 + 3 * C::kColBytes + p.xbuf_bytes + p.stg_bytes + (size_t)p.levels * 32768 + 512;
+    if (n < 1 || fixed + 2 * per_stage > limit) return false;   // (one CTA a tile always fits)
+    p.stages = std::min(kMaxStages, (int)((limit - fixed) / per_stage));
+    p.smem = fixed + (size_t)p.stages * per_stage;
+    p.rounds = (tiles + n - 1) / n;
+    p.len = LANES ? (nsb + 7) / 8 * (8 / s) : 4 * ((n_chunks + s - 1) / s);
+    p.cost = p.rounds * (p.len * (!LANES && p.stages == 2 && p.rounds > 1 ? 1.6f : 1.0f) + 1.0f);
+    return true;
+  };
+  TilePlan p;
+  best->cost = 1e30f;
+  for (int s = 1; s * PSPLIT <= kMaxCluster; s *= 2)
+    if (candidate(s, p) && p.cost < best->cost) *best = p;
+  if (!LANES) {
+    const float pow2 = best->cost;
+    for (int s : {3, 5, 6, 7})
+      if (candidate(s, p) && p.cost < 0.7f * pow2 && p.cost < best->cost) *best = p;
+  }
+  return best->cost < 1e30f ? BK_OK : bk_fail(BK_ERR_UNSUPPORTED, "tile GEMV: K=%d does not fit in shared memory", K);
+}
+
 template <int NB, bool LANES>
 int32_t launch_tile(UmmaParams& P) {
   using C = Cfg<NB, LANES>;
@@ -797,59 +886,30 @@ int32_t launch_tile(UmmaParams& P) {
   BK_ARG(ok || !LANES, "tile GEMV: the lane order needs segments of whole 32-row boxes");
   P.use_maps = ok ? 1 : 0;
 
-  auto kernel = gemv_q4k_umma_kernel<NB, LANES>;
-  static int clusters[4] = {0, 0, 0, 0};   // resident clusters of 1, 2, 4, 8 CTAs
-  const size_t limit = c.smem_optin - 1024;
+  const int tiles = (g.total_vrows + kTileM - 1) / kTileM * P.groups;
+  TilePlan t;
+  const int32_t rc = plan_tiles<NB, LANES>(tiles, g.K, &t);
+  if (rc != BK_OK) return rc;
+  const int cs = t.csplit * (4 / C::PS);
+  P.csplit = t.csplit;
+  P.levels = t.levels;
+  P.xbuf_bytes = t.xbuf_bytes;
+  P.stg_bytes = t.stg_bytes;
+  P.stages = t.stages;
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(kUT);
-  cfg.dynamicSmemBytes = limit;
   cfg.stream = c.stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cs;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  if (!clusters[0]) {
-    BK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
-    for (int i = 3; i >= 0; i--) {
-      attr[0].val.clusterDim.x = 1 << i;
-      cfg.gridDim = dim3((c.sm_count >> i) << i);
-      cfg.numAttrs = 1;
-      BK_CUDA(cudaOccupancyMaxActiveClusters(&clusters[i], kernel, &cfg));
-      if (clusters[i] < 1) return bk_fail(BK_ERR_UNSUPPORTED, "tile GEMV: a cluster of %d does not fit the device", 1 << i);
-    }
-  }
-  // How many CTAs share the classes (or chunks) of a tile: the fewest steps of the longest CTA, a tile's exchange and pipeline
-  // fill counted as one superblock.
-  const int tiles = (g.total_vrows + kTileM - 1) / kTileM * P.groups, nsb = g.K / 256, n_chunks = (nsb + 3) / 4;
-  int best = 1, best_cost = 0x7fffffff;
-  for (int s = 1; s * (4 / C::PS) <= 8; s *= 2) {
-    const int cs = s * (4 / C::PS), n = clusters[__builtin_ctz(cs)];
-    const int rounds = (tiles + n - 1) / n, len = LANES ? (nsb + 7) / 8 * (8 / s) : 4 * ((n_chunks + s - 1) / s);
-    const size_t buf = LANES ? 0 : (size_t)((s > 1 ? n_chunks * (C::N / cs) : C::N) + (s > 1 ? (n_chunks + s - 1) / s * C::N : 0)) * kXPitch * 4;
-    if (buf + (size_t)C::kTabs * kTileM * 16 + 2 * C::kStage + 5 * C::kColBytes + 512 > limit) continue;   // (one CTA a tile always fits)
-    const int cost = rounds * (len + 1);
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = s;
-    }
-  }
-  P.csplit = best;
-  const int cs = best * (4 / C::PS), n = clusters[__builtin_ctz(cs)];
-  P.levels = LANES && best <= 2 ? 2 - __builtin_ctz(best) : 0;
-  P.xbuf_bytes = (uint32_t)((LANES ? 64 : cs > 1 ? n_chunks * (C::N / cs) : C::N) * kXPitch * 4);
-  P.stg_bytes = cs == 1 ? 0 : (uint32_t)((LANES ? 64 : (n_chunks + best - 1) / best * C::N) * kXPitch * 4);
-  const size_t fixed = (size_t)C::kTabs * kTileM * 16 + 3 * C::kColBytes + P.xbuf_bytes + P.stg_bytes + (size_t)P.levels * 32768 + 512;
-  constexpr size_t per_stage = C::kStage + C::kColBytes;
-  BK_ARG(fixed + 2 * per_stage <= limit, "tile GEMV: K=%d does not fit in shared memory", g.K);
-  P.stages = (int)((limit - fixed) / per_stage);
-  if (P.stages > kMaxStages) P.stages = kMaxStages;
-  attr[0].val.clusterDim.x = cs;
-  cfg.gridDim = dim3((tiles < n ? tiles : n) * cs);
-  cfg.dynamicSmemBytes = fixed + (size_t)P.stages * per_stage;
   cfg.numAttrs = 2;
-  BK_CUDA(cudaLaunchKernelEx(&cfg, kernel, P));
+  cfg.gridDim = dim3((tiles < t.clusters ? tiles : t.clusters) * cs);
+  cfg.dynamicSmemBytes = t.smem;
+  BK_CUDA(cudaLaunchKernelEx(&cfg, gemv_q4k_umma_kernel<NB, LANES>, P));
   BK_CHECK_LAUNCH();
   return BK_OK;
 }
@@ -862,7 +922,7 @@ int32_t bk_gemv_umma_launch(void* params, int B, bool lanes) {
   UmmaParams P;
   P.g = *static_cast<GemvParams*>(params);
   P.B = B;
-  const bool split = lanes && bk_tile_split(P.g.total_vrows, B);
+  const bool split = bk_tile_split(P.g.total_vrows, P.g.K, B, lanes);
   P.groups = split ? 2 : 1;
   if (P.g.prologue == BK_PRO_Q8) {
     const size_t need = bk_tile_image_bytes(P.g.K, B);
@@ -883,5 +943,20 @@ int32_t bk_gemv_umma_launch(void* params, int B, bool lanes) {
     P.g.x = c.tile_image;
   }
   if (lanes) return B <= 32 || split ? launch_tile<2, true>(P) : launch_tile<4, true>(P);   // (17 columns and more)
-  return B <= 16 ? launch_tile<1, false>(P) : B <= 32 ? launch_tile<2, false>(P) : launch_tile<4, false>(P);
+  return B <= 16 ? launch_tile<1, false>(P) : B <= 32 || split ? launch_tile<2, false>(P) : launch_tile<4, false>(P);
+}
+
+// Two groups of 32 columns instead of one of 64, each with its own image and tiles.
+// LANES: at 64 columns a tile takes a cluster of four CTAs, so up to 18 tiles leave half of the SMs idle (clusters of eight, which would
+// share the classes too, do not fit sixteen times).  As two groups they take twice as many clusters.
+// TILE: the values that a cluster exchanges grow with columns and K; at 64 columns and K 17,408 no cluster has room for them, and one CTA walks
+// all of K (1,024 rows: 161 us).  A superblock of 64 columns takes 1.7 times one of 32 (K 17,408, 12,352 rows, one CTA a tile: 164 and 96 us).
+bool bk_tile_split(int rows, int K, int B, bool lanes) {
+  if (B <= 32) return false;
+  const int tiles = (rows + kTileM - 1) / kTileM;
+  if (lanes) return tiles * 8 <= bk_ctx().sm_count;
+  TilePlan one, two;
+  if (plan_tiles<4, false>(tiles, K, &one) != BK_OK || plan_tiles<2, false>(2 * tiles, K, &two) != BK_OK) return false;
+  // (where two groups need every SM for a few superblocks they are slower all the same: K 1024, 9,472 rows 17 us, as two groups 18 to 22)
+  return two.cost < 1.65f * one.cost && (2 * tiles * 4 <= 3 * bk_ctx().sm_count || two.len >= 16);
 }

@@ -238,9 +238,13 @@ def test_gemv_linearity_full_size(bk):
 @pytest.mark.parametrize("B,K,N", [(16, 256, 128), (16, 2048, 131), (17, 2048, 300), (31, 4096, 260), (32, 2048, 1000),
                                    (33, 2048, 150), (64, 6144, 200), (32, 17408, 140),
                                    # row counts that are multiples of 32: weights fed by tiled TMA loads
-                                   (16, 1024, 96), (32, 2048, 2080), (24, 768, 4128), (40, 4096, 1056), (32, 6144, 2048)])
+                                   (16, 1024, 96), (32, 2048, 2080), (24, 768, 4128), (40, 4096, 1056), (32, 6144, 2048),
+                                   # clusters that are no power of two: 3, 5, 6 and 7 four-superblock chunks, and 17 over at most 8 CTAs
+                                   (16, 3072, 64), (32, 2304, 640), (17, 5120, 2048), (16, 6144, 300), (64, 7168, 160), (16, 17408, 2048), (20, 17408, 1100),
+                                   # more than 32 columns in two groups where no cluster has room for the exchange, and where one group is faster
+                                   (33, 17408, 96), (64, 17408, 1056), (48, 17408, 70), (64, 2048, 2080), (40, 256, 4096)])
 def test_gemv_dense_tile_path(bk, B, K, N):
-    """16 or more columns of Q8_1 blocks: tcgen05 int8 MMA (one per 32-weight sub-block) with TMEM accumulators.  The
+    """16 or more columns of Q8_1 blocks: tcgen05 f16 MMAs (two per 32-weight sub-block) with TMEM accumulators.  The
     integer block dots are exact; the f32 chain per (row, column) is the tile order of the oracle, so results are
     bit-identical to it -- for plain f32 output, for several segments with different epilogues in one launch, and
     for the SwiGLU pair."""
