@@ -65,12 +65,15 @@ struct Model {
   cudaEvent_t pin_read[2] = {nullptr, nullptr};   // recorded after the step that reads ids slot p
   bool pin_busy[2] = {false, false};
   uint64_t pin_dev = 0;        // device address of pin_ids
+  // the launch chain by conv-state parity
   cudaGraphExec_t graph[2] = {nullptr, nullptr};       // token fed back on the device (embed reads m.ids)
   cudaGraphExec_t graph_host[2] = {nullptr, nullptr};  // token from the host (embed reads the mapped pinned ids)
   unsigned long long graph_kernels = 0;
   // persistent step (batch 1, one GPU): the phases of the plan run as one cooperative launch
   int step_mode = 0;    // 0 = library's choice, 1 = one launch per op, 2 = persistent step kernel
   uint64_t plan = 0;
+  int plan_rows = 0;    // steps at positions below this run the plan, further ones the launch chain
+  cudaGraphExec_t plan_graph[2] = {nullptr, nullptr};
   long long steps = 0;  // steps taken since the last reset (host mirror of pos)
   int conv_cur = 0;     // which of the two conv-state buffers is current (flips with every decode step / prompt pass)
   // buffers of the multi-token prompt path (bkModelPrefill), sized for `cols` = tokens x sequences columns
@@ -212,9 +215,36 @@ int32_t enqueue_step_persist(Model& m, int parity, int token = -1) {
   return bk_plan_launch(m.plan, parity, io);
 }
 
-// enqueue one decode step on the library stream; parity selects the conv-state buffer pair
-int32_t enqueue_step(Model& m, int parity, bool host_tokens = false) {
-  if (m.plan && !g_prof.on) return enqueue_step_persist(m, parity);
+// Positions below this run the persistent step.  Its attention takes an item of a split for one pair of query heads, so its rounds over
+// the SMs read a row once per pair and wait for one another, where the chain's kernel reads a row once; everything else of a layer
+// is faster in one launch.  The chain takes over where the attention layers lose more than all layers gain, in us:
+//   one launch   2 + 2.2 per round + 0.07 per row of a split and round  (splits of 64, 128, 256, 448 rows: 6.8, 10.6, 19.8, 33.6 a round)
+//   chain        9 + 0.054 per row of a split + 0.4 per MB of keys and values
+//   a layer's other launches 6, less 0.018 per MB of weights (5.0 of 24 layers of hidden 2048, 2.1 of 64 of hidden 5120)
+// Measured, chain / one launch: 24 layers, splits of 64 rows: 2,000 rows 752 / 626, 4,000 772 / 710; of 128: 8,000 rows 805 / 813, 16,000 844 / 1,063; of
+// 256: 8,000 rows 855 / 797, 32,000 915 / 1,430.  64 layers: splits of 64, 2,000 rows 4,814 / 4,745, 4,000 4,885 / 5,083.
+int plan_row_limit(const Model& m) {
+  const bkModelConfig& c = m.cfg;
+  const int pairs = (m.Hq / m.Hkv + 1) / 2;
+  int n_full = 0;
+  for (const LayerW& L : m.layers) n_full += L.full;
+  if (n_full == 0) return c.max_len;
+  const double H = c.hidden, linear = ((double)(m.Cw + 2 * m.ZD) + 2 * m.Hv) * H, full = ((double)(m.QG + 2 * m.KVD) + m.Hq * c.head_dim) * H;
+  const double weights = (n_full * full + (c.n_layers - n_full) * linear) / c.n_layers + 3.0 * m.inter * H;   // of a layer
+  const double gain = c.n_layers * std::max(0.0, 6.0 - 0.018 * weights / 256 * 144 / 1e6), split = m.split_len;
+  int rows = 0;
+  for (int round = 1; rows < c.max_len; round++) {
+    const long long end = std::min<long long>(c.max_len, (long long)bk_ctx().sm_count * round / (m.Hkv * pairs) * m.split_len);   // the last row of this round
+    const double per_split = std::min((double)end, split), mb = (double)end * m.KVD * 4 / 1e6;
+    if (n_full * (2.0 + round * (2.2 + 0.07 * per_split) - (9.0 + 0.054 * per_split + 0.4 * mb)) > gain) break;
+    rows = (int)end;
+  }
+  return rows;
+}
+bool on_plan(const Model& m) { return m.plan && m.steps < m.plan_rows; }
+
+// enqueue one decode step as one launch per op; parity selects the conv-state buffer pair
+int32_t enqueue_chain(Model& m, int parity, bool host_tokens = false) {
   const bkModelConfig& c = m.cfg;
   const int B = m.B, H = c.hidden;
   int cur = 0;
@@ -539,13 +569,17 @@ int32_t enqueue_prefill(Model& m, int T) {
   return BK_OK;
 }
 
-int32_t capture(Model& m, int parity, bool host_tokens = false) {
+// enqueue one decode step on the library stream
+int32_t enqueue_step(Model& m, int parity) { return on_plan(m) && !g_prof.on ? enqueue_step_persist(m, parity) : enqueue_chain(m, parity); }
+
+enum StepGraph { SG_PLAN, SG_CHAIN, SG_CHAIN_HOST };
+int32_t capture(Model& m, int parity, StepGraph which) {
   BkContext& c = bk_ctx();
   cudaGraph_t g = nullptr;
   BK_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
   c.capturing = true;
   c.captured = 0;
-  int32_t rc = enqueue_step(m, parity, host_tokens);
+  int32_t rc = which == SG_PLAN ? enqueue_step_persist(m, parity) : enqueue_chain(m, parity, which == SG_CHAIN_HOST);
   c.capturing = false;
   cudaError_t e = cudaStreamEndCapture(c.stream, &g);
   if (rc) {
@@ -553,8 +587,8 @@ int32_t capture(Model& m, int parity, bool host_tokens = false) {
     return rc;
   }
   if (e != cudaSuccess) return bk_fail((int32_t)e, "bkModelFinalize: graph capture -> %s", cudaGetErrorString(e));
-  m.graph_kernels = c.captured;
-  e = cudaGraphInstantiate(host_tokens ? &m.graph_host[parity] : &m.graph[parity], g, 0);
+  if (which != SG_PLAN) m.graph_kernels = c.captured;
+  e = cudaGraphInstantiate(which == SG_PLAN ? &m.plan_graph[parity] : which == SG_CHAIN ? &m.graph[parity] : &m.graph_host[parity], g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) return bk_fail((int32_t)e, "bkModelFinalize: graph instantiate -> %s", cudaGetErrorString(e));
   return BK_OK;
@@ -770,16 +804,18 @@ int32_t bkModelFinalize(uint64_t model) {
   // hand-off inside it costs one L2 store and load, a dependent launch 2 us of completion, flush and wait.
   if (m.step_mode == 2 || (m.step_mode == 0 && B == 1 && m.tp == 1)) TRY(build_plan(m));
   BK_ARG(m.step_mode != 2 || m.plan, "bkModelFinalize: this model's shapes do not fit the persistent step kernel");
+  if (m.plan) m.plan_rows = m.step_mode == 2 ? c.max_len : plan_row_limit(m);
+  const bool chain = m.plan_rows < c.max_len;   // some positions take the launch chain
   // one eager step sets the kernels' shared-memory attributes and validates every pointer, then the
   // state is cleared and the two parity graphs are captured
-  TRY(enqueue_step(m, 0));
+  if (m.plan_rows > 0) TRY(enqueue_step_persist(m, 0));
+  if (chain) TRY(enqueue_chain(m, 0));
   BK_CUDA(cudaStreamSynchronize(bk_ctx().stream));
   TRY(reset_state(m));
-  TRY(capture(m, 0));
-  TRY(capture(m, 1));
-  if (m.tp == 1 && !m.plan) {
-    TRY(capture(m, 0, true));
-    TRY(capture(m, 1, true));
+  for (int parity = 0; parity < 2; parity++) {
+    if (m.plan_rows > 0) TRY(capture(m, parity, SG_PLAN));
+    if (chain) TRY(capture(m, parity, SG_CHAIN));
+    if (chain && m.tp == 1) TRY(capture(m, parity, SG_CHAIN_HOST));
   }
   BK_CUDA(cudaStreamSynchronize(bk_ctx().stream));
   m.finalized = true;
@@ -800,7 +836,7 @@ int32_t bkModelInfo(uint64_t model, int32_t* split_len, int32_t* attn_warps, int
   Model& m = *as_model(model);
   if (split_len) *split_len = m.split_len;
   if (attn_warps) *attn_warps = 8;
-  if (kernels_per_step) *kernels_per_step = (int32_t)m.graph_kernels;
+  if (kernels_per_step) *kernels_per_step = on_plan(m) ? 1 : (int32_t)m.graph_kernels;   // at the current position
   if (steps) *steps = m.steps;
   return BK_OK;
 }
@@ -808,8 +844,9 @@ int32_t bkModelInfo(uint64_t model, int32_t* split_len, int32_t* attn_warps, int
 static int32_t launch_step(Model& m, bool host_tokens = false) {
   BkContext& c = bk_ctx();
   BK_ARG(m.steps < m.cfg.max_len, "bkDecodeStep: position %lld reached max_len=%d", m.steps, m.cfg.max_len);
-  BK_CUDA(cudaGraphLaunch((host_tokens && m.graph_host[m.conv_cur]) ? m.graph_host[m.conv_cur] : m.graph[m.conv_cur], c.stream));
-  c.launches += m.graph_kernels;
+  const bool plan = on_plan(m);
+  BK_CUDA(cudaGraphLaunch(plan ? m.plan_graph[m.conv_cur] : (host_tokens && m.graph_host[m.conv_cur]) ? m.graph_host[m.conv_cur] : m.graph[m.conv_cur], c.stream));
+  c.launches += plan ? 1 : m.graph_kernels;
   m.steps++;
   m.conv_cur ^= 1;
   return BK_OK;
@@ -824,7 +861,7 @@ int32_t bkDecodeStep(uint64_t model, const int32_t* tokens, int32_t* out_ids, fl
   const int B = m.B;
   const bool mapped_io = m.tp == 1;
   int32_t* const out_slot = m.pin_ids + 2 * B;   // ids out, then vals
-  if (tokens && m.plan) {
+  if (tokens && on_plan(m)) {
     // The token travels in the launch's parameters: read from mapped host memory by all 148 CTAs it costs 18 us.
     BK_ARG(tokens[0] >= 0 && tokens[0] < m.cfg.vocab, "bkDecodeStep: token %d outside the vocabulary", tokens[0]);
     BK_ARG(m.steps < m.cfg.max_len, "bkDecodeStep: position %lld reached max_len=%d", m.steps, m.cfg.max_len);
@@ -978,6 +1015,7 @@ int32_t bkModelDestroy(uint64_t model) {
   for (int i = 0; i < 2; i++) {
     if (m->graph[i]) cudaGraphExecDestroy(m->graph[i]);
     if (m->graph_host[i]) cudaGraphExecDestroy(m->graph_host[i]);
+    if (m->plan_graph[i]) cudaGraphExecDestroy(m->plan_graph[i]);
     if (m->pin_read[i]) cudaEventDestroy(m->pin_read[i]);
   }
   for (uint64_t p : m->owned) cudaFree(bk_ptr<void>(p));

@@ -298,7 +298,7 @@ BK_API int32_t bkModelSetTensor(uint64_t model, const char* name, uint64_t dev_p
  * bunker_b200/model.py `shard_weights`. */
 BK_API int32_t bkModelSetComm(uint64_t model, uint64_t comm);
 /* How the decode step is issued (before bkModelFinalize).  0: the library's choice (mode 2 for one sequence on one GPU where
- * the shapes fit it, else mode 1); 1: one launch per op, the shape of the reference's loop (src/runner.ts:146-149), chained
+ * the shapes fit it and as long as the context is short enough for it, else mode 1); 1: one launch per op, the shape of the reference's loop (src/runner.ts:146-149), chained
  * with programmatic dependent launch; 2: the persistent step kernel -- one cooperative launch per token that runs the ops as
  * phases handing their results to one another on the device (batch 1 on one GPU only; bkModelFinalize fails if the model's
  * shapes do not fit it).  All modes give the same bits. */

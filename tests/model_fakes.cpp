@@ -1,5 +1,6 @@
 // Host-only program around bk_model.cu: the CUDA runtime and the library's other translation units are fakes that record what the
-// model asks for.  Usage: model_fakes STEP_MODE PLAN_RC  -- the result of finishing the step plan; prints "key value" lines.
+// model asks for.  Usage: model_fakes STEP_MODE PLAN_RC [MAX_LEN STEPS]  -- the result of finishing the step plan, and a longer cache with
+// steps taken one by one; prints "key value" lines.
 #include <stdarg.h>
 #include <stdlib.h>
 #include <string.h>
@@ -11,6 +12,8 @@
 
 static BkContext g_ctx_fake;
 static int g_plan_rc, g_plans, g_plan_launches, g_gemvs, g_graphs, g_graph_launches;
+static int g_plan_graphs, g_plan_steps, g_captured_from;   // a graph that holds a plan launch, launches of one
+static std::map<cudaGraphExec_t, bool> g_is_plan;
 static uint64_t g_next = 1 << 20;
 static char g_err[256];
 
@@ -75,12 +78,16 @@ cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "fake"; }
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaSuccess; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return g_captured_from = g_plan_launches, cudaSuccess; }
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) { *g = (cudaGraph_t)1; return cudaSuccess; }
 cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
-cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) { *e = (cudaGraphExec_t)(uintptr_t)(++g_graphs); return cudaSuccess; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) {
+  *e = (cudaGraphExec_t)(uintptr_t)(++g_graphs);
+  g_plan_graphs += g_is_plan[*e] = g_plan_launches > g_captured_from;
+  return cudaSuccess;
+}
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return g_graph_launches++, cudaSuccess; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t) { return g_graph_launches++, g_plan_steps += g_is_plan[e], cudaSuccess; }
 }
 
 int main(int argc, char** argv) {
@@ -91,7 +98,7 @@ int main(int argc, char** argv) {
   bkModelConfig c;
   memset(&c, 0, sizeof(c));
   c.hidden = 256; c.n_layers = 2; c.full_attn_interval = 2; c.vocab = 300; c.gdn_k_heads = 1; c.gdn_v_heads = 2; c.attn_q_heads = 2; c.attn_kv_heads = 1;
-  c.head_dim = 256; c.rot_dim = 64; c.intermediate = 512; c.max_len = 64; c.batch = 1; c.tp_size = 1; c.eps = 1e-6f; c.rope_theta = 1e7;
+  c.head_dim = 256; c.rot_dim = 64; c.intermediate = 512; c.max_len = argc > 3 ? atoi(argv[3]) : 64; c.batch = 1; c.tp_size = 1; c.eps = 1e-6f; c.rope_theta = 1e7;
   uint64_t m = 0;
   if (bkModelCreate(&c, &m) != BK_OK) return 3;
   auto q4k = [](uint64_t n, uint64_t k) { return n * (k / 256) * 144; };
@@ -117,6 +124,21 @@ int main(int argc, char** argv) {
   int32_t tok = 5, id = 0;
   const int step = bkDecodeStep(m, &tok, &id, nullptr), eager = bkDecodeStepEager(m);
   printf("step %d\neager %d\ngraphs %d\ngraph_launches %d\nplan_launches %d\ngemvs %d\n", step, eager, g_graphs, g_graph_launches, g_plan_launches, g_gemvs);
+  if (argc > 4) {
+    bkModelReset(m);
+    g_graph_launches = g_plan_steps = g_plan_launches = 0;
+    int first_chain = -1, back = 0;   // the first position off the plan; positions that went back to it
+    for (int i = 0; i < atoi(argv[4]); i++) {
+      const int before = g_plan_steps + g_plan_launches;
+      if ((i & 1 ? bkDecodeStep(m, &tok, nullptr, nullptr) : bkDecodeRun(m, 1)) != BK_OK) return 6;
+      const bool plan = g_plan_steps + g_plan_launches > before;
+      if (!plan && first_chain < 0) first_chain = i;
+      back += plan && first_chain >= 0;
+    }
+    int32_t kernels = 0;
+    bkModelInfo(m, nullptr, nullptr, &kernels, nullptr);
+    printf("plan_graphs %d\nfirst_chain %d\nback %d\n", g_plan_graphs, first_chain, back);
+  }
   bkModelDestroy(m);
   printf("plans_left %d\n", g_plans);
   return 0;

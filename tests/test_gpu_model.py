@@ -403,6 +403,32 @@ def test_persistent_step_long_context(bk, q_heads, kv_heads, T, max_len):
     assert_same_bits(outs[1][1], outs[0][1], "logits")
 
 
+def test_step_crosses_from_one_launch_to_the_chain(bk):
+    """Eight query heads on one KV head of a model of two layers: from 7,104 cached rows on the launch chain is faster and the library's own
+    choice changes over.  Tokens fed back on the device and by the host, logits as with one launch per op throughout."""
+    cfg = M.ModelConfig(hidden=256, n_layers=2, vocab=300, gdn_k_heads=1, gdn_v_heads=2, attn_q_heads=8, attn_kv_heads=1, intermediate=512,
+                        full_attn_interval=2, max_len=7200)
+    w = M.synth_weights(cfg, seed=12)
+    prompt = np.random.default_rng(3).integers(0, cfg.vocab, (7098, 1)).astype(np.int32)
+    outs, kernels = [], []
+    for mode in (0, 1):
+        gm = M.DecodeModel(cfg, w, batch=1, step_mode=mode)
+        ids, _ = gm.prefill(prompt)
+        for i in range(12):
+            if mode == 0:
+                kernels.append(gm.info()["kernels_per_step"])
+            if i % 2:
+                ids, _ = gm.step(ids)
+            else:
+                gm.run(1)
+                ids = gm.tokens(len(prompt) + i, 1)[0]
+        outs.append((gm.tokens(len(prompt) - 1, 13), gm.logits()))
+        gm.destroy()
+    assert kernels[:6] == [1] * 6 and min(kernels[6:]) > 10
+    assert np.array_equal(outs[0][0], outs[1][0])
+    assert_same_bits(outs[0][1], outs[1][1], "logits")
+
+
 @pytest.mark.parametrize("name,value", [("model.layers.0.post_attention_layernorm.weight", 0x7fc0), ("model.layers.1.input_layernorm.weight", 0xffc0),
                                         ("model.layers.0.input_layernorm.weight", 0x7f80), ("final.norm.weight", 0x7fc0), ("final.norm.weight", 0xff80),
                                         ("final.norm.weight", 0x0001)])

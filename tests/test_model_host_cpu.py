@@ -47,3 +47,18 @@ def test_automatic_mode_goes_on_with_the_launch_chain(program):
 def test_other_failures_of_the_plan_are_reported(program, mode, rc):
     r = program(mode, rc)
     assert r["finalize"] == rc and r["plans"] == 0
+
+
+def test_long_contexts_leave_the_one_launch_step(program):
+    """One pair of query heads on one KV head and splits of 64 rows: a round of attention items is 148 * 64 = 9,472 rows and costs 6.68 us, the
+    chain's kernel 12.46 us and 0.4 us per MB (3.88 a round), the other launches of two small layers 11.97 us: eight rounds pay, the ninth does not."""
+    r = program(0, OK, 80000, 76000)
+    assert r["finalize"] == OK and r["graphs"] == 6 and r["plan_graphs"] == 2
+    assert r["first_chain"] == 8 * 9472 and r["back"] == 0
+
+
+@pytest.mark.parametrize("mode,max_len", [(0, 9000), (2, 80000)])
+def test_one_launch_step_at_every_position(program, mode, max_len):
+    """A cache that ends within the rule, and a caller who asked for the one-launch step: no graph of the chain is captured."""
+    r = program(mode, OK, max_len, min(max_len, 79000))
+    assert r["finalize"] == OK and r["graphs"] == r["plan_graphs"] == 2 and r["first_chain"] == -1
