@@ -442,13 +442,14 @@ int32_t bk_gemv_launch_tp(const bkGemvArgs& a, const BkPush* push, const BkReduc
       const size_t need = (size_t)((vr + 15) / 16) * 16384;
       if (c.gemv_carry_bytes < need) {
         if (c.capturing) return bk_fail(BK_ERR_STATE, "bkGemvQ4K: the split-K scratch must be sized by an eager launch before a capture");
-        if (c.gemv_carry) cudaFree(c.gemv_carry);
-        c.gemv_carry = nullptr;
-        c.gemv_carry_bytes = 0;
+        // The step graphs of models keep the address of the buffer they were captured with, so an outgrown one lives on until bkShutdown; at
+        // least doubling it keeps all of them together below twice the last.
+        const size_t size = need > 2 * c.gemv_carry_bytes ? need : 2 * c.gemv_carry_bytes;
         void* q = nullptr;
-        BK_CUDA(cudaMalloc(&q, need));
+        BK_CUDA(cudaMalloc(&q, size));
+        if (c.gemv_carry) c.outgrown.push_back(c.gemv_carry);
         c.gemv_carry = static_cast<float*>(q);
-        c.gemv_carry_bytes = need;
+        c.gemv_carry_bytes = size;
       }
       for (int s0 = 0, i = 0; s0 < nsb; s0 += per, i++) {
         const int s1 = s0 + per < nsb ? s0 + per : nsb;

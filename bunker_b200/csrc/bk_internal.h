@@ -5,6 +5,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <vector>
+
 #include "../../include/bunker_cuda_diag.h"
 
 struct BkContext {
@@ -34,6 +36,7 @@ struct BkContext {
   size_t gdn_ws_bytes = 0;
   float* gemv_carry = nullptr;       // class accumulators handed from one K part of a split GEMV to the next
   size_t gemv_carry_bytes = 0;
+  std::vector<void*> outgrown;       // earlier, smaller ones: captured graphs may still write to them
   char err[512] = {0};
 };
 

@@ -87,6 +87,11 @@ int32_t bkShutdown(void) {
   cudaFree(g_ctx.d_status);
   cudaFree(g_ctx.tile_image);
   cudaFree(g_ctx.gdn_ws);
+  cudaFree(g_ctx.gemv_carry);
+  for (void* p : g_ctx.outgrown) cudaFree(p);
+  g_ctx.outgrown.clear();
+  g_ctx.gemv_carry = nullptr;
+  g_ctx.gemv_carry_bytes = 0;
   g_ctx.d_status = nullptr;
   g_ctx.tile_image = nullptr;
   g_ctx.tile_image_bytes = 0;

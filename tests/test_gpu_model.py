@@ -3,6 +3,7 @@ import numpy as np
 import pytest
 
 from bunker_b200 import model as M
+from bunker_b200 import ops
 from bunker_b200 import runtime as R
 from oracle.model_oracle import OracleModel
 from tests.util import assert_same_bits
@@ -450,6 +451,34 @@ def test_persistent_step_of_values_that_are_not_finite(bk, name, value):
     nan = np.isnan(outs[0][1])
     assert np.array_equal(nan, np.isnan(outs[1][1]))
     assert_same_bits(np.where(nan, np.float32(0), outs[1][1]), np.where(nan, np.float32(0), outs[0][1]), "logits")
+
+
+def test_scratch_of_a_cut_projection_outlives_a_larger_launch(bk):
+    """An FFN of 17,408 columns is cut along K for 2 to 8 sequences, and the class sums between its parts lie in a buffer of the library whose
+    address the model's step graphs hold.  A launch of more rows that outgrows the buffer must leave it to them."""
+    cfg = M.ModelConfig(hidden=256, n_layers=1, vocab=128, gdn_k_heads=1, gdn_v_heads=2, attn_q_heads=1, attn_kv_heads=1, intermediate=17408,
+                        full_attn_interval=2, max_len=32)
+    prompt = np.random.default_rng(5).integers(0, cfg.vocab, (3, 4)).astype(np.int32)
+    gm = M.DecodeModel(cfg, M.synth_weights(cfg, seed=5), batch=4)
+    want = M.runGraphDecode(gm, prompt, 8)
+    logits = gm.logits()
+    K, B = 17408, 4
+    sizes = (2048, 8192, 30000)   # rows, each more than the buffer holds
+    for N in sizes:
+        W, xq, y = R.DeviceBuffer.zeros(N * K // 256 * 144), R.DeviceBuffer.zeros(B * K // 32 * 36), R.DeviceBuffer(B * N * 4)
+        ops.gemv(xq.ptr, K, B, [ops.gemv_seg(W.ptr, N, y.ptr)])
+        assert R.cuSync() == 0
+        assert not y.download(np.float32, (B, N)).any()
+        # memory that was given back would be handed out again here
+        filler = [R.DeviceBuffer.zeros(1 << 20) for _ in range(8)]
+        gm.reset()
+        assert np.array_equal(M.runGraphDecode(gm, prompt, 8), want)
+        assert_same_bits(gm.logits(), logits, "logits")
+        for f in filler:
+            assert not f.download(np.uint8, (1 << 20,)).any()
+            f.free()
+        W.free(), xq.free(), y.free()
+    gm.destroy()
 
 
 def test_graph_front_end_decodes_like_the_step_graph(bk):
