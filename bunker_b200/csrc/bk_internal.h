@@ -188,7 +188,7 @@ struct BkStepIO {
   uint64_t embed, ids_in, x0;
   uint64_t ids_out, val_out, pos, hist, host_out;        // as bk_argmax_launch
   int32_t token;                                         // the input token, or -1: ids_in has it
-  int32_t hist_ld, hist_rows, vocab_offset;
+  int32_t hist_ld, hist_rows;
 };
 int32_t bk_plan_create(uint64_t* out, const BkPlanDims& dims);   // *out = 0 when the shapes do not fit the kernel
 // whether a model goes on with one launch per op after its plan failed with rc: what this device cannot do is an error only to a

@@ -211,7 +211,7 @@ int32_t enqueue_step_persist(Model& m, int parity, int token = -1) {
   io.x0 = m.x[0];
   io.ids_out = m.ids; io.val_out = m.val; io.pos = m.pos; io.hist = m.hist;
   io.host_out = m.pin_dev ? m.pin_dev + (uint64_t)2 * 4 : 0;
-  io.hist_ld = 1; io.hist_rows = c.max_len; io.vocab_offset = 0;
+  io.hist_ld = 1; io.hist_rows = c.max_len;
   return bk_plan_launch(m.plan, parity, io);
 }
 

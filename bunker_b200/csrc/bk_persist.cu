@@ -44,6 +44,7 @@ namespace {
 constexpr int kCW = 8;                // consumer warps: with the producer 288 threads, 168 registers each without a spill (16 warps spill)
 constexpr int kBlock = 4;             // rows multiplied together
 constexpr int kCT = kCW * 32;
+static_assert(kCT == 256, "norms and embedded rows are in the 256-thread order");
 constexpr int kPT = kCT + 32;         // and the producer warp
 constexpr int kEnt = 64;              // ring entries (row groups requested and not yet freed), eight per consumer warp
 constexpr int kGroupMax = 128 / kCW;  // rows of a group
@@ -124,7 +125,7 @@ struct StepIO {
   int32_t* hist;
   int hist_ld, hist_rows;
   int32_t* host_out;
-  int vocab_offset, H;
+  int H;
 };
 
 struct StepParams {
@@ -559,7 +560,7 @@ BK_DEVINL uint4 embed_chunk(const uint8_t* row, int q) {
 BK_DEVINL void embed_row(const StepIO& io, uint8_t* xrow, uint32_t tag) {
   const int id = io.token >= 0 ? io.token : io.ids_in[0];
   const uint8_t* row = io.embed + (size_t)id * (io.H / 256) * 144;
-  for (int q = threadIdx.x; q < io.H / 8 && threadIdx.x < 256; q += 256) {
+  for (int q = threadIdx.x; q < io.H / 8; q += kCT) {
     const uint4 v = embed_chunk(row, q);
     reinterpret_cast<uint4*>(xrow)[q] = v;
     if (blockIdx.x == 0) {
@@ -579,14 +580,13 @@ BK_DEVINL void stage_activation(const StepParams& P, const Phase& ph, const Stag
   const uint4* nw = static_cast<const uint4*>(ph.norm_w);
   const uint32_t* in = static_cast<const uint32_t*>(ph.in);
   const uint32_t th = (base + ph.in_tag) << 16;
-  const int step = norm ? 256 : kCT;   // threads that take part
-  if (!embed && tid < step && (tid & ~31) < nchunk) sentinel16(in + (size_t)(tid & ~31) * 8, th, ctl);
+  if (!embed && (tid & ~31) < nchunk) sentinel16(in + (size_t)(tid & ~31) * 8, th, ctl);
   uint4 wv = make_uint4(0, 0, 0, 0);
-  if (norm && tid < step && tid < nchunk) wv = ld_early(nw + tid);
+  if (norm && tid < nchunk) wv = ld_early(nw + tid);
   float rstd = 1.0f, acc = 0.0f;
-  if (norm && tid < 256) {
+  if (norm) {
 #pragma unroll 1
-    for (int q = tid; q < nchunk; q += 256) {   // whole warps: nchunk is a multiple of 32
+    for (int q = tid; q < nchunk; q += kCT) {   // whole warps: nchunk is a multiple of 32
       uint4 v;
       if (!embed) {
         uint4 a, b;
@@ -618,7 +618,7 @@ BK_DEVINL void stage_activation(const StepParams& P, const Phase& ph, const Stag
     b = ld_vec(in + (size_t)tid * 8 + 4);
   }
 #pragma unroll 1
-  for (int q = tid < step ? tid : nchunk; q < nchunk; q += step) {
+  for (int q = tid; q < nchunk; q += kCT) {
     float y[8];
     if (norm) {
       if (q != tid) wv = __ldg(nw + q);
@@ -744,7 +744,7 @@ BK_DEVINL void group_rows(const StepParams& P, const Phase& ph, const Stage& st,
   if (mine) {
     if (epi == OUT_LOGITS) {
       static_cast<float*>(out)[n] = y;
-      best_merge(best[ri], y, P.io.vocab_offset + n);
+      best_merge(best[ri], y, n);
     } else if (epi == OUT_T32) {
       st_t32(static_cast<unsigned long long*>(out) + n, y, tag);
     } else if (!(swiglu && (ri & 1))) {
@@ -1611,7 +1611,6 @@ int32_t bk_plan_launch(uint64_t plan, int parity, const BkStepIO& io) {
   P.io.hist_ld = io.hist_ld;
   P.io.hist_rows = io.hist_rows;
   P.io.host_out = bk_ptr<int32_t>(io.host_out);
-  P.io.vocab_offset = io.vocab_offset;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(pl->grid);
   cfg.blockDim = dim3(kPT);
