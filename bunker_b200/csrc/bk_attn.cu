@@ -11,7 +11,7 @@
 // Per split: scores for all rows (each K row is read once for the G query heads of
 // the group), exact max, p = exp(s-m), then o = sum p*V with each V row read once.
 // The CTA that finishes a (batch, KV head) last merges its splits and applies the sigmoid output gate.
-// Orders are fixed (see the CPU checker): lane l owns dims [8l,8l+8); row jj of a
+// Orders are fixed (see the CPU oracle): lane l owns dims [8l,8l+8); row jj of a
 // split belongs to warp jj mod 8; warps and splits are added in ascending order.
 #include "bk_common.cuh"
 #include "bk_internal.h"

@@ -2,7 +2,7 @@
 //
 // Every f32 rounding point is spelled out (explicit __fmul_rn/__fadd_rn/fmaf)
 // and the file is compiled with -fmad=false, so a*b+c never fuses by accident.
-// The CPU checker mirrors the same operation sequences; that is what makes the
+// The CPU oracle mirrors the same operation sequences; that is what makes the
 // kernels bit-reproducible on a host.
 #pragma once
 #include <cuda_runtime.h>

@@ -218,8 +218,8 @@ __device__ __forceinline__ void gdn_step_body(const GdnParams& p, GdnSmem& sm, c
 // Only the recurrence itself is serial.  Convolution, norms and gates of all tokens come first (gdn_prepare_kernel, one warp per
 // token and head), then the recurrence, four CTAs per value head (32 columns of the state each, in registers for all tokens),
 // then the gated norm (gdn_finish_kernel).  Per token the recurrence is two chains of 32 dependent FMAs and two barriers of
-// four warps, 0.3 us; as one CTA per head that did everything token after token it took 2.7 us.  64 tokens, 32 value heads: 176 us
-// as one launch, 7 + 24 + 5 us as three.  The operations and their order are those of gdn_step_body.
+// four warps, 0.3 us; as one CTA per head that did everything token after token it took 2.7 us.  64 tokens, 32 value heads: 150 us
+// as one launch, 40 us as three (7 + 24 + 5 us of kernels).  The operations and their order are those of gdn_step_body.
 struct GdnTokens {
   GdnParams g;
   int T;            // tokens per sequence of this launch

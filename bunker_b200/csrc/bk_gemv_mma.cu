@@ -12,7 +12,7 @@
 //     val(s,p) = fma(d, fma(d8_1, f32(sc1*i1), d8_0*f32(sc0*i0)), -(dmin * fma(s8_1, m1, s8_0*m0)))
 // and adds them in the order the 32-lane scheme defines: class c = s mod 8 collects s = c, c+8, ... in
 // ascending order; T_p = ((P0+P4)+(P2+P6)) + ((P1+P5)+(P3+P7)); row total = (T0+T2) + (T1+T3) across the four
-// p-warps through shared memory.  The result is bit-identical to gemv_q4k_kernel and to the CPU checker.
+// p-warps through shared memory.  The result is bit-identical to gemv_q4k_kernel and to the CPU oracle.
 //
 // Rows of a tile sit in shared memory at a stride of rowb+16 bytes (one bulk copy per row): with the natural
 // stride (a multiple of 128 bytes) the eight rows of an A fragment would hit the same banks.

@@ -26,7 +26,7 @@
 //     N = 16) per wait;
 //   * two EPILOGUE warps add up what the scalers hand over and write the outputs while the scalers are at the next tile.
 //
-// Two orders of the f32 part, both fixed and mirrored by the CPU checker:
+// Two orders of the f32 part, both fixed and mirrored by the CPU oracle:
 //   LANES (the order of the batch <= 8 kernels, for prompts of 17 columns and more): per unit u = (s, p)
 //     val = fma(d, fma(d8_1, x1, d8_0*x0), -(dmin * fma(s8_1, m1, s8_0*m0))); class c = s mod 8 of pair p adds its units in
 //     ascending s; T_p = ((P0+P4)+(P2+P6)) + ((P1+P5)+(P3+P7)); y = (T0+T2) + (T1+T3).  The classes are walked in the order

@@ -440,10 +440,10 @@ int32_t alloc_prefill(Model& m, int cols) {
   return BK_OK;
 }
 
-// T prompt tokens of every sequence in one pass: the projections see T*B columns (weights streamed once per 8
-// columns instead of once per token); the recurrent parts -- conv1d + GDN state, KV append + attention -- run token
-// after token with the decode kernels.  Every column goes through the arithmetic of the decode step, so the state
-// and the logits of the last token are bit-identical to T decode steps.  Single GPU only.
+// T prompt tokens of every sequence in one pass: the projections see T*B columns (weights streamed once from 17 columns on where every
+// segment's rows are whole boxes of 32, else once per 8 columns), the GDN layers take all tokens in three launches, attention takes all
+// columns in two.  Every column goes through the arithmetic of the decode step, so the state and the logits of the last token are
+// bit-identical to T decode steps.  Single GPU only.
 int32_t enqueue_prefill(Model& m, int T) {
   const bkModelConfig& c = m.cfg;
   const int B = m.B, H = c.hidden, C = T * B;

@@ -8,10 +8,11 @@
 //
 // What bounds a step at batch 1: about 120 dependent phases, so the latency of a hand-off and of a phase's fixed part; the
 // weights alone would take 170 us (24 layers, hidden 2048).  As 123 dependent launches the step takes 726 us (5.9 us
-// each: grid completion, flush and dependency wait 2 us, activation prologue 1-2 us, then the rows); as one launch 560 us.
+// each: grid completion, flush and dependency wait 2 us, activation prologue 1-2 us, then the rows); as one launch 558 us.
 // Of the 4.5 us of a projection phase (2048 wide, 84 rows per SM) 0.7 us are the wait for the hand-off, 1.3 us norm and
-// quantisation, 1.5 us dot products, 0.4 us reduction and epilogue.  64 layers of hidden 5120: 4.74 -> 4.60 ms (HBM 2.1 ms: the
-// half-rate integer instructions of the dots bound it).
+// quantisation, 1.5 us dot products, 0.4 us reduction and epilogue.  64 layers of hidden 5120: 4.75 -> 4.6 ms.  There the projections are
+// long enough to be streams (gate and up 25 us for 100 MB, 4.0 TB/s; the others 2.6 to 2.9) and neither the dots (1.3 ms) nor HBM (2.2 ms)
+// account for the step; the ring holds 120 KB, 2.7 us of an SM's share, so it is full and stands still while a long activation is staged.
 //
 // Hand-off.  There is no grid barrier.  Every activation word carries the generation it belongs to: bf16 values as 32-bit
 // words {value, 16-bit tag}, f32 values as 64-bit words {value, 32-bit tag}.  A producer stores the word; a consumer loads

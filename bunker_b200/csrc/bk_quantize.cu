@@ -2,7 +2,7 @@
 //
 // bunker uploads its safetensors weights as they are, bf16 (loadWeights, prototypes/decode.ts:64-76); the Q4_K model
 // served here needs them quantised once at load time.  Half a warp per 256-weight superblock, lane l of it holding weights
-// [16l, 16l+16) (half of sub-block l/2).  The arithmetic is the CPU checker's, operation for operation:
+// [16l, 16l+16) (half of sub-block l/2).  The arithmetic is the CPU oracle's, operation for operation:
 //   sub-block:  lo = min(min x, 0), scale = (max x - lo) / 15, mn = 0 - lo
 //   superblock: d = f16_rn(max scale / 63), dmin = f16_rn(max mn / 63), sc = floor(scale * (1/d) + 0.5) (<= 63),
 //               m = floor(mn * (1/dmin) + 0.5) (<= 63)

@@ -102,7 +102,7 @@ BK_API uint64_t bkStagedBytes(int32_t K, int32_t B);
 
 /* f32 accumulation order of a row's result (the integer block dots are exact either way).  LANES: the order of the
  * batch <= 8 kernels (64-weight units over 32 lanes, butterfly).  TILE: from 16 columns on, with BK_PRO_Q8 input, the
- * dense tile kernel (tcgen05 int8 MMA, accumulators in tensor memory) and its order: one chain per (row, column),
+ * dense tile kernel (tcgen05 f16 MMA, accumulators in tensor memory) and its order: one chain per (row, column),
  * sub-blocks ascending, superblocks ascending within a chunk of four, chunks ascending; below 16 columns TILE means
  * LANES.  AUTO: TILE when the launch has at least 4096 rows (all segments together, a SwiGLU pair counting twice), or
  * at least 1024 rows and K >= 2048; else LANES -- a rule of the shapes alone, so a host can mirror it.  Both orders are
@@ -258,7 +258,7 @@ BK_API int32_t bkArgmaxStatic(uint64_t logits, int32_t V, int32_t B, uint64_t id
  * top_p * total; u in [0,1) from splitmix64(splitmix64(seed ^ (step << 20)) + sequence) >> 40; the first candidate whose
  * running sum exceeds u * (prefix total).  step = (step_dev ? step_dev[b] : 0) + step_add (step_dev: device int32 [B],
  * e.g. the model's position buffer, or 0).  temperature 0 or top_k 1 is the argmax.  idx int32 [B]; val f32 [B] (the
- * chosen logit; 0 to skip).  Deterministic: the same inputs give the same tokens, on any GPU and on the CPU checker. */
+ * chosen logit; 0 to skip).  Deterministic: the same inputs give the same tokens, on any GPU and on the CPU oracle. */
 BK_API int32_t bkSample(uint64_t logits, int32_t V, int32_t B, float temperature, int32_t top_k, float top_p, uint64_t seed,
                         uint64_t step_dev, uint32_t step_add, uint64_t idx, uint64_t val);
 
@@ -328,6 +328,7 @@ BK_API int32_t bkDecodeRun(uint64_t model, int32_t n_steps);
 BK_API int32_t bkDecodeStepProfiled(uint64_t model, float* ms_out, int32_t* count_out, int32_t n_classes);
 /* Tokens produced by steps [first_step, first_step+n_steps): out[n_steps][B] host ints. */
 BK_API int32_t bkModelTokens(uint64_t model, int32_t first_step, int32_t n_steps, int32_t* out);
+/* kernels_per_step: launches of a step at the current position (1 while the one-launch step serves it). */
 BK_API int32_t bkModelInfo(uint64_t model, int32_t* split_len, int32_t* attn_warps, int32_t* kernels_per_step,
                            int64_t* steps);
 /* Device address of an internal buffer: "logits" f32 [B][vocab], "ids", "pos", "x0", "x1". */

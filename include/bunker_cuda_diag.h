@@ -37,7 +37,7 @@ BK_API int32_t bkTuneTileMinRows(int32_t rows);
 BK_API int32_t bkStepTraceEnable(uint64_t dev_buf, int32_t max_phases);
 /* Polls a bounded device-side wait may take before it gives up and sets the status word that bkSync reports as
  * BK_ERR_TIMEOUT (0 restores the built-in limits).  Applies to the tensor-parallel exchange consumer
- * (bkReduceRmsNormQuantQ8_1 and the model's reducing launches) and the persistent step kernel's waits for tagged words, for
+ * (bkReduceRmsNormQuantQ8_1 and the model's reducing launches) and all waits of the persistent step kernel, for
  * launches issued after the call.  Lets a test make a wait run out in microseconds without hanging anything. */
 BK_API int32_t bkSetSpinLimit(int32_t polls);
 /* Kept for hosts that bind it: the persistent step kernel has no grid barrier any more (its phases hand tagged words to
