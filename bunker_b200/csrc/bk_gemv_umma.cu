@@ -18,8 +18,7 @@
 //     of the 128 rows and the activations of that superblock, which are ready-made operand B tiles (see the image below);
 //   * eight EXPANDER warps (two per 32 rows, taking turns; thread <-> row) turn a row's 32 bytes into 64 f16 in tensor memory
 //     (operand A; the shared-memory bandwidth that it would cost is needed by the scalers) and its header into {d, -dmin, m0, m1};
-//   * one MMA warp issues four MMAs (M = 128, N = columns, K = 16) per step into two accumulators of N tensor-memory columns
-//     (measured: 47 cycles each whatever N, 43 for a commit, both of them the issuing thread's);
+//   * one MMA warp issues four MMAs (M = 128, N = columns, K = 16) per step into two accumulators of N tensor-memory columns;
 //   * eight SCALER warps (two per TMEM lane quarter, half of the columns each) read the accumulators as 16x256b fragments (a thread
 //     holds 4 rows x 2 columns of every 8 columns, so that a column's d8 and s8 are loaded once for 4 rows and a row's minima
 //     once for all columns) and run the f32 part, two columns per instruction; four such blocks (one step at N = 64, four at
@@ -40,9 +39,10 @@
 // that owns the column (one bulk copy through distributed shared memory per owner; the first 1, 2, 4 or 8 CTAs own columns); the owner adds
 // them in the fixed order and runs the epilogue.
 //
-// Weight feed: tiled TMA loads of 32-row boxes (cp.async.bulk.tensor.2d) where every segment's row count is a multiple of 32; a
-// SwiGLU launch then keeps its 64 gate rows in tile rows 0..63 and their up rows in 64..127.  Other shapes (TILE only)
-// copy row by row.  No multicast.  Every wait is bounded; TMEM is released on every path out of the kernel.
+// Weight feed: one tiled TMA load (cp.async.bulk.tensor.2d) of the tile's 128 rows per stage, two where headers and quants are apart; a SwiGLU
+// launch keeps 64 gate rows in tile rows 0..63 and their up rows in 64..127.  A tile with rows of several segments takes boxes of 32,
+// 16 or 8 rows, whatever divides the segments' first rows; other shapes (TILE only) copy row by row.  No multicast.  Every wait is
+// bounded; TMEM is released on every path out of the kernel.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -82,12 +82,14 @@ struct UmmaParams {
   GemvParams g;       // K, segments, total_vrows, x = image (see bk_tile_image_bytes), status
   int B;              // activation columns, 1..64
   int groups;         // column groups (N > 32 columns of few rows: two groups of 32, each with its own image and its own tiles)
-  int use_maps;       // weights come by tiled TMA loads through maps[]
+  int use_maps;       // weights come by tiled TMA loads through maps[] and part[]
   int stages;         // ring stages
   int csplit;         // LANES: CTAs that share the classes of a pair; TILE: CTAs that share the chunks (= cluster size, 1 to 8)
   int levels;         // LANES: stack levels in shared memory
   uint32_t xbuf_bytes, stg_bytes;   // received values; values to send (clusters of more than one)
-  CUtensorMap maps[10];   // [2i], [2i+1]: headers and quants of segment i (whole superblocks: only [2i]); i = 4: the up matrix
+  CUtensorMap maps[10];   // [2i], [2i+1]: headers and quants of segment i (whole superblocks: only [2i]); i = 4: the up matrix.  Boxes of a tile's rows
+  CUtensorMap part[8];    // the same in boxes of part_rows rows, for tiles that more than one segment has rows in
+  int part_rows;
 };
 
 BK_DEVINL uint64_t umma_desc(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
@@ -157,6 +159,19 @@ BK_DEVINL void umma_f16(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc) 
   asm volatile("{\n\t.reg .pred pz;\n\tsetp.ne.b32 pz, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, pz;\n\t}" ::"r"(d), "r"(a), "l"(bdesc),
                "r"(idesc), "n"(ACC ? 1 : 0)
                : "memory");
+}
+BK_DEVINL bool elect_one() {
+  uint32_t p;
+  asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(p));
+  return p != 0;
+}
+// the same wait for a whole warp that stays together, as the roles of one warp do whose instructions take uniform registers
+BK_DEVINL void mbar_wait_warp(uint32_t bar, uint32_t parity, int* status, volatile int* dead) {
+#pragma unroll 1
+  for (int it = 0; it < (1 << 22); it++)
+    if (__all_sync(0xffffffffu, mbar_poll(bar, parity, true) || *dead)) return;
+  *dead = 1;
+  if (status) atomicExch(status, 10003 /* BK_ERR_TIMEOUT */);
 }
 BK_DEVINL void scalers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kScalers) : "memory"); }
 BK_DEVINL void cluster_sync() {
@@ -258,7 +273,7 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
     *dead = 0;
     for (int i = 0; i < nst; i++) {
       mbar_init(smem_u32(wfull + i), 1);
-      mbar_init(smem_u32(wempty + i), (PS == 1 ? 4 : 8) + 1);   // expander warps, and a scaler for the MMAs
+      mbar_init(smem_u32(wempty + i), (PS == 1 ? 4 : 8) + 1);   // expander warps, and the MMAs
     }
     for (int i = 0; i < 2; i++) {
       mbar_init(smem_u32(a_full + i), C::kHalf * kTileM);
@@ -462,48 +477,53 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
       }
     } else if (warp == kMmaWarp) {
       // ================= MMA issue: per step two sub-blocks of K = 32 =================
-      // One lane only, and few instructions: this thread has to keep up with four warps per scheduler.
+      // The warp stays together and one elected lane issues, so that addresses and descriptors are uniform values: with one lane that runs
+      // alone every MMA first moves its operands there (tile order, 32 columns, 152k rows: 110 us, so 105).
       // f32 accumulators, f16 operands, both K-major
       constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
-      if (lane == 0) {
-        int stage = 0, batch = 0, g = 0;
-        uint32_t spar = 0, bpar = 1;   // a fresh barrier counts as freed
-        {
-          for (int i = 0; i < total; i++) {
-            mbar_wait_idle(smem_u32(wfull + stage), spar, p.status, dead);   // operand B and the column factors
-            uint64_t bd = umma_desc(smem_u32(raw + (size_t)stage * C::kStage + C::kWBytes), N * 16, 128);
+      const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+      const uint64_t bd0 = umma_desc(smem_u32(raw) + C::kWBytes, N * 16, 128);
+      int stage = 0, batch = 0, g = 0;
+      uint32_t spar = 0, bpar = 1;   // a fresh barrier counts as freed
+      for (int i = 0; i < total; i++) {
+        mbar_wait_warp(smem_u32(wfull + stage), spar, p.status, dead);   // operand B and the column factors
+        const uint64_t bs = bd0 + (uint32_t)(stage * (C::kStage >> 4));   // (an address below 256 KB: no carry into the other fields)
 #pragma unroll
-            for (int pi = 0; pi < PS; pi++, g++) {
-              const int bi = pi % BT;
-              if (bi == 0) mbar_wait_idle(smem_u32(d_free + batch), bpar, p.status, dead);
-              if (g % C::kHalf == 0) mbar_wait_idle(smem_u32(a_full + ((g / C::kHalf) & 1)), (uint32_t)(g / C::kA) & 1u, p.status, dead);
-              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              const uint32_t a0 = tmem_a + (g % C::kA) * 32, d0 = tmem + batch * 128 + bi * 2 * N;
-              umma_f16<false>(d0, a0, bd, idesc);
-              umma_f16<true>(d0, a0 + 8, bd + N * 2, idesc);
-              umma_f16<false>(d0 + N, a0 + 16, bd + N * 4, idesc);
-              umma_f16<true>(d0 + N, a0 + 24, bd + N * 6, idesc);
-              bd += N * 8;
-              if (bi == BT - 1) {
-                umma_commit(smem_u32(d_full + batch));
-                mbar_arrive(smem_u32(d_full + batch));   // passes on what the expanders and the copies have written
-                if (++batch == C::kBatches) {
-                  batch = 0;
-                  bpar ^= 1u;
-                }
-              }
-              if (g % C::kHalf == C::kHalf - 1) umma_commit(smem_u32(a_free + ((g / C::kHalf) & 1)));
+        for (int pi = 0; pi < PS; pi++, g++) {
+          const int bi = pi % BT;
+          if (bi == 0) mbar_wait_warp(smem_u32(d_free + batch), bpar, p.status, dead);
+          if (g % C::kHalf == 0) mbar_wait_warp(smem_u32(a_full + ((g / C::kHalf) & 1)), (uint32_t)(g / C::kA) & 1u, p.status, dead);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a0 = tm + C::kBatches * 128 + (g % C::kA) * 32, d0 = tm + batch * 128 + bi * 2 * N;
+          const uint64_t bd = bs + pi * (N * 8);
+          if (elect_one()) {
+            umma_f16<false>(d0, a0, bd, idesc);
+            umma_f16<true>(d0, a0 + 8, bd + N * 2, idesc);
+            umma_f16<false>(d0 + N, a0 + 16, bd + N * 4, idesc);
+            umma_f16<true>(d0 + N, a0 + 24, bd + N * 6, idesc);
+            if (pi == PS - 1) umma_commit(smem_u32(wempty + stage));   // operand B has been read
+            if (bi == BT - 1) {
+              umma_commit(smem_u32(d_full + batch));
+              mbar_arrive(smem_u32(d_full + batch));   // passes on what the expanders and the copies have written
             }
-            if (++stage == nst) {
-              stage = 0;
-              spar ^= 1u;
-            }
+            if (g % C::kHalf == C::kHalf - 1) umma_commit(smem_u32(a_free + ((g / C::kHalf) & 1)));
           }
+          __syncwarp();
+          if (bi == BT - 1 && ++batch == C::kBatches) {
+            batch = 0;
+            bpar ^= 1u;
+          }
+        }
+        if (++stage == nst) {
+          stage = 0;
+          spar ^= 1u;
         }
       }
       __syncwarp();
     } else {
       // ================= producer: superblock after superblock, tile after tile =================
+      // One elected lane issues and few copies make a stage: whatever its size a copy costs the issuing warp about 100 cycles, and with
+      // a box per 32 rows, one per lane, the issue bound the whole kernel in the lane order (64 columns: 1,940 of 1,960 cycles a step).
       int cslot = 0;
       Walk<LANES> w, wx;
       const int first = min(total, nst);
@@ -511,9 +531,10 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
       const uint8_t* img_b = static_cast<const uint8_t*>(p.x) + (size_t)p0 * C::kBBytes;   // image: operand B of all units, then their factors
       const uint8_t* img_c = static_cast<const uint8_t*>(p.x) + (size_t)(p.K / 64) * C::kBBytes + (size_t)p0 * (N * 16);
       const size_t img_bytes = (size_t)(p.K / 64) * (C::kBBytes + N * 16);
+      const bool leader = elect_one();
       auto fill_x = [&](int s, int stage, int vt) {
         const size_t go = two ? (size_t)(vt & 1) * img_bytes : 0;
-        if (lane == 0) {
+        if (leader) {
           const uint32_t bar = smem_u32(wfull + stage);
           bulk_g2s(smem_u32(raw + (size_t)stage * C::kStage + C::kWBytes), img_b + go + (size_t)s * 4 * C::kBBytes, PS * C::kBBytes, bar);
           bulk_g2s(smem_u32(cols + cslot * C::kColBytes), img_c + go + (size_t)s * (4 * N * 16), C::kColBytes, bar);
@@ -521,45 +542,68 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
         if (++cslot == ncols) cslot = 0;   // (three superblocks more than stages: the scalers are at most that far behind the MMAs)
       };
       constexpr uint32_t kXBytes = PS * C::kBBytes + C::kColBytes;
-      int vt = tile0, stage = 0;
+      constexpr uint32_t kRowW = C::kWBytes / kTileM;   // bytes of a tile row in a stage
+      auto load_box = [&](const CUtensorMap* m, uint32_t dst, int x, int row, uint32_t bar) {
+        asm volatile(
+            "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;" ::"r"(dst),
+            "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(row), "r"(bar), "l"(policy)
+            : "memory");
+      };
+      // the segment of the tile's first row, that row in it, and whether the tile has rows of no other segment
+      int vt = tile0, tile = 0, mi = 0, row0 = 0;
+      bool whole = true;
+      auto enter_tile = [&]() {
+        tile = two ? vt >> 1 : vt;
+        mi = 0;
+        int next = p.total_vrows;
+#pragma unroll
+        for (int si = 3; si >= 1; si--)
+          if (si < p.n_segs && mi == 0) {
+            if (tile * kTileM >= p.segs[si].vrow_begin) mi = si;
+            else next = p.segs[si].vrow_begin;
+          }
+        row0 = swiglu_halves ? tile * 64 : tile * kTileM - p.segs[mi].vrow_begin;
+        whole = next == p.total_vrows || (tile + 1) * kTileM <= next;
+      };
+      int stage = 0;
       uint32_t spar = 1;   // parity of the readers' arrivals on the previous use
       w.start(pos0, pos1, nsb);
+      enter_tile();
       for (int i = 0; i < total; i++) {
-        if (i >= nst) mbar_wait_idle(smem_u32(wempty + stage), spar, p.status, dead);
+        if (i >= nst) mbar_wait_warp(smem_u32(wempty + stage), spar, p.status, dead);
         const uint32_t bar = smem_u32(wfull + stage), dst0 = smem_u32(raw + (size_t)stage * C::kStage);
-        const int tile = two ? vt >> 1 : vt;
-        if (P.use_maps) {
-          // lanes 0..3: the 32-row boxes of the tile (whole superblocks, or headers); lanes 4..7: their quants
-          const int bx = lane & 3;
-          bool valid = lane < (PS == 4 ? 4 : 8);
-          int mi = 0, row0 = 0;
-          if (swiglu_halves) {   // boxes 0, 1: gate rows tile*64 + 32k; boxes 2, 3: the same rows of the up matrix
-            row0 = tile * 64 + 32 * (bx & 1);
-            mi = bx < 2 ? 0 : 4;
-            valid = valid && row0 < p.segs[0].n_rows;
-          } else {
-            const int v0 = tile * kTileM + 32 * bx;
-            valid = valid && v0 < p.total_vrows;
-#pragma unroll
-            for (int si = 1; si < 4; si++)
-              if (si < p.n_segs && v0 >= p.segs[si].vrow_begin) mi = si;
-            row0 = v0 - p.segs[mi].vrow_begin;
+        const int x = w.s * 144, xq = x + 16 + 32 * p0;
+        if (P.use_maps && whole) {   // rows past the last one are filled with zeros
+          if (leader) {
+            mbar_expect_tx(bar, C::kWBytes + kXBytes);
+            const CUtensorMap* m = P.maps + 2 * mi;
+            load_box(m, dst0, x, row0, bar);
+            if (PS < 4) load_box(m + 1, dst0 + kTileM * 16, xq, row0, bar);
+            if (swiglu_halves) {   // the maps' boxes have 64 rows: the gate's, and here the same rows of the up matrix
+              load_box(P.maps + 8, dst0 + (PS == 4 ? 64 * 144 : 64 * 16), x, row0, bar);
+              if (PS < 4) load_box(P.maps + 9, dst0 + kTileM * 16 + 64 * 32 * PS, xq, row0, bar);
+            }
           }
-          const unsigned boxes = __popc(__ballot_sync(0xffffffffu, valid && lane < 4));
-          if (lane == 0) mbar_expect_tx(bar, boxes * (uint32_t)(C::kWBytes / 4) + kXBytes);
+        } else if (P.use_maps) {
+          // lanes 0..15: the tile's boxes (whole superblocks, or headers); lanes 16..31: their quants
+          const int bx = lane & 15, v0 = tile * kTileM + P.part_rows * bx;
+          const bool valid = P.part_rows * bx < kTileM && v0 < p.total_vrows && (PS < 4 || lane < 16);
+          int si = 0;
+#pragma unroll
+          for (int k = 1; k < 4; k++)
+            if (k < p.n_segs && v0 >= p.segs[k].vrow_begin) si = k;
+          const uint32_t boxes = __popc(__ballot_sync(0xffffffffu, valid && lane < 16));
+          if (leader) mbar_expect_tx(bar, boxes * (uint32_t)P.part_rows * kRowW + kXBytes);
           __syncwarp();
           if (valid) {
-            const bool quants = lane >= 4;
-            const int x = w.s * 144 + (quants ? 16 + 32 * p0 : 0);
-            const uint32_t dst = dst0 + (PS == 4 ? bx * 32 * 144 : quants ? kTileM * 16 + bx * 32 * 32 * PS : bx * 32 * 16);
-            asm volatile(
-                "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;" ::"r"(dst),
-                "l"(reinterpret_cast<uint64_t>(&P.maps[2 * mi + (quants ? 1 : 0)])), "r"(x), "r"(row0), "r"(bar), "l"(policy)
-                : "memory");
+            const bool quants = lane >= 16;
+            const int at = P.part_rows * bx;
+            load_box(P.part + 2 * si + (quants ? 1 : 0), dst0 + (PS == 4 ? at * 144 : quants ? kTileM * 16 + at * 32 * PS : at * 16), quants ? xq : x,
+                     v0 - p.segs[si].vrow_begin, bar);
           }
         } else {
           const int rows_here = min(kTileM, p.total_vrows - tile * kTileM);
-          if (lane == 0) mbar_expect_tx(bar, (uint32_t)rows_here * 144 + kXBytes);
+          if (leader) mbar_expect_tx(bar, (uint32_t)rows_here * 144 + kXBytes);
           __syncwarp();
 #pragma unroll 1
           for (int r = lane; r < rows_here; r += 32) bulk_g2s(dst0 + r * 144, decode_vrow(p, tile * kTileM + r).row + (size_t)w.s * 144, 144, bar);
@@ -575,6 +619,7 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
         if (w.done()) {
           vt += tile_step;
           w.start(pos0, pos1, nsb);
+          enter_tile();
         }
         if (++stage == nst) {
           stage = 0;
@@ -590,7 +635,7 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
     const int col0 = half * (N / 2) + 2 * (lane & 3);   // and columns: col0 + 8cb and the next
     const int own_shift = __ffs(own) - 1;
     const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + half * (N / 2);
-    int batch = 0, tab = 0, col = 0, stage = 0;
+    int batch = 0, tab = 0, col = 0;
     uint32_t bpar = 0;
     // One batch: BT steps from the current row table and pair pi0 of the current column factors on, as four blocks of 8 columns;
     // f(m, i, x0, x1, c0, c1, r): the two columns of block m = step * NB + column block, row i, accumulators of both sub-blocks,
@@ -634,8 +679,6 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
       }
     };
     auto next_superblock = [&]() {
-      if (st == 0) mbar_arrive(smem_u32(wempty + stage));   // its MMAs are through with operand B
-      if (++stage == nst) stage = 0;
       if (++col == ncols) col = 0;
     };
     // value v (of nv that this CTA sends) of column block cb and row i into the buffer the owners read or are sent
@@ -773,12 +816,12 @@ __global__ void __launch_bounds__(256) tile_image_kernel(const uint32_t* x, int 
   bk_tile_store_factors(img, nblk * 32, B, b, blk, d8, __fmul_rn(d8, (float)qsum));
 }
 
-// Matrix of Q4_K rows; header < 0: whole superblock columns (box 32 rows x 144 bytes), 1: their headers (x 16 bytes), 0: the quants
+// Matrix of Q4_K rows; header < 0: whole superblock columns (box rows x 144 bytes), 1: their headers (x 16 bytes), 0: the quants
 // of `pairs` sub-block pairs (x 32 * pairs bytes, swizzled so that the expanders' 16-byte reads hit all banks).
-bool encode_weight_map(CUtensorMap* m, const uint8_t* W, int n_rows, size_t row_bytes, int header, int pairs) {
+bool encode_weight_map(CUtensorMap* m, const uint8_t* W, int n_rows, size_t row_bytes, int box_rows, int header, int pairs) {
   const uint32_t box = header < 0 ? 144 : header ? 16 : 32 * pairs;
   const CUtensorMapSwizzle sw = header == 0 ? (pairs == 1 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B) : CU_TENSOR_MAP_SWIZZLE_NONE;
-  return bk_encode_map_2d(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, (uint64_t)(uintptr_t)W, row_bytes, (uint64_t)n_rows, row_bytes, box, 32, sw);
+  return bk_encode_map_2d(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, (uint64_t)(uintptr_t)W, row_bytes, (uint64_t)n_rows, row_bytes, box, box_rows, sw);
 }
 
 // How a launch of `tiles` tiles is cut: CTAs of a cluster that share the classes (or chunks) of a tile.
@@ -871,19 +914,26 @@ int32_t launch_tile(UmmaParams& P) {
   using C = Cfg<NB, LANES>;
   BkContext& c = bk_ctx();
   GemvParams& g = P.g;
-  // tensor-map feed: 32-row boxes that never straddle two segments
-  bool ok = true;
-  for (int i = 0; i < g.n_segs; i++) ok = ok && g.segs[i].n_rows % 32 == 0;
-  const size_t row_bytes = (size_t)(g.K / 256) * 144;
-  for (int i = 0; ok && i < g.n_segs; i++) {
-    for (int up = 0; ok && up < (g.segs[i].epi == BK_EPI_SWIGLU ? 2 : 1); up++) {
-      const uint8_t* W = up ? g.segs[i].W2 : g.segs[i].W;
-      CUtensorMap* m = P.maps + (up ? 8 : 2 * i);
-      ok = C::PS == 4 ? encode_weight_map(m, W, g.segs[i].n_rows, row_bytes, -1, 4)
-                      : encode_weight_map(m, W, g.segs[i].n_rows, row_bytes, 1, 0) && encode_weight_map(m + 1, W, g.segs[i].n_rows, row_bytes, 0, C::PS);
-    }
+  // tensor-map feed: boxes that never straddle two segments
+  P.part_rows = 32;
+  bool ok = true, mixed = false;
+  for (int i = 1; i < g.n_segs; i++) {
+    while (P.part_rows > 8 && g.segs[i].vrow_begin % P.part_rows != 0) P.part_rows /= 2;
+    ok = ok && g.segs[i].vrow_begin % P.part_rows == 0;
+    mixed = mixed || g.segs[i].vrow_begin % kTileM != 0;
   }
-  BK_ARG(ok || !LANES, "tile GEMV: the lane order needs segments of whole 32-row boxes");
+  const size_t row_bytes = (size_t)(g.K / 256) * 144;
+  auto encode = [&](CUtensorMap* m, const uint8_t* W, int n_rows, int box_rows) {
+    return C::PS == 4 ? encode_weight_map(m, W, n_rows, row_bytes, box_rows, -1, 4)
+                      : encode_weight_map(m, W, n_rows, row_bytes, box_rows, 1, 0) && encode_weight_map(m + 1, W, n_rows, row_bytes, box_rows, 0, C::PS);
+  };
+  for (int i = 0; ok && i < g.n_segs; i++) {
+    const bool swiglu = g.segs[i].epi == BK_EPI_SWIGLU;   // (alone in its launch)
+    ok = encode(P.maps + 2 * i, g.segs[i].W, g.segs[i].n_rows, swiglu ? 64 : kTileM);
+    if (ok && swiglu) ok = encode(P.maps + 8, g.segs[i].W2, g.segs[i].n_rows, 64);
+    if (ok && mixed) ok = encode(P.part + 2 * i, g.segs[i].W, g.segs[i].n_rows, P.part_rows);
+  }
+  BK_ARG(ok || !LANES, "tile GEMV: the lane order needs segments that begin at multiples of 8 rows");
   P.use_maps = ok ? 1 : 0;
 
   const int tiles = (g.total_vrows + kTileM - 1) / kTileM * P.groups;

@@ -351,3 +351,30 @@ def test_gemv_refuses_internal_prologues(bk, B, prologue):
         ops.gemv(x.ptr, K, B, [ops.gemv_seg(dW.ptr, N, y.ptr)], prologue=prologue, norm_w=x.ptr)
     assert e.value.code == R.BK_ERR_ARG
     assert R.cuSync() == 0
+
+
+@pytest.mark.parametrize("order", [R.BK_GEMV_ORDER_LANES, R.BK_GEMV_ORDER_TILE])
+@pytest.mark.parametrize("B,K,rows", [(32, 512, (128, 128)),              # every tile has rows of one segment
+                                      (24, 2304, (256, 96, 32, 32)),      # the last tile has three: boxes of 32 rows
+                                      (64, 768, (384, 48, 48)),           # of 16
+                                      (17, 2048, (200, 8, 24, 71)),       # of 8, all but the first in the second tile, and a last box past the end
+                                      (40, 1024, (136, 130)),             # a segment that begins in mid-tile and ends in a later one
+                                      (32, 256, (130, 60)),               # no box divides the second segment's first row
+                                      (64, 17408, (40, 8)), (33, 2048, (1000,)), (16, 512, (33,))])
+def test_gemv_tiles_of_several_segments(bk, order, B, K, rows):
+    """Tiles whose rows belong to one segment are one box of weights, others several, of as many rows as divide the segments' first rows; rows past
+    the end of a matrix are not read."""
+    rng = np.random.default_rng(1300 + B + K)
+    xq = O.q8_1_quantize(rng.normal(0, 1, (B, K)).astype(np.float32))
+    dxq = dev(xq)
+    W = [synth.q4k_weights(rng, n, K) for n in rows]
+    dW, y = [dev(w) for w in W], [R.DeviceBuffer(B * n * 4) for n in rows]
+    ops.gemv(dxq.ptr, K, B, [ops.gemv_seg(w.ptr, n, o.ptr) for w, n, o in zip(dW, rows, y)], order=order)
+    oracle = O.gemv_q4k_q8_tile if order == R.BK_GEMV_ORDER_TILE else O.gemv_q4k_q8
+    for i, n in enumerate(rows):
+        assert_same_bits(y[i].download(np.float32, (B, n)), oracle(W[i], n, K, xq), f"segment {i}")
+    n = rows[0]
+    act, up = R.DeviceBuffer(B * n * 2), dev(synth.q4k_weights(rng, n, K))
+    ops.gemv(dxq.ptr, K, B, [ops.gemv_seg(dW[0].ptr, n, act.ptr, R.BK_EPI_SWIGLU, W2=up.ptr)], order=order)
+    g, u = oracle(W[0], n, K, xq), oracle(up.download(np.uint8, W[0].shape), n, K, xq)
+    assert_same_bits(act.download(np.uint16, (B, n)), O.swiglu(g, u), "SwiGLU pair")
