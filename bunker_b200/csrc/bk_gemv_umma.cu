@@ -638,8 +638,8 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
     int batch = 0, tab = 0, col = 0;
     uint32_t bpar = 0;
     // One batch: BT steps from the current row table and pair pi0 of the current column factors on, as four blocks of 8 columns;
-    // f(m, i, x0, x1, c0, c1, r): the two columns of block m = step * NB + column block, row i, accumulators of both sub-blocks,
-    // column factors {d8, d8', s8, s8'} of both, row factors
+    // f(bi, cb, i, x0, x1, c0, c1, r): step bi, the two columns of block cb, row i, accumulators of both sub-blocks, column factors
+    // {d8, d8', s8, s8'} of both, row factors
     auto run_batch = [&](int pi0, auto&& f) {
       mbar_wait_idle(smem_u32(d_full + batch), bpar, p.status, dead);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
         const float4 c0 = ct[bi * N + cb * 4], c1 = ct[bi * N + N / 2 + cb * 4];
 #pragma unroll
         for (int i = 0; i < 4; i++)
-          f(m, i, make_float2(x[u][0][i >> 1][2 * (i & 1)], x[u][0][i >> 1][2 * (i & 1) + 1]),
+          f(bi, cb, i, make_float2(x[u][0][i >> 1][2 * (i & 1)], x[u][0][i >> 1][2 * (i & 1) + 1]),
             make_float2(x[u][1][i >> 1][2 * (i & 1)], x[u][1][i >> 1][2 * (i & 1) + 1]), c0, c1, r4[i]);
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -700,22 +700,27 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
 
     for (int k = 0; k < n_my; k++) {
       if constexpr (LANES) {
-        float2 S[16], L0[16];
+        float2 S[16], L0[16];   // [step of the batch = pair][column block][row]
         int sp = 0;
-        for (int lp = 0; lp < pos1 - pos0; lp++) {
+        auto run_class = [&](int pos, float2 (&T)[16]) {
 #pragma unroll
-          for (int e = 0; e < 16; e++) S[e] = make_float2(0.0f, 0.0f);
-          for (int s = Walk<LANES>::cls(pos0 + lp); s < nsb; s += 8) {
-            run_batch(0, [&](int m, int i, float2 x0, float2 x1, const float4& c0, const float4& c1, const float4& r) {
+          for (int e = 0; e < 16; e++) T[e] = make_float2(0.0f, 0.0f);
+          for (int s = Walk<LANES>::cls(pos); s < nsb; s += 8) {
+            run_batch(0, [&](int bi, int cb, int i, float2 x0, float2 x1, const float4& c0, const float4& c1, const float4& r) {
               float2 a = mul2(make_float2(c0.x, c0.y), x0);
               a = bk_fma2(make_float2(c1.x, c1.y), x1, a);
               float2 mm = mul2(make_float2(c0.z, c0.w), dup2(r.z));
               mm = bk_fma2(make_float2(c1.z, c1.w), dup2(r.w), mm);
-              S[m * 4 + i] = bk_add2(S[m * 4 + i], bk_fma2(dup2(r.x), a, mul2(dup2(r.y), mm)));
+              const int e = (bi * NB + cb) * 4 + i;
+              T[e] = bk_add2(T[e], bk_fma2(dup2(r.x), a, mul2(dup2(r.y), mm)));
             });
             next_superblock();
           }
-          if (lp & 1) {
+        };
+        for (int lp = 0; lp < pos1 - pos0; lp += 2) {   // (classes are shared by powers of two: one, or a whole number of pairs)
+          run_class(pos0 + lp, L0);
+          if (lp + 1 < pos1 - pos0) {
+            run_class(pos0 + lp + 1, S);
 #pragma unroll
             for (int e = 0; e < 16; e++) S[e] = bk_add2(L0[e], S[e]);
             for (int m = lp >> 1; m & 1; m >>= 1) {
@@ -723,37 +728,35 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
 #pragma unroll
               for (int e = 0; e < 16; e++) S[e] = bk_add2(stack[(sp * 16 + e) * kScalers + st], S[e]);
             }
-            if (lp + 1 < pos1 - pos0) {
+            if (lp + 2 < pos1 - pos0) {
 #pragma unroll
               for (int e = 0; e < 16; e++) stack[(sp * 16 + e) * kScalers + st] = S[e];
               sp++;
             }
-          } else {
-#pragma unroll
-            for (int e = 0; e < 16; e++) L0[e] = S[e];
           }
         }
         if (k > 0) mbar_wait_idle<true>(smem_u32(xempty), (uint32_t)(k - 1) & 1u, p.status, dead);   // what was sent before has been read
 #pragma unroll
         for (int e = 0; e < 16; e++) {
-          float* o = place(e / (4 * NB), PS, (e / 4) % NB, e & 3);
+          float* o = place(e / (4 * NB), PS, e / 4 % NB, e & 3);
           o[0] = pos1 - pos0 == 1 ? L0[e].x : S[e].x;
           o[kXPitch] = pos1 - pos0 == 1 ? L0[e].y : S[e].y;
         }
         send((int)rank * PS, PS);
       } else {
-        float2 yc[NB * 4];
+        constexpr int E = 4 * NB;
+        float2 yc[E];
         const int ch0 = pos0 >> 2, nv = CS > 1 ? (pos1 + 3) / 4 - ch0 : 1;
         if (k > 0 && pos0 >= pos1) mbar_wait_idle<true>(smem_u32(xempty), (uint32_t)(k - 1) & 1u, p.status, dead);
         for (int s = pos0; s < pos1; s++) {
-          float2 A[NB * 4], M[NB * 4];
+          float2 A[E], M[E];
 #pragma unroll
-          for (int e = 0; e < NB * 4; e++) A[e] = M[e] = make_float2(0.0f, 0.0f);
+          for (int e = 0; e < E; e++) A[e] = M[e] = make_float2(0.0f, 0.0f);
           float rd[4], rm[4];
 #pragma unroll 1
           for (int pi = 0; pi < 4; pi += BT)
-            run_batch(pi, [&](int m, int i, float2 x0, float2 x1, const float4& c0, const float4& c1, const float4& r) {
-              const int e = (m % NB) * 4 + i;
+            run_batch(pi, [&](int bi, int cb, int i, float2 x0, float2 x1, const float4& c0, const float4& c1, const float4& r) {
+              const int e = cb * 4 + i;
               A[e] = bk_fma2(make_float2(c0.x, c0.y), x0, A[e]);
               M[e] = bk_fma2(make_float2(c0.z, c0.w), dup2(r.z), M[e]);
               A[e] = bk_fma2(make_float2(c1.x, c1.y), x1, A[e]);
@@ -763,13 +766,13 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
             });
           next_superblock();
 #pragma unroll
-          for (int e = 0; e < NB * 4; e++)
+          for (int e = 0; e < E; e++)
             yc[e] = bk_add2((s & 3) == 0 ? make_float2(0.0f, 0.0f) : yc[e], bk_fma2(dup2(rd[e & 3]), A[e], mul2(dup2(rm[e & 3]), M[e])));
           if ((s & 3) == 3 || s == nsb - 1) {   // a chunk ends: its own value, or y += yc in place
             if (k > 0 && s - pos0 < 4) mbar_wait_idle<true>(smem_u32(xempty), (uint32_t)(k - 1) & 1u, p.status, dead);
             const bool first = CS > 1 || s < 4;
 #pragma unroll
-            for (int e = 0; e < NB * 4; e++) {
+            for (int e = 0; e < E; e++) {
               float* o = place(CS > 1 ? (s >> 2) - ch0 : 0, nv, e / 4, e & 3);
               o[0] = __fadd_rn(first ? 0.0f : o[0], yc[e].x);
               o[kXPitch] = __fadd_rn(first ? 0.0f : o[kXPitch], yc[e].y);
