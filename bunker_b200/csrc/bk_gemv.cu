@@ -372,14 +372,14 @@ int32_t bk_gemv_launch_tp(const bkGemvArgs& a, const BkPush* push, const BkReduc
   // Ready-made Q8_1 blocks of many columns go to the dense tile kernel (tcgen05, bk_gemv_umma.cu), which streams the weights
   // once for all columns.  From 16 columns on it has an f32 order of its own (see there), which order = BK_GEMV_ORDER_LANES
   // declines and AUTO takes for launches of many rows; the rule depends on the shapes only.  In the lane order it takes
-  // 17 columns and more of rows in whole boxes of 32: two launches of 8 columns on the mma.sync kernel are as fast at 16 (K 2048,
+  // 17 columns and more of segments that begin at multiples of 8 rows: two launches of 8 columns on the mma.sync kernel are as fast at 16 (K 2048,
   // 12,352 rows: 18 us, here 20), three or four are not (32 columns: 37 us, here 27; 64: 74 us, here 36).  A caller's Q8_1 blocks have to be
   // made into its image first, which few columns of a short K do not pay back (dense_blocks_pay).
   int launch_rows = 0;
-  bool whole_boxes = true;
+  bool whole_boxes = true;   // (a box of 8 rows of weights belongs to one segment)
   for (int i = 0; i < a.n_segs && i < 4; i++) {
+    whole_boxes = whole_boxes && launch_rows % 8 == 0;
     launch_rows += a.segs[i].n_rows * (a.segs[i].epilogue == BK_EPI_SWIGLU ? 2 : 1);
-    whole_boxes = whole_boxes && a.segs[i].n_rows % 32 == 0;
   }
   const bool dense = a.B > 8 && (a.prologue == BK_PRO_Q8 || a.prologue == BK_PRO_TILE) && !push && !reduce && !g_view;
   const bool tile_order = dense && a.B >= 16 && (a.order == BK_GEMV_ORDER_TILE || (a.order == BK_GEMV_ORDER_AUTO && bk_gemv_auto_tile(launch_rows, a.K)));
