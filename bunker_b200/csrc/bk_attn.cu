@@ -85,32 +85,17 @@ __device__ __forceinline__ void norm_rope_256(const uint16_t* src, const uint16_
   __syncwarp();
 }
 
-// Sum 8 per-lane values over the warp with 9 shuffles instead of 40: at each of the
-// first three levels a lane keeps half of its values and trades the other half with
-// its xor partner.  The additions are the butterfly's, so the bits are too.
-// On return lane l holds the total of value index 4*bit4(l) + 2*bit3(l) + bit2(l).
-__device__ __forceinline__ float warp_sum8(const float (&v)[8]) {
-  const int lane = threadIdx.x & 31;
-  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
-  float w[4], x[2];
+// One level of a warp's xor butterfly over N values at once: a lane keeps half of its values and sends the other half to its partner
+// `off` lanes away.  SWAPPED: the lanes with that bit set hold the two halves exchanged, so there is nothing to select; otherwise
+// they do not.  The additions are the butterfly's, so the bits are too.
+template <int N, bool SWAPPED>
+__device__ __forceinline__ void butterfly_level(float (&v)[N], int off) {
+  const bool upper = threadIdx.x & off;
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    float send = b4 ? v[i] : v[i + 4];
-    float keep = b4 ? v[i + 4] : v[i];
-    w[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, 16));
+  for (int i = 0; i < N / 2; i++) {
+    const float send = !SWAPPED && upper ? v[i] : v[i + N / 2], keep = !SWAPPED && upper ? v[i + N / 2] : v[i];
+    v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, off));
   }
-#pragma unroll
-  for (int i = 0; i < 2; i++) {
-    float send = b3 ? w[i] : w[i + 2];
-    float keep = b3 ? w[i + 2] : w[i];
-    x[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, 8));
-  }
-  float send = b2 ? x[0] : x[1];
-  float keep = b2 ? x[1] : x[0];
-  float y = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, 4));
-  y = __fadd_rn(y, __shfl_xor_sync(0xffffffffu, y, 2));
-  y = __fadd_rn(y, __shfl_xor_sync(0xffffffffu, y, 1));
-  return y;
 }
 
 // merge the splits of one (batch, q head) by one warp; lane l owns output dims [8l, 8l+8).
@@ -167,15 +152,20 @@ __device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, flo
 
 // dynamic shared memory layout (bytes):
 //   q_st  : 8*256 bf16                 4096
-//   k_st  : 256 bf16                    512
+//   k_st  : 256 bf16                    512   (the row this launch appends)
+//   v_st  : 256 bf16                    512
 //   m_s   : 8 f32 (+8 spare)             64
 //   l_s   : kW*8 f32                    256
-//   s_s   : split_len*8 f32
-//   o_s   : kW*8*256 f32              65536   (reused by the split merge)
-// One CTA per (split, KV head, batch).  Rows of the cache that were written in earlier steps do not depend on
-// the kernel running just before this one, so (p.settled) the first chunk of K rows and of V rows of every warp is
-// requested before the dependency wait; longer splits stream further chunks with the next
-// chunk in flight while the current one is reduced.  The CTA that finishes a (batch, KV head) last merges the splits.
+//   s_s   : split_len * heads (rounded up to a power of two) pairs of f32: the score, then p twice
+//   o_s   : kW*8*256 f32              65536   (the rings of rows, then the warps' sums, then the split merge)
+// One CTA per (split, KV head, batch).  Every warp streams its K rows and then its V rows through a ring of its own in shared memory,
+// 16 rows of 512 bytes, by asynchronous copies: a lane copies and reads back its own 16 bytes of a row, so nothing has to be
+// synchronised, the copies of the first V rows run under the scores and the softmax, and 16 warps keep up to 128 KB on the way.  (Rows in
+// registers, three of a warp on their way, 200 instructions per K row and V row: 8 sequences, 32,768 rows, 8 heads per KV head 209 us = 0.39 of
+// the copy rate, 6 heads and 4 KV heads 330 us, 4 and 1 90 us.  Now 157, 257 and 68 us; 163 instructions, 55 % of the issue slots, and what is
+// waited for are results of the instruction before: FMAs of one chain, shuffles.)  Rows of the
+// cache that were written in earlier steps do not depend on the kernel running just before this one, so (p.settled) the first rows are
+// requested before the dependency wait.  The CTA that finishes a (batch, KV head) last merges the splits.
 // Two CTAs per SM (at most 128 registers): with one CTA of 8 warps an SM cannot hide the latency of the per-row
 // shuffle reductions and the stream stalls.
 // Prompt columns: every column's K row (head norm + RoPE at its own position, the arithmetic of the decode step) and V
@@ -198,35 +188,23 @@ __global__ void __launch_bounds__(32) attn_append_kernel(const AttnParams p) {
       *reinterpret_cast<const uint4*>(p.v + ((size_t)b * p.Hkv + kvh) * kHD + lane * 8);
 }
 
-// warp_sum8 of values in the order g ^ (4 bit4 + 2 bit3 + bit2 of the lane): the same sums, addition for addition
-__device__ __forceinline__ float warp_sum8_swapped(const float (&v)[8]) {
-  float w[4], x[2];
-#pragma unroll
-  for (int i = 0; i < 4; i++) w[i] = __fadd_rn(v[i], __shfl_xor_sync(0xffffffffu, v[i + 4], 16));
-#pragma unroll
-  for (int i = 0; i < 2; i++) x[i] = __fadd_rn(w[i], __shfl_xor_sync(0xffffffffu, w[i + 2], 8));
-  float y = __fadd_rn(x[0], __shfl_xor_sync(0xffffffffu, x[1], 4));
-  y = __fadd_rn(y, __shfl_xor_sync(0xffffffffu, y, 2));
-  return __fadd_rn(y, __shfl_xor_sync(0xffffffffu, y, 1));
-}
+constexpr int kRows = 4;      // rows requested together
+constexpr int kBatches = 4;   // such batches of a warp on their way or in use
+static_assert(kRows * kBatches * kHD * 2 == 8 * kHD * 4, "a warp's ring is its part of o_s");
 
-template <int G, bool LONG>
+template <int G>
 __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams p) {
-  // Rows of one warp per register chunk (two chunks are live, the one in use and the next): as many as 128 registers hold
-  // without spilling, since the bytes in flight bound the few-head case (8 sequences, 20,000 rows, 4 heads: 4 rows 84 us, 6 rows 78) and
-  // the FMAs the many-head one (32,768 rows, 8 heads: 4 rows with 24 bytes spilled 218 us, 3 rows and the head order below 208).
-  // A short split of few heads takes 4 rows all the same: it has 8 to 32 rows a warp, and what a chunk of six holds beyond them is
-  // cleared and tested for nothing (launch_split).
-  constexpr int kCh = G <= 4 ? (LONG ? 6 : 4) : G >= 7 ? 3 : 4;
+  constexpr int GP = G <= 1 ? 1 : G <= 2 ? 2 : G <= 4 ? 4 : 8;   // heads, up to a power of two
   bk_pdl_trigger();
   bk_stamp(p.trace, 0);
   extern __shared__ __align__(16) uint8_t smem[];
   uint16_t* q_st = reinterpret_cast<uint16_t*>(smem);
   uint16_t* k_st = q_st + 8 * kHD;
-  float* m_s = reinterpret_cast<float*>(k_st + kHD);
+  uint16_t* v_st = k_st + kHD;
+  float* m_s = reinterpret_cast<float*>(v_st + kHD);
   float* l_s = m_s + 16;
-  float* s_s = l_s + kW * 8;
-  float* o_s = s_s + (size_t)p.split_len * 8;
+  float2* s_s = reinterpret_cast<float2*>(l_s + kW * 8);
+  float* o_s = reinterpret_cast<float*>(s_s + (size_t)p.split_len * GP);
   __shared__ int s_last;
 
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
@@ -236,25 +214,47 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   uint16_t* Vb = p.v_cache + ((size_t)cb * p.Hkv + kvh) * (size_t)p.max_len * kHD;
   const int j0 = split * p.split_len;
 
-  // rows of this warp: jj = warp + 8*i; chunk c holds i in [kCh*c, kCh*c + kCh)
-  uint4 kc[kCh], vc[kCh];
-  int pos = 0, ns = 0;
-  auto load_chunk = [&](const uint16_t* base, int c, uint4 (&dst)[kCh], bool skip_pos) {
-#pragma unroll
-    for (int e = 0; e < kCh; e++) {
-      const int jj = warp + 8 * (kCh * c + e);
-      const bool ok = jj < ns && !(skip_pos && j0 + jj == pos);
-      dst[e] = ok ? *reinterpret_cast<const uint4*>(base + (size_t)(j0 + jj) * kHD + lane * 8) : make_uint4(0, 0, 0, 0);
-    }
-  };
-  bool early = false;   // the first chunks were requested before the dependency wait and are still the right ones
-  if (p.settled) {
-    pos = p.pos[b];
+  // rows of this warp: jj = warp + 8*i, i < nr; its stream is nb batches of K rows, then as many of V rows
+  uint4* const ring = reinterpret_cast<uint4*>(o_s + (size_t)warp * 8 * kHD) + lane;   // this lane's 16 bytes of a row: ring[32 * slot]
+  const uint16_t* const Kw = Kb + (size_t)(j0 + warp) * kHD + lane * 8;
+  const uint16_t* const Vw = Vb + (size_t)(j0 + warp) * kHD + lane * 8;
+  int pos = 0, ns = 0, nr = 0, nb = 0, np = 0;   // np: rows that come from the cache
+  bool mine = false;                             // row np is the one at pos, which this launch may append
+  auto set_pos = [&](int at) {
+    pos = at;
     ns = min(pos + 1, j0 + p.split_len) - j0;   // <= 0: nothing to do for this split
-    if (ns > 0) {
-      load_chunk(Kb, 0, kc, true);
-      load_chunk(Vb, 0, vc, true);
+    nr = max(0, (ns - warp + 7) >> 3);
+    nb = (nr + kRows - 1) / kRows;
+    mine = nr > 0 && j0 + warp + 8 * (nr - 1) == pos;
+    np = nr - (mine ? 1 : 0);
+  };
+  auto copy = [&](uint32_t dst, const uint16_t* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+  };
+  // request batch q; own: the row at pos comes from shared memory, once it is there
+  auto request = [&](int q, bool own) {
+    if (q < 2 * nb) {
+      const bool is_v = q >= nb;
+      const int i = kRows * (is_v ? q - nb : q);
+      const uint16_t* src = (is_v ? Vw : Kw) + (uint32_t)i * (8 * kHD);
+      uint4* dst = ring + 32 * kRows * (q % kBatches);
+      if (i + kRows <= np) {
+#pragma unroll
+        for (int e = 0; e < kRows; e++) copy(smem_u32(dst) + e * 512, src + e * (8 * kHD));
+      } else {
+#pragma unroll 1
+        for (int e = 0; e < kRows && i + e < nr; e++) {
+          if (i + e < np) copy(smem_u32(dst) + e * 512, src + e * (8 * kHD));
+          else if (own) dst[32 * e] = *reinterpret_cast<const uint4*>((is_v ? v_st : k_st) + lane * 8);
+        }
+      }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  bool early = false;   // the first rows were requested before the dependency wait and are still the right ones
+  if (p.settled) {
+    set_pos(p.pos[b]);
+    for (int q = 0; q < kBatches; q++) request(q, false);
     early = true;
   }
   bk_pdl_wait();
@@ -264,13 +264,17 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
     // still have been running when the early part above read it.  A changed value discards the early loads.
     const int pos_now = __ldcg(p.pos + b);
     if (!early || pos_now != pos) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
       early = false;
-      pos = pos_now;
-      ns = min(pos + 1, j0 + p.split_len) - j0;
+      set_pos(pos_now);
     }
   }
-  if (ns <= 0) return;
+  if (ns <= 0) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    return;
+  }
   const int nsplits = (pos + p.split_len) / p.split_len;
+  const bool owner = pos >= j0 && pos < j0 + ns;
 
   // ---- phase 0: q (and, in the split that owns row pos, k/v append) ----
   if (p.fused) {
@@ -280,46 +284,48 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
       const uint16_t* src = p.qg + ((size_t)b * p.Hq + kvh * G + warp) * 2 * kHD;
       norm_rope_256(src, p.q_norm_w, cr, sr, p.rot_half, q_st + warp * kHD);
     }
-    if (p.n_seq == 0 && warp == kW - 1 && pos >= j0 && pos < j0 + ns) {
+    if (p.n_seq == 0 && warp == kW - 1 && owner) {
+      const uint4 v = *reinterpret_cast<const uint4*>(p.v + ((size_t)b * p.Hkv + kvh) * kHD + lane * 8);
       norm_rope_256(p.k + ((size_t)b * p.Hkv + kvh) * kHD, p.k_norm_w, cr, sr, p.rot_half, k_st);
       *reinterpret_cast<uint4*>(Kb + (size_t)pos * kHD + lane * 8) = *reinterpret_cast<const uint4*>(k_st + lane * 8);
-      *reinterpret_cast<uint4*>(Vb + (size_t)pos * kHD + lane * 8) =
-          *reinterpret_cast<const uint4*>(p.v + ((size_t)b * p.Hkv + kvh) * kHD + lane * 8);
+      *reinterpret_cast<uint4*>(Vb + (size_t)pos * kHD + lane * 8) = v;
+      *reinterpret_cast<uint4*>(v_st + lane * 8) = v;
     }
   } else {
     if (warp < G)
       *reinterpret_cast<uint4*>(q_st + warp * kHD + lane * 8) =
           *reinterpret_cast<const uint4*>(p.qg + ((size_t)b * p.Hq + kvh * G + warp) * kHD + lane * 8);
   }
-  __syncthreads();  // the appended K/V row is visible to this CTA from here on
+  if ((!p.fused || p.n_seq > 0) && warp == kW - 1 && owner) {   // the row is in the cache
+    *reinterpret_cast<uint4*>(k_st + lane * 8) = *reinterpret_cast<const uint4*>(Kb + (size_t)pos * kHD + lane * 8);
+    *reinterpret_cast<uint4*>(v_st + lane * 8) = *reinterpret_cast<const uint4*>(Vb + (size_t)pos * kHD + lane * 8);
+  }
+  __syncthreads();   // q and the row at pos are in shared memory
   bk_stamp(p.trace, 3);
   if (!early) {
-    load_chunk(Kb, 0, kc, false);
-    load_chunk(Vb, 0, vc, false);
-  } else {
-    // the row appended above was left out of the early loads
-    const int jp = pos - j0;
-    if (jp >= 0 && jp < ns && (jp & 7) == warp && (jp >> 3) < kCh) {
-      const int e = jp >> 3;
-#pragma unroll
-      for (int i = 0; i < kCh; i++)
-        if (i == e) {
-          kc[i] = *reinterpret_cast<const uint4*>(Kb + (size_t)pos * kHD + lane * 8);
-          vc[i] = *reinterpret_cast<const uint4*>(Vb + (size_t)pos * kHD + lane * 8);
-        }
-    }
+    for (int q = 0; q < kBatches; q++) request(q, true);
+  } else if (mine) {   // left out of the early requests
+    const int q = np / kRows, e = np % kRows;
+    if (q < kBatches) ring[32 * (kRows * q + e)] = *reinterpret_cast<const uint4*>(k_st + lane * 8);
+    if (q + nb < kBatches) ring[32 * (kRows * (q + nb) + e)] = *reinterpret_cast<const uint4*>(v_st + lane * 8);
   }
-  const int nchunks = (ns + 8 * kCh - 1) / (8 * kCh);
 
   // ---- phase 1: scores ----
   {
     // query heads in pairs {q_g[d], q_g+1[d]}: one packed FMA advances the dot products of two heads (each its own
     // chain over d, as before)
-    float2 qp[(G + 1) / 2][8];
-    const int hsel = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);   // the head whose score this lane ends up with
-    // Eight heads: a lane takes them in the order g ^ hsel, so that in each of the first three levels of the reduction it keeps the
-    // first half of its values and sends the second -- nothing to select.
-    const int swap = G == 8 ? hsel : 0;
+    // The 5 levels of the warp's butterfly halve what a lane still holds, the scores of four rows: with heads a power of two in number
+    // first a row's heads, then the rows, otherwise the rows first, so that 4 rows of 8 heads take 31 shuffles (one by one 36).  A
+    // lane takes what the first levels halve in an order of its own, g ^ hsel or r ^ rsel, so that in each of them it keeps the first half
+    // and sends the second.
+    constexpr bool kHeadsFirst = G == GP;
+    constexpr int kTurn = GP <= 2 ? 2 : 1, R = kRows * kTurn;   // batches, rows scored together: eight where they have few heads (latency, not work)
+    constexpr int HB = GP == 8 ? 3 : GP == 4 ? 2 : GP == 2 ? 1 : 0, RB = kTurn + 1, kPlain = 5 - HB - RB;   // levels that halve heads, rows, nothing
+    const int hsel = kHeadsFirst ? lane >> (5 - HB) : (lane >> kPlain) & (GP - 1);   // the head and the row whose score this lane ends up with
+    const int rsel = kHeadsFirst ? (lane >> kPlain) & (R - 1) : lane >> 3;
+    const int swap = kHeadsFirst ? hsel : 0;
+    constexpr int GH = (G + 1) / 2;
+    float2 qp[GH][8];
 #pragma unroll
     for (int g = 0; g < G; g += 2) {
       float q0[8], q1[8];
@@ -328,33 +334,75 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
 #pragma unroll
       for (int d = 0; d < 8; d++) qp[g >> 1][d] = make_float2(q0[d], g + 1 < G ? q1[d] : 0.0f);
     }
-    for (int c = 0; c < nchunks; c++) {
-      uint4 kn[kCh];
-      if (c + 1 < nchunks) load_chunk(Kb, c + 1, kn, false);
+#pragma unroll 1
+    for (int q = 0; q < nb; q += kTurn) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kBatches - kTurn) : "memory");   // batches q and, of two, q + 1 have landed
+      // this lane's part of the dot products of row r ^ rsel (a row past the last is whatever the ring holds: its scores are not stored)
+      auto dots = [&](int r, float (&pa)[GP]) {
+        float kf[8];
+        bf16x8_to_f32(ring[32 * ((kRows * q + (r ^ rsel)) % (kRows * kBatches))], kf);
+        float2 a2[GH];
 #pragma unroll
-      for (int e = 0; e < kCh; e++) {
-        const int jj = warp + 8 * (kCh * c + e);
-        if (jj < ns) {   // warp-uniform
-          float kf[8], pa[8];
-          bf16x8_to_f32(kc[e], kf);
+        for (int g = 0; g < GH; g++) a2[g] = make_float2(0.0f, 0.0f);
 #pragma unroll
-          for (int g = 0; g < 8; g += 2) {
-            float2 a2 = make_float2(0.0f, 0.0f);
-            if (g < G) {
+        for (int d = 0; d < 8; d++)
 #pragma unroll
-              for (int d = 0; d < 8; d++) a2 = bk_fma2(qp[(g < G ? g : 0) >> 1][d], make_float2(kf[d], kf[d]), a2);
-            }
-            pa[g] = a2.x;
-            pa[g + 1] = a2.y;
+          for (int g = 0; g < GH; g++) a2[g] = bk_fma2(qp[g][d], make_float2(kf[d], kf[d]), a2[g]);
+#pragma unroll
+        for (int g = 0; g < GP; g++) pa[g] = g / 2 >= GH ? 0.0f : g & 1 ? a2[g / 2 < GH ? g / 2 : 0].y : a2[g / 2 < GH ? g / 2 : 0].x;
+      };
+      float s1;
+      if constexpr (kHeadsFirst) {
+        float y[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          float pa[GP];
+          dots(r, pa);
+          if constexpr (GP == 8) {
+            butterfly_level<8, true>(pa, 16);
+            butterfly_level<4, true>(reinterpret_cast<float(&)[4]>(pa), 8);
+            butterfly_level<2, true>(reinterpret_cast<float(&)[2]>(pa), 4);
+          } else if constexpr (GP == 4) {
+            butterfly_level<4, true>(pa, 16);
+            butterfly_level<2, true>(reinterpret_cast<float(&)[2]>(pa), 8);
+          } else if constexpr (GP == 2) {
+            butterfly_level<2, true>(pa, 16);
           }
-          const float s1 = G == 8 ? warp_sum8_swapped(pa) : warp_sum8(pa);
-          if ((lane & 3) == 0) s_s[(size_t)jj * 8 + hsel] = __fmul_rn(s1, p.scale);
+          y[r] = pa[0];
         }
-      }
-      if (c + 1 < nchunks) {
+        if constexpr (kTurn == 2) butterfly_level<8, true>(y, 16 >> HB);
+        butterfly_level<4, true>(reinterpret_cast<float(&)[4]>(y), (1 << kPlain) * 2);
+        butterfly_level<2, true>(reinterpret_cast<float(&)[2]>(y), 1 << kPlain);
+        s1 = y[0];
+      } else {
+        float lo[GP], hi[GP];   // rows 0, 1 of the lane's order, plus what their partners have of them
+        auto two_rows = [&](int r, float (&v)[GP]) {   // rows r and r + 2
+          float w[GP];
+          dots(r, v);
+          dots(r + 2, w);
 #pragma unroll
-        for (int e = 0; e < kCh; e++) kc[e] = kn[e];
+          for (int g = 0; g < G; g++) v[g] = __fadd_rn(v[g], __shfl_xor_sync(0xffffffffu, w[g], 16));
+        };
+        two_rows(0, lo);
+        two_rows(1, hi);
+#pragma unroll
+        for (int g = 0; g < G; g++) lo[g] = __fadd_rn(lo[g], __shfl_xor_sync(0xffffffffu, hi[g], 8));
+        if constexpr (GP == 8) {
+          butterfly_level<8, false>(lo, 4);
+          butterfly_level<4, false>(reinterpret_cast<float(&)[4]>(lo), 2);
+          butterfly_level<2, false>(reinterpret_cast<float(&)[2]>(lo), 1);
+        } else {
+          butterfly_level<4, false>(lo, 4);
+          butterfly_level<2, false>(reinterpret_cast<float(&)[2]>(lo), 2);
+        }
+        s1 = lo[0];
       }
+#pragma unroll
+      for (int off = (1 << kPlain) >> 1; off >= 1; off >>= 1) s1 = __fadd_rn(s1, __shfl_xor_sync(0xffffffffu, s1, off));
+      const int i = kRows * q + rsel;
+      if ((lane & ((1 << kPlain) - 1)) == 0 && i < nr) s_s[(size_t)(warp + 8 * i) * GP + hsel].x = __fmul_rn(s1, p.scale);
+      request(q + kBatches, true);
+      if (kTurn == 2 && q + 1 < nb) request(q + 1 + kBatches, true);   // (else batch q + 1 is the first of the V rows)
     }
   }
   __syncthreads();
@@ -362,14 +410,15 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
 
   // ---- phase 2: exact max per head, p = exp(s - m) in place ----
   {
-    const int g = tid & 7;
+    constexpr int kStep = kW * 32 / GP;
+    const int g = tid & (GP - 1);
     float m = -INFINITY;
-    for (int jj = tid >> 3; jj < ns; jj += (kW * 32) >> 3) m = fmaxf(m, s_s[(size_t)jj * 8 + g]);
-    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
-    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
-    if (lane < 8) l_s[warp * 8 + lane] = m;  // l_s doubles as the cross-warp max buffer
+    for (int jj = tid / GP; jj < ns; jj += kStep) m = fmaxf(m, s_s[(size_t)jj * GP + g].x);
+#pragma unroll
+    for (int off = GP; off < 32; off <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+    if (lane < GP) l_s[warp * 8 + lane] = m;  // l_s doubles as the cross-warp max buffer
     __syncthreads();
-    if (tid < 8) {
+    if (tid < GP) {
       float mm = l_s[tid];
 #pragma unroll
       for (int w = 1; w < kW; w++) mm = fmaxf(mm, l_s[w * 8 + tid]);
@@ -377,9 +426,9 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
     }
     __syncthreads();
     const float mg = m_s[g];
-    for (int jj = tid >> 3; jj < ns; jj += (kW * 32) >> 3) {
-      float sv = s_s[(size_t)jj * 8 + g];
-      s_s[(size_t)jj * 8 + g] = (g < G) ? bk_expf(__fsub_rn(sv, mg)) : 0.0f;
+    for (int jj = tid / GP; jj < ns; jj += kStep) {
+      const float e = g < G ? bk_expf(__fsub_rn(s_s[(size_t)jj * GP + g].x, mg)) : 0.0f;
+      s_s[(size_t)jj * GP + g] = make_float2(e, e);   // twice: the factor of a packed FMA
     }
   }
   __syncthreads();
@@ -387,48 +436,51 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   // ---- phase 3: o = sum p * V ----
   {
     float2 acc[G][4];   // dims (2i, 2i+1) side by side: one packed FMA per pair
-    float2 lw[(G + 1) / 2];   // heads 2i, 2i+1
-#pragma unroll
-    for (int g = 0; g < (G + 1) / 2; g++) lw[g] = make_float2(0.0f, 0.0f);
+    float lw = 0.0f;    // of head lane mod GP
 #pragma unroll
     for (int g = 0; g < G; g++) {
 #pragma unroll
       for (int e = 0; e < 4; e++) acc[g][e] = make_float2(0.0f, 0.0f);
     }
-    for (int c = 0; c < nchunks; c++) {
-      uint4 vn[kCh];
-      if (c + 1 < nchunks) load_chunk(Vb, c + 1, vn, false);
+#pragma unroll 1
+    for (int q = 0; q < nb; q++) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kBatches - 1) : "memory");   // batch nb + q has landed
+      const uint4* rows = ring + 32 * kRows * ((nb + q) % kBatches);
 #pragma unroll
-      for (int e = 0; e < kCh; e++) {
-        const int jj = warp + 8 * (kCh * c + e);
-        if (jj < ns) {
+      for (int r = 0; r < kRows; r++) {
+        const int i = kRows * q + r;
+        if (i < nr) {   // warp-uniform
           float vf[8];
-          bf16x8_to_f32(vc[e], vf);
-          const float4 p0 = *reinterpret_cast<const float4*>(s_s + (size_t)jj * 8);
-          const float4 p1 = *reinterpret_cast<const float4*>(s_s + (size_t)jj * 8 + 4);
-          const float pp[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+          bf16x8_to_f32(rows[32 * r], vf);
+          const float2* ps = s_s + (size_t)(warp + 8 * i) * GP;
+          lw = __fadd_rn(lw, ps[lane & (GP - 1)].x);
 #pragma unroll
-          for (int g = 0; g < G; g += 2) lw[g >> 1] = bk_add2(lw[g >> 1], make_float2(pp[g], pp[g + 1]));
+          for (int g = 0; g < G; g += 2) {
+            float2 pg[2];
+            if (GP > 1) {
+              const float4 pp = *reinterpret_cast<const float4*>(ps + g);
+              pg[0] = make_float2(pp.x, pp.y);
+              pg[1] = make_float2(pp.z, pp.w);
+            } else pg[0] = ps[0];
 #pragma unroll
-          for (int g = 0; g < G; g++) {
-            const float2 p2 = make_float2(pp[g], pp[g]);
+            for (int h = 0; h < 2; h++)
+              if (g + h < G) {
 #pragma unroll
-            for (int d = 0; d < 4; d++) acc[g][d] = bk_fma2(p2, make_float2(vf[2 * d], vf[2 * d + 1]), acc[g][d]);
+                for (int d = 0; d < 4; d++) acc[g + h < G ? g + h : 0][d] = bk_fma2(pg[h], make_float2(vf[2 * d], vf[2 * d + 1]), acc[g + h < G ? g + h : 0][d]);
+              }
           }
         }
       }
-      if (c + 1 < nchunks) {
-#pragma unroll
-        for (int e = 0; e < kCh; e++) vc[e] = vn[e];
-      }
+      request(nb + q + kBatches, true);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll
-    for (int g = 0; g < G; g++) {
+    for (int g = 0; g < G; g++) {   // over this warp's ring
       float4* d = reinterpret_cast<float4*>(o_s + ((size_t)(warp * 8 + g)) * kHD + lane * 8);
       d[0] = make_float4(acc[g][0].x, acc[g][0].y, acc[g][1].x, acc[g][1].y);
       d[1] = make_float4(acc[g][2].x, acc[g][2].y, acc[g][3].x, acc[g][3].y);
-      if (lane == 0) l_s[warp * 8 + g] = g & 1 ? lw[g >> 1].y : lw[g >> 1].x;
     }
+    if (lane < G) l_s[warp * 8 + lane] = lw;
   }
   __syncthreads();
   bk_stamp(p.trace, 6);
@@ -469,26 +521,22 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   bk_stamp(p.trace, 5);
 }
 
-size_t attn_smem_bytes(int split_len) { return 4096 + 512 + 64 + 256 + (size_t)split_len * 32 + (size_t)kW * 8 * kHD * 4; }
+size_t attn_smem_bytes(int split_len, int heads) {
+  const int gp = heads <= 1 ? 1 : heads <= 2 ? 2 : heads <= 4 ? 4 : 8;
+  return 4096 + 1024 + 64 + 256 + (size_t)split_len * gp * 8 + (size_t)kW * 8 * kHD * 4;
+}
 
-template <int G, bool LONG>
-int32_t launch_split_rows(const AttnParams& p, dim3 grid, size_t smem) {
+template <int G>
+int32_t launch_split(const AttnParams& p, dim3 grid) {
   static size_t configured = 0;
+  const size_t smem = attn_smem_bytes(p.split_len, G);
   if (smem > configured) {
-    BK_CUDA(cudaFuncSetAttribute(attn_split_kernel<G, LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BK_CUDA(cudaFuncSetAttribute(attn_split_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = smem;
   }
-  BK_CUDA(bk_launch_pdl(attn_split_kernel<G, LONG>, grid, dim3(kW * 32), smem, p));
+  BK_CUDA(bk_launch_pdl(attn_split_kernel<G>, grid, dim3(kW * 32), smem, p));
   BK_CHECK_LAUNCH();
   return BK_OK;
-}
-// Chunks of six rows from splits of more than 256 rows on.  Two heads per KV head, 2 KV heads, chunks of 4 / 6 rows: splits of 64 rows (1
-// sequence, 1,000 rows) 10.5 / 11.1 us, of 256 (8 sequences, 4,096 rows) 23.2 / 22.8, of 512 (8 sequences, 32,768 rows) 163 / 149.
-template <int G>
-int32_t launch_split(const AttnParams& p, dim3 grid, size_t smem) {
-  if constexpr (G <= 4)
-    if (p.split_len > 256) return launch_split_rows<G, true>(p, grid, smem);
-  return launch_split_rows<G, false>(p, grid, smem);
 }
 
 }  // namespace
@@ -598,18 +646,17 @@ int32_t bk_attn_launch(const bkAttnArgs& args, int n_seq, int layout_B) {
     BK_CUDA(bk_launch_pdl(attn_append_kernel, dim3(a.Hkv, a.B), dim3(32), 0, p));
     BK_CHECK_LAUNCH();
   }
-  size_t smem = attn_smem_bytes(split_len);
   dim3 grid(nsplit, a.Hkv, a.B);
   int32_t rc;
   switch (a.Hq / a.Hkv) {
-    case 1: rc = launch_split<1>(p, grid, smem); break;
-    case 2: rc = launch_split<2>(p, grid, smem); break;
-    case 3: rc = launch_split<3>(p, grid, smem); break;
-    case 4: rc = launch_split<4>(p, grid, smem); break;
-    case 5: rc = launch_split<5>(p, grid, smem); break;
-    case 6: rc = launch_split<6>(p, grid, smem); break;
-    case 7: rc = launch_split<7>(p, grid, smem); break;
-    default: rc = launch_split<8>(p, grid, smem); break;
+    case 1: rc = launch_split<1>(p, grid); break;
+    case 2: rc = launch_split<2>(p, grid); break;
+    case 3: rc = launch_split<3>(p, grid); break;
+    case 4: rc = launch_split<4>(p, grid); break;
+    case 5: rc = launch_split<5>(p, grid); break;
+    case 6: rc = launch_split<6>(p, grid); break;
+    case 7: rc = launch_split<7>(p, grid); break;
+    default: rc = launch_split<8>(p, grid); break;
   }
   if (rc) return rc;
   return BK_OK;

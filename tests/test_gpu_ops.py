@@ -329,6 +329,22 @@ def test_attn_decode_ragged_positions_and_plain(bk):
     assert rel_err(synth.bf16_to_f32(got[b, h * HD:(h + 1) * HD]), plain) < 5e-3  # bf16 output rounding
 
 
+@pytest.mark.parametrize("Hq,Hkv", [(1, 1), (4, 2), (6, 2), (8, 2), (5, 1), (6, 1), (7, 1), (8, 1)])
+def test_attn_decode_row_lists(bk, Hq, Hkv):
+    """Lists of rows of a warp that end in every place of a batch of four and of a ring of sixteen, the appended row among the first sixteen and after
+    them, splits of one row, for every number of query heads per KV head."""
+    cos_t, sin_t = ops.rope_tables(1024)
+    B, L, split_len = 6, 640, 320   # 40 rows a warp
+    c = synth.attn_case(B, L, Hq=Hq, Hkv=Hkv, max_len=640, config_id=70 + Hq)
+    for pos in ([0, 7, 8, 30, 33, 63], [96, 127, 128, 130, 167, 200], [319, 320, 327, 450, 452, 639]):
+        c["pos"] = np.array(pos, np.int32)
+        got, Kg, Vg, split_len, W = _run_attn(c, cos_t, sin_t, split_len=split_len)
+        q, Kc, Vc, want = _attn_oracle(c, cos_t, sin_t, split_len, W)
+        assert_same_bits(Kg, Kc, "k cache after append")
+        assert_same_bits(Vg, Vc, "v cache after append")
+        assert_same_bits(got, want, f"attention, {Hq} heads on {Hkv}, positions {pos}")
+
+
 @pytest.mark.parametrize("B,L", [(1, 32768), (8, 4096), (8, 32768)])
 def test_attn_decode_long_context(bk, B, L):
     """configs[2] long caches (4096 and 32768 rows) at batch 1 and 8, default plan; bit-exact against the oracle."""
