@@ -1,82 +1,159 @@
 // bk_quantize.cu -- f32 / bf16 weight rows -> Q4_K superblocks on the device: the quantiser behind the weight loader.
 //
 // bunker uploads its safetensors weights as they are, bf16 (loadWeights, prototypes/decode.ts:64-76); the Q4_K model
-// served here needs them quantised once at load time.  Half a warp per 256-weight superblock, lane l of it holding weights
-// [16l, 16l+16) (half of sub-block l/2).  The arithmetic is the CPU oracle's, operation for operation:
+// served here needs them quantised once at load time.  A lane takes a sub-block of 32 weights, a warp four superblocks of 256.  The
+// arithmetic is the CPU oracle's, operation for operation:
 //   sub-block:  lo = min(min x, 0), scale = (max x - lo) / 15, mn = 0 - lo
 //   superblock: d = f16_rn(max scale / 63), dmin = f16_rn(max mn / 63), sc = floor(scale * (1/d) + 0.5) (<= 63),
 //               m = floor(mn * (1/dmin) + 0.5) (<= 63)
 //   weight:     q = clamp(floor((x + dmin*m) / (d*sc) + 0.5), 0, 15)
 // Output layout: bytes [0,2) d, [2,4) dmin, [4,16) the twelve 6-bit scale/min bytes, [16,144) quants, every 32 bytes
 // serving sub-blocks 2p (low nibbles) and 2p+1 (high nibbles).
+#include <algorithm>
+
 #include "bk_common.cuh"
 #include "bk_internal.h"
 
 namespace {
 
-constexpr int kQWarps = 8;   // warps of a CTA, two superblocks each
+constexpr int kQWarps = 4;   // warps of a CTA
+constexpr int kQSb = 4;      // superblocks of a warp
 
-// floor(t / dl + 0.5) clamped to 0..15, the division and the addition each rounded once.  The quotient is first formed
-// with the approximate reciprocal (relative error below 2^-21): unless it lies within kTieBand of a rounding boundary
-// the integer is already the exact one.
-constexpr float kTieBand = 2e-5f;
-BK_DEVINL int quant4_exact(float t, float dl) { return max(0, min(15, (int)floorf(__fadd_rn(__fdiv_rn(t, dl), 0.5f)))); }
+// floor(t / dl + 0.5) clamped to 0..15, t = w + ml, the sum, the division and the addition each rounded once.  The quotient is first formed as
+// w * r + ml * r with the approximate reciprocal r (off by at most 2^-23 of it) and rounded to the nearest integer.  With ml * r up to 32 it
+// is off by less than 4e-6 for r and ml * r and 1e-6 for its own rounding, and the exact one by 2.4e-6 for its three, below 16: unless it
+// lies within kTieBand of a half the integer is already the exact one.
+constexpr float kTieBand = 1e-5f, kMaxMlr = 32.0f;
+BK_DEVINL uint32_t quant4_exact(float t, float dl) { return (uint32_t)max(0, min(15, (int)floorf(__fadd_rn(__fdiv_rn(t, dl), 0.5f)))); }
 
-BK_DEVINL float2 add2_rd(float2 a, float2 b) {   // rounding down
-  unsigned long long ra, rb, rd;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
-  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
-  float2 d;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
+BK_DEVINL uint32_t min_bf2(uint32_t a, uint32_t b) {   // like fminf: a NaN loses
+  uint32_t d;
+  asm("min.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
-
-// 16 lanes per superblock, 16 weights each (half a sub-block): two superblocks per warp share the scalar work, and a
-// superblock leaves through shared memory as 16-byte stores.  Issue-bound, the half-rate minima and maxima above all: 17408 x
-// 5120 bf16 took 123 us with eight IEEE divisions per thread and byte stores (1.86 TB/s), 78 us with one weight at a time, 73 us with
-// two (3.1 TB/s).
+BK_DEVINL uint32_t max_nan_bf2(uint32_t a, uint32_t b) {   // a NaN wins
+  uint32_t d;
+  asm("max.NaN.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+BK_DEVINL float max_nan(float a, float b) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
+// chunk c of a row of 16-byte chunks: rows are permuted so that the lanes' reads hit all banks
 template <bool BF16>
-__global__ void __launch_bounds__(kQWarps * 32) quantize_q4k_kernel(const void* x, size_t n_superblocks, uint8_t* out) {
-  __shared__ __align__(16) uint8_t stage[kQWarps][2 * 144];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4, l = lane & 15;
-  const size_t first = ((size_t)blockIdx.x * kQWarps + warp) * 2;
-  if (first >= n_superblocks) return;   // whole warps leave together
-  const size_t sb_idx = min(first + half, n_superblocks - 1);   // a last odd superblock is computed twice and stored once
-  float v[16];
+BK_DEVINL int chunk_slot(int row, int c) {
+  return BF16 ? row * 4 + (c ^ ((row >> 1) & 3)) : row * 8 + (c ^ (row & 7));
+}
+// weight e of this lane's sub-block, for what hardly ever runs
+template <bool BF16>
+BK_DEVINL float one_weight(const uint4* rows, int e) {
+  const int lane = threadIdx.x & 31;
+  if (BF16) return bk_bf16_to_f32(reinterpret_cast<const uint16_t*>(rows + chunk_slot<BF16>(lane, e >> 3))[e & 7]);
+  return reinterpret_cast<const float*>(rows + chunk_slot<BF16>(lane, e >> 2))[e & 3];
+}
+template <bool BF16>
+__device__ __noinline__ float largest_number(const uint4* rows) {
+  float hi = one_weight<BF16>(rows, 0);
+#pragma unroll 1
+  for (int e = 1; e < 32; e++) hi = fmaxf(hi, one_weight<BF16>(rows, e));
+  return hi;
+}
+// the exact quants of weights 8c to 8c + 7, a byte each
+template <bool BF16>
+__device__ __noinline__ uint2 exact_quants(const uint4* rows, int c, float ml, float dl) {
+  uint32_t q[2] = {0u, 0u};
+#pragma unroll 1
+  for (int e = 0; e < 4; e++) {
+    q[0] |= quant4_exact(__fadd_rn(one_weight<BF16>(rows, 8 * c + e), ml), dl) << (8 * e);
+    q[1] |= quant4_exact(__fadd_rn(one_weight<BF16>(rows, 8 * c + 4 + e), ml), dl) << (8 * e);
+  }
+  return make_uint2(q[0], q[1]);
+}
+
+// The quants of this lane's sub-block, with the neighbour's, into their 32 bytes.  PLAIN: no weight of the warp leaves 0..15, none is a NaN, and
+// ml * r is small.  Rounding without conversions: y + 1.5 * 2^23 has the integer in its low bits; two weights per instruction.
+template <bool BF16, bool PLAIN>
+BK_DEVINL void write_quants(const uint4* rows, uint8_t* quants, float r, float mlr, float ml, float dl) {
+  constexpr float kMagic = 12582912.0f;
+  const int lane = threadIdx.x & 31;
+  const bool odd = lane & 1;
+  const float2 magic2 = make_float2(kMagic, kMagic), minus2 = make_float2(-1.0f, -1.0f), r2 = make_float2(r, r), c2 = PLAIN ? make_float2(mlr, mlr) : make_float2(0.0f, 0.0f);
+#pragma unroll
+  for (int c = 0; c < 4; c++) {   // eight weights, read again: kept in registers since the first pass they cost a third of the warps
+    float w[8];
+    if (BF16) {
+      const uint4 v = rows[chunk_slot<BF16>(lane, c)];
+      w[0] = __uint_as_float(v.x << 16); w[1] = __uint_as_float(v.x & 0xffff0000u);
+      w[2] = __uint_as_float(v.y << 16); w[3] = __uint_as_float(v.y & 0xffff0000u);
+      w[4] = __uint_as_float(v.z << 16); w[5] = __uint_as_float(v.z & 0xffff0000u);
+      w[6] = __uint_as_float(v.w << 16); w[7] = __uint_as_float(v.w & 0xffff0000u);
+    } else {
+      const uint4 v = rows[chunk_slot<BF16>(lane, 2 * c)], u = rows[chunk_slot<BF16>(lane, 2 * c + 1)];
+      w[0] = __uint_as_float(v.x); w[1] = __uint_as_float(v.y); w[2] = __uint_as_float(v.z); w[3] = __uint_as_float(v.w);
+      w[4] = __uint_as_float(u.x); w[5] = __uint_as_float(u.y); w[6] = __uint_as_float(u.z); w[7] = __uint_as_float(u.w);
+    }
+    uint32_t t[8];
+    float tie = 0.0f;   // largest distance from an integer
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+      float2 x = make_float2(w[e], w[e + 1]);
+      if (!PLAIN) x = bk_add2(x, make_float2(ml, ml));
+      const float2 y = bk_fma2(x, r2, c2);
+      float2 f = bk_add2(y, magic2);
+      const float2 o = bk_add2(y, bk_fma2(f, minus2, magic2));
+      tie = fmaxf(tie, fmaxf(fabsf(o.x), fabsf(o.y)));
+      if (!PLAIN) f = make_float2(fminf(fmaxf(f.x, kMagic), kMagic + 15.0f), fminf(fmaxf(f.y, kMagic), kMagic + 15.0f));   // (a NaN becomes 0)
+      t[e] = __float_as_uint(f.x);
+      t[e + 1] = __float_as_uint(f.y);
+    }
+    uint2 q;   // a quant per byte
+    q.x = __byte_perm(__byte_perm(t[0], t[1], 0x0040), __byte_perm(t[2], t[3], 0x0040), 0x5410);
+    q.y = __byte_perm(__byte_perm(t[4], t[5], 0x0040), __byte_perm(t[6], t[7], 0x0040), 0x5410);
+    if (tie > 0.5f - kTieBand) q = exact_quants<BF16>(rows, c, ml, dl);
+    if (!PLAIN && !(dl > 0.0f)) q = make_uint2(0u, 0u);
+    // of the pair of lanes the even one writes the first four bytes, the odd one the others
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, odd ? q.x : q.y, 1);
+    *reinterpret_cast<uint32_t*>(quants + 8 * c) = odd ? other | (q.y << 4) : q.x | (other << 4);
+  }
+}
+
+// the 1,024 weights in `rows` to four superblocks in `stage`; sub-block `lane` is this lane's
+template <bool BF16>
+BK_DEVINL void quantize_superblocks(const uint4* rows, uint8_t* stage) {
+  constexpr int kChunks = BF16 ? 4 : 8;
+  const int lane = threadIdx.x & 31, l = lane & 7;
+  float lo, hi;
   if (BF16) {
-    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(x) + sb_idx * 256 + l * 16);
+    uint32_t mn2, mx2;   // of the even and of the odd weights, as the bf16 pairs that they are
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const uint4 r = __ldcs(src + k);
-      v[8 * k + 0] = __uint_as_float(r.x << 16); v[8 * k + 1] = __uint_as_float(r.x & 0xffff0000u);
-      v[8 * k + 2] = __uint_as_float(r.y << 16); v[8 * k + 3] = __uint_as_float(r.y & 0xffff0000u);
-      v[8 * k + 4] = __uint_as_float(r.z << 16); v[8 * k + 5] = __uint_as_float(r.z & 0xffff0000u);
-      v[8 * k + 6] = __uint_as_float(r.w << 16); v[8 * k + 7] = __uint_as_float(r.w & 0xffff0000u);
+    for (int c = 0; c < kChunks; c++) {
+      const uint4 v = rows[chunk_slot<BF16>(lane, c)];
+      const uint32_t mn = min_bf2(min_bf2(v.x, v.y), min_bf2(v.z, v.w)), mx = max_nan_bf2(max_nan_bf2(v.x, v.y), max_nan_bf2(v.z, v.w));
+      mn2 = c == 0 ? mn : min_bf2(mn2, mn);
+      mx2 = c == 0 ? mx : max_nan_bf2(mx2, mx);
     }
+    lo = fminf(__uint_as_float(mn2 << 16), __uint_as_float(mn2 & 0xffff0000u));
+    hi = max_nan(__uint_as_float(mx2 << 16), __uint_as_float(mx2 & 0xffff0000u));
   } else {
-    const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + sb_idx * 256 + l * 16);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const float4 r = __ldcs(src + k);
-      v[4 * k] = r.x; v[4 * k + 1] = r.y; v[4 * k + 2] = r.z; v[4 * k + 3] = r.w;
+    for (int c = 0; c < kChunks; c++) {
+      const float4 v = *reinterpret_cast<const float4*>(rows + chunk_slot<BF16>(lane, c));
+      const float mn = fminf(fminf(v.x, v.y), fminf(v.z, v.w)), mx = max_nan(max_nan(v.x, v.y), max_nan(v.z, v.w));
+      lo = c == 0 ? mn : fminf(lo, mn);
+      hi = c == 0 ? mx : max_nan(hi, mx);
     }
   }
-  float lo = v[0], hi = v[0];
-#pragma unroll
-  for (int e = 1; e < 16; e++) {
-    lo = fminf(lo, v[e]);
-    hi = fmaxf(hi, v[e]);
-  }
-  lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, 1));   // the two lanes of a sub-block
-  hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, 1));
+  const bool has_nan = hi != hi;   // a NaN counts for neither end and becomes 0
+  if (has_nan) hi = largest_number<BF16>(rows);
   if (lo > 0.0f) lo = 0.0f;
   float scale = __fdiv_rn(__fsub_rn(hi, lo), 15.0f);
   if (!(scale > 0.0f)) scale = 0.0f;
   const float mn = __fsub_rn(0.0f, lo);   // 0 - lo, not -lo: a zero minimum stays +0 (its sign would reach the f16 dmin)
   float max_scale = scale, max_min = mn;
 #pragma unroll
-  for (int off = 2; off <= 8; off <<= 1) {
+  for (int off = 1; off <= 4; off <<= 1) {
     max_scale = fmaxf(max_scale, __shfl_xor_sync(0xffffffffu, max_scale, off));
     max_min = fmaxf(max_min, __shfl_xor_sync(0xffffffffu, max_min, off));
   }
@@ -88,56 +165,63 @@ __global__ void __launch_bounds__(kQWarps * 32) quantize_q4k_kernel(const void* 
   const int sc = min(63, (int)floorf(__fadd_rn(__fmul_rn(scale, inv_d), 0.5f)));
   const int m6 = min(63, (int)floorf(__fadd_rn(__fmul_rn(mn, inv_dm), 0.5f)));
   const float dl = __fmul_rn(d, (float)sc), ml = __fmul_rn(dm, (float)m6);
-  uint32_t q[4] = {0u, 0u, 0u, 0u};   // sixteen 4-bit quants, one per byte
-  if (dl > 0.0f) {
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(dl));
-    // floor without conversions: y + 1.5 * 2^23 rounded down has floor(y) in its low bits, and the clamp to 0..15 is one of floats
-    float off_tie = 0.0f;   // largest distance of a fraction from 1/2
-    uint32_t t[16];
-    const float2 ml2 = make_float2(ml, ml), r2 = make_float2(r, r), half2 = make_float2(0.5f, 0.5f);
-#pragma unroll
-    for (int e = 0; e < 16; e += 2) {   // two weights per instruction
-      const float2 y = bk_fma2(bk_add2(make_float2(v[e], v[e + 1]), ml2), r2, half2);
-      const float2 f = add2_rd(y, make_float2(12582912.0f, 12582912.0f));
-      const float2 fl = bk_add2(f, make_float2(-12582912.0f, -12582912.0f));
-      const float2 o = bk_add2(bk_fma2(fl, make_float2(-1.0f, -1.0f), y), make_float2(-0.5f, -0.5f));
-      off_tie = fmaxf(off_tie, fmaxf(fabsf(o.x), fabsf(o.y)));
-      t[e] = __float_as_uint(fminf(fmaxf(f.x, 12582912.0f), 12582927.0f));
-      t[e + 1] = __float_as_uint(fminf(fmaxf(f.y, 12582912.0f), 12582927.0f));
-    }
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-      q[k] = __byte_perm(__byte_perm(t[4 * k], t[4 * k + 1], 0x0040), __byte_perm(t[4 * k + 2], t[4 * k + 3], 0x0040), 0x5410);
-    const bool near_tie = off_tie > 0.5f - kTieBand;
-    if (near_tie) {
-      q[0] = q[1] = q[2] = q[3] = 0u;
-#pragma unroll
-      for (int e = 0; e < 16; e++) q[e >> 2] |= (uint32_t)quant4_exact(__fadd_rn(v[e], ml), dl) << (8 * (e & 3));
-    }
-  }
-  // quant bytes: lanes 4p, 4p+1 hold sub-block 2p (low nibbles), lanes 4p+2, 4p+3 sub-block 2p+1 (high nibbles) of the
-  // same 32 bytes
-  uint32_t hn[4];
-#pragma unroll
-  for (int k = 0; k < 4; k++) hn[k] = __shfl_down_sync(0xffffffffu, q[k], 2);
-  uint8_t* sb = stage[warp] + half * 144;
-  if ((l & 2) == 0)
-    *reinterpret_cast<uint4*>(sb + 16 + (l >> 2) * 32 + (l & 1) * 16) =
-        make_uint4(q[0] | (hn[0] << 4), q[1] | (hn[1] << 4), q[2] | (hn[2] << 4), q[3] | (hn[3] << 4));
-  // header: sub-block j's scale and min sit in lane 2j; lanes 0..3 assemble bytes j, j+4, j+8 of the twelve
-  const int j = (lane & 16) + 2 * (l & 3);
-  const int sc_lo = __shfl_sync(0xffffffffu, sc, j), sc_hi = __shfl_sync(0xffffffffu, sc, j + 8);
-  const int m_lo = __shfl_sync(0xffffffffu, m6, j), m_hi = __shfl_sync(0xffffffffu, m6, j + 8);
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(dl));
+  uint8_t* const sb = stage + (lane >> 3) * 144;
+  uint8_t* const quants = sb + 16 + (l >> 1) * 32 + (lane & 1 ? 4 : 0);   // 32 bytes hold sub-block 2p in their low and 2p + 1 in their high nibbles
+  // The smallest and the largest weight (rounding is monotonic) show whether any lane needs the clamp to 0..15, or t before its product.
+  const float mlr = __fmul_rn(ml, r);
+  const bool plain = dl > 0.0f && mlr <= kMaxMlr && !has_nan && fmaf(lo, r, mlr) > -0.49f && fmaf(hi, r, mlr) < 15.49f;
+  if (__all_sync(0xffffffffu, plain)) write_quants<BF16, true>(rows, quants, r, mlr, ml, dl);
+  else write_quants<BF16, false>(rows, quants, r, mlr, ml, dl);
+  // header: lanes 0..3 of a superblock assemble bytes j, j+4, j+8 of the twelve
+  const int upper = __shfl_down_sync(0xffffffffu, sc | (m6 << 8), 4), sc_hi = upper & 0xff, m_hi = upper >> 8;
   if (l < 4) {
-    sb[4 + l] = (uint8_t)(sc_lo | ((sc_hi >> 4) << 6));
-    sb[8 + l] = (uint8_t)(m_lo | ((m_hi >> 4) << 6));
+    sb[4 + l] = (uint8_t)(sc | ((sc_hi >> 4) << 6));
+    sb[8 + l] = (uint8_t)(m6 | ((m_hi >> 4) << 6));
     sb[12 + l] = (uint8_t)((sc_hi & 0x0f) | ((m_hi & 0x0f) << 4));
   }
   if (l == 0) *reinterpret_cast<uint32_t*>(sb) = (uint32_t)dh | ((uint32_t)mh << 16);
-  __syncwarp();
-  const int n16 = first + 1 < n_superblocks ? 18 : 9;
-  if (lane < n16) reinterpret_cast<uint4*>(out + first * 144)[lane] = reinterpret_cast<const uint4*>(stage[warp])[lane];
+}
+
+// Bound: instruction issue, 79 % of the slots with half a sub-block a lane.  Of the 363 instructions per 512 weights that that took, more than
+// half were a sub-block's and a superblock's scalar work (five divisions, the maxima, the header), done by every lane; with a whole sub-block
+// a lane each of them serves twice as many weights.  A lane's weights are 64 or 128 contiguous bytes, so they come through shared memory:
+// 16-byte chunks by asynchronous copies in the order of memory.  The grid fills the device once and a warp requests its next superblocks
+// before it quantises the present ones (24,000 f32 superblocks 11.3 us, so 9.3).  64 registers for bf16, as many as eight CTAs of an SM
+// leave: fewer cost more than the warps they allow give (11 CTAs 68 us).  17,408 x 5,120 weights: bf16 73.5 -> 58 us (3.9 TB/s), f32 80 -> 68.
+template <bool BF16>
+__global__ void __launch_bounds__(kQWarps * 32, BF16 ? 8 : 5) quantize_q4k_kernel(const void* x, size_t n_superblocks, uint8_t* out) {
+  constexpr int kChunks = BF16 ? 4 : 8;   // 16-byte chunks of a sub-block
+  __shared__ __align__(16) uint4 rows[kQWarps][2][32 * kChunks];   // the weights in use and the next ones
+  __shared__ __align__(16) uint8_t stage[kQWarps][kQSb * 144];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto request = [&](size_t first, int buffer) {
+    if (first < n_superblocks) {
+      const int n_sb = (int)min((size_t)kQSb, n_superblocks - first);
+#pragma unroll
+      for (int k = 0; k < kChunks; k++) {   // chunk `at` of the warp's weights; superblocks past the end are the last one again, and not stored
+        const int at = lane + 32 * k, sb = at / (8 * kChunks);
+        const uint8_t* src = static_cast<const uint8_t*>(x) + (first + min(sb, n_sb - 1)) * (8 * kChunks * 16) + (at % (8 * kChunks)) * 16;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&rows[warp][buffer][chunk_slot<BF16>(at / kChunks, at % kChunks)])), "l"(src) : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const size_t step = (size_t)gridDim.x * kQWarps * kQSb;
+  size_t first = ((size_t)blockIdx.x * kQWarps + warp) * kQSb;
+  request(first, 0);
+#pragma unroll 1
+  for (int buffer = 0; first < n_superblocks; first += step, buffer ^= 1) {
+    request(first + step, buffer ^ 1);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    quantize_superblocks<BF16>(rows[warp][buffer], stage[warp]);
+    __syncwarp();
+    const int n16 = 9 * (int)min((size_t)kQSb, n_superblocks - first);
+    for (int i = lane; i < n16; i += 32) reinterpret_cast<uint4*>(out + first * 144)[i] = reinterpret_cast<const uint4*>(stage[warp])[i];
+    __syncwarp();
+  }
 }
 
 }  // namespace
@@ -148,7 +232,15 @@ extern "C" int32_t bkQuantizeQ4K(uint64_t x, int32_t dtype, int64_t n_rows, int3
   BK_ARG(n_rows > 0 && K > 0 && K % 256 == 0, "bkQuantizeQ4K: bad shape rows=%lld K=%d (K a multiple of 256)", (long long)n_rows, K);
   BK_ARG(x && out && (x & 15) == 0 && (out & 15) == 0, "bkQuantizeQ4K: null or misaligned pointer");
   const size_t nsb = (size_t)n_rows * (K / 256);
-  const unsigned grid = (unsigned)((nsb + 2 * kQWarps - 1) / (2 * kQWarps));
+  static int resident[2] = {0, 0};   // CTAs of an SM
+  int& n = resident[dtype == BK_DTYPE_BF16];
+  if (!n) {
+    if (dtype == BK_DTYPE_BF16) BK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, quantize_q4k_kernel<true>, kQWarps * 32, 0));
+    else BK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, quantize_q4k_kernel<false>, kQWarps * 32, 0));
+    if (n < 1) n = 1;
+  }
+  const size_t ctas = (nsb + kQSb * kQWarps - 1) / (kQSb * kQWarps);
+  const unsigned grid = (unsigned)std::min<size_t>(ctas, (size_t)n * bk_ctx().sm_count);
   if (dtype == BK_DTYPE_BF16)
     quantize_q4k_kernel<true><<<grid, kQWarps * 32, 0, bk_ctx().stream>>>(bk_ptr<void>(x), nsb, bk_ptr<uint8_t>(out));
   else

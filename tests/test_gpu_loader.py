@@ -57,6 +57,28 @@ def test_quantize_q4k_odd_superblock_counts_and_ties(bk, N, K):
     dx.free(), out.free()
 
 
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("n_sb", [1, 2, 3, 5, 31, 33])
+def test_quantize_q4k_partial_groups_clamps_and_nans(bk, n_sb, bf16):
+    """Four superblocks share a warp and 32 a thread block, the last of them incomplete here.  Sub-blocks whose scale is rounded far down (the clamp
+    to 15), whose minimum is (the clamp to 0), and with NaNs, which become 0 and count for neither end."""
+    rng = np.random.default_rng(40 + n_sb)
+    x = rng.normal(0, 0.02, (n_sb, 256)).astype(np.float32)
+    x[:, 32:64] *= 0.02 * rng.random((n_sb, 1)).astype(np.float32)      # scales of a few steps beside one of 63
+    x[:, 64:96] = np.abs(x[:, 64:96]) * 0.05                            # no minimum, a small scale
+    x[:, 96] = -0.3
+    x[:, 129:160:3] = np.nan
+    if bf16:
+        xb = synth.f32_to_bf16(x)
+        xb[:, 129:160:3] = 0x7FC0
+        x = synth.bf16_to_f32(xb)
+    dx, out = R.DeviceBuffer.from_numpy(xb if bf16 else x), R.DeviceBuffer(n_sb * 144)
+    ops.quantize_q4k(dx.ptr, n_sb, 256, out.ptr, bf16=bf16)
+    assert R.cuSync() == 0
+    assert_same_bits(out.download(np.uint8, (n_sb, 144)), O.q4k_quantize(x), "Q4_K superblocks")
+    dx.free(), out.free()
+
+
 def test_checkpoint_load_matches_host_quantised_model(bk, tmp_path):
     """A bf16 checkpoint with the reference's tensor names (model.language_model.layers.L...., tied embed_tokens) is
     loaded through the device quantiser; the model must decode exactly like one built from the same weights quantised
