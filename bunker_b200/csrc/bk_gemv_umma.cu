@@ -26,7 +26,7 @@
 //   * two EPILOGUE warps add up what the scalers hand over and write the outputs while the scalers are at the next tile.
 //
 // Two orders of the f32 part, both fixed and mirrored by the CPU oracle:
-//   LANES (the order of the batch <= 8 kernels, for prompts of 17 columns and more): per unit u = (s, p)
+//   LANES (the order of the batch <= 8 kernels, for prompts of many columns and for 9 to 15 sequences): per unit u = (s, p)
 //     val = fma(d, fma(d8_1, x1, d8_0*x0), -(dmin * fma(s8_1, m1, s8_0*m0))); class c = s mod 8 of pair p adds its units in
 //     ascending s; T_p = ((P0+P4)+(P2+P6)) + ((P1+P5)+(P3+P7)); y = (T0+T2) + (T1+T3).  The classes are walked in the order
 //     0,4,2,6,1,5,3,7, so that a stack of three values per (row, column, pair) holds what is still to be added: one in
@@ -995,7 +995,7 @@ int32_t bk_gemv_umma_launch(void* params, int B, bool lanes) {
     BK_CHECK_LAUNCH();
     P.g.x = c.tile_image;
   }
-  if (lanes) return B <= 32 || split ? launch_tile<2, true>(P) : launch_tile<4, true>(P);   // (17 columns and more)
+  if (lanes) return B <= 16 ? launch_tile<1, true>(P) : B <= 32 || split ? launch_tile<2, true>(P) : launch_tile<4, true>(P);   // (nine columns and more)
   return B <= 16 ? launch_tile<1, false>(P) : B <= 32 || split ? launch_tile<2, false>(P) : launch_tile<4, false>(P);
 }
 

@@ -121,7 +121,7 @@ bool bk_encode_map_2d(CUtensorMap* m, CUtensorMapDataType type, uint64_t base, u
 bool bk_gemv_mma_fits(int K, int B);   // whether the batch-3..8 tensor-core GEMV can hold this K (else column pairs)
 // whether a dense launch of B columns takes them as two groups of 32 (launch rows `rows`; lanes: in the lane order)
 bool bk_tile_split(int rows, int K, int B, bool lanes);
-bool bk_gemv_dense_lanes(int B);           // whether B columns are enough for the dense tile kernel in the lane order
+bool bk_gemv_dense_lanes(int B, int rows, int K, bool staged);   // whether B columns of a launch are enough for the dense tile kernel in the lane order; staged: the other path would take a staged activation
 bool bk_gemv_auto_tile(int rows, int K);   // whether BK_GEMV_ORDER_AUTO sends a launch of these shapes (>= 16 columns) to the dense tile path
 int32_t bk_gemv_launch(const bkGemvArgs& a);
 int32_t bk_gdn_launch(const bkGdnArgs& a);   // bkGdnStep, also with out_q8_layout BK_Q8_TILE

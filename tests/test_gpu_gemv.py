@@ -378,3 +378,19 @@ def test_gemv_tiles_of_several_segments(bk, order, B, K, rows):
     ops.gemv(dxq.ptr, K, B, [ops.gemv_seg(dW[0].ptr, n, act.ptr, R.BK_EPI_SWIGLU, W2=up.ptr)], order=order)
     g, u = oracle(W[0], n, K, xq), oracle(up.download(np.uint8, W[0].shape), n, K, xq)
     assert_same_bits(act.download(np.uint16, (B, n)), O.swiglu(g, u), "SwiGLU pair")
+
+
+@pytest.mark.parametrize("B,K,rows", [(10, 4096, 3096), (16, 4096, 3104), (16, 6144, 1376), (11, 6144, 1384), (13, 17408, 168), (13, 17408, 256), (9, 17408, 656),
+                                      (9, 17408, 664), (10, 2048, 12392), (15, 2048, 12400), (16, 2304, 24640)])
+def test_gemv_nine_to_sixteen_columns_in_lane_order(bk, B, K, rows):
+    """Both sides of the line between two launches of 8 columns and the dense tile kernel (rows * K^2), two segments of which the second begins at
+    a multiple of 8 rows, and one tile shared by the classes of up to eight thread blocks."""
+    rng = np.random.default_rng(1500 + B + K)
+    xq = O.q8_1_quantize(rng.normal(0, 1, (B, K)).astype(np.float32))
+    n = [rows - 48, 48]
+    W = [synth.q4k_weights(rng, k, K) for k in n]
+    dxq, dW, y = dev(xq), [dev(w) for w in W], [R.DeviceBuffer(B * k * 4) for k in n]
+    for _ in range(2):
+        ops.gemv(dxq.ptr, K, B, [ops.gemv_seg(w.ptr, k, o.ptr) for w, k, o in zip(dW, n, y)], order=R.BK_GEMV_ORDER_LANES)
+    for i, k in enumerate(n):
+        assert_same_bits(y[i].download(np.float32, (B, k)), O.gemv_q4k_q8(W[i], k, K, xq), f"segment {i}")
