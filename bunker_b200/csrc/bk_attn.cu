@@ -58,13 +58,18 @@ __device__ __forceinline__ void bf16x8_to_f32(uint4 v, float (&y)[8]) {
   y[7] = __uint_as_float(v.w & 0xffff0000u);
 }
 
-// head RMSNorm*(1+w) -> bf16 -> rotary on the first 2*rot_half dims, result in `stage`
-__device__ __forceinline__ void norm_rope_256(const uint16_t* src, const uint16_t* w, const float* cos_row,
-                                              const float* sin_row, int rot_half, uint16_t* stage) {
+// head RMSNorm*(1+w) -> bf16 -> rotary on the first 2*rot_half dims, result in `stage`.  x and w: the row and the norm weights, 8 dims a lane;
+// the first 32 angles are requested before the norm that they wait for.
+__device__ __forceinline__ void norm_rope_256(uint4 xr, uint4 wr, const float* cos_row, const float* sin_row, int rot_half, uint16_t* stage) {
   const int lane = threadIdx.x & 31;
+  float c = 0.0f, s = 0.0f;
+  if (lane < rot_half) {
+    c = cos_row[lane];
+    s = sin_row[lane];
+  }
   float x[8], wv[8];
-  bf16x8_to_f32(*reinterpret_cast<const uint4*>(src + lane * 8), x);
-  bf16x8_to_f32(*reinterpret_cast<const uint4*>(w + lane * 8), wv);
+  bf16x8_to_f32(xr, x);
+  bf16x8_to_f32(wr, wv);
   float acc = 0.0f;
 #pragma unroll
   for (int e = 0; e < 8; e++) acc = fmaf(x[e], x[e], acc);
@@ -75,8 +80,11 @@ __device__ __forceinline__ void norm_rope_256(const uint16_t* src, const uint16_
     stage[lane * 8 + e] = bk_f32_to_bf16(__fmul_rn(__fmul_rn(x[e], rstd), __fadd_rn(1.0f, wv[e])));
   __syncwarp();
   for (int i = lane; i < rot_half; i += 32) {
+    if (i >= 32) {
+      c = cos_row[i];
+      s = sin_row[i];
+    }
     float x1 = bk_bf16_to_f32(stage[i]), x2 = bk_bf16_to_f32(stage[i + rot_half]);
-    float c = cos_row[i], s = sin_row[i];
     uint16_t r1 = bk_f32_to_bf16(__fsub_rn(__fmul_rn(x1, c), __fmul_rn(x2, s)));
     uint16_t r2 = bk_f32_to_bf16(__fadd_rn(__fmul_rn(x2, c), __fmul_rn(x1, s)));
     stage[i] = r1;
@@ -101,34 +109,15 @@ __device__ __forceinline__ void butterfly_level(float (&v)[N], int off) {
 // merge the splits of one (batch, q head) by one warp; lane l owns output dims [8l, 8l+8).
 // w_s: ns floats of shared memory private to the warp.  M = max m_s; w_s = exp(m_s - M);
 // L = fma(w_s, l_s, L) and O = fma(w_s, o_s, O) in ascending s; out = (O/L) * sigmoid(gate).
-__device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, float* w_s) {
+__device__ __forceinline__ uint4 head_gate(const AttnParams& p, int b, int h) {
   const int lane = threadIdx.x & 31;
-  const float* sc_ml = p.part_ml + ((size_t)b * p.Hq + h) * p.max_splits * 2;
-  const float* sc_o = p.part_o + ((size_t)b * p.Hq + h) * p.max_splits * kHD;
-  float m = -INFINITY;
-  for (int s = lane; s < ns; s += 32) {
-    float ms = __ldcg(sc_ml + 2 * s);
-    w_s[s] = ms;
-    m = fmaxf(m, ms);
-  }
-  const float M = bk_warp_max(m);
-  for (int s = lane; s < ns; s += 32) w_s[s] = bk_expf(__fsub_rn(w_s[s], M));
-  __syncwarp();
-  float L = 0.0f, O[8];
-#pragma unroll
-  for (int e = 0; e < 8; e++) O[e] = 0.0f;
-  for (int s = 0; s < ns; s++) {
-    const float w = w_s[s];
-    L = fmaf(w, __ldcg(sc_ml + 2 * s + 1), L);
-    const float4 a = __ldcg(reinterpret_cast<const float4*>(sc_o + (size_t)s * kHD + lane * 8));
-    const float4 c = __ldcg(reinterpret_cast<const float4*>(sc_o + (size_t)s * kHD + lane * 8) + 1);
-    O[0] = fmaf(w, a.x, O[0]); O[1] = fmaf(w, a.y, O[1]); O[2] = fmaf(w, a.z, O[2]); O[3] = fmaf(w, a.w, O[3]);
-    O[4] = fmaf(w, c.x, O[4]); O[5] = fmaf(w, c.y, O[5]); O[6] = fmaf(w, c.z, O[6]); O[7] = fmaf(w, c.w, O[7]);
-  }
-  const uint16_t* gp = p.fused ? p.qg + ((size_t)b * p.Hq + h) * 2 * kHD + kHD + lane * 8
-                               : p.gate + ((size_t)b * p.Hq + h) * kHD + lane * 8;
+  return *reinterpret_cast<const uint4*>(p.fused ? p.qg + ((size_t)b * p.Hq + h) * 2 * kHD + kHD + lane * 8 : p.gate + ((size_t)b * p.Hq + h) * kHD + lane * 8);
+}
+// out = (O/L) * sigmoid(gate) of this lane's dims
+__device__ void store_head_warp(const AttnParams& p, int b, int h, const float (&O)[8], float L, uint4 gate) {
+  const int lane = threadIdx.x & 31;
   float gf[8];
-  bf16x8_to_f32(*reinterpret_cast<const uint4*>(gp), gf);
+  bf16x8_to_f32(gate, gf);
   uint32_t o[4];
 #pragma unroll
   for (int e = 0; e < 8; e += 2) {
@@ -148,6 +137,34 @@ __device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, flo
     else if (p.out_q8_layout == BK_Q8_STAGED) bk_staged_store<8>(p.out_q8, p.Hq * kHD, p.B, b, (h * kHD + lane * 8) >> 5, y, (lane & 3) * 8);
     else bk_q8_1_store<8>(p.out_q8 + ((((size_t)b * p.Hq + h) * kHD + lane * 8) >> 5) * 36, y, (lane & 3) * 8);
   }
+}
+
+__device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, float* w_s, uint4 gate) {
+  const int lane = threadIdx.x & 31;
+  const float* sc_ml = p.part_ml + ((size_t)b * p.Hq + h) * p.max_splits * 2;
+  const float* sc_o = p.part_o + ((size_t)b * p.Hq + h) * p.max_splits * kHD;
+  float m = -INFINITY;
+  for (int s = lane; s < ns; s += 32) {
+    float ms = __ldcg(sc_ml + 2 * s);
+    w_s[s] = ms;
+    m = fmaxf(m, ms);
+  }
+  const float M = bk_warp_max(m);
+  for (int s = lane; s < ns; s += 32) w_s[s] = bk_expf(__fsub_rn(w_s[s], M));
+  __syncwarp();
+  float L = 0.0f, O[8];
+#pragma unroll
+  for (int e = 0; e < 8; e++) O[e] = 0.0f;
+#pragma unroll 4
+  for (int s = 0; s < ns; s++) {
+    const float w = w_s[s];
+    L = fmaf(w, __ldcg(sc_ml + 2 * s + 1), L);
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(sc_o + (size_t)s * kHD + lane * 8));
+    const float4 c = __ldcg(reinterpret_cast<const float4*>(sc_o + (size_t)s * kHD + lane * 8) + 1);
+    O[0] = fmaf(w, a.x, O[0]); O[1] = fmaf(w, a.y, O[1]); O[2] = fmaf(w, a.z, O[2]); O[3] = fmaf(w, a.w, O[3]);
+    O[4] = fmaf(w, c.x, O[4]); O[5] = fmaf(w, c.y, O[5]); O[6] = fmaf(w, c.z, O[6]); O[7] = fmaf(w, c.w, O[7]);
+  }
+  store_head_warp(p, b, h, O, L, gate);
 }
 
 // dynamic shared memory layout (bytes):
@@ -180,8 +197,8 @@ __global__ void __launch_bounds__(32) attn_append_kernel(const AttnParams p) {
   const int cb = b % p.n_seq;
   uint16_t* Kb = p.k_cache + ((size_t)cb * p.Hkv + kvh) * (size_t)p.max_len * kHD;
   uint16_t* Vb = p.v_cache + ((size_t)cb * p.Hkv + kvh) * (size_t)p.max_len * kHD;
-  norm_rope_256(p.k + ((size_t)b * p.Hkv + kvh) * kHD, p.k_norm_w, p.cos_t + (size_t)pos * p.rot_half,
-                p.sin_t + (size_t)pos * p.rot_half, p.rot_half, k_st);
+  norm_rope_256(*reinterpret_cast<const uint4*>(p.k + ((size_t)b * p.Hkv + kvh) * kHD + lane * 8), *reinterpret_cast<const uint4*>(p.k_norm_w + lane * 8),
+                p.cos_t + (size_t)pos * p.rot_half, p.sin_t + (size_t)pos * p.rot_half, p.rot_half, k_st);
   __syncwarp();
   *reinterpret_cast<uint4*>(Kb + (size_t)pos * kHD + lane * 8) = *reinterpret_cast<const uint4*>(k_st + lane * 8);
   *reinterpret_cast<uint4*>(Vb + (size_t)pos * kHD + lane * 8) =
@@ -251,22 +268,24 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  bool early = false;   // the first rows were requested before the dependency wait and are still the right ones
   if (p.settled) {
     set_pos(p.pos[b]);
     for (int q = 0; q < kBatches; q++) request(q, false);
-    early = true;
   }
+  uint4 wrow = make_uint4(0, 0, 0, 0);
+  if (p.fused && (warp < G || warp == kW - 1)) wrow = *reinterpret_cast<const uint4*>((warp < G ? p.q_norm_w : p.k_norm_w) + lane * 8);
   bk_pdl_wait();
   bk_stamp(p.trace, 2);
+  uint4 xrow = make_uint4(0, 0, 0, 0);   // this warp's query head: it does not wait for the position
+  if (warp < G) xrow = *reinterpret_cast<const uint4*>(p.qg + ((size_t)b * p.Hq + kvh * G + warp) * (p.fused ? 2 : 1) * kHD + lane * 8);
   {
     // The position is taken (again) after the wait: the kernel that advances it may be only a few launches back and
     // still have been running when the early part above read it.  A changed value discards the early loads.
     const int pos_now = __ldcg(p.pos + b);
-    if (!early || pos_now != pos) {
+    if (!p.settled || pos_now != pos) {
       asm volatile("cp.async.wait_all;" ::: "memory");
-      early = false;
       set_pos(pos_now);
+      for (int q = 0; q < kBatches; q++) request(q, false);
     }
   }
   if (ns <= 0) {
@@ -280,21 +299,17 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   if (p.fused) {
     const float* cr = p.cos_t + (size_t)pos * p.rot_half;
     const float* sr = p.sin_t + (size_t)pos * p.rot_half;
-    if (warp < G) {
-      const uint16_t* src = p.qg + ((size_t)b * p.Hq + kvh * G + warp) * 2 * kHD;
-      norm_rope_256(src, p.q_norm_w, cr, sr, p.rot_half, q_st + warp * kHD);
-    }
     if (p.n_seq == 0 && warp == kW - 1 && owner) {
+      const uint4 k = *reinterpret_cast<const uint4*>(p.k + ((size_t)b * p.Hkv + kvh) * kHD + lane * 8);
       const uint4 v = *reinterpret_cast<const uint4*>(p.v + ((size_t)b * p.Hkv + kvh) * kHD + lane * 8);
-      norm_rope_256(p.k + ((size_t)b * p.Hkv + kvh) * kHD, p.k_norm_w, cr, sr, p.rot_half, k_st);
+      norm_rope_256(k, G == kW ? *reinterpret_cast<const uint4*>(p.k_norm_w + lane * 8) : wrow, cr, sr, p.rot_half, k_st);
       *reinterpret_cast<uint4*>(Kb + (size_t)pos * kHD + lane * 8) = *reinterpret_cast<const uint4*>(k_st + lane * 8);
       *reinterpret_cast<uint4*>(Vb + (size_t)pos * kHD + lane * 8) = v;
       *reinterpret_cast<uint4*>(v_st + lane * 8) = v;
     }
+    if (warp < G) norm_rope_256(xrow, wrow, cr, sr, p.rot_half, q_st + warp * kHD);
   } else {
-    if (warp < G)
-      *reinterpret_cast<uint4*>(q_st + warp * kHD + lane * 8) =
-          *reinterpret_cast<const uint4*>(p.qg + ((size_t)b * p.Hq + kvh * G + warp) * kHD + lane * 8);
+    if (warp < G) *reinterpret_cast<uint4*>(q_st + warp * kHD + lane * 8) = xrow;
   }
   if ((!p.fused || p.n_seq > 0) && warp == kW - 1 && owner) {   // the row is in the cache
     *reinterpret_cast<uint4*>(k_st + lane * 8) = *reinterpret_cast<const uint4*>(Kb + (size_t)pos * kHD + lane * 8);
@@ -302,9 +317,7 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   }
   __syncthreads();   // q and the row at pos are in shared memory
   bk_stamp(p.trace, 3);
-  if (!early) {
-    for (int q = 0; q < kBatches; q++) request(q, true);
-  } else if (mine) {   // left out of the early requests
+  if (mine) {   // left out of the first requests
     const int q = np / kRows, e = np % kRows;
     if (q < kBatches) ring[32 * (kRows * q + e)] = *reinterpret_cast<const uint4*>(k_st + lane * 8);
     if (q + nb < kBatches) ring[32 * (kRows * (q + nb) + e)] = *reinterpret_cast<const uint4*>(v_st + lane * 8);
@@ -485,6 +498,31 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   __syncthreads();
   bk_stamp(p.trace, 6);
 
+  if (nsplits == 1) {   // nothing to merge with: the partials need not leave the CTA
+    if (warp < G) {
+      const uint4 gate = head_gate(p, b, kvh * G + warp);
+      float L = l_s[warp], O[8];
+#pragma unroll
+      for (int w = 1; w < kW; w++) L = __fadd_rn(L, l_s[w * 8 + warp]);
+#pragma unroll
+      for (int e = 0; e < 8; e += 4) {
+        float4 o = *reinterpret_cast<const float4*>(o_s + (size_t)warp * kHD + lane * 8 + e);
+#pragma unroll
+        for (int w = 1; w < kW; w++) {
+          const float4 t = *reinterpret_cast<const float4*>(o_s + ((size_t)(w * 8 + warp)) * kHD + lane * 8 + e);
+          o = make_float4(__fadd_rn(o.x, t.x), __fadd_rn(o.y, t.y), __fadd_rn(o.z, t.z), __fadd_rn(o.w, t.w));
+        }
+        O[e] = o.x; O[e + 1] = o.y; O[e + 2] = o.z; O[e + 3] = o.w;
+      }
+      const float w = bk_expf(__fsub_rn(m_s[warp], m_s[warp]));   // the merge of one split, operation for operation
+      L = fmaf(w, L, 0.0f);
+#pragma unroll
+      for (int e = 0; e < 8; e++) O[e] = fmaf(w, O[e], 0.0f);
+      store_head_warp(p, b, kvh * G + warp, O, L, gate);
+    }
+    bk_stamp(p.trace, 5);
+    return;
+  }
   // ---- cross-warp sums in warp order, partial out ----
   float *sc_ml = p.part_ml, *sc_o = p.part_o;
   for (int idx = tid; idx < G * kHD; idx += kW * 32) {
@@ -504,6 +542,8 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   }
 
   // ---- the CTA that completes this (batch, KV head) merges its splits ----
+  uint4 gate = make_uint4(0, 0, 0, 0);   // (requested before it is known whether it is this one)
+  if (warp < G) gate = head_gate(p, b, kvh * G + warp);
   __threadfence();
   __syncthreads();
   bk_stamp(p.trace, 7);
@@ -515,7 +555,7 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   __syncthreads();
   if (s_last) {
     __threadfence();
-    if (warp < G) combine_head_warp(p, b, kvh * G + warp, nsplits, o_s + warp * kMaxSplits);  // one head per warp
+    if (warp < G) combine_head_warp(p, b, kvh * G + warp, nsplits, o_s + warp * kMaxSplits, gate);  // one head per warp
     if (tid == 0) *cnt = 0;
   }
   bk_stamp(p.trace, 5);
