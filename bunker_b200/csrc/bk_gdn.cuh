@@ -38,16 +38,25 @@ struct GdnParams {
 // Two builds of this body.  gdn_step_kernel: launched with 576 threads when the grid has at most one CTA per SM; the
 // two extra warps only keep a second CTA of this grid off the SM (register file), so no SM finishes last with two.
 // gdn_step_kernel_x2: 64 registers, two CTAs per SM, for grids larger than the SM count (batch 8: 256 CTAs, one wave).
+// gdn_step_kernel_x3: the state in shared memory instead of registers, three CTAs per SM, for grids of more than one such wave.  Bound: the
+// state, 128 KB a head in and out, and while a CTA goes through its chain of norms and sums it neither loads nor stores.  In the step, us, two /
+// three CTAs an SM: 13 sequences of 32 heads 17.1 / 13.4, 16 19.8 / 15.3, 32 35.2 / 26.6 (5.1 TB/s), 64 67.5 / 51.9, 8 of 48 heads 14.3 / 11.3.  (Quarter
+// heads, eight CTAs of 128 threads an SM and the norm's sums through a cluster: as slow as two whole ones.  One CTA an SM that walks the heads
+// behind a ring of copies: 34.5 us for 32 sequences, the chain of a head being 4.9.)
+enum { kGdnOne, kGdnMulti, kGdnShared };
+constexpr uint32_t kGdnHeadBytes = 128 * 128 * 4;
 struct GdnSmem {
   float s_q[128], s_k[128], s_v[128], s_o[128];
   float s_part[4][128];
   float s_scal[4];  // q scale, k rstd, decay, beta
 };
 
-// MULTI: a few tokens one after the other (T of them), the state and the three conv taps in registers between them.
-template <bool MULTI>
-__device__ __forceinline__ void gdn_step_body(const GdnParams& p, GdnSmem& sm, const int hv, const int b) {
+// kGdnMulti: a few tokens one after the other (T of them), the state and the three conv taps in registers between them.
+// kGdnShared: the state comes by one bulk copy into `state`, and what is read twice of it is scaled by the decay twice.
+template <int MODE>
+__device__ __forceinline__ void gdn_step_body(const GdnParams& p, GdnSmem& sm, const int hv, const int b, float* state = nullptr, uint64_t* bar = nullptr, int* status = nullptr) {
   constexpr int D = 128;
+  constexpr bool MULTI = MODE == kGdnMulti, SHARED = MODE == kGdnShared;
   float (&s_q)[D] = sm.s_q;
   float (&s_k)[D] = sm.s_k;
   float (&s_v)[D] = sm.s_v;
@@ -73,14 +82,19 @@ __device__ __forceinline__ void gdn_step_body(const GdnParams& p, GdnSmem& sm, c
   // State, conv taps and per-head constants do not come from the kernel that runs just before this one
   // (p.early != 0 asserts that), so they are requested before the dependency wait and arrive while the
   // projection GEMV is still finishing.
-  float sd[32];
+  float sd[SHARED ? 1 : 32];
   uint16_t h0 = 0, h1 = 0, h2 = 0;
   uint2 cw = make_uint2(0, 0);
   float alog = 0.0f, dtb = 0.0f, nw = 0.0f;
   auto load_static = [&]() {
-    if (active) {
+    if (SHARED) {
+      if (t == 0) {
+        mbar_expect_tx(smem_u32(bar), kGdnHeadBytes);
+        bulk_g2s(smem_u32(state), p.S_in + ((size_t)b * p.Hv + hv) * (D * D), kGdnHeadBytes, smem_u32(bar));
+      }
+    } else if (active) {
 #pragma unroll
-      for (int i = 0; i < 32; i++) sd[i] = S[(size_t)i * D];
+      for (int i = 0; i < 32; i++) sd[SHARED ? 0 : i] = S[(size_t)i * D];
     }
     if (t < 3 * D && p.apply_conv) {
       const uint16_t* st = p.cs_in + (size_t)b * 3 * C;
@@ -160,7 +174,13 @@ __device__ __forceinline__ void gdn_step_body(const GdnParams& p, GdnSmem& sm, c
 
     const float decay = s_scal[2], beta = s_scal[3];
     float acc = 0.0f;
-    if (active) {
+    const float* st = state + 32 * r * D + j;
+    if constexpr (SHARED) {
+      mbar_wait_bounded(smem_u32(bar), 0, status);
+#pragma unroll 16
+      for (int i = 0; i < 32; i++) acc = fmaf(s_k[32 * r + i], __fmul_rn(st[i * D], decay), acc);
+      s_part[r][j] = acc;
+    } else if (active) {
 #pragma unroll
       for (int i = 0; i < 32; i++) {
         sd[i] = __fmul_rn(sd[i], decay);
@@ -173,7 +193,15 @@ __device__ __forceinline__ void gdn_step_body(const GdnParams& p, GdnSmem& sm, c
     float delta = __fmul_rn(__fsub_rn(s_v[j], kS), beta);
     __syncthreads();
     acc = 0.0f;
-    if (active) {
+    if constexpr (SHARED) {
+#pragma unroll 16
+      for (int i = 0; i < 32; i++) {
+        const float v = fmaf(s_k[32 * r + i], delta, __fmul_rn(st[i * D], decay));
+        Sn[(size_t)i * D] = v;
+        acc = fmaf(s_q[32 * r + i], v, acc);
+      }
+      s_part[r][j] = acc;
+    } else if (active) {
 #pragma unroll
       for (int i = 0; i < 32; i++) {
         sd[i] = fmaf(s_k[32 * r + i], delta, sd[i]);

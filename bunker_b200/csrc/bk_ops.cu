@@ -178,15 +178,26 @@ __global__ void conv1d_step_kernel(const uint16_t* x, const uint16_t* st, const 
 
 __global__ void __launch_bounds__(576) gdn_step_kernel(const GdnParams p) {
   __shared__ GdnSmem sm;
-  gdn_step_body<false>(p, sm, blockIdx.x, blockIdx.y);
+  gdn_step_body<kGdnOne>(p, sm, blockIdx.x, blockIdx.y);
 }
 __global__ void __launch_bounds__(512, 2) gdn_step_kernel_x2(const GdnParams p) {
   __shared__ GdnSmem sm;
-  gdn_step_body<false>(p, sm, blockIdx.x, blockIdx.y);
+  gdn_step_body<kGdnOne>(p, sm, blockIdx.x, blockIdx.y);
 }
 __global__ void __launch_bounds__(576) gdn_step_kernel_multi(const GdnParams p) {
   __shared__ GdnSmem sm;
-  gdn_step_body<true>(p, sm, blockIdx.x, blockIdx.y);
+  gdn_step_body<kGdnMulti>(p, sm, blockIdx.x, blockIdx.y);
+}
+__global__ void __launch_bounds__(512, 3) gdn_step_kernel_x3(const GdnParams p, int* status) {
+  extern __shared__ __align__(128) float gdn_state[];
+  __shared__ GdnSmem sm;
+  __shared__ uint64_t bar;
+  if (threadIdx.x == 0) {
+    mbar_init(smem_u32(&bar), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  gdn_step_body<kGdnShared>(p, sm, blockIdx.x, blockIdx.y, gdn_state, &bar, status);   // (its barriers make the mbarrier visible before it is waited for)
 }
 // ---- q/k head RMSNorm + partial rotary, one warp per (batch, head) ----------------
 // (src/emitters.ts:123-183).  Lane l owns the HD/32 contiguous dims of the head.
@@ -553,7 +564,17 @@ int32_t bk_gdn_launch(const bkGdnArgs& a) {
     }
     return BK_OK;
   }
-  if (a.Hv * a.B > bk_ctx().sm_count) BK_CUDA(bk_launch_pdl(gdn_step_kernel_x2, dim3(a.Hv, a.B), dim3(512), 0, p));
+  // One wave of two CTAs an SM is the faster one as long as it is one (8 sequences of 32 heads, in the step, 10.5 us, with three an SM 11.2); the state must
+  // be on the boundary that a bulk copy needs.
+  const int n_heads = a.Hv * a.B, sms = bk_ctx().sm_count;
+  if (n_heads > 2 * sms && (a.S_in & 15) == 0) {
+    static bool configured = false;
+    if (!configured) {
+      BK_CUDA(cudaFuncSetAttribute(gdn_step_kernel_x3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGdnHeadBytes));
+      configured = true;
+    }
+    BK_CUDA(bk_launch_pdl(gdn_step_kernel_x3, dim3(a.Hv, a.B), dim3(512), kGdnHeadBytes, p, bk_ctx().d_status));
+  } else if (n_heads > sms) BK_CUDA(bk_launch_pdl(gdn_step_kernel_x2, dim3(a.Hv, a.B), dim3(512), 0, p));
   else BK_CUDA(bk_launch_pdl(gdn_step_kernel, dim3(a.Hv, a.B), dim3(576), 0, p));
   BK_CHECK_LAUNCH();
   return BK_OK;

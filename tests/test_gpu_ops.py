@@ -132,6 +132,29 @@ def test_gdn_step_config1(bk, B):
     assert rel_err(w_S[0, hv], Sp) < 1e-3 and rel_err(w_o[0, hv], op) < 1e-3
 
 
+@pytest.mark.parametrize("B,Hk,Hv,off", [(9, 16, 32, 0), (10, 16, 32, 0), (10, 16, 32, 8), (64, 4, 8, 0), (7, 16, 48, 0)])
+def test_gdn_step_of_more_heads_than_a_wave(bk, B, Hk, Hv, off):
+    """Heads up to two per SM and more of them, which take their state by bulk copies; a state off the 16-byte boundary those need; two steps in
+    place, the second with the outputs of the first."""
+    c = synth.gdn_case(B, Hk=Hk, Hv=Hv, config_id=90 + B)
+    d = {k: dev(v) for k, v in c.items() if isinstance(v, np.ndarray)}
+    n, C = c["S"].size * 4, c["qkv"].shape[1]
+    S = R.DeviceBuffer.zeros(n + 16)
+    R.cuHtoD(S.ptr + off, c["S"])
+    cs = [d["conv_state"], R.DeviceBuffer(B * 3 * C * 2)]
+    out = R.DeviceBuffer(B * Hv * 128 * 2)
+    state, conv = c["S"], c["conv_state"]
+    for step in range(2):
+        ops.gdn_step(qkv=d["qkv"].ptr, z=d["z"].ptr, a=d["a"].ptr, b=d["b"].ptr, conv_w=d["conv_w"].ptr, conv_state_in=cs[step].ptr, conv_state_new=cs[step ^ 1].ptr,
+                     A_log=d["A_log"].ptr, dt_bias=d["dt_bias"].ptr, norm_w=d["norm_w"].ptr, S_in=S.ptr + off, S_new=S.ptr + off, out=out.ptr, B=B, Hk=Hk, Hv=Hv, apply_conv=1)
+        _, conv, state, _, want = _gdn_oracle(dict(c, S=state, conv_state=conv))
+        assert_same_bits(out.download(np.uint16, (B, Hv * 128)), want, f"out of step {step}")
+    got = np.empty_like(c["S"])
+    R.cuDtoH(got, S.ptr + off)
+    assert_same_bits(got, state, "state")
+    assert_same_bits(cs[0].download(np.uint16, conv.shape), conv, "conv state")
+
+
 def test_gdn_step_several_tokens_in_one_launch(bk):
     """n_tokens = 3: three consecutive tokens of two sequences in one launch (state and conv taps stay in registers)
     equal three single-token launches: outputs of every token, final state, final conv state; staged output too."""
