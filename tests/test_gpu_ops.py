@@ -214,6 +214,13 @@ def test_gdn_step_many_tokens(bk, B, T, Hk, Hv):
         assert_same_bits(a.download(np.float32, (n,)), b.download(np.float32, (n,)), what)
 
 
+@pytest.mark.parametrize("B,T,Hk,Hv", [(9, 5, 8, 8), (10, 5, 8, 8), (2, 65, 16, 32), (1, 7, 16, 48), (10, 6, 2, 8)])
+def test_gdn_step_many_tokens_of_few_and_many_heads(bk, B, T, Hk, Hv):
+    """Both sides of the line between the recurrence that packs a token's output with the next token's k.S (up to two CTAs an SM) and the one that
+    does not, even and odd numbers of tokens, and a second launch of one token."""
+    test_gdn_step_many_tokens(bk, B, T, Hk, Hv)
+
+
 def test_gdn_step_without_conv(bk):
     c = synth.gdn_case(2, Hk=2, Hv=4, config_id=21)
     Hk, Hv, B = 2, 4, 2
