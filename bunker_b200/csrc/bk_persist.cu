@@ -585,14 +585,20 @@ BK_DEVINL void stage_activation(const StepParams& P, const Phase& ph, const Stag
   uint4 wv = make_uint4(0, 0, 0, 0);
   if (norm && tid < nchunk) wv = ld_early(nw + tid);
   float rstd = 1.0f, acc = 0.0f;
+  uint4 a = make_uint4(0, 0, 0, 0), b = a;   // a plain row's words, one pass ahead, and the first of a normalised one
+  if (!embed && tid < nchunk) {
+    a = ld_vec(in + (size_t)tid * 8);
+    b = ld_vec(in + (size_t)tid * 8 + 4);
+  }
   if (norm) {
 #pragma unroll 1
     for (int q = tid; q < nchunk; q += kCT) {   // whole warps: nchunk is a multiple of 32
       uint4 v;
       if (!embed) {
-        uint4 a, b;
-        a = ld_vec(in + (size_t)q * 8);
-        b = ld_vec(in + (size_t)q * 8 + 4);
+        if (q != tid) {
+          a = ld_vec(in + (size_t)q * 8);
+          b = ld_vec(in + (size_t)q * 8 + 4);
+        }
         wait_chunk(in, q, th, a, b, ctl);
         v = pack_words(a, b);
         reinterpret_cast<uint4*>(xrow)[q] = v;
@@ -612,11 +618,6 @@ BK_DEVINL void stage_activation(const StepParams& P, const Phase& ph, const Stag
     float total = __fadd_rn(__fadd_rn(__fadd_rn(r0.x, r0.y), r0.z), r0.w);
     total = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(total, r1.x), r1.y), r1.z), r1.w);
     rstd = bk_rcp_sqrt(__fadd_rn(__fdiv_rn(total, (float)K), ph.eps));
-  }
-  uint4 a = make_uint4(0, 0, 0, 0), b = a;   // a plain row's words, one pass ahead
-  if (!norm && tid < nchunk) {
-    a = ld_vec(in + (size_t)tid * 8);
-    b = ld_vec(in + (size_t)tid * 8 + 4);
   }
 #pragma unroll 1
   for (int q = tid; q < nchunk; q += kCT) {
