@@ -702,17 +702,28 @@ __global__ void __launch_bounds__(kUT, 1) gemv_q4k_umma_kernel(const __grid_cons
       if constexpr (LANES) {
         float2 S[16], L0[16];   // [step of the batch = pair][column block][row]
         int sp = 0;
+        auto unit = [&](float2 x0, float2 x1, const float4& c0, const float4& c1, const float4& r) {
+          float2 a = mul2(make_float2(c0.x, c0.y), x0);
+          a = bk_fma2(make_float2(c1.x, c1.y), x1, a);
+          float2 mm = mul2(make_float2(c0.z, c0.w), dup2(r.z));
+          mm = bk_fma2(make_float2(c1.z, c1.w), dup2(r.w), mm);
+          return bk_fma2(dup2(r.x), a, mul2(dup2(r.y), mm));
+        };
         auto run_class = [&](int pos, float2 (&T)[16]) {
-#pragma unroll
-          for (int e = 0; e < 16; e++) T[e] = make_float2(0.0f, 0.0f);
-          for (int s = Walk<LANES>::cls(pos); s < nsb; s += 8) {
+          int s = Walk<LANES>::cls(pos);
+          if (s < nsb) {   // the first superblock of the class, onto zero
             run_batch(0, [&](int bi, int cb, int i, float2 x0, float2 x1, const float4& c0, const float4& c1, const float4& r) {
-              float2 a = mul2(make_float2(c0.x, c0.y), x0);
-              a = bk_fma2(make_float2(c1.x, c1.y), x1, a);
-              float2 mm = mul2(make_float2(c0.z, c0.w), dup2(r.z));
-              mm = bk_fma2(make_float2(c1.z, c1.w), dup2(r.w), mm);
+              T[(bi * NB + cb) * 4 + i] = bk_add2(make_float2(0.0f, 0.0f), unit(x0, x1, c0, c1, r));
+            });
+            next_superblock();
+          } else {
+#pragma unroll
+            for (int e = 0; e < 16; e++) T[e] = make_float2(0.0f, 0.0f);
+          }
+          for (s += 8; s < nsb; s += 8) {
+            run_batch(0, [&](int bi, int cb, int i, float2 x0, float2 x1, const float4& c0, const float4& c1, const float4& r) {
               const int e = (bi * NB + cb) * 4 + i;
-              T[e] = bk_add2(T[e], bk_fma2(dup2(r.x), a, mul2(dup2(r.y), mm)));
+              T[e] = bk_add2(T[e], unit(x0, x1, c0, c1, r));
             });
             next_superblock();
           }
