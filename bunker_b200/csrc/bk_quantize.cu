@@ -46,30 +46,35 @@ template <bool BF16>
 BK_DEVINL int chunk_slot(int row, int c) {
   return BF16 ? row * 4 + (c ^ ((row >> 1) & 3)) : row * 8 + (c ^ (row & 7));
 }
-// weight e of this lane's sub-block, for what hardly ever runs
+// weight e of sub-block `sub`, for what seldom runs
 template <bool BF16>
-BK_DEVINL float one_weight(const uint4* rows, int e) {
-  const int lane = threadIdx.x & 31;
-  if (BF16) return bk_bf16_to_f32(reinterpret_cast<const uint16_t*>(rows + chunk_slot<BF16>(lane, e >> 3))[e & 7]);
-  return reinterpret_cast<const float*>(rows + chunk_slot<BF16>(lane, e >> 2))[e & 3];
+BK_DEVINL float one_weight(const uint4* rows, int sub, int e) {
+  if (BF16) return bk_bf16_to_f32(reinterpret_cast<const uint16_t*>(rows + chunk_slot<BF16>(sub, e >> 3))[e & 7]);
+  return reinterpret_cast<const float*>(rows + chunk_slot<BF16>(sub, e >> 2))[e & 3];
 }
 template <bool BF16>
 __device__ __noinline__ float largest_number(const uint4* rows) {
-  float hi = one_weight<BF16>(rows, 0);
+  const int lane = threadIdx.x & 31;
+  float hi = one_weight<BF16>(rows, lane, 0);
 #pragma unroll 1
-  for (int e = 1; e < 32; e++) hi = fmaxf(hi, one_weight<BF16>(rows, e));
+  for (int e = 1; e < 32; e++) hi = fmaxf(hi, one_weight<BF16>(rows, lane, e));
   return hi;
 }
-// the exact quants of weights 8c to 8c + 7, a byte each
+// q of the lanes in `todo` becomes the exact quants of their weights 8c to 8c + 7, a byte each: eight lanes divide for one.  Of 1,024 weights
+// one lies near a tie in 50 cases, and a small launch waits for its slowest warp: with the lane's own eight divisions one after the other 64 x
+// 1,536 weights took 4.6 us, 301 x 2,304 5.3.
 template <bool BF16>
-__device__ __noinline__ uint2 exact_quants(const uint4* rows, int c, float ml, float dl) {
-  uint32_t q[2] = {0u, 0u};
+__device__ __noinline__ uint2 exact_quants(const uint4* rows, int c, uint32_t todo, uint2 q, float ml, float dl) {
+  const int lane = threadIdx.x & 31, e = lane & 7;
 #pragma unroll 1
-  for (int e = 0; e < 4; e++) {
-    q[0] |= quant4_exact(__fadd_rn(one_weight<BF16>(rows, 8 * c + e), ml), dl) << (8 * e);
-    q[1] |= quant4_exact(__fadd_rn(one_weight<BF16>(rows, 8 * c + 4 + e), ml), dl) << (8 * e);
+  for (; todo; todo &= todo - 1) {
+    const int sub = __ffs(todo) - 1;
+    const float t = __fadd_rn(one_weight<BF16>(rows, sub, 8 * c + e), __shfl_sync(0xffffffffu, ml, sub));
+    const uint32_t v = quant4_exact(t, __shfl_sync(0xffffffffu, dl, sub)) << (8 * (e & 3));
+    const uint32_t x = __reduce_or_sync(0xffffffffu, e < 4 ? v : 0u), y = __reduce_or_sync(0xffffffffu, e < 4 ? 0u : v);
+    if (lane == sub) q = make_uint2(x, y);
   }
-  return make_uint2(q[0], q[1]);
+  return q;
 }
 
 // The quants of this lane's sub-block, with the neighbour's, into their 32 bytes.  PLAIN: no weight of the warp leaves 0..15, none is a NaN, and
@@ -111,7 +116,8 @@ BK_DEVINL void write_quants(const uint4* rows, uint8_t* quants, float r, float m
     uint2 q;   // a quant per byte
     q.x = __byte_perm(__byte_perm(t[0], t[1], 0x0040), __byte_perm(t[2], t[3], 0x0040), 0x5410);
     q.y = __byte_perm(__byte_perm(t[4], t[5], 0x0040), __byte_perm(t[6], t[7], 0x0040), 0x5410);
-    if (tie > 0.5f - kTieBand) q = exact_quants<BF16>(rows, c, ml, dl);
+    const uint32_t near_tie = __ballot_sync(0xffffffffu, tie > 0.5f - kTieBand);
+    if (near_tie) q = exact_quants<BF16>(rows, c, near_tie, q, ml, dl);
     if (!PLAIN && !(dl > 0.0f)) q = make_uint2(0u, 0u);
     // of the pair of lanes the even one writes the first four bytes, the odd one the others
     const uint32_t other = __shfl_xor_sync(0xffffffffu, odd ? q.x : q.y, 1);

@@ -79,6 +79,23 @@ def test_quantize_q4k_partial_groups_clamps_and_nans(bk, n_sb, bf16):
     dx.free(), out.free()
 
 
+@pytest.mark.parametrize("bf16", [False, True])
+def test_quantize_q4k_many_near_ties(bk, bf16):
+    """Weights of 0, 1/2, .. 15 with a largest scale of 1: d * sc is 1 - 4e-6, so 0.5, 1.5 and 2.5 lie within 1e-5 of a tie, in some sub-blocks of
+    a warp and not in others, in every chunk of eight."""
+    rng = np.random.default_rng(77)
+    x = rng.integers(0, 31, (33, 256)).astype(np.float32) / 2
+    x[:, ::32] = 0.0
+    x[:, 31::32] = 15.0
+    x[::3, 64:128] = np.round(x[::3, 64:128])       # no ties
+    x[1::4] -= 2.0                                  # a minimum as well
+    dx, out = R.DeviceBuffer.from_numpy(synth.f32_to_bf16(x) if bf16 else x), R.DeviceBuffer(33 * 144)
+    ops.quantize_q4k(dx.ptr, 33, 256, out.ptr, bf16=bf16)
+    assert R.cuSync() == 0
+    assert_same_bits(out.download(np.uint8, (33, 144)), O.q4k_quantize(x), "Q4_K superblocks")
+    dx.free(), out.free()
+
+
 def test_checkpoint_load_matches_host_quantised_model(bk, tmp_path):
     """A bf16 checkpoint with the reference's tensor names (model.language_model.layers.L...., tied embed_tokens) is
     loaded through the device quantiser; the model must decode exactly like one built from the same weights quantised
