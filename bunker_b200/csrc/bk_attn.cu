@@ -59,14 +59,10 @@ __device__ __forceinline__ void bf16x8_to_f32(uint4 v, float (&y)[8]) {
 }
 
 // head RMSNorm*(1+w) -> bf16 -> rotary on the first 2*rot_half dims, result in `stage`.  x and w: the row and the norm weights, 8 dims a lane;
-// the first 32 angles are requested before the norm that they wait for.
-__device__ __forceinline__ void norm_rope_256(uint4 xr, uint4 wr, const float* cos_row, const float* sin_row, int rot_half, uint16_t* stage) {
+// c and s: the lane's of the first 32 angles, which the caller has requested.
+__device__ __forceinline__ float first_angles(const float* row, int rot_half) { return (threadIdx.x & 31) < rot_half ? row[threadIdx.x & 31] : 0.0f; }
+__device__ __forceinline__ void norm_rope_256(uint4 xr, uint4 wr, float c, float s, const float* cos_row, const float* sin_row, int rot_half, uint16_t* stage) {
   const int lane = threadIdx.x & 31;
-  float c = 0.0f, s = 0.0f;
-  if (lane < rot_half) {
-    c = cos_row[lane];
-    s = sin_row[lane];
-  }
   float x[8], wv[8];
   bf16x8_to_f32(xr, x);
   bf16x8_to_f32(wr, wv);
@@ -173,7 +169,7 @@ __device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, flo
 //   v_st  : 256 bf16                    512
 //   m_s   : 8 f32 (+8 spare)             64
 //   l_s   : kW*8 f32                    256
-//   s_s   : split_len * heads (rounded up to a power of two) pairs of f32: the score, then p twice
+//   s_s   : split_len * heads (rounded up to a power of two) f32: the score, then p
 //   o_s   : kW*8*256 f32              65536   (the rings of rows, then the warps' sums, then the split merge)
 // One CTA per (split, KV head, batch).  Every warp streams its K rows and then its V rows through a ring of its own in shared memory,
 // 16 rows of 512 bytes, by asynchronous copies: a lane copies and reads back its own 16 bytes of a row, so nothing has to be
@@ -197,8 +193,9 @@ __global__ void __launch_bounds__(32) attn_append_kernel(const AttnParams p) {
   const int cb = b % p.n_seq;
   uint16_t* Kb = p.k_cache + ((size_t)cb * p.Hkv + kvh) * (size_t)p.max_len * kHD;
   uint16_t* Vb = p.v_cache + ((size_t)cb * p.Hkv + kvh) * (size_t)p.max_len * kHD;
+  const float *cr = p.cos_t + (size_t)pos * p.rot_half, *sr = p.sin_t + (size_t)pos * p.rot_half;
   norm_rope_256(*reinterpret_cast<const uint4*>(p.k + ((size_t)b * p.Hkv + kvh) * kHD + lane * 8), *reinterpret_cast<const uint4*>(p.k_norm_w + lane * 8),
-                p.cos_t + (size_t)pos * p.rot_half, p.sin_t + (size_t)pos * p.rot_half, p.rot_half, k_st);
+                first_angles(cr, p.rot_half), first_angles(sr, p.rot_half), cr, sr, p.rot_half, k_st);
   __syncwarp();
   *reinterpret_cast<uint4*>(Kb + (size_t)pos * kHD + lane * 8) = *reinterpret_cast<const uint4*>(k_st + lane * 8);
   *reinterpret_cast<uint4*>(Vb + (size_t)pos * kHD + lane * 8) =
@@ -220,7 +217,7 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   uint16_t* v_st = k_st + kHD;
   float* m_s = reinterpret_cast<float*>(v_st + kHD);
   float* l_s = m_s + 16;
-  float2* s_s = reinterpret_cast<float2*>(l_s + kW * 8);
+  float* s_s = l_s + kW * 8;
   float* o_s = reinterpret_cast<float*>(s_s + (size_t)p.split_len * GP);
   __shared__ int s_last;
 
@@ -278,14 +275,30 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   bk_stamp(p.trace, 2);
   uint4 xrow = make_uint4(0, 0, 0, 0);   // this warp's query head: it does not wait for the position
   if (warp < G) xrow = *reinterpret_cast<const uint4*>(p.qg + ((size_t)b * p.Hq + kvh * G + warp) * (p.fused ? 2 : 1) * kHD + lane * 8);
+  // What the query heads and the new row wait for is requested ahead of the cache's rows, and of those only the first batch: a warp gives out
+  // requests no faster than the SM takes them in, so with all four (two CTAs, 128 KB) the heads were ready 2.8 us after the start, with one 1.8.  8
+  // sequences, 6 heads, 4 KV heads, 450 rows 14.0 -> 13.5 us, 1,600 rows 22.3 -> 21.3; with two 13.7 and 21.5, with none 13.7 and 21.6.
+  float cos0 = 0.0f, sin0 = 0.0f;
+  uint4 krow = make_uint4(0, 0, 0, 0), vrow = krow, kw = wrow;
+  bool rest = false;   // the batches after the first have not been requested yet
   {
     // The position is taken (again) after the wait: the kernel that advances it may be only a few launches back and
     // still have been running when the early part above read it.  A changed value discards the early loads.
     const int pos_now = __ldcg(p.pos + b);
+    if (p.fused && pos_now >= j0 && (warp < G || warp == kW - 1)) {
+      cos0 = first_angles(p.cos_t + (size_t)pos_now * p.rot_half, p.rot_half);
+      sin0 = first_angles(p.sin_t + (size_t)pos_now * p.rot_half, p.rot_half);
+      if (p.n_seq == 0 && warp == kW - 1 && pos_now < j0 + p.split_len) {
+        krow = *reinterpret_cast<const uint4*>(p.k + ((size_t)b * p.Hkv + kvh) * kHD + lane * 8);
+        vrow = *reinterpret_cast<const uint4*>(p.v + ((size_t)b * p.Hkv + kvh) * kHD + lane * 8);
+        if (G == kW) kw = *reinterpret_cast<const uint4*>(p.k_norm_w + lane * 8);
+      }
+    }
     if (!p.settled || pos_now != pos) {
       asm volatile("cp.async.wait_all;" ::: "memory");
       set_pos(pos_now);
-      for (int q = 0; q < kBatches; q++) request(q, false);
+      request(0, false);
+      rest = true;
     }
   }
   if (ns <= 0) {
@@ -300,14 +313,12 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
     const float* cr = p.cos_t + (size_t)pos * p.rot_half;
     const float* sr = p.sin_t + (size_t)pos * p.rot_half;
     if (p.n_seq == 0 && warp == kW - 1 && owner) {
-      const uint4 k = *reinterpret_cast<const uint4*>(p.k + ((size_t)b * p.Hkv + kvh) * kHD + lane * 8);
-      const uint4 v = *reinterpret_cast<const uint4*>(p.v + ((size_t)b * p.Hkv + kvh) * kHD + lane * 8);
-      norm_rope_256(k, G == kW ? *reinterpret_cast<const uint4*>(p.k_norm_w + lane * 8) : wrow, cr, sr, p.rot_half, k_st);
+      norm_rope_256(krow, kw, cos0, sin0, cr, sr, p.rot_half, k_st);
       *reinterpret_cast<uint4*>(Kb + (size_t)pos * kHD + lane * 8) = *reinterpret_cast<const uint4*>(k_st + lane * 8);
-      *reinterpret_cast<uint4*>(Vb + (size_t)pos * kHD + lane * 8) = v;
-      *reinterpret_cast<uint4*>(v_st + lane * 8) = v;
+      *reinterpret_cast<uint4*>(Vb + (size_t)pos * kHD + lane * 8) = vrow;
+      *reinterpret_cast<uint4*>(v_st + lane * 8) = vrow;
     }
-    if (warp < G) norm_rope_256(xrow, wrow, cr, sr, p.rot_half, q_st + warp * kHD);
+    if (warp < G) norm_rope_256(xrow, wrow, cos0, sin0, cr, sr, p.rot_half, q_st + warp * kHD);
   } else {
     if (warp < G) *reinterpret_cast<uint4*>(q_st + warp * kHD + lane * 8) = xrow;
   }
@@ -315,6 +326,8 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
     *reinterpret_cast<uint4*>(k_st + lane * 8) = *reinterpret_cast<const uint4*>(Kb + (size_t)pos * kHD + lane * 8);
     *reinterpret_cast<uint4*>(v_st + lane * 8) = *reinterpret_cast<const uint4*>(Vb + (size_t)pos * kHD + lane * 8);
   }
+  if (rest)
+    for (int q = 1; q < kBatches; q++) request(q, false);
   __syncthreads();   // q and the row at pos are in shared memory
   bk_stamp(p.trace, 3);
   if (mine) {   // left out of the first requests
@@ -413,7 +426,7 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
 #pragma unroll
       for (int off = (1 << kPlain) >> 1; off >= 1; off >>= 1) s1 = __fadd_rn(s1, __shfl_xor_sync(0xffffffffu, s1, off));
       const int i = kRows * q + rsel;
-      if ((lane & ((1 << kPlain) - 1)) == 0 && i < nr) s_s[(size_t)(warp + 8 * i) * GP + hsel].x = __fmul_rn(s1, p.scale);
+      if ((lane & ((1 << kPlain) - 1)) == 0 && i < nr) s_s[(size_t)(warp + 8 * i) * GP + hsel] = __fmul_rn(s1, p.scale);
       request(q + kBatches, true);
       if (kTurn == 2 && q + 1 < nb) request(q + 1 + kBatches, true);   // (else batch q + 1 is the first of the V rows)
     }
@@ -426,7 +439,7 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
     constexpr int kStep = kW * 32 / GP;
     const int g = tid & (GP - 1);
     float m = -INFINITY;
-    for (int jj = tid / GP; jj < ns; jj += kStep) m = fmaxf(m, s_s[(size_t)jj * GP + g].x);
+    for (int jj = tid / GP; jj < ns; jj += kStep) m = fmaxf(m, s_s[(size_t)jj * GP + g]);
 #pragma unroll
     for (int off = GP; off < 32; off <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
     if (lane < GP) l_s[warp * 8 + lane] = m;  // l_s doubles as the cross-warp max buffer
@@ -439,10 +452,7 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
     }
     __syncthreads();
     const float mg = m_s[g];
-    for (int jj = tid / GP; jj < ns; jj += kStep) {
-      const float e = g < G ? bk_expf(__fsub_rn(s_s[(size_t)jj * GP + g].x, mg)) : 0.0f;
-      s_s[(size_t)jj * GP + g] = make_float2(e, e);   // twice: the factor of a packed FMA
-    }
+    for (int jj = tid / GP; jj < ns; jj += kStep) s_s[(size_t)jj * GP + g] = g < G ? bk_expf(__fsub_rn(s_s[(size_t)jj * GP + g], mg)) : 0.0f;
   }
   __syncthreads();
 
@@ -465,23 +475,19 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
         if (i < nr) {   // warp-uniform
           float vf[8];
           bf16x8_to_f32(rows[32 * r], vf);
-          const float2* ps = s_s + (size_t)(warp + 8 * i) * GP;
-          lw = __fadd_rn(lw, ps[lane & (GP - 1)].x);
+          const float* ps = s_s + (size_t)(warp + 8 * i) * GP;
+          lw = __fadd_rn(lw, ps[lane & (GP - 1)]);
+          float pp[GP];
+          if constexpr (GP >= 4) {
 #pragma unroll
-          for (int g = 0; g < G; g += 2) {
-            float2 pg[2];
-            if (GP > 1) {
-              const float4 pp = *reinterpret_cast<const float4*>(ps + g);
-              pg[0] = make_float2(pp.x, pp.y);
-              pg[1] = make_float2(pp.z, pp.w);
-            } else pg[0] = ps[0];
+            for (int g = 0; g < GP; g += 4) *reinterpret_cast<float4*>(pp + g) = *reinterpret_cast<const float4*>(ps + g);
+          } else if constexpr (GP == 2) {
+            *reinterpret_cast<float2*>(pp) = *reinterpret_cast<const float2*>(ps);
+          } else pp[0] = ps[0];
 #pragma unroll
-            for (int h = 0; h < 2; h++)
-              if (g + h < G) {
+          for (int g = 0; g < G; g++)
 #pragma unroll
-                for (int d = 0; d < 4; d++) acc[g + h < G ? g + h : 0][d] = bk_fma2(pg[h], make_float2(vf[2 * d], vf[2 * d + 1]), acc[g + h < G ? g + h : 0][d]);
-              }
-          }
+            for (int d = 0; d < 4; d++) acc[g][d] = bk_fma2(make_float2(pp[g], pp[g]), make_float2(vf[2 * d], vf[2 * d + 1]), acc[g][d]);
         }
       }
       request(nb + q + kBatches, true);
@@ -542,8 +548,6 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   }
 
   // ---- the CTA that completes this (batch, KV head) merges its splits ----
-  uint4 gate = make_uint4(0, 0, 0, 0);   // (requested before it is known whether it is this one)
-  if (warp < G) gate = head_gate(p, b, kvh * G + warp);
   __threadfence();
   __syncthreads();
   bk_stamp(p.trace, 7);
@@ -555,7 +559,7 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   __syncthreads();
   if (s_last) {
     __threadfence();
-    if (warp < G) combine_head_warp(p, b, kvh * G + warp, nsplits, o_s + warp * kMaxSplits, gate);  // one head per warp
+    if (warp < G) combine_head_warp(p, b, kvh * G + warp, nsplits, o_s + warp * kMaxSplits, head_gate(p, b, kvh * G + warp));  // one head per warp
     if (tid == 0) *cnt = 0;
   }
   bk_stamp(p.trace, 5);
@@ -563,7 +567,7 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
 
 size_t attn_smem_bytes(int split_len, int heads) {
   const int gp = heads <= 1 ? 1 : heads <= 2 ? 2 : heads <= 4 ? 4 : 8;
-  return 4096 + 1024 + 64 + 256 + (size_t)split_len * gp * 8 + (size_t)kW * 8 * kHD * 4;
+  return 4096 + 1024 + 64 + 256 + (size_t)split_len * gp * 4 + (size_t)kW * 8 * kHD * 4;
 }
 
 template <int G>
