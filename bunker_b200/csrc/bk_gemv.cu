@@ -660,17 +660,7 @@ int32_t bk_gemv_launch_tp(const bkGemvArgs& a, const BkPush* push, const BkReduc
   return tp ? launch_gemv<2, gemv_gmax(2), true>(p, grid, threads, smem) : launch_gemv<2, gemv_gmax(2), false>(p, grid, threads, smem);
 }
 
-// 9 to 16 columns are two launches on the mma.sync kernel, which is the faster the longer the rows: where rows * K^2 is small two of those are
-// faster, nine columns (the second launch is the batch-1 kernel) four times as long.  Measured with the image launch, 16 columns, two
-// launches / dense, us: K 1024, 24,576 rows 19.0 / 22.6, 49,152 32.3 / 26.3; K 2048, 9,216 rows 14.0 / 14.4, 12,288 18.9 / 17.8; K 4096, 2,048 rows
-// 13.7 / 13.3, 4,096 16.0 / 14.1; K 6144, 1,024 rows 17.5 / 12.5; K 17,408, 2,048 rows 53 / 26.  Nine columns: K 2048, 24,576 rows 23.3 / 25.3, 49,152
-// 37.7 / 34.2; K 6144, 2,048 rows 14.0 / 14.6, 9,216 28.3 / 22.3; K 17,408, 1,024 rows 34.7 / 17.4.  Where the two would copy a staged activation
-// instead of Q8_1 blocks (the steps and prompts of a model) they are faster and the line is further up: 13 sequences, in the step, K 6144, 2,048
-// rows 10.5 / 13.3, K 2048, 12,288 rows 15.2 / 15.9, 151,936 rows 142 / 83; 12 sequences, 64 layers 17.6 / 10.5 ms a step.
-bool bk_gemv_dense_lanes(int B, int rows, int K, bool staged) {
-  if (B <= 8 || B > 16) return B > 16;
-  return (double)rows * K * K >= (B == 9 ? 2e11 : staged ? 1.2e11 : 5.2e10);
-}
+bool bk_gemv_dense_lanes(int B) { return B > 16; }
 bool bk_gemv_auto_tile(int rows, int K) { return rows >= g_tile_min_rows || (rows >= g_tile_min_rows_cut && K >= 2048); }
 
 extern "C" {
