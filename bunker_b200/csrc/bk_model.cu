@@ -219,10 +219,11 @@ int32_t enqueue_step_persist(Model& m, int parity, int token = -1) {
 // the SMs read a row once per pair and wait for one another, where the chain's kernel reads a row once; everything else of a layer
 // is faster in one launch.  The chain takes over where the attention layers lose more than all layers gain, in us:
 //   one launch   2 + 2.2 per round + 0.07 per row of a split and round  (splits of 64, 128, 256, 448 rows: 6.8, 10.6, 19.8, 33.6 a round)
-//   chain        9 + 0.054 per row of a split + 0.4 per MB of keys and values
+//   chain        11.3 + 0.0185 per row of a split + 0.4 per MB of keys and values
 //   a layer's other launches 6, less 0.018 per MB of weights (5.0 of 24 layers of hidden 2048, 2.1 of 64 of hidden 5120)
-// Measured, chain / one launch: 24 layers, splits of 64 rows: 2,000 rows 752 / 626, 4,000 772 / 710; of 128: 8,000 rows 805 / 813, 16,000 844 / 1,063; of
-// 256: 8,000 rows 855 / 797, 32,000 915 / 1,430.  64 layers: splits of 64, 2,000 rows 4,814 / 4,745, 4,000 4,885 / 5,083.
+// Measured, chain / one launch: 24 layers, splits of 64 rows: 2,000 rows 755 / 618, 4,000 772 / 709; of 128: 8,000 rows 792 / 808, 16,000 830 / 1,056; of
+// 256: 8,000 rows 824 / 795, 32,000 882 / 1,427.  64 layers, splits of 64: 1,000 rows 4,740 / 4,597, 2,000 4,773 / 4,721, 4,000 4,845 / 5,025 (another B200:
+// 4,793 / 4,817, 4,826 / 4,936, 4,900 / 5,243); of 448: 8,000 rows 5,134 / 5,551.
 int plan_row_limit(const Model& m) {
   const bkModelConfig& c = m.cfg;
   const int pairs = (m.Hq / m.Hkv + 1) / 2;
@@ -236,7 +237,7 @@ int plan_row_limit(const Model& m) {
   for (int round = 1; rows < c.max_len; round++) {
     const long long end = std::min<long long>(c.max_len, (long long)bk_ctx().sm_count * round / (m.Hkv * pairs) * m.split_len);   // the last row of this round
     const double per_split = std::min((double)end, split), mb = (double)end * m.KVD * 4 / 1e6;
-    if (n_full * (2.0 + round * (2.2 + 0.07 * per_split) - (9.0 + 0.054 * per_split + 0.4 * mb)) > gain) break;
+    if (n_full * (2.0 + round * (2.2 + 0.07 * per_split) - (11.3 + 0.0185 * per_split + 0.4 * mb)) > gain) break;
     rows = (int)end;
   }
   return rows;
