@@ -175,8 +175,8 @@ __device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, flo
 // 16 rows of 512 bytes, by asynchronous copies: a lane copies and reads back its own 16 bytes of a row, so nothing has to be
 // synchronised, the copies of the first V rows run under the scores and the softmax, and 16 warps keep up to 128 KB on the way.  (Rows in
 // registers, three of a warp on their way, 200 instructions per K row and V row: 8 sequences, 32,768 rows, 8 heads per KV head 209 us = 0.39 of
-// the copy rate, 6 heads and 4 KV heads 330 us, 4 and 1 90 us.  Now 157, 257 and 68 us; 163 instructions, 55 % of the issue slots, and what is
-// waited for are results of the instruction before: FMAs of one chain, shuffles.)  Rows of the
+// the copy rate, 6 heads and 4 KV heads 330 us, 4 and 1 90 us.  Now 143, 239 and 65 us; 163 instructions with the probabilities stored in pairs,
+// 55 % of the issue slots, and what is waited for are results of the instruction before: FMAs of one chain, shuffles.)  Rows of the
 // cache that were written in earlier steps do not depend on the kernel running just before this one, so (p.settled) the first rows are
 // requested before the dependency wait.  The CTA that finishes a (batch, KV head) last merges the splits.
 // Two CTAs per SM (at most 128 registers): with one CTA of 8 warps an SM cannot hide the latency of the per-row

@@ -66,7 +66,7 @@ struct Cfg {
   static constexpr int PS = LANES ? 4 / NB : 4;                       // sub-block pairs of a superblock that a CTA handles
   // TMEM: kBatches batches of accumulators (128 columns each) and kA steps of operand A (32 each), handed over kHalf at a time.
   // What a step costs the MMA thread beside its MMAs is mostly waits, so few columns take larger halves and fewer batches -- but in the
-  // lane order, whose scalers pause at the end of a class, three batches are better (32 columns, 152k rows: 176 us, with two 199).
+  // lane order, whose scalers pause at the end of a class, three batches are better (32 columns, 152k rows, when that took 176 us: with two 199; now 137).
   static constexpr int kBatches = LANES || NB == 4 ? 3 : 2, kA = LANES || NB == 4 ? 4 : 8, kHalf = kA / 2;
   static constexpr int BT = 4 / NB;                                   // steps per batch of the scalers: 128 TMEM columns
   static constexpr int kTabs = kA + kBatches * BT;               // row tables: a step's is read before its successor's is written (see there)
