@@ -173,7 +173,7 @@ __device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, flo
 //   o_s   : kW*8*256 f32              65536   (the rings of rows, then the warps' sums, then the split merge)
 // One CTA per (split, KV head, batch).  Every warp streams its K rows and then its V rows through a ring of its own in shared memory,
 // 16 rows of 512 bytes, by asynchronous copies: a lane copies and reads back its own 16 bytes of a row, so nothing has to be
-// synchronised, the copies of the first V rows run under the scores and the softmax, and 16 warps keep up to 128 KB on the way.  (Rows in
+// synchronised until the sums take the ring's place, the copies of the first V rows run under the scores and the softmax, and 16 warps keep up to 128 KB on the way.  (Rows in
 // registers, three of a warp on their way, 200 instructions per K row and V row: 8 sequences, 32,768 rows, 8 heads per KV head 209 us = 0.39 of
 // the copy rate, 6 heads and 4 KV heads 330 us, 4 and 1 90 us.  Now 143, 239 and 65 us; 163 instructions with the probabilities stored in pairs,
 // 55 % of the issue slots, and what is waited for are results of the instruction before: FMAs of one chain, shuffles.)  Rows of the
@@ -493,6 +493,7 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
       request(nb + q + kBatches, true);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();   // a lane's sums go over other lanes' bytes of the ring, which those have read by now
 #pragma unroll
     for (int g = 0; g < G; g++) {   // over this warp's ring
       float4* d = reinterpret_cast<float4*>(o_s + ((size_t)(warp * 8 + g)) * kHD + lane * 8);

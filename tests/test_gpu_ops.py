@@ -375,6 +375,40 @@ def test_attn_decode_row_lists(bk, Hq, Hkv):
         assert_same_bits(got, want, f"attention, {Hq} heads on {Hkv}, positions {pos}")
 
 
+@pytest.mark.parametrize("Hq,Hkv", [(1, 1), (4, 2), (3, 1), (4, 1), (5, 1), (6, 1), (7, 1), (8, 1)])
+@pytest.mark.parametrize("fused", [1, 0])
+@pytest.mark.parametrize("settled", [1, 0])
+def test_attn_decode_entry_forms(bk, Hq, Hkv, fused, settled):
+    """The rows before the dependency wait or after it, the row at the position made here or already in the cache: lists of rows that end in
+    every place of a batch and of the ring, a position at each end of a split, the buffers of one call taken on by the next."""
+    cos_t, sin_t = ops.rope_tables(1024)
+    B, HD, ml, split_len = 6, 256, 640, 320   # 40 rows a warp
+    c = synth.attn_case(B, ml, Hq=Hq, Hkv=Hkv, max_len=ml, config_id=90 + Hq)
+    W = ops.attn_plan(ml, B, Hkv)[1]
+    d = {k: dev(v) for k, v in c.items() if isinstance(v, np.ndarray)}
+    dc, ds, out = dev(cos_t), dev(sin_t), R.DeviceBuffer(B * Hq * HD * 2)
+    gate = np.ascontiguousarray(c["qg"].reshape(B, Hq, 2, HD)[:, :, 1])
+    dgate, dq = dev(gate), R.DeviceBuffer(B * Hq * HD * 2)
+    scratch = R.DeviceBuffer.zeros(ops.attn_scratch_bytes(B, Hq, HD, ml, split_len))
+    for pos in ([0, 7, 8, 30, 33, 63], [96, 127, 128, 130, 167, 200], [319, 320, 327, 450, 452, 639], [640 - 8, 0, 319, 31, 511, 576]):
+        c["pos"] = np.array(pos, np.int32)
+        q, Kc, Vc, want = _attn_oracle(c, cos_t, sin_t, split_len, W)
+        if not fused:   # the row at the position is there, the heads are normalised and rotated
+            d["k_cache"].upload(Kc), d["v_cache"].upload(Vc), dq.upload(q)
+        d["pos"].upload(c["pos"])
+        for _ in range(2):
+            ops.attn_decode(qg=d["qg"].ptr if fused else dq.ptr, k=d["k"].ptr, v=d["v"].ptr, q_norm_w=d["q_norm_w"].ptr, k_norm_w=d["k_norm_w"].ptr,
+                            gate=dgate.ptr, cos_t=dc.ptr, sin_t=ds.ptr, k_cache=d["k_cache"].ptr, v_cache=d["v_cache"].ptr, pos=d["pos"].ptr, out=out.ptr,
+                            scratch=scratch.ptr, B=B, Hq=Hq, Hkv=Hkv, HD=HD, rot_half=32, max_len=ml, split_len=split_len, max_pos=ml - 1, scale=1.0 / 16.0,
+                            fused_norm_rope=fused, cache_is_settled=settled)
+        assert_same_bits(out.download(np.uint16, (B, Hq * HD)), want, f"attention, {Hq} heads on {Hkv}, positions {pos}")
+        assert_same_bits(d["k_cache"].download(np.uint16, Kc.shape), Kc, "k cache")
+        assert_same_bits(d["v_cache"].download(np.uint16, Vc.shape), Vc, "v cache")
+        c["k_cache"], c["v_cache"] = Kc, Vc
+    for b in list(d.values()) + [dc, ds, out, dgate, dq, scratch]:
+        b.free()
+
+
 @pytest.mark.parametrize("B,L", [(1, 32768), (8, 4096), (8, 32768)])
 def test_attn_decode_long_context(bk, B, L):
     """configs[2] long caches (4096 and 32768 rows) at batch 1 and 8, default plan; bit-exact against the oracle."""
