@@ -102,9 +102,6 @@ __device__ __forceinline__ void butterfly_level(float (&v)[N], int off) {
   }
 }
 
-// merge the splits of one (batch, q head) by one warp; lane l owns output dims [8l, 8l+8).
-// w_s: ns floats of shared memory private to the warp.  M = max m_s; w_s = exp(m_s - M);
-// L = fma(w_s, l_s, L) and O = fma(w_s, o_s, O) in ascending s; out = (O/L) * sigmoid(gate).
 __device__ __forceinline__ uint4 head_gate(const AttnParams& p, int b, int h) {
   const int lane = threadIdx.x & 31;
   return *reinterpret_cast<const uint4*>(p.fused ? p.qg + ((size_t)b * p.Hq + h) * 2 * kHD + kHD + lane * 8 : p.gate + ((size_t)b * p.Hq + h) * kHD + lane * 8);
@@ -135,32 +132,101 @@ __device__ void store_head_warp(const AttnParams& p, int b, int h, const float (
   }
 }
 
-__device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, float* w_s, uint4 gate) {
-  const int lane = threadIdx.x & 31;
-  const float* sc_ml = p.part_ml + ((size_t)b * p.Hq + h) * p.max_splits * 2;
-  const float* sc_o = p.part_o + ((size_t)b * p.Hq + h) * p.max_splits * kHD;
-  float m = -INFINITY;
-  for (int s = lane; s < ns; s += 32) {
-    float ms = __ldcg(sc_ml + 2 * s);
-    w_s[s] = ms;
-    m = fmaxf(m, ms);
-  }
-  const float M = bk_warp_max(m);
-  for (int s = lane; s < ns; s += 32) w_s[s] = bk_expf(__fsub_rn(w_s[s], M));
-  __syncwarp();
-  float L = 0.0f, O[8];
+// Merge the splits of one (batch, KV head), all threads of a CTA: M = max m_s; w_s = exp(m_s - M); L = fma(w_s, l_s, L) and O = fma(w_s, o_s, O) in
+// ascending s; out = (O/L) * sigmoid(gate).  wl: G * ns pairs of shared memory; where a head has more than one warp they then take its sums.
+// Bound: latency of L2, with one CTA at work.  The heads' dims are spread over all eight warps, so that 64 values a thread (32 where 80 registers
+// are all there are) are on their way at a time, the first of them while the weights are made.  With a head a warp and four splits requested
+// together the whole kernel took, us, so now: one head, 141 splits 25.7, 14.4, 157 splits 26.2, 16.3; 4 heads on 4, 40 splits 14.1, 11.7; 16 on 2, 63 splits 20.9,
+// 19.9.  Few splits leave a head to its warp (V = 8), which then meets nobody: 8 heads on 8, 8 sequences, four
+// splits of 128 12.7, 12.1.
+template <int G, int V>   // V: dims of a thread
+__device__ __forceinline__ void merge_splits(const AttnParams& p, int b, int kvh, int ns, float2* wl, float* l_s) {
+  constexpr int T = kHD / V, U = (G == 1 || (G <= 4 && V == 8) ? 32 : 64) / V;   // threads of a head, splits requested together
+  constexpr int kHeads = kW * 32 / T, kPasses = (G + kHeads - 1) / kHeads;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, col = tid % T * V;
+  const float* src = nullptr;
+  float o[U][V];
+  auto request = [&](int s0) {
 #pragma unroll
-  for (int e = 0; e < 8; e++) O[e] = 0.0f;
-#pragma unroll 4
-  for (int s = 0; s < ns; s++) {
-    const float w = w_s[s];
-    L = fmaf(w, __ldcg(sc_ml + 2 * s + 1), L);
-    const float4 a = __ldcg(reinterpret_cast<const float4*>(sc_o + (size_t)s * kHD + lane * 8));
-    const float4 c = __ldcg(reinterpret_cast<const float4*>(sc_o + (size_t)s * kHD + lane * 8) + 1);
-    O[0] = fmaf(w, a.x, O[0]); O[1] = fmaf(w, a.y, O[1]); O[2] = fmaf(w, a.z, O[2]); O[3] = fmaf(w, a.w, O[3]);
-    O[4] = fmaf(w, c.x, O[4]); O[5] = fmaf(w, c.y, O[5]); O[6] = fmaf(w, c.z, O[6]); O[7] = fmaf(w, c.w, O[7]);
+    for (int i = 0; i < U; i++)
+      if (s0 + i < ns) {
+        const float* at = src + (size_t)(s0 + i) * kHD;
+        if constexpr (V >= 4) {
+#pragma unroll
+          for (int e = 0; e < V; e += 4) *reinterpret_cast<float4*>(o[i] + e) = __ldcg(reinterpret_cast<const float4*>(at + e));
+        } else if constexpr (V == 2) {
+          *reinterpret_cast<float2*>(o[i]) = __ldcg(reinterpret_cast<const float2*>(at));
+        } else {
+          o[i][0] = __ldcg(at);
+        }
+      }
+  };
+  auto enter = [&](int g) {
+    src = p.part_o + ((size_t)b * p.Hq + kvh * G + min(g, G - 1)) * p.max_splits * kHD + col;
+    if (g < G) request(0);
+  };
+  enter(tid / T);
+  uint4 gate = make_uint4(0, 0, 0, 0);
+  if (warp < G) {
+    gate = head_gate(p, b, kvh * G + warp);
+    const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + ((size_t)b * p.Hq + kvh * G + warp) * p.max_splits;
+    float2* mine = wl + warp * ns;
+    float m = -INFINITY;
+    for (int s = lane; s < ns; s += 32) {
+      const float2 v = __ldcg(ml + s);
+      mine[s] = v;
+      m = fmaxf(m, v.x);
+    }
+    const float M = bk_warp_max(m);
+    for (int s = lane; s < ns; s += 32) mine[s].x = bk_expf(__fsub_rn(mine[s].x, M));
   }
-  store_head_warp(p, b, h, O, L, gate);
+  if (T > 32) __syncthreads();
+  else __syncwarp();
+  float L[kPasses], O[kPasses][V];
+#pragma unroll
+  for (int pass = 0; pass < kPasses; pass++) {
+    const int g = pass * kHeads + tid / T;
+    if (pass) enter(g);
+    L[pass] = 0.0f;
+#pragma unroll
+    for (int e = 0; e < V; e++) O[pass][e] = 0.0f;
+    if (g < G) {
+#pragma unroll 1
+      for (int s0 = 0; s0 < ns; s0 += U) {
+        if (s0) request(s0);
+#pragma unroll
+        for (int i = 0; i < U; i++)
+          if (s0 + i < ns) {
+            const float2 w = wl[g * ns + s0 + i];
+            L[pass] = fmaf(w.x, w.y, L[pass]);
+#pragma unroll
+            for (int e = 0; e < V; e++) O[pass][e] = fmaf(w.x, o[i][e], O[pass][e]);
+          }
+      }
+    }
+  }
+  if constexpr (V == 8) {
+    if (warp < G) store_head_warp(p, b, kvh * G + warp, O[0], L[0], gate);
+  } else {
+    __syncthreads();   // the weights have been read
+    float* sums = reinterpret_cast<float*>(wl);
+#pragma unroll
+    for (int pass = 0; pass < kPasses; pass++) {
+      const int g = pass * kHeads + tid / T;
+      if (g < G) {
+#pragma unroll
+        for (int e = 0; e < V; e++) sums[g * kHD + col + e] = O[pass][e];
+        if (col == 0) l_s[g] = L[pass];
+      }
+    }
+    __syncthreads();
+    if (warp < G) {
+      float out[8];
+#pragma unroll
+      for (int e = 0; e < 8; e++) out[e] = sums[warp * kHD + lane * 8 + e];
+      store_head_warp(p, b, kvh * G + warp, out, l_s[warp], gate);
+    }
+  }
 }
 
 // dynamic shared memory layout (bytes):
@@ -175,8 +241,8 @@ __device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, flo
 // 16 rows of 512 bytes, by asynchronous copies: a lane copies and reads back its own 16 bytes of a row, so nothing has to be
 // synchronised until the sums take the ring's place, the copies of the first V rows run under the scores and the softmax, and 16 warps keep up to 128 KB on the way.  (Rows in
 // registers, three of a warp on their way, 200 instructions per K row and V row: 8 sequences, 32,768 rows, 8 heads per KV head 209 us = 0.39 of
-// the copy rate, 6 heads and 4 KV heads 330 us, 4 and 1 90 us.  Now 143, 239 and 65 us; 163 instructions with the probabilities stored in pairs,
-// 55 % of the issue slots, and what is waited for are results of the instruction before: FMAs of one chain, shuffles.)  Rows of the
+// the copy rate, 6 heads and 4 KV heads 330 us, 4 and 1 90 us.  Now 139, 236 and 62 us; 163 instructions,
+// 58 % of the issue slots, and what is waited for are results of the instruction before: FMAs of one chain, shuffles.)  Rows of the
 // cache that were written in earlier steps do not depend on the kernel running just before this one, so (p.settled) the first rows are
 // requested before the dependency wait.  The CTA that finishes a (batch, KV head) last merges the splits.
 // Two CTAs per SM (at most 128 registers): with one CTA of 8 warps an SM cannot hide the latency of the per-row
@@ -204,10 +270,10 @@ __global__ void __launch_bounds__(32) attn_append_kernel(const AttnParams p) {
 
 constexpr int kRows = 4;      // rows requested together
 constexpr int kBatches = 4;   // such batches of a warp on their way or in use
-static_assert(kRows * kBatches * kHD * 2 == 8 * kHD * 4, "a warp's ring is its part of o_s");
 
 template <int G>
-__global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams p) {
+__global__ void __launch_bounds__(kW * 32, G == 1 ? 3 : 2) attn_split_kernel(const AttnParams p) {
+  static_assert(kRows * kBatches * kHD * 2 <= 8 * kHD * 4, "a warp's ring is its part of o_s");
   constexpr int GP = G <= 1 ? 1 : G <= 2 ? 2 : G <= 4 ? 4 : 8;   // heads, up to a power of two
   bk_pdl_trigger();
   bk_stamp(p.trace, 0);
@@ -345,7 +411,7 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
     // lane takes what the first levels halve in an order of its own, g ^ hsel or r ^ rsel, so that in each of them it keeps the first half
     // and sends the second.
     constexpr bool kHeadsFirst = G == GP;
-    constexpr int kTurn = GP <= 2 ? 2 : 1, R = kRows * kTurn;   // batches, rows scored together: eight where they have few heads (latency, not work)
+    constexpr int kTurn = GP <= 2 && kBatches > 2 ? 2 : 1, R = kRows * kTurn;   // batches, rows scored together: eight where they have few heads (latency, not work)
     constexpr int HB = GP == 8 ? 3 : GP == 4 ? 2 : GP == 2 ? 1 : 0, RB = kTurn + 1, kPlain = 5 - HB - RB;   // levels that halve heads, rows, nothing
     const int hsel = kHeadsFirst ? lane >> (5 - HB) : (lane >> kPlain) & (GP - 1);   // the head and the row whose score this lane ends up with
     const int rsel = kHeadsFirst ? (lane >> kPlain) & (R - 1) : lane >> 3;
@@ -560,7 +626,9 @@ __global__ void __launch_bounds__(kW * 32, 2) attn_split_kernel(const AttnParams
   __syncthreads();
   if (s_last) {
     __threadfence();
-    if (warp < G) combine_head_warp(p, b, kvh * G + warp, nsplits, o_s + warp * kMaxSplits, head_gate(p, b, kvh * G + warp));  // one head per warp
+    constexpr int V = G <= 2 ? G : G <= 4 || kBatches != 2 ? 4 : 8;
+    if (V < 8 && nsplits <= 8) merge_splits<G, 8>(p, b, kvh, nsplits, reinterpret_cast<float2*>(o_s), l_s);
+    else merge_splits<G, V>(p, b, kvh, nsplits, reinterpret_cast<float2*>(o_s), l_s);
     if (tid == 0) *cnt = 0;
   }
   bk_stamp(p.trace, 5);
@@ -572,14 +640,14 @@ size_t attn_smem_bytes(int split_len, int heads) {
 }
 
 template <int G>
-int32_t launch_split(const AttnParams& p, dim3 grid) {
+int32_t launch_split(const AttnParams& p, int nsplit) {
   static size_t configured = 0;
   const size_t smem = attn_smem_bytes(p.split_len, G);
   if (smem > configured) {
     BK_CUDA(cudaFuncSetAttribute(attn_split_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = smem;
   }
-  BK_CUDA(bk_launch_pdl(attn_split_kernel<G>, grid, dim3(kW * 32), smem, p));
+  BK_CUDA(bk_launch_pdl(attn_split_kernel<G>, dim3(nsplit, p.Hkv, p.B), dim3(kW * 32), smem, p));
   BK_CHECK_LAUNCH();
   return BK_OK;
 }
@@ -691,17 +759,16 @@ int32_t bk_attn_launch(const bkAttnArgs& args, int n_seq, int layout_B) {
     BK_CUDA(bk_launch_pdl(attn_append_kernel, dim3(a.Hkv, a.B), dim3(32), 0, p));
     BK_CHECK_LAUNCH();
   }
-  dim3 grid(nsplit, a.Hkv, a.B);
   int32_t rc;
   switch (a.Hq / a.Hkv) {
-    case 1: rc = launch_split<1>(p, grid); break;
-    case 2: rc = launch_split<2>(p, grid); break;
-    case 3: rc = launch_split<3>(p, grid); break;
-    case 4: rc = launch_split<4>(p, grid); break;
-    case 5: rc = launch_split<5>(p, grid); break;
-    case 6: rc = launch_split<6>(p, grid); break;
-    case 7: rc = launch_split<7>(p, grid); break;
-    default: rc = launch_split<8>(p, grid); break;
+    case 1: rc = launch_split<1>(p, nsplit); break;
+    case 2: rc = launch_split<2>(p, nsplit); break;
+    case 3: rc = launch_split<3>(p, nsplit); break;
+    case 4: rc = launch_split<4>(p, nsplit); break;
+    case 5: rc = launch_split<5>(p, nsplit); break;
+    case 6: rc = launch_split<6>(p, nsplit); break;
+    case 7: rc = launch_split<7>(p, nsplit); break;
+    default: rc = launch_split<8>(p, nsplit); break;
   }
   if (rc) return rc;
   return BK_OK;

@@ -409,6 +409,20 @@ def test_attn_decode_entry_forms(bk, Hq, Hkv, fused, settled):
         b.free()
 
 
+@pytest.mark.parametrize("Hq,Hkv", [(1, 1), (4, 2), (3, 1), (4, 1), (5, 1), (6, 1), (7, 1), (8, 1)])
+def test_attn_decode_merge_of_many_splits(bk, Hq, Hkv):
+    """Splits of 8 rows, one to 141 of them to merge: either side of what a warp merges alone, whole and partial groups of splits requested together,
+    for every number of query heads per KV head."""
+    cos_t, sin_t = ops.rope_tables(2048)
+    L, split_len = 1128, 8
+    c = synth.attn_case(9, L, Hq=Hq, Hkv=Hkv, max_len=L, config_id=110 + Hq)
+    c["pos"] = np.array([n * split_len - 1 - i % 8 for i, n in enumerate([1, 2, 8, 9, 16, 33, 64, 65, 141])], np.int32)
+    got, Kg, Vg, split_len, W = _run_attn(c, cos_t, sin_t, split_len=split_len)
+    q, Kc, Vc, want = _attn_oracle(c, cos_t, sin_t, split_len, W)
+    assert_same_bits(Kg, Kc, "k cache after append")
+    assert_same_bits(got, want, f"attention, {Hq} heads on {Hkv}")
+
+
 @pytest.mark.parametrize("B,L", [(1, 32768), (8, 4096), (8, 32768)])
 def test_attn_decode_long_context(bk, B, L):
     """configs[2] long caches (4096 and 32768 rows) at batch 1 and 8, default plan; bit-exact against the oracle."""
