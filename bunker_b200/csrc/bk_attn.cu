@@ -16,6 +16,8 @@
 #include "bk_common.cuh"
 #include "bk_internal.h"
 
+#include <algorithm>
+
 namespace {
 
 constexpr int kW = 8;        // warps per split CTA
@@ -238,8 +240,8 @@ __device__ __forceinline__ void merge_splits(const AttnParams& p, int b, int kvh
 //   s_s   : split_len * heads (rounded up to a power of two) f32: the score, then p
 //   o_s   : kW*8*256 f32              65536   (the rings of rows, then the warps' sums, then the split merge)
 // One CTA per (split, KV head, batch).  Every warp streams its K rows and then its V rows through a ring of its own in shared memory,
-// 16 rows of 512 bytes, by asynchronous copies: a lane copies and reads back its own 16 bytes of a row, so nothing has to be
-// synchronised until the sums take the ring's place, the copies of the first V rows run under the scores and the softmax, and 16 warps keep up to 128 KB on the way.  (Rows in
+// 8 or 16 rows of 512 bytes, by asynchronous copies: a lane copies and reads back its own 16 bytes of a row, so nothing has to be
+// synchronised until the sums take the ring's place, the copies of the first V rows run under the scores and the softmax, and 16 warps keep 64 or 128 KB on the way.  (Rows in
 // registers, three of a warp on their way, 200 instructions per K row and V row: 8 sequences, 32,768 rows, 8 heads per KV head 209 us = 0.39 of
 // the copy rate, 6 heads and 4 KV heads 330 us, 4 and 1 90 us.  Now 139, 236 and 62 us; 163 instructions,
 // 58 % of the issue slots, and what is waited for are results of the instruction before: FMAs of one chain, shuffles.)  Rows of the
@@ -269,9 +271,9 @@ __global__ void __launch_bounds__(32) attn_append_kernel(const AttnParams p) {
 }
 
 constexpr int kRows = 4;      // rows requested together
-constexpr int kBatches = 4;   // such batches of a warp on their way or in use
 
-template <int G>
+// kBatches: batches of rows of a warp on their way or in use
+template <int G, int kBatches>
 __global__ void __launch_bounds__(kW * 32, G == 1 ? 3 : 2) attn_split_kernel(const AttnParams p) {
   static_assert(kRows * kBatches * kHD * 2 <= 8 * kHD * 4, "a warp's ring is its part of o_s");
   constexpr int GP = G <= 1 ? 1 : G <= 2 ? 2 : G <= 4 ? 4 : 8;   // heads, up to a power of two
@@ -639,17 +641,31 @@ size_t attn_smem_bytes(int split_len, int heads) {
   return 4096 + 1024 + 64 + 256 + (size_t)split_len * gp * 4 + (size_t)kW * 8 * kHD * 4;
 }
 
-template <int G>
-int32_t launch_split(const AttnParams& p, int nsplit) {
+template <int G, int kBatches>
+int32_t launch_split_batches(const AttnParams& p, dim3 grid, size_t smem) {
   static size_t configured = 0;
-  const size_t smem = attn_smem_bytes(p.split_len, G);
   if (smem > configured) {
-    BK_CUDA(cudaFuncSetAttribute(attn_split_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BK_CUDA(cudaFuncSetAttribute(attn_split_kernel<G, kBatches>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = smem;
   }
-  BK_CUDA(bk_launch_pdl(attn_split_kernel<G>, dim3(nsplit, p.Hkv, p.B), dim3(kW * 32), smem, p));
+  BK_CUDA(bk_launch_pdl(attn_split_kernel<G, kBatches>, grid, dim3(kW * 32), smem, p));
   BK_CHECK_LAUNCH();
   return BK_OK;
+}
+
+// Two batches of rows on their way where the splits are short or two CTAs an SM hold all of them, else four.  There more requests bring no more bytes, but
+// the query heads come later behind them and some CTAs run far ahead of others (24 heads on 4, four / two batches, us: 8 sequences, 900 rows, 256 splits of 128
+// 17.6 / 17.1, 2,000 rows, 256 of 256 25.1 / 24.2, 600 rows, 320 of 64 21.0 / 19.7; but 5 sequences, 9,000 rows, 360 of 512 60.1 / 67.3).
+// One head per KV head leaves room for three CTAs an SM, which many splits want (16 sequences, 8 heads, 560 rows, 384 splits 18.5 us, two an SM 25.4).  What two an
+// SM hold gets two at most, by shared memory that it does not use: three make an uneven spread, since the launch before still holds some SMs (6
+// sequences, 8 heads, 1,100 rows, 288 splits 18.2 us, so 15.2).
+template <int G>
+int32_t launch_split(const AttnParams& p, int nsplit) {
+  const bool two_an_sm = (long long)nsplit * p.Hkv * p.B <= 2 * bk_ctx().sm_count;
+  size_t smem = attn_smem_bytes(p.split_len, G);
+  if (G == 1 && two_an_sm) smem = std::max<size_t>(smem, bk_ctx().smem_optin / 3);
+  const dim3 grid(nsplit, p.Hkv, p.B);
+  return p.split_len <= 128 || (p.split_len <= 256 && two_an_sm) ? launch_split_batches<G, 2>(p, grid, smem) : launch_split_batches<G, 4>(p, grid, smem);
 }
 
 }  // namespace

@@ -423,6 +423,20 @@ def test_attn_decode_merge_of_many_splits(bk, Hq, Hkv):
     assert_same_bits(got, want, f"attention, {Hq} heads on {Hkv}")
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,L,split_len", [(1, 8, 1, 8185, 8),       # the most splits there may be, for the most heads
+                                                  (148, 2, 1, 16, 8), (149, 2, 1, 16, 8), (74, 6, 2, 16, 8), (75, 6, 2, 16, 8),   # as many as two an SM hold and more
+                                                  (98, 1, 1, 270, 136), (99, 1, 1, 270, 136), (149, 1, 1, 270, 136),             # the same, and three an SM
+                                                  (3, 8, 2, 130, 128), (3, 8, 2, 270, 136), (3, 8, 2, 260, 256), (3, 8, 2, 300, 264)])   # longer splits
+def test_attn_decode_at_the_edges_of_its_rule(bk, B, Hq, Hkv, L, split_len):
+    cos_t, sin_t = ops.rope_tables(max(L, 64))
+    c = synth.attn_case(B, L, Hq=Hq, Hkv=Hkv, config_id=130 + Hq)
+    c["pos"] = np.array([L - 1 - (3 * b) % min(L, 9) for b in range(B)], np.int32)
+    got, Kg, Vg, split_len, W = _run_attn(c, cos_t, sin_t, split_len=split_len)
+    q, Kc, Vc, want = _attn_oracle(c, cos_t, sin_t, split_len, W)
+    assert_same_bits(Kg, Kc, "k cache after append")
+    assert_same_bits(got, want, f"attention B={B} L={L} split_len={split_len}")
+
+
 @pytest.mark.parametrize("B,L", [(1, 32768), (8, 4096), (8, 32768)])
 def test_attn_decode_long_context(bk, B, L):
     """configs[2] long caches (4096 and 32768 rows) at batch 1 and 8, default plan; bit-exact against the oracle."""
