@@ -79,16 +79,40 @@ def test_quantize_q4k_partial_groups_clamps_and_nans(bk, n_sb, bf16):
     dx.free(), out.free()
 
 
+def _near_tie_weights(bf16: bool):
+    """33 superblocks with d = dmin = 2^-5 exactly: sub-block 0 has the largest scale, 63 steps, sub-block 1 the largest minimum, the others whole
+    numbers of both.  Weights on integers and on ties, all of them bf16 numbers; as f32 a third of those on ties is moved by an ulp to either side.
+    Returns the weights and how far each quotient is from a tie."""
+    rng = np.random.default_rng(77)
+    x, off = np.empty((33, 8, 32), np.float32), np.empty((33, 8, 32))
+    for sb in range(33):
+        for j in range(8):
+            s, m = (63, 1) if j == 0 else (8, 63) if j == 1 else (rng.choice([1, 2, 3, 4, 5, 6, 7, 8, 12, 16, 24, 32]), 0) if j < 6 else (rng.choice([2, 4, 8]), rng.integers(0, 63))
+            n = rng.integers(0, 15, 32) + (0.5 if (sb + j) % 3 else rng.choice([0.0, 0.5], 32))
+            if j == 0:
+                n = rng.choice([0.5, 1.5], 32)
+            if sb % 4 == 2 and j > 3:
+                n = np.floor(n)      # no ties
+            v = (n * s - m).astype(np.float32)
+            v[rng.integers(0, 16)], v[16 + rng.integers(0, 16)] = -m, 15 * s - m
+            if not bf16:
+                t = (v + m) / s
+                on = t != np.floor(t)
+                v = np.where(on & (rng.random(32) < 1 / 3), np.nextafter(v, np.float32(rng.choice([-1e9, 1e9]))), v).astype(np.float32)
+            x[sb, j] = v / 32
+            t = (v.astype(np.float64) + m) / s
+            off[sb, j] = np.abs(t - np.floor(t) - 0.5)
+    return x.reshape(33, 256), off
+
+
 @pytest.mark.parametrize("bf16", [False, True])
 def test_quantize_q4k_many_near_ties(bk, bf16):
-    """Weights of 0, 1/2, .. 15 with a largest scale of 1: d * sc is 1 - 4e-6, so 0.5, 1.5 and 2.5 lie within 1e-5 of a tie, in some sub-blocks of
-    a warp and not in others, in every chunk of eight."""
-    rng = np.random.default_rng(77)
-    x = rng.integers(0, 31, (33, 256)).astype(np.float32) / 2
-    x[:, ::32] = 0.0
-    x[:, 31::32] = 15.0
-    x[::3, 64:128] = np.round(x[::3, 64:128])       # no ties
-    x[1::4] -= 2.0                                  # a minimum as well
+    """Several lanes of a warp (32 sub-blocks) have a quotient within 1e-5 of a tie, in each of the four chunks of eight weights, and others have none."""
+    x, off = _near_tie_weights(bf16)
+    assert np.array_equal(synth.bf16_to_f32(synth.f32_to_bf16(x)), x) == bf16
+    near = off[:32].reshape(8, 32, 4, 8).min(axis=3) < 1e-5   # warp, lane, chunk
+    assert near.sum(axis=1).min() >= 8 and (~near).sum(axis=1).min() >= 4
+    assert (O.q4k_quantize(x).reshape(33, 144)[:, :4].copy().view(np.float16) == 2.0 ** -5).all()
     dx, out = R.DeviceBuffer.from_numpy(synth.f32_to_bf16(x) if bf16 else x), R.DeviceBuffer(33 * 144)
     ops.quantize_q4k(dx.ptr, 33, 256, out.ptr, bf16=bf16)
     assert R.cuSync() == 0
