@@ -330,6 +330,45 @@ def test_scaled_model_shapes_batch32_tile_path(bk):
     gm.destroy()
 
 
+# A GDN and an attention layer of the 64-layer configuration's widths with a small FFN and vocabulary: from ten columns on the input and the output
+# projections (16,480 and 14,336 rows of 5,120, 5,120 rows of 6,144) take the dense tile kernel, whose image the norm, GDN and attention kernels
+# write; with nine only the input projections do.  The FFN and the vocabulary (2,048 rows and fewer) go in groups of eight columns.
+WIDE = M.CONFIG_HYBRID_64L.with_(n_layers=2, full_attn_interval=2, intermediate=512, vocab=2048, max_len=64)
+
+
+@pytest.mark.parametrize("B", [9, 10, 13, 15])
+def test_nine_to_fifteen_sequences_of_wide_projections(bk, B):
+    w = M.synth_weights(WIDE, seed=80)
+    gm = M.DecodeModel(WIDE, w, batch=B)
+    info = gm.info()
+    om = OracleModel(WIDE, w, batch=B, split_len=info["split_len"], attn_warps=info["attn_warps"])
+    prompt = np.random.default_rng(81).integers(0, WIDE.vocab, (2, B)).astype(np.int32)
+    ids_g = ids_o = None
+    for t in range(3):
+        ids_o, _ = om.step(prompt[t] if t < 2 else ids_o)
+        ids_g, _ = gm.step(prompt[t] if t < 2 else ids_g)
+        assert_same_bits(gm.logits(), om.logits, f"logits at step {t}")
+    gm.destroy()
+
+
+@pytest.mark.parametrize("B,T", [(1, 9), (1, 11), (1, 15), (2, 5), (3, 5)])
+def test_prefill_of_nine_to_fifteen_columns_of_wide_projections(bk, B, T):
+    w = M.synth_weights(WIDE, seed=82)
+    prompt = np.random.default_rng(83).integers(0, WIDE.vocab, (T, B)).astype(np.int32)
+    ga, gb = M.DecodeModel(WIDE, w, batch=B), M.DecodeModel(WIDE, w, batch=B)
+    ia, va = ga.prefill(prompt)
+    for t in range(T):
+        ib, vb = gb.step(prompt[t])
+    assert_same_bits(va, vb, "max logit after the prompt")
+    assert_same_bits(ga.logits(), gb.logits(), "logits after the prompt")
+    for t in range(2):
+        ia, _ = ga.step(ia)
+        ib, _ = gb.step(ib)
+    assert_same_bits(ga.logits(), gb.logits(), "logits after two more steps")
+    ga.destroy()
+    gb.destroy()
+
+
 @pytest.mark.parametrize("interval,n_layers", [(4, 4), (1, 2), (2, 3), (4, 3)])
 def test_persistent_step_equals_per_op_step_and_oracle(bk, interval, n_layers):
     """Batch 1 on one GPU can run as a persistent kernel (phases + device-side barriers, step mode 2).  The same model
