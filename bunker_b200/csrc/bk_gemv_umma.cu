@@ -184,7 +184,7 @@ BK_DEVINL void cluster_sync() {
 template <bool LANES>
 struct Walk {
   int pos, pos1, s, nsb;
-  BK_DEVINL static int cls(int pos) { return (int)((0x73516240u >> (4 * pos)) & 7u); }
+  __host__ __device__ __forceinline__ static int cls(int pos) { return (int)((0x73516240u >> (4 * pos)) & 7u); }
   BK_DEVINL void start(int pos0, int end, int n) {
     nsb = n;
     pos1 = end;
@@ -882,11 +882,14 @@ int32_t resident_clusters(const int** out) {
 
 template <int NB, bool LANES>
 int32_t plan_tiles(int tiles, int K, TilePlan* best) {
-  // The cheapest of 1, 2, 4 and 8 parts: the steps of the longest CTA, a tile's exchange and pipeline fill counted as one superblock; with
-  // two stages only, superblocks of one tile after another come half as fast (17 chunks, 48 tiles of 32 columns: 1.8 times, rounds of
-  // one tile hardly at all).  The lane order shares its classes by powers of two; other numbers of parts are taken in the tile order
-  // where they save 30 % (K 5120, 2,048 rows, 32 columns: five parts of one chunk 15.4 us, four of one or two 20.2): by less they are
-  // slower, since fewer CTAs own columns.
+  // LANES: the cheapest of 1, 2, 4 and 8 parts: the superblocks of the longest CTA, 0.2 for each of its classes, and 3 (64 columns 3.5) for a tile's
+  // exchange and pipeline fill.  Fitted to 365 launches of 16, 32 and 64 columns: ten are up to 9 % slower than with the best number of parts.  With
+  // eight classes of ceil(K / 2048) and 1 for a tile 32 were, by up to 38 % (64 columns, 9,472 rows, K 256 29.4 us, so 21.2, K 2048 34.3, so 29.6; 32
+  // columns, 20,480 rows, K 256 28.5, so 21.2; 16 columns, 24,576 rows, K 256 19.5, so 14.9).
+  // TILE: the same with the steps of the longest CTA and one superblock for a tile; with two stages only, superblocks of one tile after another come
+  // half as fast (17 chunks, 48 tiles of 32 columns: 1.8 times, rounds of one tile hardly at all).  The lane order shares its classes by powers of
+  // two; other numbers of parts are taken in the tile order where they save 30 % (K 5120, 2,048 rows, 32 columns: five parts of one chunk 15.4 us,
+  // four of one or two 20.2): by less they are slower, since fewer CTAs own columns.
   using C = Cfg<NB, LANES>;
   constexpr int PSPLIT = 4 / C::PS;
   constexpr size_t per_stage = C::kStage + C::kColBytes;
@@ -907,8 +910,18 @@ int32_t plan_tiles(int tiles, int K, TilePlan* best) {
     p.stages = std::min(kMaxStages, (int)((limit - fixed) / per_stage));
     p.smem = fixed + (size_t)p.stages * per_stage;
     p.rounds = (tiles + n - 1) / n;
-    p.len = LANES ? (nsb + 7) / 8 * (8 / s) : 4 * ((n_chunks + s - 1) / s);
-    p.cost = p.rounds * (p.len * (!LANES && p.stages == 2 && p.rounds > 1 ? 1.6f : 1.0f) + 1.0f);
+    if (LANES) {
+      p.len = 0;
+      for (int part = 0; part < s; part++) {
+        int n_sb = 0;
+        for (int pos = part * 8 / s; pos < (part + 1) * 8 / s; pos++) n_sb += std::max(0, (nsb - Walk<true>::cls(pos) + 7) / 8);
+        p.len = std::max(p.len, n_sb);
+      }
+      p.cost = p.rounds * (p.len + 0.2f * (8 / s) + (NB == 4 ? 3.5f : 3.0f));
+    } else {
+      p.len = 4 * ((n_chunks + s - 1) / s);
+      p.cost = p.rounds * (p.len * (p.stages == 2 && p.rounds > 1 ? 1.6f : 1.0f) + 1.0f);
+    }
     return true;
   };
   TilePlan p;
