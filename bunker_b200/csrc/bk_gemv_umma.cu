@@ -882,10 +882,11 @@ int32_t resident_clusters(const int** out) {
 
 template <int NB, bool LANES>
 int32_t plan_tiles(int tiles, int K, TilePlan* best) {
-  // LANES: the cheapest of 1, 2, 4 and 8 parts: the superblocks of the longest CTA, 0.2 for each of its classes, and 3 (64 columns 3.5) for a tile's
-  // exchange and pipeline fill.  Fitted to 365 launches of 16, 32 and 64 columns: ten are up to 9 % slower than with the best number of parts.  With
-  // eight classes of ceil(K / 2048) and 1 for a tile 32 were, by up to 38 % (64 columns, 9,472 rows, K 256 29.4 us, so 21.2, K 2048 34.3, so 29.6; 32
-  // columns, 20,480 rows, K 256 28.5, so 21.2; 16 columns, 24,576 rows, K 256 19.5, so 14.9).
+  // LANES: the cheapest of 1, 2, 4 and 8 parts.  A tile costs the superblocks of its longest CTA, 0.1 for each of that CTA's classes and kEnd for the
+  // exchange; its end runs beside the next tile's superblocks, but however few those are no tile after the first takes less than kTile.  Fitted to
+  // 1,071 launches of 16, 32 and 64 columns: 14 are 4 to 9 % slower than with the best number of parts.  With eight classes of ceil(K / 2048)
+  // superblocks and one for a tile's end 85 were, by up to 62 % (64 columns, 9,472 rows, K 256 29.4 us, so 21.2, K 2048 34.3, so 29.6; 32 columns, 20,480
+  // rows, K 256 28.5, so 21.2; 16 columns, 24,576 rows, K 256 19.5, so 14.9).
   // TILE: the same with the steps of the longest CTA and one superblock for a tile; with two stages only, superblocks of one tile after another come
   // half as fast (17 chunks, 48 tiles of 32 columns: 1.8 times, rounds of one tile hardly at all).  The lane order shares its classes by powers of
   // two; other numbers of parts are taken in the tile order where they save 30 % (K 5120, 2,048 rows, 32 columns: five parts of one chunk 15.4 us,
@@ -898,6 +899,7 @@ int32_t plan_tiles(int tiles, int K, TilePlan* best) {
   const int32_t rc = resident_clusters<NB, LANES>(&clusters);
   if (rc != BK_OK) return rc;
   const int nsb = K / 256, n_chunks = (nsb + 3) / 4;
+  constexpr float kEnd = NB == 1 ? 0.5f : NB == 2 ? 1.5f : 3.5f, kTile = NB == 1 ? 6.0f : NB == 2 ? 7.0f : 9.0f;
   auto candidate = [&](int s, TilePlan& p) {
     const int cs = s * PSPLIT, n = clusters[cs], own = C::N / owners_of(cs);
     p.csplit = s;
@@ -917,7 +919,8 @@ int32_t plan_tiles(int tiles, int K, TilePlan* best) {
         for (int pos = part * 8 / s; pos < (part + 1) * 8 / s; pos++) n_sb += std::max(0, (nsb - Walk<true>::cls(pos) + 7) / 8);
         p.len = std::max(p.len, n_sb);
       }
-      p.cost = p.rounds * (p.len + 0.2f * (8 / s) + (NB == 4 ? 3.5f : 3.0f));
+      const float tile = p.len + 0.1f * (8 / s) + kEnd;
+      p.cost = tile + (p.rounds - 1) * std::max(tile, kTile);
     } else {
       p.len = 4 * ((n_chunks + s - 1) / s);
       p.cost = p.rounds * (p.len * (p.stages == 2 && p.rounds > 1 ? 1.6f : 1.0f) + 1.0f);
