@@ -355,17 +355,23 @@ static const KView* g_view = nullptr;
 
 int32_t bk_gemv_launch(const bkGemvArgs& a) { return bk_gemv_launch_tp(a, nullptr, nullptr, nullptr); }
 
-// Whether the lane-order dense kernel, with the launch that makes its image (2 us), is faster than one launch per 8 columns.  A short K is
-// few steps per tile and row round, so the kernel's fixed part weighs more the more rounds there are.  Measured (groups of 8 / dense, us):
-// 24 columns, K 2048: 4,096 rows 16.0 / 15.4, 9,472 20.2 / 24.9; K 2560: 12,352 rows 34.0 / 28.7; K 256: 1,024 rows 11.1 / 9.3, 12,352 14.5 / 20.8.
-// 32 columns, K 256: 8,192 rows 14.3 / 12.9, 20,480 23.6 / 31.3; K 1024: 12,352 rows 24.4 / 24.7.  40 columns, K 1024: 4,096 rows 19.7 / 16.4, 49,152
-// 76.8 / 84.1; K 2048: 49,152 rows 118.7 / 110.4.  48 columns, K 256: 12,352 rows 28.5 / 24.9, 49,152 62.4 / 74.2.
+// Whether a caller's Q8_1 blocks of 9 columns and more go to the dense kernel in the lane order, with the launch that makes its image (2 us), or to one
+// launch per 8 columns.  The dense kernel pays for a tile's end what three superblocks cost, so a short K wants many columns; where either
+// kernel has just started another round over the SMs (2,048, 9,472 rows) the line moves.  Measured (groups of 8 / dense, us), 9 columns: K 6144,
+// 9,216 rows 30.5 / 26.0, 2,048 16.1 / 16.6; K 2048, 24,576 25.0 / 26.8, 49,152 39.4 / 36.3.  10 columns: K 4096, 2,048 rows 13.4 / 14.7; K 2048, 9,216 15.7 /
+// 16.4, 12,288 20.3 / 19.4; K 1024, 49,152 34.5 / 26.0.  16 columns: K 8192, 512 rows 28.7 / 14.7; K 6144, 1,024 18.9 / 13.7; K 4096, 1,024 14.7 / 12.6, 3,072
+// 17.2 / 15.6; K 1024, 24,576 21.1 / 22.4.  24 columns: K 1024, 9,472 rows 17.1 / 18.6; K 2048, 12,288 30.8 / 26.0.  32 columns: K 256, 12,288 rows 20.5 / 18.8.  33
+// columns: K 512, 12,288 rows 27.5 / 25.3, 24,576 37.5 / 41.1.  Of 5,244 shapes (9 to 64 columns, K 256 to 17,408, 512 to 98,304 rows) 42 take more than
+// 4.5 % longer than on the other path, none of them by more than 13 % in two measurements.
 static bool dense_blocks_pay(int rows, int K, int B) {
+  if (B == 9) return K >= 8192 || (K >= 5120 && rows >= 6144) || (K >= 4096 && rows >= 12288) || (K >= 2304 && rows >= 16384) || rows > 24576;
   switch ((B + 7) / 8) {
-    case 3: return K >= 2560 || rows <= 1024 || (K >= 2048 && rows <= 4096);
-    case 4: return K > 512 || rows <= 8192;
-    case 5: return K > 1024 || rows <= 8192;
-    case 6: return K > 512 || rows <= 16384;
+    case 2:
+      return K >= 5120 || (K >= 3072 && (rows <= 1024 || rows >= 3072)) || (K >= 2560 && rows >= 8192) || (K >= 2048 && rows >= 10240) ||
+             (K >= 1536 && rows > 20480) || (K > 512 && rows > 24576) || rows >= 49152;
+    case 3: return rows <= 1024 || K >= 2304 || (K >= 1536 && (B > 17 || rows <= 8192 || rows > 12288)) || (K >= 768 && (rows <= 4096 || rows >= 16384));
+    case 5: return K >= 1536 || rows <= 8448 || (rows >= 10240 && rows <= (K >= 768 ? 24576 : 12288));
+    case 6: return K > 512 || rows <= 24576;
     default: return true;
   }
 }
@@ -376,10 +382,9 @@ int32_t bk_gemv_launch_tp(const bkGemvArgs& a, const BkPush* push, const BkReduc
   BK_ARG(a.B >= 1 && a.B <= 64, "bkGemvQ4K: B=%d outside 1..64", a.B);
   // Ready-made Q8_1 blocks of many columns go to the dense tile kernel (tcgen05, bk_gemv_umma.cu), which streams the weights
   // once for all columns.  From 16 columns on it has an f32 order of its own (see there), which order = BK_GEMV_ORDER_LANES
-  // declines and AUTO takes for launches of many rows; the rule depends on the shapes only.  In the lane order it takes
-  // 17 columns and more of segments that begin at multiples of 8 rows, and nine and more of many or long rows (bk_gemv_dense_lanes): a launch of 8
-  // columns each on the mma.sync kernel takes longer (K 2048, 12,352 rows, 32 columns: 37 us, here 23; 64: 74 us, here 31).  A caller's Q8_1 blocks have to be
-  // made into its image first, which few columns of a short K do not pay back (dense_blocks_pay).
+  // declines and AUTO takes for launches of many rows; the rule depends on the shapes only.  In the lane order it takes nine columns
+  // and more of segments that begin at multiples of 8 rows where it is the faster one (bk_gemv_dense_lanes, for a caller's blocks dense_blocks_pay; K 2048,
+  // 12,352 rows, 32 columns: 23 us, in launches of 8 columns each 37; 64: 31 and 74).
   int launch_rows = 0;
   bool whole_boxes = true;   // (a box of 8 rows of weights belongs to one segment)
   for (int i = 0; i < a.n_segs && i < 4; i++) {
@@ -388,8 +393,7 @@ int32_t bk_gemv_launch_tp(const bkGemvArgs& a, const BkPush* push, const BkReduc
   }
   const bool dense = a.B > 8 && (a.prologue == BK_PRO_Q8 || a.prologue == BK_PRO_TILE) && !push && !reduce && !g_view;
   const bool tile_order = dense && a.B >= 16 && (a.order == BK_GEMV_ORDER_TILE || (a.order == BK_GEMV_ORDER_AUTO && bk_gemv_auto_tile(launch_rows, a.K)));
-  const bool tile_path = tile_order || (dense && whole_boxes && (a.prologue == BK_PRO_TILE ||
-                                                                 (bk_gemv_dense_lanes(a.B, launch_rows, a.K, false) && dense_blocks_pay(launch_rows, a.K, a.B))));
+  const bool tile_path = tile_order || (dense && whole_boxes && (a.prologue == BK_PRO_TILE || dense_blocks_pay(launch_rows, a.K, a.B)));
   BK_ARG(a.prologue != BK_PRO_TILE || tile_path, "bkGemvQ4K: unknown prologue %d", a.prologue);
   if (a.B > 8 && !tile_path) {
     // Everything else of more than 8 columns: groups of 8 on the mma.sync kernel, one launch per group (the weights
@@ -660,7 +664,15 @@ int32_t bk_gemv_launch_tp(const bkGemvArgs& a, const BkPush* push, const BkReduc
   return tp ? launch_gemv<2, gemv_gmax(2), true>(p, grid, threads, smem) : launch_gemv<2, gemv_gmax(2), false>(p, grid, threads, smem);
 }
 
-bool bk_gemv_dense_lanes(int B) { return B > 16; }
+// From 17 columns on always.  9 to 16 columns are two launches on the mma.sync kernel, with a staged activation; those are the faster the longer the rows, and
+// the dense kernel leaves no room for the next launch's CTA beside its own.  In the step, all of one projection moved to the dense kernel, us a step: 24
+// layers, 10 to 15 sequences: 18 x 12,352 rows of K 2048 +42 to 50, 24 x 12,288 of 2048 +98 to 145, 24 x 2,048 of 6144 +156 to 187, 24 x 2,048 of 4096 +174 to 233, 151,936 of
+// 2048 -42 to 44.  64 layers, 12 sequences, everything dense 10.16 ms, all but 5,120 rows of 6144 10.34, all but 14,336 of 5120 10.48, nothing 14.58.  Nine columns
+// (the second launch is the batch-1 kernel) have their line further up; a K too wide for the mma.sync kernel goes to the dense one.
+bool bk_gemv_dense_lanes(int B, int rows, int K) {
+  if (B <= 8 || B > 16) return B > 16;
+  return !bk_gemv_mma_fits(K, 8) || (double)rows * K * K >= (B == 9 ? 2e11 : 1.2e11);
+}
 bool bk_gemv_auto_tile(int rows, int K) { return rows >= g_tile_min_rows || (rows >= g_tile_min_rows_cut && K >= 2048); }
 
 extern "C" {

@@ -121,19 +121,7 @@ bool bk_encode_map_2d(CUtensorMap* m, CUtensorMapDataType type, uint64_t base, u
 bool bk_gemv_mma_fits(int K, int B);   // whether the batch-3..8 tensor-core GEMV can hold this K (else column pairs)
 // whether a dense launch of B columns takes them as two groups of 32 (launch rows `rows`; lanes: in the lane order)
 bool bk_tile_split(int rows, int K, int B, bool lanes);
-bool bk_gemv_dense_lanes(int B);           // whether B columns are enough for the dense tile kernel in the lane order whatever the launch
-// Whether B columns of a launch are; staged: the other path would take a staged activation.
-// 9 to 16 columns are two launches on the mma.sync kernel, which is the faster the longer the rows: where rows * K^2 is small two of those are
-// faster, nine columns (the second launch is the batch-1 kernel) four times as long.  Measured with the image launch, 16 columns, two
-// launches / dense, us: K 1024, 24,576 rows 19.0 / 22.6, 49,152 32.3 / 26.3; K 2048, 9,216 rows 14.0 / 14.4, 12,288 18.9 / 17.8; K 4096, 2,048 rows
-// 13.7 / 13.3, 4,096 16.0 / 14.1; K 6144, 1,024 rows 17.5 / 12.5; K 17,408, 2,048 rows 53 / 26.  Nine columns: K 2048, 24,576 rows 23.3 / 25.3, 49,152
-// 37.7 / 34.2; K 6144, 2,048 rows 14.0 / 14.6, 9,216 28.3 / 22.3; K 17,408, 1,024 rows 34.7 / 17.4.  Where the two would copy a staged activation
-// instead of Q8_1 blocks (the steps and prompts of a model) they are faster and the line is further up: 13 sequences, in the step, K 6144, 2,048
-// rows 10.5 / 13.3, K 2048, 12,288 rows 15.2 / 15.9, 151,936 rows 142 / 83; 12 sequences, 64 layers 17.6 / 10.5 ms a step.
-inline bool bk_gemv_dense_lanes(int B, int rows, int K, bool staged) {
-  if (B <= 8 || B > 16) return bk_gemv_dense_lanes(B);
-  return (double)rows * K * K >= (B == 9 ? 2e11 : staged ? 1.2e11 : 5.2e10);
-}
+bool bk_gemv_dense_lanes(int B, int rows, int K);   // whether the steps and prompts of a model take B columns to the dense tile kernel in the lane order
 bool bk_gemv_auto_tile(int rows, int K);   // whether BK_GEMV_ORDER_AUTO sends a launch of these shapes (>= 16 columns) to the dense tile path
 int32_t bk_gemv_launch(const bkGemvArgs& a);
 int32_t bk_gdn_launch(const bkGdnArgs& a);   // bkGdnStep, also with out_q8_layout BK_Q8_TILE

@@ -264,7 +264,7 @@ int32_t enqueue_chain(Model& m, int parity, bool host_tokens = false) {
   // A projection that goes to the dense tile kernel (bk_gemv_launch_tp has the rule) reads that kernel's image.
   auto layout_for = [&](int K, int rows, int row_gcd) {
     if (tile_path && bk_gemv_auto_tile(rows, K)) return bk_tile_split(rows, K, B, false) ? BK_Q8_TILE32 : BK_Q8_TILE;
-    if (m.tp == 1 && row_gcd % 8 == 0 && bk_gemv_dense_lanes(B, rows, K, staged_ok(K, rows))) return bk_tile_split(rows, K, B, true) ? BK_Q8_TILE32 : BK_Q8_TILE;
+    if (m.tp == 1 && row_gcd % 8 == 0 && bk_gemv_dense_lanes(B, rows, K)) return bk_tile_split(rows, K, B, true) ? BK_Q8_TILE32 : BK_Q8_TILE;
     return staged_ok(K, rows) ? BK_Q8_STAGED : BK_Q8_BLOCKS;
   };
   auto prologue_of = [](int layout) { return layout >= BK_Q8_TILE ? BK_PRO_TILE : layout == BK_Q8_STAGED ? BK_PRO_STAGED : BK_PRO_Q8; };
@@ -452,7 +452,7 @@ int32_t enqueue_prefill(Model& m, int T) {
   auto staged_ok = [&](int K, int cols) { return cols >= 2 && bk_gemv_mma_fits(K, cols < 8 ? cols : 8) && !(cols > 8 && cols % 8 == 1); };
   // many columns: the dense tile kernel, in the lane order, where every segment begins at a multiple of 8 rows
   auto layout_for = [&](int K, int cols, int rows, int row_gcd) {
-    if (bk_gemv_dense_lanes(cols, rows, K, staged_ok(K, cols)) && row_gcd % 8 == 0) return bk_tile_split(rows, K, cols, true) ? BK_Q8_TILE32 : BK_Q8_TILE;
+    if (bk_gemv_dense_lanes(cols, rows, K) && row_gcd % 8 == 0) return bk_tile_split(rows, K, cols, true) ? BK_Q8_TILE32 : BK_Q8_TILE;
     return staged_ok(K, cols) ? BK_Q8_STAGED : BK_Q8_BLOCKS;
   };
   auto point_at = [&](bkGemvArgs& g, int K, int cols, int layout) {

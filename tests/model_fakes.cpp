@@ -39,7 +39,7 @@ int32_t bk_argmax_launch(uint64_t, int32_t, int32_t, uint64_t, uint64_t, uint64_
 int32_t bk_quant_rows_launch(uint64_t, uint64_t, int32_t, int32_t, float, uint64_t, int32_t, const BkReduce*) { return BK_OK; }
 bool bk_gemv_mma_fits(int, int) { return true; }
 bool bk_tile_split(int, int, int, bool) { return false; }
-bool bk_gemv_dense_lanes(int) { return false; }
+bool bk_gemv_dense_lanes(int, int, int) { return false; }
 bool bk_gemv_auto_tile(int, int) { return false; }
 int32_t bk_plan_create(uint64_t* out, const BkPlanDims&) { return g_plans++, *out = 77, BK_OK; }
 void bk_plan_add_layer(uint64_t, const BkPlanLayer&) {}

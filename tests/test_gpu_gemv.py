@@ -394,3 +394,11 @@ def test_gemv_nine_to_sixteen_columns_in_lane_order(bk, B, K, rows):
         ops.gemv(dxq.ptr, K, B, [ops.gemv_seg(w.ptr, k, o.ptr) for w, k, o in zip(dW, n, y)], order=R.BK_GEMV_ORDER_LANES)
     for i, k in enumerate(n):
         assert_same_bits(y[i].download(np.float32, (B, k)), O.gemv_q4k_q8(W[i], k, K, xq), f"segment {i}")
+
+
+@pytest.mark.parametrize("B,K,rows", [(9, 5120, 6136), (9, 5120, 6144), (9, 8192, 56), (9, 4096, 12280), (9, 4096, 12288), (9, 2304, 16384), (9, 256, 24584), (10, 5120, 56), (10, 3072, 1024), (10, 3072, 1032),
+                                      (10, 3072, 3072), (12, 2560, 8192), (16, 2048, 10240), (14, 1536, 20488), (16, 768, 24584), (11, 512, 49152), (17, 1536, 12296),
+                                      (18, 1536, 9000), (24, 768, 4104), (20, 1024, 16384), (25, 256, 9000), (33, 512, 8456), (33, 512, 10240), (40, 1024, 24584), (48, 512, 24584),
+                                      (40, 2048, 9472), (32, 256, 20480), (16, 256, 20480)])   # (the last three: tiles that fewer thread blocks share)
+def test_gemv_blocks_at_the_lines_of_the_lane_order(bk, B, K, rows):
+    test_gemv_nine_to_sixteen_columns_in_lane_order(bk, B, K, rows)
