@@ -42,6 +42,7 @@ struct AttnParams {
   unsigned int* counters;    // splits done per (entry, KV head); they reset themselves
   const uint16_t* gate;
   int B, Hq, Hkv, rot_half, max_len, split_len, max_splits, fused;
+  int splits_first;   // the grid is (split, KV head, entry), not (KV head, entry, split)
   int settled;  // cache rows of earlier steps and pos[] are not outputs of the immediately preceding launch
   int n_seq;    // > 0: prompt columns.  Entry b of the launch is token b / n_seq of sequence b mod n_seq: it reads that
                 // sequence's cache, and its own K/V row has already been appended (attn_append_kernel)
@@ -132,6 +133,35 @@ __device__ void store_head_warp(const AttnParams& p, int b, int h, const float (
     else if (p.out_q8_layout == BK_Q8_STAGED) bk_staged_store<8>(p.out_q8, p.Hq * kHD, p.B, b, (h * kHD + lane * 8) >> 5, y, (lane & 3) * 8);
     else bk_q8_1_store<8>(p.out_q8 + ((((size_t)b * p.Hq + h) * kHD + lane * 8) >> 5) * 36, y, (lane & 3) * 8);
   }
+}
+
+// merge the splits of one (batch, q head) by one warp, as little code as there can be; w_s: ns floats of shared memory private to the warp
+__device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, float* w_s, uint4 gate) {
+  const int lane = threadIdx.x & 31;
+  const float* sc_ml = p.part_ml + ((size_t)b * p.Hq + h) * p.max_splits * 2;
+  const float* sc_o = p.part_o + ((size_t)b * p.Hq + h) * p.max_splits * kHD;
+  float m = -INFINITY;
+  for (int s = lane; s < ns; s += 32) {
+    float ms = __ldcg(sc_ml + 2 * s);
+    w_s[s] = ms;
+    m = fmaxf(m, ms);
+  }
+  const float M = bk_warp_max(m);
+  for (int s = lane; s < ns; s += 32) w_s[s] = bk_expf(__fsub_rn(w_s[s], M));
+  __syncwarp();
+  float L = 0.0f, O[8];
+#pragma unroll
+  for (int e = 0; e < 8; e++) O[e] = 0.0f;
+#pragma unroll 4
+  for (int s = 0; s < ns; s++) {
+    const float w = w_s[s];
+    L = fmaf(w, __ldcg(sc_ml + 2 * s + 1), L);
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(sc_o + (size_t)s * kHD + lane * 8));
+    const float4 c = __ldcg(reinterpret_cast<const float4*>(sc_o + (size_t)s * kHD + lane * 8) + 1);
+    O[0] = fmaf(w, a.x, O[0]); O[1] = fmaf(w, a.y, O[1]); O[2] = fmaf(w, a.z, O[2]); O[3] = fmaf(w, a.w, O[3]);
+    O[4] = fmaf(w, c.x, O[4]); O[5] = fmaf(w, c.y, O[5]); O[6] = fmaf(w, c.z, O[6]); O[7] = fmaf(w, c.w, O[7]);
+  }
+  store_head_warp(p, b, h, O, L, gate);
 }
 
 // Merge the splits of one (batch, KV head), all threads of a CTA: M = max m_s; w_s = exp(m_s - M); L = fma(w_s, l_s, L) and O = fma(w_s, o_s, O) in
@@ -272,8 +302,8 @@ __global__ void __launch_bounds__(32) attn_append_kernel(const AttnParams p) {
 
 constexpr int kRows = 4;      // rows requested together
 
-// kBatches: batches of rows of a warp on their way or in use
-template <int G, int kBatches>
+// kBatches: batches of rows of a warp on their way or in use; MANY: the merge for many splits
+template <int G, int kBatches, bool MANY>
 __global__ void __launch_bounds__(kW * 32, G == 1 ? 3 : 2) attn_split_kernel(const AttnParams p) {
   static_assert(kRows * kBatches * kHD * 2 <= 8 * kHD * 4, "a warp's ring is its part of o_s");
   constexpr int GP = G <= 1 ? 1 : G <= 2 ? 2 : G <= 4 ? 4 : 8;   // heads, up to a power of two
@@ -289,7 +319,8 @@ __global__ void __launch_bounds__(kW * 32, G == 1 ? 3 : 2) attn_split_kernel(con
   float* o_s = reinterpret_cast<float*>(s_s + (size_t)p.split_len * GP);
   __shared__ int s_last;
 
-  const int kvh = blockIdx.x, b = blockIdx.y, split = blockIdx.z;
+  const bool splits_first = p.splits_first;
+  const int split = splits_first ? blockIdx.x : blockIdx.z, kvh = splits_first ? blockIdx.y : blockIdx.x, b = splits_first ? blockIdx.z : blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
   const int cb = p.n_seq > 0 ? b % p.n_seq : b;   // whose cache
   uint16_t* Kb = p.k_cache + ((size_t)cb * p.Hkv + kvh) * (size_t)p.max_len * kHD;
@@ -628,9 +659,13 @@ __global__ void __launch_bounds__(kW * 32, G == 1 ? 3 : 2) attn_split_kernel(con
   __syncthreads();
   if (s_last) {
     __threadfence();
-    constexpr int V = G <= 2 ? G : G <= 4 || kBatches != 2 ? 4 : 8;
-    if (V < 8 && nsplits <= 8) merge_splits<G, 8>(p, b, kvh, nsplits, reinterpret_cast<float2*>(o_s), l_s);
-    else merge_splits<G, V>(p, b, kvh, nsplits, reinterpret_cast<float2*>(o_s), l_s);
+    if constexpr (!MANY) {
+      if (warp < G) combine_head_warp(p, b, kvh * G + warp, nsplits, o_s + warp * kMaxSplits, head_gate(p, b, kvh * G + warp));
+    } else {
+      constexpr int V = G <= 2 ? G : G <= 4 || kBatches != 2 ? 4 : 8;
+      if (V < 8 && nsplits <= 8) merge_splits<G, 8>(p, b, kvh, nsplits, reinterpret_cast<float2*>(o_s), l_s);
+      else merge_splits<G, V>(p, b, kvh, nsplits, reinterpret_cast<float2*>(o_s), l_s);
+    }
     if (tid == 0) *cnt = 0;
   }
   bk_stamp(p.trace, 5);
@@ -641,14 +676,14 @@ size_t attn_smem_bytes(int split_len, int heads) {
   return 4096 + 1024 + 64 + 256 + (size_t)split_len * gp * 4 + (size_t)kW * 8 * kHD * 4;
 }
 
-template <int G, int kBatches>
-int32_t launch_split_batches(const AttnParams& p, dim3 grid, size_t smem) {
+template <int G, int kBatches, bool MANY>
+int32_t launch_split_as(const AttnParams& p, dim3 grid, size_t smem) {
   static size_t configured = 0;
   if (smem > configured) {
-    BK_CUDA(cudaFuncSetAttribute(attn_split_kernel<G, kBatches>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BK_CUDA(cudaFuncSetAttribute(attn_split_kernel<G, kBatches, MANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = smem;
   }
-  BK_CUDA(bk_launch_pdl(attn_split_kernel<G, kBatches>, grid, dim3(kW * 32), smem, p));
+  BK_CUDA(bk_launch_pdl(attn_split_kernel<G, kBatches, MANY>, grid, dim3(kW * 32), smem, p));
   BK_CHECK_LAUNCH();
   return BK_OK;
 }
@@ -656,18 +691,27 @@ int32_t launch_split_batches(const AttnParams& p, dim3 grid, size_t smem) {
 // Two batches of rows on their way where the splits are short or two CTAs an SM hold all of them, else four.  There more requests bring no more bytes, but
 // the query heads come later behind them and some CTAs run far ahead of others (24 heads on 4, four / two batches, us: 8 sequences, 900 rows, 256 splits of 128
 // 17.6 / 17.1, 2,000 rows, 256 of 256 25.1 / 24.2, 600 rows, 320 of 64 21.0 / 19.7; but 5 sequences, 9,000 rows, 360 of 512 60.1 / 67.3).
-// One head per KV head leaves room for three CTAs an SM, which many splits want (16 sequences, 8 heads, 560 rows, 384 splits 18.5 us, two an SM 25.4).  What two an
-// SM hold gets two at most, by shared memory that it does not use: three make an uneven spread, since the launch before still holds some SMs (6
-// sequences, 8 heads, 1,100 rows, 288 splits 18.2 us, so 15.2).
+// One or two heads per KV head leave room for three CTAs an SM, which many splits want (16 sequences, 8 heads on 8, 560 rows, 384 splits 18.5 us, two an SM
+// 25.4).  What two an SM hold gets two at most, by shared memory that it does not use: three make an uneven spread, since the launch before still holds
+// some SMs (6 sequences, 8 heads on 8, 1,100 rows, 288 splits 18.2 us, so 15.2; 16 on 8, 450 rows 16.3, so 13.9).
 // The grid walks the splits last: a second wave is then made of last splits, which are short (8 sequences, 24 heads on 4, 320 splits of 64: 600 rows 20.2 us, so
 // 19.0, 577 rows 19.3, so 17.4), and prompt columns of a sequence read the same rows at the same time.
+// Settled rows (the steps of a model) are requested while the launch before still runs, and of those four batches are better; a single wave of them walks the
+// splits first; and a launch of at most eight splits, or of many heads, takes the kernel with the short merge, since code is cold in a step.  24 layers, 8
+// sequences, splits of 64, up to five of them: each of the three is worth 4 to 7 us of 1,135 a step; up to 15 of them: the short merge 1,158, the other 1,184.
+template <int G, int kBatches>
+int32_t launch_split_batches(const AttnParams& p, dim3 grid, size_t smem, int nsplit) {
+  return nsplit > 8 && (!p.settled || G <= 4) ? launch_split_as<G, kBatches, true>(p, grid, smem) : launch_split_as<G, kBatches, false>(p, grid, smem);
+}
 template <int G>
-int32_t launch_split(const AttnParams& p, int nsplit) {
+int32_t launch_split(AttnParams& p, int nsplit) {
   const bool two_an_sm = (long long)nsplit * p.Hkv * p.B <= 2 * bk_ctx().sm_count;
   size_t smem = attn_smem_bytes(p.split_len, G);
-  if (G == 1 && two_an_sm) smem = std::max<size_t>(smem, bk_ctx().smem_optin / 3);
-  const dim3 grid(p.Hkv, p.B, nsplit);
-  return p.split_len <= 128 || (p.split_len <= 256 && two_an_sm) ? launch_split_batches<G, 2>(p, grid, smem) : launch_split_batches<G, 4>(p, grid, smem);
+  if (two_an_sm) smem = std::max<size_t>(smem, bk_ctx().smem_optin / 3);
+  p.splits_first = p.settled && two_an_sm;
+  const dim3 grid = p.splits_first ? dim3(nsplit, p.Hkv, p.B) : dim3(p.Hkv, p.B, nsplit);
+  if (!p.settled && (p.split_len <= 128 || (p.split_len <= 256 && two_an_sm))) return launch_split_batches<G, 2>(p, grid, smem, nsplit);
+  return launch_split_batches<G, 4>(p, grid, smem, nsplit);
 }
 
 }  // namespace
