@@ -105,6 +105,7 @@ __device__ __forceinline__ void butterfly_level(float (&v)[N], int off) {
   }
 }
 
+// the sigmoid gate of a head, 8 dims a lane
 __device__ __forceinline__ uint4 head_gate(const AttnParams& p, int b, int h) {
   const int lane = threadIdx.x & 31;
   return *reinterpret_cast<const uint4*>(p.fused ? p.qg + ((size_t)b * p.Hq + h) * 2 * kHD + kHD + lane * 8 : p.gate + ((size_t)b * p.Hq + h) * kHD + lane * 8);
@@ -135,7 +136,8 @@ __device__ void store_head_warp(const AttnParams& p, int b, int h, const float (
   }
 }
 
-// merge the splits of one (batch, q head) by one warp, as little code as there can be; w_s: ns floats of shared memory private to the warp
+// Merge the splits of one (batch, q head) by one warp; lane l owns output dims [8l, 8l+8).  w_s: ns floats of shared memory private to the warp.  M = max m_s; w_s =
+// exp(m_s - M); L = fma(w_s, l_s, L) and O = fma(w_s, o_s, O) in ascending s; out = (O/L) * sigmoid(gate).  As little code as there can be (see launch_split).
 __device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, float* w_s, uint4 gate) {
   const int lane = threadIdx.x & 31;
   const float* sc_ml = p.part_ml + ((size_t)b * p.Hq + h) * p.max_splits * 2;
@@ -164,8 +166,7 @@ __device__ void combine_head_warp(const AttnParams& p, int b, int h, int ns, flo
   store_head_warp(p, b, h, O, L, gate);
 }
 
-// Merge the splits of one (batch, KV head), all threads of a CTA: M = max m_s; w_s = exp(m_s - M); L = fma(w_s, l_s, L) and O = fma(w_s, o_s, O) in
-// ascending s; out = (O/L) * sigmoid(gate).  wl: G * ns pairs of shared memory; where a head has more than one warp they then take its sums.
+// The same for many splits, all threads of a CTA for the heads of one (batch, KV head).  wl: G * ns pairs of shared memory; where a head has more than one warp they then take its sums.
 // Bound: latency of L2, with one CTA at work.  The heads' dims are spread over all eight warps, so that 64 values a thread (32 where 80 registers
 // are all there are) are on their way at a time, the first of them while the weights are made.  With a head a warp and four splits requested
 // together the whole kernel took, us, so now: one head, 141 splits 25.7, 14.4, 157 splits 26.2, 16.3; 4 heads on 4, 40 splits 14.1, 11.7; 16 on 2, 63 splits 20.9,

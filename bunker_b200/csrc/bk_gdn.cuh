@@ -8,8 +8,8 @@ namespace {
 
 // ---- fused conv1d + gated DeltaNet step ------------------------------------------
 // One CTA of 512 threads per (batch, value head).  Thread (r = t>>7, j = t&127)
-// keeps rows 32r..32r+31 of column j of the 128x128 state in registers: one read
-// and one write of the state per step.  Column sums over the 128 rows use the four
+// has rows 32r..32r+31 of column j of the 128x128 state, in registers or (more than
+// two heads an SM) in shared memory: one read and one write of the state per step.  Column sums over the 128 rows use the four
 // row groups in order ((g0+g1)+g2)+g3.
 struct GdnParams {
   const uint16_t* qkv;
@@ -30,7 +30,7 @@ struct GdnParams {
   uint8_t* out_q8;
   int out_q8_layout;
   int B, Hk, Hv, apply_conv;
-  int T;      // tokens per sequence (gdn_step_body<true>)
+  int T;      // tokens per sequence (gdn_step_body<kGdnMulti>)
   int early;  // state / conv state / weights are not outputs of the immediately preceding launch
   unsigned long long* trace;
 };

@@ -282,7 +282,7 @@ __global__ void block_dots_kernel(const uint8_t* W, int N, int K, const uint32_t
 
 // packQ8_1 on the device: one aligned group of 4 lanes per 32-element block
 // Bound: launch latency.  Launched programmatically it starts while the launch before it drains, and the projection that follows requests its weights
-// while it runs: the pair at 4,096 x 4,096, one column 8.4 -> 7.7 us, twelve columns 18.5 -> 15.1, 17,000 x 5,120, two columns 26.7 -> 24.2.
+// while it runs: the pair at 4,096 x 4,096, one column 8.2 -> 6.7 to 7.5 us by host, twelve columns 18.5 -> 15.1, 17,000 x 5,120, two columns 26.7 -> 24.2.
 template <bool BF16>
 __global__ void quant_q8_1_kernel(const void* x, int K, int B, uint8_t* out) {
   // The wait comes first: what the next launch reads before its own wait (weights, settled states) may come from the launch before this one.

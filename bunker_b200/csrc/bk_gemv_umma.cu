@@ -1,7 +1,7 @@
-// bk_gemv_umma.cu -- Q4_K x Q8_1 GEMM for 16 to 64 activation columns on the 5th-generation tensor cores (tcgen05.mma kind::f16,
+// bk_gemv_umma.cu -- Q4_K x Q8_1 GEMM for 9 to 64 activation columns on the 5th-generation tensor cores (tcgen05.mma kind::f16,
 // operand A and the accumulators in tensor memory).
 //
-// From 16 columns on the product is a dense contraction: the weights are streamed ONCE for all columns (the batch 2..8 kernel
+// With so many columns the product is a dense contraction: the weights are streamed ONCE for all columns (the batch 2..8 kernel
 // streams them once per group of 8).  The reference's nearest thing is its int8 tensor-core GEMM experiment
 // (src/kernel.ts:396-456: 4-bit blocks expanded to int8 tiles, int32 accumulators, scales applied afterwards,
 // experiments/q4k_q81_final.ts:217); this is that idea on the 144-byte Q4_K layout.
@@ -996,7 +996,7 @@ int32_t launch_tile(UmmaParams& P) {
 
 }  // namespace
 
-// 16 to 64 columns (17 in the lane order); p: a filled GemvParams whose x is an image, or Q8_1 blocks (prologue BK_PRO_Q8).
+// 16 to 64 columns (9 to 64 in the lane order); p: a filled GemvParams whose x is an image, or Q8_1 blocks (prologue BK_PRO_Q8).
 int32_t bk_gemv_umma_launch(void* params, int B, bool lanes) {
   BkContext& c = bk_ctx();
   UmmaParams P;

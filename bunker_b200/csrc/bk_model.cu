@@ -221,9 +221,9 @@ int32_t enqueue_step_persist(Model& m, int parity, int token = -1) {
 //   one launch   2 + 2.2 per round + 0.07 per row of a split and round  (splits of 64, 128, 256, 448 rows: 6.8, 10.6, 19.8, 33.6 a round)
 //   chain        11.3 + 0.0185 per row of a split + 0.4 per MB of keys and values
 //   a layer's other launches 6, less 0.018 per MB of weights (5.0 of 24 layers of hidden 2048, 2.1 of 64 of hidden 5120)
-// Measured, chain / one launch: 24 layers, splits of 64 rows: 2,000 rows 755 / 618, 4,000 772 / 709; of 128: 8,000 rows 792 / 808, 16,000 830 / 1,056; of
-// 256: 8,000 rows 824 / 795, 32,000 882 / 1,427.  64 layers, splits of 64: 1,000 rows 4,740 / 4,597, 2,000 4,773 / 4,721, 4,000 4,845 / 5,025 (another B200:
-// 4,793 / 4,817, 4,826 / 4,936, 4,900 / 5,243); of 448: 8,000 rows 5,134 / 5,551.
+// Measured, chain / one launch: 24 layers, splits of 64 rows: 2,000 rows 746 / 615, 4,000 764 / 704; of 128: 8,000 rows 789 / 810, 16,000 824 / 1,056; of
+// 256: 8,000 rows 819 / 787, 32,000 876 / 1,419.  64 layers, splits of 64: 1,000 rows 4,778 / 4,674, 2,000 4,812 / 4,799, 4,000 4,881 / 5,103 (other B200s differ by
+// up to 4 %, most at one launch); of 448: 8,000 rows 5,170 / 5,569.
 int plan_row_limit(const Model& m) {
   const bkModelConfig& c = m.cfg;
   const int pairs = (m.Hq / m.Hkv + 1) / 2;
@@ -332,7 +332,7 @@ int32_t enqueue_chain(Model& m, int parity, bool host_tokens = false) {
       ga.qkv = m.qkv; ga.z = m.z; ga.a = m.a; ga.b = m.b;
       ga.conv_w = L.conv_w; ga.conv_state_in = L.conv_state[parity]; ga.conv_state_new = L.conv_state[parity ^ 1];
       ga.A_log = L.A_log; ga.dt_bias = L.dt_bias; ga.norm_w = L.gnorm;
-      ga.S_in = L.S; ga.S_new = L.S;  // in place: each thread rewrites exactly the rows it read
+      ga.S_in = L.S; ga.S_new = L.S;  // in place: a CTA has read what it rewrites, in registers, or waited for its copy of the whole head, before it stores
       const int zd_layout = q8_handoff ? layout_for(m.ZD, H, H) : BK_Q8_BLOCKS;
       ga.out = m.attn_out; ga.out_q8 = q8_handoff ? m.attn_q8 : 0; ga.out_q8_layout = zd_layout;
       ga.B = B; ga.Hk = m.Hk; ga.Hv = m.Hv; ga.apply_conv = 1;
